@@ -447,6 +447,7 @@ int hm_autotune(hm_handle* h, int64_t ncols, int32_t calls, double* times) {
   // single right-hand side: phase-2 split x phase-1 waves
   float best = -1.f;
   hm_handle::Tune keep = h->tune;
+  const bool slabs = keep.p2_split == 1;
   const int splits[3] = {2, 4, 8}, waves[3] = {1, 2, 4};
   if (times)
     for (int i = 0; i < 15; ++i) times[i] = -1.0;
@@ -461,8 +462,8 @@ int hm_autotune(hm_handle* h, int64_t ncols, int32_t calls, double* times) {
   };
   for (int a = 0; a < 3; ++a)
     for (int b = 0; b < 3; ++b) HM_TRY(try_shape(splits[a], b, 3 * a + b));
-  // phase 2 by tree clusters (FP64 and FP32 factors; BF16 factors have their own phase 2)
-  if (h->storage != HM_BF16)
+  // phase 2 by row slabs (BF16 factors: where it is the default, on trees off the 64-row grid)
+  if (h->storage != HM_BF16 || slabs)
     for (int b = 0; b < 3; ++b) HM_TRY(try_shape(1, b, 12 + b));
   h->tune = keep;
   // several columns on the tensor cores: the column block

@@ -381,6 +381,18 @@ int partition_only(hm_handle* h, int64_t ncl, const int64_t* cl_s, const int64_t
 // y = sum A z + sum C x_seg.  The forward plan uses the pools in row-group
 // order; the transposed plan reads the same data with A and B swapped.
 // ---------------------------------------------------------------------------
+// The leaves by row group, in leaf order within a group (a counting sort):
+// the order of the pools and of the z slots.
+std::vector<int64_t> pool_order(const hm_handle* h) {
+  int32_t ng = 0;
+  for (const Leaf& L : h->leaves) ng = std::max(ng, L.group + 1);
+  std::vector<int64_t> at((size_t)ng + 1, 0), order(h->leaves.size());
+  for (const Leaf& L : h->leaves) ++at[L.group + 1];
+  for (int32_t g = 0; g < ng; ++g) at[g + 1] += at[g];
+  for (size_t i = 0; i < h->leaves.size(); ++i) order[at[h->leaves[i].group]++] = (int64_t)i;
+  return order;
+}
+
 int build_matvec_plans(hm_handle* h) {
   const int eb = elem_bytes(h->storage), deb = dense_elem_bytes(h->storage);
   const int64_t ncl = (int64_t)h->cl_s.size();
@@ -411,11 +423,7 @@ int build_matvec_plans(hm_handle* h) {
   for (auto& L : h->leaves) L.group = grank[grp[L.s]];
 
   // leaf order in the pools: by group, then leaf order
-  std::vector<int64_t> order(h->leaves.size());
-  std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int64_t a, int64_t b) {
-    return h->leaves[a].group < h->leaves[b].group;
-  });
+  const std::vector<int64_t> order = pool_order(h);
   int64_t rk_off = 0, dn_off = 0;
   h->kmax = 0;
   for (int64_t li : order) {
@@ -446,15 +454,18 @@ int build_matvec_plans(hm_handle* h) {
   }
   HM_TRY(build_mv_descriptors(h, order, /*trans=*/0));
   HM_TRY(build_mv_descriptors(h, order, /*trans=*/1));
-  // phase-2 shape until hm_autotune: row windows when every leaf starts on a
-  // 64-row boundary (bisection of 2^k points), where a window's leaves tile it
-  // in aligned pieces; otherwise (KMeans trees, other sizes) by tree clusters,
-  // which keeps every load aligned and every lane busy whatever the
-  // boundaries (BF16 factors have their own phase 2)
+  // phase-2 shape until hm_autotune: row slabs, which read leaves that start at
+  // any row and fill the SMs at every size; row windows only for n > 2^18 with
+  // every leaf on a 64-row boundary (bisection of 2^k points), where a lane's
+  // four rows come in one vector load.  Matvec, slabs against windows: 103 and
+  // 236 us at n = 65536, 1068 and 1102 us at n = 2^18, 3813 and 3767 us at
+  // n = 2^19 (FP64), 2154 and 2040 us (FP32); off the grid, n = 100003, 262 and
+  // 957 us
   if (!h->tune.tuned) {
-    bool aligned = true;
-    for (const Leaf& L : h->leaves) aligned = aligned && (L.row0 % 64 == 0) && (L.col0 % 64 == 0);
-    h->tune.p2_split = (aligned || h->storage == HM_BF16) ? 4 : 1;
+    bool aligned = h->n > 1 << 18;
+    if (aligned)
+      for (const Leaf& L : h->leaves) aligned = aligned && (L.row0 % 64 == 0) && (L.col0 % 64 == 0);
+    h->tune.p2_split = aligned ? 4 : 1;
   }
   return HM_OK;
 }

@@ -159,6 +159,19 @@ struct MvWin {
   uint32_t begin, end;     // P2Desc range
 };
 
+// Phase 2 by row slabs: the entries (one column of one leaf, over the slab's
+// rows it covers) of a slab of at most 224 output rows.
+struct __align__(16) SlabEnt {         // 16 bytes
+  uint64_t off;            // element offset of the value in row lo (40 bits); P2_DENSE_T: row stride << 40
+  uint32_t zi;             // z slot (low-rank) or first input index (dense)
+  uint32_t meta;           // lo | last << 8 (rows lo .. last of the slab) | P2_* << 16 | input indices << 24 (P2_DENSE_T: <= 32)
+};
+constexpr uint64_t SLAB_OFF_MASK = ((uint64_t)1 << 40) - 1;
+struct Slab {
+  uint32_t row0, nrows;    // output rows of the slab
+  uint32_t begin, dense, mid, end;   // entries: low-rank, dense from `dense`, P2_DENSE_T from `mid`
+};
+
 constexpr int MV_WROWS = 1024;         // rows per phase-2 window (8 warps x 32 lanes x 4 rows)
 
 struct MvPlan {
@@ -178,13 +191,11 @@ struct MvPlan {
   MvWin* d_wind = nullptr;         // windows over d_p2d (nwin of them)
   P2Desc* d_p2r = nullptr;         // the low-rank descriptors alone, window by window (built with d_p2d)
   MvWin* d_winr = nullptr;         // windows over d_p2r
-  // phase 2 by tree clusters (hm_autotune's phase-2 shape 1; built on first
-  // use): a unit is a 128-row chunk of an output cluster that is some leaf's
-  // cluster, with exactly the leaves of that cluster; one warp per unit
-  bool cl_built = false;
-  P2Desc* d_cd = nullptr;          // descriptors, unit by unit (offsets moved to the chunk's first row)
-  MvWin* d_cu = nullptr;           // units: rows [row0, row0 + nrows), descriptors [begin, end)
-  std::vector<int32_t> cl_level;   // units of tree level i: [cl_level[i], cl_level[i + 1])
+  // phase 2 by row slabs (phase-2 shape 1; built on first use)
+  Slab* d_slab = nullptr;          // nslab slabs
+  SlabEnt* d_ent = nullptr;        // (in the allocation of d_slab)
+  int32_t nslab = 0;
+  bool no_slab = false;            // the lists could not be had
 };
 
 struct LuState;            // H-LU data (hm_lu.cu)
@@ -241,7 +252,7 @@ struct hm_handle {
   int64_t piv_count = 0;
 
   struct Tune {                    // launch shapes chosen by hm_autotune (hm_api.cu)
-    int p2_split = 4;              // phase-2 CTAs per 1024-row window (2, 4, 8); 1: by tree clusters
+    int p2_split = 4;              // phase-2 CTAs per 1024-row window (2, 4, 8); 1: by row slabs
     int p1_waves = 1;              // phase-1 grid in resident waves (1, 2, 4)
     int tc_nc[3] = {0, 0, 0};      // tensor-core column block for c <= 16, <= 32, > 32 (0: by c)
     int tuned = 0;
@@ -276,6 +287,7 @@ int build_handle(hm_handle* h, const double* geom, int64_t ncluster,
                  const int64_t* cl_s, const int64_t* cl_e, const int64_t* cl_left,
                  const int64_t* cl_right, int64_t n_nb, const int64_t* nb_pairs);
 int build_matvec_plans(hm_handle* h);
+std::vector<int64_t> pool_order(const hm_handle* h);   // leaves in the order of the pools
 int build_like(hm_handle* h, const hm_handle* ref);
 int partition_only(hm_handle* h, int64_t ncl, const int64_t* cl_s, const int64_t* cl_e, const int64_t* cl_left,
                    const int64_t* cl_right, int64_t n_nb, const int64_t* nb_pairs);

@@ -53,6 +53,30 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
   return s;
 }
 
+// Sums NV values over the warp.  Each round halves the values a lane keeps
+// (it sends the other half to the partner lane), so 2*CB sums cost NV-1
+// shuffles instead of 5*NV.  On return the lane holds the total of value idx;
+// the lanes that agree in their low log2(32/NV) bits hold the same total.
+template <int NV>
+__device__ __forceinline__ double warp_reduce_scatter(double (&v)[NV], int lane, int& idx) {
+  idx = 0;
+#pragma unroll
+  for (int h = NV / 2, o = 16; h >= 1; h >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const double send = up ? v[i] : v[i + h];
+      const double keep = up ? v[i + h] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+    if (up) idx += h;
+  }
+  double s = v[0];
+#pragma unroll
+  for (int o = 16 / NV; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
 // ---------------------------------------------------------------------------
 // host-side helpers implemented in hm_lowrank.cu
 // ---------------------------------------------------------------------------

@@ -395,173 +395,166 @@ __global__ void __launch_bounds__(P2Shape<SPLIT>::WARPS * 32) mv_phase2_kernel(c
 }
 
 // ---------------------------------------------------------------------------
-// phase 2 by tree clusters: one warp per unit (at most 128 rows of one output
-// cluster and all the leaves of that cluster), R = 1, 2 or 4 consecutive rows
-// a lane by the unit's size.  Every entry starts on the unit's first row, so a
-// lane's R values come in one aligned load (columns are padded to a multiple
-// of 4 elements and 16 bytes; values past the unit's last row are loaded but
-// never stored).  The result is added into y.
+// phase 2 by row slabs: the output rows are cut at cluster boundaries into
+// slabs of at most 224 rows; one CTA per slab, R = ceil(rows / 32) rows a lane
+// (32 apart), its 8 warps splitting the slab's entries (one entry: one column
+// of a leaf over the slab's rows) and adding their sums in shared memory, in
+// one launch that writes every row once.  A lane reads single elements, 32
+// consecutive rows per warp load, so a leaf may start at any row: no alignment
+// to honour, and few idle lanes since leaves end where slabs end.  The next 32
+// entries and their z values are fetched while the current ones are summed.
+// Bound: HBM (R x 32 elements per entry).  Why slabs: grouped by tree cluster
+// (one warp per 128 rows of a cluster, a launch per tree level) a level of
+// n = 100003 has about 1000 warps with 760 dependent entries each, a fifth of
+// what the SMs hold, and the levels run one after another.
 // ---------------------------------------------------------------------------
-constexpr int CL_E = 64;       // expanded (leaf, column) entries per warp round
-constexpr int CL_WARPS = 8;
+constexpr int SL_WARPS = 8;
+constexpr int SL_RMAX = 7;                     // rows a lane at most
 
-template <int R> __device__ __forceinline__ void cl_ld(const double* p, double (&v)[R]) {
-  if constexpr (R == 1) {
-    v[0] = __ldcs(p);
-  } else if constexpr (R == 2) {
-    const double2 a = __ldcs(reinterpret_cast<const double2*>(p));
-    v[0] = a.x; v[1] = a.y;
-  } else {
-    const double2 a = __ldcs(reinterpret_cast<const double2*>(p));
-    const double2 b = __ldcs(reinterpret_cast<const double2*>(p) + 1);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-  }
-}
-template <int R> __device__ __forceinline__ void cl_ld(const float* p, float (&v)[R]) {
-  if constexpr (R == 1) {
-    v[0] = __ldcs(p);
-  } else if constexpr (R == 2) {
-    const float2 a = __ldcs(reinterpret_cast<const float2*>(p));
-    v[0] = a.x; v[1] = a.y;
-  } else {
-    const float4 a = __ldcs(reinterpret_cast<const float4*>(p));
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-  }
-}
-
-struct ClSmem {                 // one warp's staging
-  P2Desc sd[32];
-  int spre[33];
-  uint32_t e_rs[CL_E];
-  uint64_t e_off[CL_E];
-  double e_z[CL_E];
+// one element of a factor or dense leaf: how it is loaded and its value in the
+// kernel's arithmetic (FP64 factors: FP64, the others FP32 products)
+template <typename E> struct SlT {
+  using Raw = E;
+  __device__ static Raw ld(const E* p) { return __ldcs(p); }
+  __device__ static E val(Raw r) { return r; }
+};
+template <> struct SlT<__nv_bfloat16> {
+  using Raw = unsigned short;
+  __device__ static Raw ld(const __nv_bfloat16* p) { return __ldcs(reinterpret_cast<const unsigned short*>(p)); }
+  __device__ static float val(Raw r) { return __uint_as_float((uint32_t)r << 16); }
 };
 
-template <typename T, int R>
-__device__ __forceinline__ void cl_unit(const MvWin& W, const P2Desc* __restrict__ d, const T* __restrict__ rk,
-                                        const T* __restrict__ dn, const double* __restrict__ z,
-                                        const double* __restrict__ x, double* __restrict__ y, ClSmem& sm, int lane) {
-  constexpr int U0 = (sizeof(T) == 8 ? 16 : 32) / R;   // 128 bytes in flight a lane, 8 entries at most
-  constexpr int U = U0 > 8 ? 8 : U0;
-  const int base = R * lane;
-  const int nrows = (int)W.nrows;
-  const bool act = base < nrows;
+// acc[q] += the entries [begin, begin + ne) of one kind, this warp's share of
+// them in whole groups of 8: E the element type, v the array zi indexes
+template <typename E, typename A, int R>
+__device__ __forceinline__ void slab_sum(const SlabEnt* __restrict__ ents, uint32_t begin, uint32_t ne,
+                                         const E* __restrict__ pool, const double* __restrict__ v, int warp, int lane,
+                                         double (&acc)[R]) {
+  // entries whose loads are in flight together: 16 to 56 loads, 64 registers at most
+  constexpr int U = (sizeof(A) == 8 ? 32 : 64) / R >= 16 ? 16 : (sizeof(A) == 8 ? 32 : 64) / R >= 8 ? 8 : 4;
+  const uint32_t per = (ne + SL_WARPS * 8 - 1) / (SL_WARPS * 8) * 8;
+  const uint32_t e0 = begin + min(ne, warp * per), e1 = begin + min(ne, (warp + 1) * per);
+  const SlabEnt none{0, 0, 255u | 255u << 8};            // row 255: in no slab
+  SlabEnt cur = e0 + lane < e1 ? ents[e0 + lane] : none;
+  A zc = e0 + lane < e1 ? (A)__ldg(v + cur.zi) : A(0);
+  for (uint32_t e = e0; e < e1; e += 32) {
+    const bool more = e + 32 + lane < e1;
+    const SlabEnt nxt = more ? ents[e + 32 + lane] : none;
+    const int n32 = (int)min(32u, e1 - e);
+    const E* mine = pool + (cur.off & SLAB_OFF_MASK);
+    A zn = A(0);
+    for (int u0 = 0; u0 < n32; u0 += U) {
+      typename SlT<E>::Raw raw[U][R];
+      uint32_t first[U], span[U];                        // lane - lo, last - lo
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const E* p = reinterpret_cast<const E*>(__shfl_sync(0xffffffffu, (unsigned long long)mine, u0 + u));
+        const uint32_t mt = __shfl_sync(0xffffffffu, cur.meta, u0 + u);
+        first[u] = lane - (mt & 255u);
+        span[u] = (mt >> 8 & 255u) - (mt & 255u);
+        // no branch around the loads, or the compiler moves each beside its use:
+        // rows not covered read the entry's last row
+#pragma unroll
+        for (int q = 0; q < R; ++q) raw[u][q] = SlT<E>::ld(p + min(first[u] + 32 * q, span[u]));
+      }
+      if (u0 == 0 && more) zn = (A)__ldg(v + nxt.zi);     // behind this group's loads
+      A part[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) part[q] = A(0);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const A zz = __shfl_sync(0xffffffffu, zc, u0 + u);
+#pragma unroll
+        for (int q = 0; q < R; ++q)
+          if (first[u] + 32 * q <= span[u]) {            // rows not covered: an infinite z stays out
+            if constexpr (std::is_same<A, double>::value) acc[q] = fma(SlT<E>::val(raw[u][q]), zz, acc[q]);
+            else part[q] = fmaf(SlT<E>::val(raw[u][q]), zz, part[q]);
+          }
+        // FP32 products and partial sums over 8 entries, folded into the FP64
+        // row sums
+        if (!std::is_same<A, double>::value && u % 8 == 7) {
+#pragma unroll
+          for (int q = 0; q < R; ++q) {
+            acc[q] += (double)part[q];
+            part[q] = A(0);
+          }
+        }
+      }
+    }
+    cur = nxt;
+    zc = zn;
+  }
+}
+
+// one slab's sums over this warp's entries, into its rows of part_sh
+template <typename T, typename TD, int R>
+__device__ __forceinline__ void slab_rows(const Slab& S, const SlabEnt* __restrict__ ents, const T* __restrict__ rk,
+                                          const TD* __restrict__ dn, const double* __restrict__ z,
+                                          const double* __restrict__ x, double* __restrict__ part_sh, int warp, int lane) {
+  using A = typename std::conditional<std::is_same<T, double>::value, double, float>::type;
   double acc[R];
 #pragma unroll
   for (int q = 0; q < R; ++q) acc[q] = 0.0;
-  for (uint32_t b0 = W.begin; b0 < W.end; b0 += 32) {
-    const int nb = (int)min(32u, W.end - b0);
-    __syncwarp();
-    int cnt = 0;
-    if (lane < nb) {
-      sm.sd[lane] = d[b0 + lane];
-      cnt = (int)sm.sd[lane].cnt;
-    }
-    int incl = cnt;
+  slab_sum<T, A, R>(ents, S.begin, S.dense - S.begin, rk, z, warp, lane, acc);
+  slab_sum<TD, A, R>(ents, S.dense, S.mid - S.dense, dn, x, warp, lane, acc);
+  // dense leaves read along their rows (H'x): an entry is 32 input indices of
+  // one leaf; lane = input index (coalesced), 16 rows at a time, whose sums
+  // over the lanes a reduce-scatter leaves in lanes 2 i and 2 i + 1
+  for (uint32_t e = S.mid + warp; e < S.end; e += SL_WARPS) {
+    const SlabEnt E = ents[e];
+    const int lo = (int)(E.meta & 255u), last = (int)(E.meta >> 8 & 255u), cnt = (int)(E.meta >> 24);
+    const int64_t ld = (int64_t)(E.off >> 40);
+    const TD* base = dn + (E.off & SLAB_OFF_MASK) + lane;
+    const double xv = lane < cnt ? __ldg(x + E.zi + lane) : 0.0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    sm.spre[lane + 1] = incl;
-    if (lane == 0) sm.spre[0] = 0;
-    __syncwarp();
-    const int total = sm.spre[nb];
-    for (int e0 = 0; e0 < total; e0 += CL_E) {
-      const int ne = min(CL_E, total - e0);
-      __syncwarp();
-      for (int e = lane; e < ne; e += 32) {
-        const int ge = e0 + e;
-        int lo = 0, hi = nb - 1;
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (sm.spre[mid] <= ge) lo = mid; else hi = mid - 1;
-        }
-        const P2Desc& D = sm.sd[lo];
-        const int c = ge - sm.spre[lo];
-        if (D.type == P2_RK) {
-          sm.e_off[e] = D.off + (uint64_t)c * D.ld;
-          sm.e_rs[e] = 1;
-          sm.e_z[e] = z[D.aux + c];
-        } else if (D.type == P2_DENSE) {
-          sm.e_off[e] = (D.off + (uint64_t)c * D.ld) | P2_DENSE_FLAG;
-          sm.e_rs[e] = 1;
-          sm.e_z[e] = x[D.aux + c];
-        } else {
-          sm.e_off[e] = (D.off + (uint64_t)c) | P2_DENSE_FLAG;
-          sm.e_rs[e] = D.ld;
-          sm.e_z[e] = x[D.aux + c];
-        }
+    for (int g = 0; g < 2 * R; ++g) {
+      const int g0 = 16 * g;                             // rows g0 .. g0 + 15
+      if (g0 > last || g0 + 15 < lo) continue;
+      double v[16];
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {
+        const bool in = lane < cnt && g0 + r >= lo && g0 + r <= last;
+        v[r] = in ? (double)__ldcs(base + (g0 + r - lo) * ld) : 0.0;
       }
-      __syncwarp();
-      if (!act) continue;
-      for (int e = 0; e < ne; e += U) {
-        T v[U][R];
-        T zz[U];                               // the FP32 path multiplies by z rounded to FP32
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-#pragma unroll
-          for (int q = 0; q < R; ++q) v[u][q] = T(0);
-          zz[u] = T(0);
-          const int ee = e + u;
-          if (ee < ne) {
-            const uint64_t o = sm.e_off[ee];
-            const uint32_t rs = sm.e_rs[ee];
-            const T* p = (o & P2_DENSE_FLAG) ? dn + (o & ~P2_DENSE_FLAG) : rk + o;
-            zz[u] = (T)sm.e_z[ee];
-            if (rs == 1) {
-              cl_ld<R>(p + base, v[u]);
-            } else {
-#pragma unroll
-              for (int q = 0; q < R; ++q)
-                if (base + q < nrows) v[u][q] = __ldg(p + (uint64_t)(base + q) * rs);
-            }
-          }
-        }
-        if constexpr (std::is_same<T, double>::value) {
-#pragma unroll
-          for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int q = 0; q < R; ++q) acc[q] = fma(v[u][q], zz[u], acc[q]);
-        } else {
-          // FP32 products and partial sums over the U entries in flight,
-          // folded into the FP64 row sums once per group
-          float part[R];
-#pragma unroll
-          for (int q = 0; q < R; ++q) part[q] = 0.f;
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-#pragma unroll
-            for (int q = 0; q < R; ++q) part[q] = fmaf(v[u][q], zz[u], part[q]);
-          }
-#pragma unroll
-          for (int q = 0; q < R; ++q) acc[q] += (double)part[q];
-        }
-      }
+      for (int r = 0; r < 16; ++r)
+        if (lane < cnt && g0 + r >= lo && g0 + r <= last) v[r] *= xv;
+      int idx;
+      const double sum = warp_reduce_scatter<16>(v, lane, idx);
+      const double got = __shfl_sync(0xffffffffu, sum, 2 * (lane & 15));
+      if ((lane >> 4) == (g & 1)) acc[g >> 1] += got;
     }
   }
-  if (act) {
 #pragma unroll
-    for (int q = 0; q < R; ++q)
-      if (base + q < nrows) y[W.row0 + base + q] += acc[q];
-  }
+  for (int q = 0; q < R; ++q) part_sh[warp * 32 * SL_RMAX + lane + 32 * q] = acc[q];
 }
 
-template <typename T>
-__global__ void __launch_bounds__(CL_WARPS * 32, 3) mv_phase2c_kernel(const MvWin* __restrict__ units, int nu,
-                                                                   const P2Desc* __restrict__ d,
-                                                                   const T* __restrict__ rk, const T* __restrict__ dn,
-                                                                   const double* __restrict__ z,
-                                                                   const double* __restrict__ x,
-                                                                   double* __restrict__ y) {
-  __shared__ ClSmem sm[CL_WARPS];
+template <typename T, typename TD>
+__global__ void __launch_bounds__(SL_WARPS * 32, 2) mv_slab_kernel(const Slab* __restrict__ slabs,
+                                                                const SlabEnt* __restrict__ ents,
+                                                                const T* __restrict__ rk, const TD* __restrict__ dn,
+                                                                const double* __restrict__ z,
+                                                                const double* __restrict__ x,
+                                                                double* __restrict__ y) {
+  __shared__ double part_sh[SL_WARPS * 32 * SL_RMAX];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int u = blockIdx.x * CL_WARPS + warp;
-  if (u >= nu) return;                         // warps are independent: no block barrier follows
-  const MvWin W = units[u];
-  if (W.nrows > 64) cl_unit<T, 4>(W, d, rk, dn, z, x, y, sm[warp], lane);
-  else if (W.nrows > 32) cl_unit<T, 2>(W, d, rk, dn, z, x, y, sm[warp], lane);
-  else cl_unit<T, 1>(W, d, rk, dn, z, x, y, sm[warp], lane);
+  const Slab S = slabs[blockIdx.x];
+  switch ((S.nrows + 31) / 32) {
+    case 1: slab_rows<T, TD, 1>(S, ents, rk, dn, z, x, part_sh, warp, lane); break;
+    case 2: slab_rows<T, TD, 2>(S, ents, rk, dn, z, x, part_sh, warp, lane); break;
+    case 3: slab_rows<T, TD, 3>(S, ents, rk, dn, z, x, part_sh, warp, lane); break;
+    case 4: slab_rows<T, TD, 4>(S, ents, rk, dn, z, x, part_sh, warp, lane); break;
+    case 5: slab_rows<T, TD, 5>(S, ents, rk, dn, z, x, part_sh, warp, lane); break;
+    case 6: slab_rows<T, TD, 6>(S, ents, rk, dn, z, x, part_sh, warp, lane); break;
+    default: slab_rows<T, TD, 7>(S, ents, rk, dn, z, x, part_sh, warp, lane);
+  }
+  __syncthreads();
+  for (int r = threadIdx.x; r < (int)S.nrows; r += SL_WARPS * 32) {
+    double s = part_sh[r];
+#pragma unroll
+    for (int w = 1; w < SL_WARPS; ++w) s += part_sh[w * 32 * SL_RMAX + r];
+    y[S.row0 + r] = s;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -578,90 +571,219 @@ void free_mv_plan(MvPlan& p) {
   if (p.d_wind) cudaFree(p.d_wind);
   if (p.d_p2r) cudaFree(p.d_p2r);
   if (p.d_winr) cudaFree(p.d_winr);
-  if (p.d_cd) cudaFree(p.d_cd);
-  if (p.d_cu) cudaFree(p.d_cu);
+  if (p.d_slab) cudaFree(p.d_slab);
   p = MvPlan{};
 }
 
-// Phase 2 by tree clusters (MvPlan::cl_*).  The leaves are grouped by their
-// output cluster (the row cluster for H*x, the column cluster for H'*x) and the
-// cluster is cut into 128-row units, so every entry of a unit covers all the
-// unit's rows from its first: each lane's rows come in one aligned vector load
-// wherever the cluster boundaries fall.  Units of one tree level are disjoint;
-// the levels run one launch after another and add into y.  z offsets follow
-// the pool order of the low-rank leaves, as in build_mv_descriptors.
-constexpr int CL_ROWS = 128;                   // rows of a unit at most (32 lanes x 4 rows)
-static int build_cluster_plan(hm_handle* h, int trans, MvPlan& P) {
-  const int eb = elem_bytes(h->storage), deb = dense_elem_bytes(h->storage);
-  std::vector<int64_t> rk;                       // low-rank leaves in pool order
-  for (size_t i = 0; i < h->leaves.size(); ++i)
-    if (h->leaves[i].type == T_RK) rk.push_back((int64_t)i);
-  std::stable_sort(rk.begin(), rk.end(), [&](int64_t a, int64_t b) { return h->leaves[a].off < h->leaves[b].off; });
-  std::vector<uint32_t> zoff(h->leaves.size(), 0);
-  int64_t z = 0;
-  for (int64_t li : rk) { zoff[li] = (uint32_t)z; z += h->leaves[li].k; }
-  const int64_t ncl = (int64_t)h->cl_s.size();
-  std::vector<std::vector<int64_t>> by(ncl);     // leaves by output cluster
-  int32_t maxdepth = 0;
-  for (size_t i = 0; i < h->leaves.size(); ++i) {
-    const Leaf& L = h->leaves[i];
-    if (L.type == T_RK && L.k == 0) continue;
-    const int32_t c = trans ? L.t : L.s;
-    by[c].push_back((int64_t)i);
-    maxdepth = std::max(maxdepth, h->cl_depth[c]);
-  }
-  std::vector<std::vector<int64_t>> lev(maxdepth + 1);   // clusters by tree level, in row order
-  for (int64_t c = 0; c < ncl; ++c)
-    if (!by[c].empty()) lev[h->cl_depth[c]].push_back(c);
-  for (auto& v : lev)
-    std::sort(v.begin(), v.end(), [&](int64_t a, int64_t b) { return h->cl_s[a] < h->cl_s[b]; });
-  std::vector<P2Desc> d;
-  std::vector<MvWin> w;
-  P.cl_level.assign(1, 0);
-  for (int32_t l = maxdepth; l >= 0; --l) {
-    for (int64_t c : lev[l]) {
-      const int64_t c0 = h->cl_s[c], m = h->cl_e[c] - h->cl_s[c];
-      for (int64_t r0 = 0; r0 < m; r0 += CL_ROWS) {
-        MvWin W{};
-        W.row0 = (uint32_t)(c0 + r0);
-        W.nrows = (uint32_t)std::min<int64_t>(CL_ROWS, m - r0);
-        W.begin = (uint32_t)d.size();
-        for (int64_t li : by[c]) {
-          const Leaf& L = h->leaves[li];
-          const int64_t npad = col_pad(L.n, eb), mpad = col_pad(L.m, eb);
-          P2Desc D{};
-          D.m = W.nrows;
-          if (L.type == T_RK) {
-            D.type = P2_RK;
-            D.off = (trans ? L.off : L.off + npad * L.k) + r0;
-            D.ld = (uint32_t)(trans ? npad : mpad);
-            D.aux = zoff[li];
-            D.cnt = (uint32_t)L.k;
-          } else {
-            const int64_t ldc = col_pad(L.m, deb);
-            D.type = trans ? P2_DENSE_T : P2_DENSE;
-            D.off = L.off + (trans ? r0 * ldc : r0);
-            D.ld = (uint32_t)ldc;
-            D.aux = (uint32_t)(trans ? L.row0 : L.col0);
-            D.cnt = (uint32_t)(trans ? L.m : L.n);
-          }
-          d.push_back(D);
-        }
-        W.end = (uint32_t)d.size();
-        w.push_back(W);
+// One leaf of a slab plan: its factor (low-rank) or block (dense) over the
+// output rows [row0, row0 + m), which are (part of) the slabs [w0, w1]; slot:
+// index of its first (leaf, slab) pair
+struct SlabLeaf {
+  int64_t off;
+  uint32_t row0, m, ld, zi, cnt, slot, w0, w1;
+  uint16_t type;
+};
+// entries of one leaf, a warp per leaf: pos[slot + w - w0] is its first entry
+// in slab w
+__global__ void __launch_bounds__(256) slab_fill_kernel(const SlabLeaf* __restrict__ leaf, int64_t nleaf,
+                                                        const uint32_t* __restrict__ pos,
+                                                        const Slab* __restrict__ slabs, SlabEnt* __restrict__ ent) {
+  const int lane = threadIdx.x & 31;
+  const int64_t li = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (li >= nleaf) return;
+  const SlabLeaf L = leaf[li];
+  const uint32_t ne = L.type == P2_DENSE_T ? (L.cnt + 31) / 32 : L.cnt;
+  for (uint32_t w = L.w0; w <= L.w1; ++w) {
+    const uint32_t s0 = slabs[w].row0, s1 = s0 + slabs[w].nrows;
+    const uint32_t a = max(L.row0, s0), b = min(L.row0 + L.m, s1);
+    const uint32_t p = pos[L.slot + (w - L.w0)];
+    for (uint32_t c = lane; c < ne; c += 32) {
+      SlabEnt E;
+      E.meta = (a - s0) | (b - 1 - s0) << 8 | (uint32_t)L.type << 16;
+      if (L.type == P2_DENSE_T) {
+        E.off = (uint64_t)(L.off + (int64_t)(a - L.row0) * L.ld + 32 * c) | (uint64_t)L.ld << 40;
+        E.zi = L.zi + 32 * c;
+        E.meta |= min(32u, L.cnt - 32 * c) << 24;
+      } else {
+        E.off = (uint64_t)(L.off + (int64_t)c * L.ld + (a - L.row0));
+        E.zi = L.zi + c;
       }
+      ent[p + c] = E;
     }
-    P.cl_level.push_back((int32_t)w.size());
   }
-  if (d.size() > (size_t)UINT32_MAX || w.size() > (size_t)INT32_MAX)
-    return fail(HM_ERR_UNSUPPORTED, "too many cluster descriptors");
-  if (d.empty()) d.push_back(P2Desc{});
-  if (w.empty()) w.push_back(MvWin{});
-  HM_CUDA_TRY(cudaMalloc(&P.d_cd, sizeof(P2Desc) * d.size()));
-  HM_CUDA_TRY(h2d_sync(P.d_cd, d.data(), sizeof(P2Desc) * d.size()));
-  HM_CUDA_TRY(cudaMalloc(&P.d_cu, sizeof(MvWin) * w.size()));
-  HM_CUDA_TRY(h2d_sync(P.d_cu, w.data(), sizeof(MvWin) * w.size()));
-  P.cl_built = true;
+}
+
+// The slab boundaries for slabs of at most `most` rows: the highest clusters
+// that small, a leaf cluster above that size in equal pieces.  Leaves of the
+// block tree sit on clusters, so they end where slabs do.
+static void slab_cuts(const hm_handle* h, int64_t most, std::vector<Slab>& out) {
+  out.clear();
+  std::vector<int64_t> todo(1, 0);
+  while (!todo.empty()) {
+    const int64_t c = todo.back();
+    todo.pop_back();
+    const int64_t s = h->cl_s[c], m = h->cl_e[c] - s;
+    if (m > most && h->cl_left[c] >= 0) {
+      todo.push_back(h->cl_right[c]);
+      todo.push_back(h->cl_left[c]);
+      continue;
+    }
+    const int64_t np = (m + most - 1) / most;
+    for (int64_t i = 0; i < np; ++i) {
+      Slab S{};
+      S.row0 = (uint32_t)(s + m * i / np);
+      S.nrows = (uint32_t)(s + m * (i + 1) / np - S.row0);
+      out.push_back(S);
+    }
+  }
+}
+
+// The slab size: of 32, 64, .. 224 rows at most, the one whose slabs leave the
+// fewest lanes idle (the larger one on a tie: fewer entries per factor byte),
+// among those that give every SM four slabs; 32 rows for matrices too small
+// for that.
+static void choose_slabs(const hm_handle* h, std::vector<Slab>& best) {
+  slab_cuts(h, 32, best);
+  double eff = 0.0;
+  std::vector<Slab> v;
+  for (int r = 1; r <= SL_RMAX; ++r) {
+    slab_cuts(h, 32 * r, v);
+    if (v.size() < 4 * 148) break;
+    int64_t lanes = 0;
+    for (const Slab& S : v) lanes += (S.nrows + 31) / 32 * 32;
+    const double e = (double)h->n / (double)lanes;
+    if (e >= eff * 0.999) {
+      eff = std::max(eff, e);
+      best = v;
+    }
+  }
+}
+
+// The slab lists of one direction.  z offsets follow the pool order of the
+// low-rank leaves, as in build_mv_descriptors; a slab lists its leaves in pool
+// order, low-rank ones first, those read along their rows (dense, H'x) last.
+static int build_slab_plan(hm_handle* h, int trans, MvPlan& P) {
+  const int eb = elem_bytes(h->storage), deb = dense_elem_bytes(h->storage);
+  std::vector<Slab> slab;
+  choose_slabs(h, slab);
+  const int64_t nslab = (int64_t)slab.size();
+  auto slab_of = [&](int64_t row) {
+    return (uint32_t)(std::upper_bound(slab.begin(), slab.end(), row,
+                                       [](int64_t r, const Slab& S) { return r < (int64_t)S.row0; }) - slab.begin() - 1);
+  };
+  // per cluster: leaves of one cluster share its slabs
+  const int64_t ncl = (int64_t)h->cl_s.size();
+  std::vector<uint32_t> c0((size_t)ncl), c1((size_t)ncl);
+  for (int64_t c = 0; c < ncl; ++c) {
+    c0[c] = slab_of(h->cl_s[c]);
+    c1[c] = slab_of(h->cl_e[c] - 1);
+  }
+  const std::vector<int64_t> order = pool_order(h);
+  std::vector<SlabLeaf> leaf;
+  leaf.reserve(order.size());
+  std::vector<uint64_t> cnt[3];                          // entries per slab: low-rank, dense, along rows
+  for (auto& v : cnt) v.assign((size_t)nslab, 0);
+  auto section = [](uint16_t type) { return type == P2_RK ? 0 : type == P2_DENSE ? 1 : 2; };
+  uint64_t slots = 0, z = 0;
+  for (int64_t li : order) {
+    const Leaf& L = h->leaves[li];
+    const int64_t npad = col_pad(L.n, eb), mpad = col_pad(L.m, eb);
+    SlabLeaf D{};
+    D.row0 = (uint32_t)(trans ? L.col0 : L.row0);
+    D.m = (uint32_t)(trans ? L.n : L.m);
+    if (L.type == T_RK) {
+      D.type = P2_RK;
+      D.off = trans ? L.off : L.off + npad * L.k;
+      D.ld = (uint32_t)(trans ? npad : mpad);
+      D.zi = (uint32_t)z;
+      D.cnt = (uint32_t)L.k;
+      z += (uint64_t)L.k;
+      if (L.k == 0) continue;
+    } else {
+      const int64_t ldc = col_pad(L.m, deb);
+      D.type = trans ? P2_DENSE_T : P2_DENSE;
+      D.off = L.off;
+      D.ld = (uint32_t)ldc;
+      D.zi = (uint32_t)(trans ? L.row0 : L.col0);
+      D.cnt = (uint32_t)(trans ? L.m : L.n);
+      if (trans && ldc >= (int64_t)1 << 24) return HM_ERR_UNSUPPORTED;   // the entry's stride field
+    }
+    D.slot = (uint32_t)slots;
+    D.w0 = c0[trans ? L.t : L.s];
+    D.w1 = c1[trans ? L.t : L.s];
+    slots += (uint64_t)(D.w1 - D.w0 + 1);
+    for (uint32_t w = D.w0; w <= D.w1; ++w) cnt[section(D.type)][w] += D.type == P2_DENSE_T ? (D.cnt + 31) / 32 : D.cnt;
+    leaf.push_back(D);
+  }
+  uint64_t tot = 0;
+  for (int64_t w = 0; w < nslab; ++w) {
+    Slab& S = slab[w];
+    uint32_t* at[3] = {&S.dense, &S.mid, &S.end};
+    S.begin = (uint32_t)tot;
+    for (int k = 0; k < 3; ++k) {
+      const uint64_t first = tot;
+      tot += cnt[k][w];
+      *at[k] = (uint32_t)tot;
+      cnt[k][w] = first;                                 // from here on: next free entry
+    }
+  }
+  if (tot > (uint64_t)UINT32_MAX || slots > (uint64_t)UINT32_MAX) return HM_ERR_UNSUPPORTED;
+  std::vector<uint32_t> pos((size_t)slots);
+  for (const SlabLeaf& D : leaf) {
+    for (uint32_t w = D.w0; w <= D.w1; ++w) {
+      uint64_t& next = cnt[section(D.type)][w];
+      pos[D.slot + (w - D.w0)] = (uint32_t)next;
+      next += D.type == P2_DENSE_T ? (D.cnt + 31) / 32 : D.cnt;
+    }
+  }
+  // one upload: leaves, first entries, slabs; the entries are written by the device
+  const size_t lb = sizeof(SlabLeaf) * leaf.size(), pb = sizeof(uint32_t) * pos.size();
+  const size_t sb = sizeof(Slab) * slab.size(), so = pad_to((int64_t)sb, 256);
+  void* keep = nullptr;                                  // slabs and entries
+  void* tmp = nullptr;
+  if (cudaMalloc(&keep, so + sizeof(SlabEnt) * std::max<size_t>(tot, 1)) != cudaSuccess) {
+    cudaGetLastError();
+    return HM_ERR_OOM;
+  }
+  if (cudaMallocAsync(&tmp, std::max<size_t>(lb + pb, 8), h->stream) != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(keep);
+    return HM_ERR_OOM;
+  }
+  cudaError_t e = cudaMemcpyAsync(keep, slab.data(), sb, cudaMemcpyHostToDevice, h->stream);
+  if (!leaf.empty()) {
+    if (e == cudaSuccess) e = cudaMemcpyAsync(tmp, leaf.data(), lb, cudaMemcpyHostToDevice, h->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync((char*)tmp + lb, pos.data(), pb, cudaMemcpyHostToDevice, h->stream);
+    const int64_t nl = (int64_t)leaf.size();
+    if (e == cudaSuccess) {
+      slab_fill_kernel<<<(unsigned)((nl + 7) / 8), 256, 0, h->stream>>>(
+          (const SlabLeaf*)tmp, nl, (const uint32_t*)((char*)tmp + lb), (const Slab*)keep,
+          (SlabEnt*)((char*)keep + so));
+      e = cudaGetLastError();
+    }
+  }
+  cudaFreeAsync(tmp, h->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);   // the caller's stream reads the entries next
+  if (e != cudaSuccess) {
+    cudaFree(keep);
+    return fail(HM_ERR_CUDA, std::string("row slabs: ") + cudaGetErrorString(e));
+  }
+  P.d_slab = (Slab*)keep;
+  P.d_ent = (SlabEnt*)((char*)keep + so);
+  P.nslab = (int32_t)nslab;
+  return HM_OK;
+}
+
+// Builds the slab lists on first use; false: this plan cannot have them (no
+// memory left for them, or an entry field too narrow) and the caller takes
+// the window lists, which every plan has.
+static int ensure_slabs(hm_handle* h, int trans, MvPlan& P, bool* usable) {
+  if (!P.d_slab && !P.no_slab) {
+    const int s = build_slab_plan(h, trans, P);
+    if (s == HM_ERR_OOM || s == HM_ERR_UNSUPPORTED) P.no_slab = true;
+    else if (s != HM_OK) return s;
+  }
+  *usable = P.d_slab != nullptr;
   return HM_OK;
 }
 
@@ -969,7 +1091,6 @@ static int matvec_t(hm_handle* h, const double* d_x, double* d_y, int trans, cud
   using TX = typename MvT<T>::X;
   constexpr int XA = 16 / (int)sizeof(TX);
   MvPlan& P = trans ? h->bwd : h->fwd;
-  if (std::is_same<T, __nv_bfloat16>::value) HM_TRY(split_p2(P));
   const int64_t stride = pad_to(h->n + 64, 64);
   HM_TRY(ensure_xs(h, sizeof(TX) * stride * XA));
   TX* xs = (TX*)h->d_xs;
@@ -995,8 +1116,14 @@ static int matvec_t(hm_handle* h, const double* d_x, double* d_y, int trans, cud
   if (ev) HM_CUDA_TRY(cudaEventRecord(ev[2], st));
   // dense leaves are FP64 with FP64 factors and FP32 otherwise
   using TD = typename std::conditional<std::is_same<T, double>::value, double, float>::type;
-  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+  bool slabs = false;
+  if (h->tune.p2_split == 1) HM_TRY(ensure_slabs(h, trans, P, &slabs));
+  if (slabs) {
+    mv_slab_kernel<T, TD><<<(unsigned)P.nslab, SL_WARPS * 32, 0, st>>>(
+        P.d_slab, P.d_ent, (const T*)h->d_rk, (const TD*)h->d_dense, h->d_z, d_x, d_y);
+  } else if constexpr (std::is_same<T, __nv_bfloat16>::value) {
     // dense leaves (FP32) first, written into y; then the BF16 low-rank part added
+    HM_TRY(split_p2(P));
     const int64_t nslab = (h->n + 31) / 32;
     mv_dense1_kernel<float><<<(unsigned)((nslab + 7) / 8), 256, 0, st>>>(P.d_wind, P.d_p2d,
                                                                          (const float*)h->d_dense, d_x, nslab, d_y);
@@ -1006,15 +1133,6 @@ static int matvec_t(hm_handle* h, const double* d_x, double* d_y, int trans, cud
     else                                       // splits 4 and 8: one warp a quarter window
       mv_phase2_bf16_kernel<4><<<(unsigned)(P.nwin * 4), P2Shape8<4>::WARPS * 32, 0, st>>>(
           P.d_winr, P.d_p2r, (const __nv_bfloat16*)h->d_rk, h->d_z, d_y);
-  } else if (h->tune.p2_split == 1) {
-    if (!P.cl_built) HM_TRY(build_cluster_plan(h, trans, P));
-    HM_CUDA_TRY(cudaMemsetAsync(d_y, 0, sizeof(double) * h->n, st));
-    for (size_t l = 0; l + 1 < P.cl_level.size(); ++l) {
-      const int u0 = P.cl_level[l], nu = P.cl_level[l + 1] - u0;
-      if (nu == 0) continue;
-      mv_phase2c_kernel<T><<<(unsigned)((nu + CL_WARPS - 1) / CL_WARPS), CL_WARPS * 32, 0, st>>>(
-          P.d_cu + u0, nu, P.d_cd, (const T*)h->d_rk, (const T*)h->d_dense, h->d_z, d_x, d_y);
-    }
   } else {
     auto p2 = [&](auto split) {
       constexpr int S = decltype(split)::value;
@@ -1091,46 +1209,98 @@ __global__ void __launch_bounds__(256) mvdd_phase1_kernel(const P1Desc* __restri
   }
 }
 
-// r = b - (sum over the window's leaves) per output row, one thread a row; a
-// window is split over MVDD_SPLIT CTAs of MV_WROWS / MVDD_SPLIT rows (the
-// double-double sums are latency-bound: one CTA per window left most SMs idle)
-constexpr int MVDD_SPLIT = 8;
-constexpr int MVDD_ROWS = MV_WROWS / MVDD_SPLIT;
+// r = b - (sum over the window's leaves) per output row.  A CTA owns 32 rows
+// (lane = row) and its 8 warps split the window's descriptors, every eighth
+// one each, so the dense near-field leaves, neighbours in the list, spread over
+// the warps; the warps' double-double sums are added in shared memory in warp
+// order.  The sums are chains of dependent FP64 operations: one thread a row
+// walking every descriptor kept an SM at two warps and took 380 us at
+// n = 20000.
+constexpr int MVDD_WARPS = 8;
+constexpr int MVDD_SPLIT = MV_WROWS / 32;
 template <typename T, typename TD>
-__global__ void __launch_bounds__(MVDD_ROWS) mvdd_phase2_kernel(const MvWin* __restrict__ win,
+__global__ void __launch_bounds__(MVDD_WARPS * 32) mvdd_phase2_kernel(const MvWin* __restrict__ win,
                                                                 const P2Desc* __restrict__ d, const T* __restrict__ rk,
                                                                 const TD* __restrict__ dn, const double* __restrict__ zh,
                                                                 const double* __restrict__ zl,
                                                                 const double* __restrict__ x,
                                                                 const double* __restrict__ bvec, double* __restrict__ rvec) {
+  __shared__ double sp[MVDD_WARPS][32], sc[MVDD_WARPS][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const MvWin W = win[blockIdx.x / MVDD_SPLIT];
-  const int r0 = (int)(blockIdx.x % MVDD_SPLIT) * MVDD_ROWS;      // this CTA's rows [r0, r0 + MVDD_ROWS)
-  const uint32_t row = (uint32_t)(r0 + threadIdx.x);
-  if (row < W.nrows) {
-    double p = 0.0, c = 0.0;
-    for (uint32_t e = W.begin; e < W.end; ++e) {
-      const P2Desc D = d[e];
-      if (D.row_off >= r0 + MVDD_ROWS || D.row_off + (int)D.m <= r0) continue;   // the whole CTA skips it
-      const int lr = (int)row - D.row_off;
-      if (lr < 0 || lr >= (int)D.m) continue;
-      if (D.type == P2_RK) {
-        for (uint32_t q = 0; q < D.cnt; ++q) {
-          const double v = from_store<T>(rk[D.off + (uint64_t)q * D.ld + lr]);
-          dd_add_prod(p, c, v, zh[D.aux + q]);
-          c = fma(v, zl[D.aux + q], c);
+  const int r0 = (int)(blockIdx.x % MVDD_SPLIT) * 32;             // this CTA's rows [r0, r0 + 32)
+  if (r0 >= (int)W.nrows) return;
+  double p = 0.0, c = 0.0;
+  for (uint32_t b0 = W.begin; b0 < W.end; b0 += 32 * MVDD_WARPS) {
+    const uint32_t b = b0 + lane * MVDD_WARPS + warp;
+    P2Desc D{};
+    bool cov = false;
+    if (b < W.end) {
+      D = d[b];
+      cov = D.row_off < r0 + 32 && D.row_off + (int)D.m > r0;
+    }
+    for (unsigned todo = __ballot_sync(0xffffffffu, cov); todo; todo &= todo - 1) {
+      const int src = __ffs(todo) - 1;
+      const uint64_t off = __shfl_sync(0xffffffffu, (unsigned long long)D.off, src);
+      const int lr = r0 + lane - __shfl_sync(0xffffffffu, D.row_off, src);
+      const int m = (int)__shfl_sync(0xffffffffu, D.m, src);
+      const uint32_t ld = __shfl_sync(0xffffffffu, D.ld, src), aux = __shfl_sync(0xffffffffu, D.aux, src);
+      const uint32_t cnt = __shfl_sync(0xffffffffu, D.cnt, src);
+      const uint32_t type = __shfl_sync(0xffffffffu, (uint32_t)D.type, src);
+      const bool mine = lr >= 0 && lr < m;
+      if (type == P2_RK) {
+        const T* f = rk + off + (mine ? lr : 0);
+        for (uint32_t q = 0; q < cnt; q += 4) {
+          double v[4], h[4], l[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const bool in = q + u < cnt;
+            v[u] = in && mine ? from_store<T>(f[(uint64_t)(q + u) * ld]) : 0.0;
+            h[u] = in ? __ldg(zh + aux + q + u) : 0.0;
+            l[u] = in ? __ldg(zl + aux + q + u) : 0.0;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (mine && q + u < cnt) {
+              dd_add_prod(p, c, v[u], h[u]);
+              c = fma(v[u], l[u], c);
+            }
         }
-      } else if (D.type == P2_DENSE) {
-        for (uint32_t q = 0; q < D.cnt; ++q)
-          dd_add_prod(p, c, (double)dn[D.off + (uint64_t)q * D.ld + lr], x[D.aux + q]);
       } else {
-        for (uint32_t q = 0; q < D.cnt; ++q)
-          dd_add_prod(p, c, (double)dn[D.off + (uint64_t)q + (uint64_t)lr * D.ld], x[D.aux + q]);
+        // dense: column by column, or along the rows of the leaf (H'x)
+        const bool tr = type == P2_DENSE_T;
+        const TD* f = dn + off + (mine ? (tr ? (uint64_t)lr * ld : (uint64_t)lr) : 0);
+        const uint64_t cs = tr ? 1 : ld;
+        for (uint32_t q = 0; q < cnt; q += 8) {
+          double v[8], h[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const bool in = q + u < cnt;
+            v[u] = in && mine ? (double)f[(q + u) * cs] : 0.0;
+            h[u] = in ? __ldg(x + aux + q + u) : 0.0;
+          }
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (mine && q + u < cnt) dd_add_prod(p, c, v[u], h[u]);
+        }
       }
     }
-    const uint32_t i = W.row0 + row;
+  }
+  sp[warp][lane] = p;
+  sc[warp][lane] = c;
+  __syncthreads();
+  if (warp == 0 && r0 + lane < (int)W.nrows) {
+    double ps = sp[0][lane], cs = sc[0][lane];
+#pragma unroll
+    for (int w = 1; w < MVDD_WARPS; ++w) {
+      double q;
+      two_sum(ps, sp[w][lane], ps, q);
+      cs += q + sc[w][lane];
+    }
+    const uint32_t i = W.row0 + (uint32_t)(r0 + lane);
     double t, q;
-    two_sum(bvec[i], -p, t, q);
-    rvec[i] = t + (q - c);
+    two_sum(bvec[i], -ps, t, q);
+    rvec[i] = t + (q - cs);
   }
 }
 
@@ -1155,7 +1325,7 @@ static int residual_t(hm_handle* h, const double* d_x, const double* d_b, double
     const int64_t blocks = std::min<int64_t>((P.np1 + 7) / 8, (int64_t)nsm * 8);
     mvdd_phase1_kernel<T><<<(unsigned)blocks, 256, 0, st>>>(P.d_p1, P.np1, (const T*)h->d_rk, d_x, zh, zl);
   }
-  mvdd_phase2_kernel<T, TD><<<(unsigned)(P.nwin * MVDD_SPLIT), MVDD_ROWS, 0, st>>>(
+  mvdd_phase2_kernel<T, TD><<<(unsigned)(P.nwin * MVDD_SPLIT), MVDD_WARPS * 32, 0, st>>>(
       P.d_win, P.d_p2, (const T*)h->d_rk, (const TD*)h->d_dense, zh, zl, d_x, d_b, d_r);
   HM_CUDA_TRY(cudaGetLastError());
   return HM_OK;

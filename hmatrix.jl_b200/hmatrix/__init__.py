@@ -233,7 +233,7 @@ class Hmat:
 
     def set_tune(self, p2_split, p1_waves=1):
         """Pin the single-column matvec launch shapes (hm_set_tune): p2_split
-        2, 4 or 8 CTAs per phase-2 window, or 1 for phase 2 by tree clusters."""
+        2, 4 or 8 CTAs per phase-2 window, or 1 for phase 2 by row slabs."""
         check(lib().hm_set_tune(self._h, int(p2_split), int(p1_waves)))
 
     def residual(self, x, b, trans=False):
