@@ -11,12 +11,14 @@
 // multiplied and summed in FP32 over the few vectors (phase 1) or entries
 // (phase 2) a lane has in flight, and those FP32 partial sums are added in
 // FP64: one conversion per group instead of one per element.
-// The input is staged as 16-byte aligned shifted copies so that every
-// x-segment load in phase 1 is a vector load, whatever the segment start.
+// For FP32 and BF16 factors the input is staged as 16-byte aligned shifted
+// copies in FP32, so that every x-segment load in phase 1 is a vector load,
+// whatever the segment start; with FP64 factors phase 1 reads x itself.
 #include "hm_internal.h"
 #include "hm_lowrank.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 #include <cstring>
 
@@ -27,19 +29,18 @@ namespace hm {
 // ---------------------------------------------------------------------------
 template <typename T> struct MvT;
 template <> struct MvT<double> {
-  static constexpr int VW = 2, U = 4, NR = 2;       // NR: factor columns a warp streams together
+  static constexpr int VW = 2, U = 2;
   using X = double;
   using R = double2;
   struct XV { double2 a; };
   __device__ static R ld(const double* p) { return __ldcs(reinterpret_cast<const double2*>(p)); }
-  __device__ static XV ldx(const double* p) { return XV{__ldg(reinterpret_cast<const double2*>(p))}; }
   __device__ static double dot(const R& f, const XV& x, double s) {
     s = fma(f.x, x.a.x, s);
     return fma(f.y, x.a.y, s);
   }
 };
 template <> struct MvT<float> {
-  static constexpr int VW = 4, U = 4, NR = 2;
+  static constexpr int VW = 4, U = 2;
   using X = float;
   using R = float4;
   struct XV { float4 a; };
@@ -56,7 +57,7 @@ template <> struct MvT<float> {
 __device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 template <> struct MvT<__nv_bfloat16> {
-  static constexpr int VW = 8, U = 2, NR = 4;       // a BF16 vector is half the bytes: twice the columns
+  static constexpr int VW = 8, U = 2;
   using X = float;
   using R = uint4;
   struct XV { float4 a, b; };
@@ -91,81 +92,95 @@ __global__ void xcopy_kernel(const double* __restrict__ x, int64_t n, TX* __rest
 // ---------------------------------------------------------------------------
 // phase 1: z = F1' x_seg, one warp per low-rank leaf
 // ---------------------------------------------------------------------------
-#ifndef HM_P1_MINB
-#define HM_P1_MINB 1
-#endif
+// A leaf's columns r .. r + NR - 1 (1 to 4 of them, all in flight together).
+// z of the NR columns is summed over the warp by one reduce-scatter.
+template <typename T, int NR>
+__device__ __forceinline__ void p1_columns(const T* __restrict__ F, uint32_t stride, uint32_t len,
+                                           const typename MvT<T>::X* __restrict__ xb, double* __restrict__ z,
+                                           int lane) {
+  using Tr = MvT<T>;
+  constexpr int VW = Tr::VW, U = Tr::U, NV = NR == 3 ? 4 : NR;
+  const int nvec = (int)(stride / VW);
+  double sc[NV];
+#pragma unroll
+  for (int j = 0; j < NV; ++j) sc[j] = 0.0;
+  for (int v0 = lane; v0 < nvec; v0 += 32 * U) {
+    typename Tr::R a[NR][U];
+    typename Tr::XV xv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int v = min(v0 + 32 * u, nvec - 1);          // past the end: the last vector, not summed
+#pragma unroll
+      for (int j = 0; j < NR; ++j) a[j][u] = Tr::ld(F + (int64_t)j * stride + (int64_t)v * VW);
+      if constexpr (std::is_same<T, double>::value) {
+        // the padding elements multiply no x (there may be none behind the last)
+        xv[u].a.x = 2 * v < (int)len ? __ldg(xb + 2 * v) : 0.0;
+        xv[u].a.y = 2 * v + 1 < (int)len ? __ldg(xb + 2 * v + 1) : 0.0;
+      } else {
+        xv[u] = Tr::ldx(xb + (int64_t)v * VW);
+      }
+    }
+    if constexpr (std::is_same<T, double>::value) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (v0 + 32 * u < nvec) {
+#pragma unroll
+          for (int j = 0; j < NR; ++j) sc[j] = Tr::dot(a[j][u], xv[u], sc[j]);
+        }
+    } else {
+      // FP32 products and partial sums over the U vectors in flight, folded
+      // into the FP64 sums once per group
+#pragma unroll
+      for (int j = 0; j < NR; ++j) {
+        float fp = 0.f;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (v0 + 32 * u < nvec) fp = Tr::dotf(a[j][u], xv[u], fp);
+        sc[j] += (double)fp;
+      }
+    }
+  }
+  int idx;
+  const double sum = warp_reduce_scatter<NV>(sc, lane, idx);
+  if ((lane & (32 / NV - 1)) == 0 && idx < NR) z[idx] = sum;
+}
+
+// One warp per low-rank leaf, the next leaf's descriptor fetched while this
+// one's columns stream; columns in groups of 4 or less, as even as they go.
+// Bound: HBM.  Three columns at a time instead of two and one repeated column,
+// and a third of the shuffles: the FP32 kernel had 16 warps an SM waiting on
+// 2 x 4 vectors each and spent as many instructions reducing as loading.
 template <typename T>
-__global__ void __launch_bounds__(256, HM_P1_MINB) mv_phase1_kernel(const P1Desc* __restrict__ d, int64_t nd,
+__global__ void __launch_bounds__(256, 3) mv_phase1_kernel(const P1Desc* __restrict__ d, int64_t nd,
                                                         const T* __restrict__ pool,
                                                         const typename MvT<T>::X* __restrict__ xs,
                                                         int64_t xs_stride, double* __restrict__ z) {
-  using Tr = MvT<T>;
-  using TX = typename Tr::X;
-  constexpr int VW = Tr::VW, U = Tr::U, NR = Tr::NR;
+  using TX = typename MvT<T>::X;
   constexpr int XA = 16 / (int)sizeof(TX);
   const int lane = threadIdx.x & 31;
   const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  P1Desc N{};
+  if (gw < nd) N = d[gw];
   for (int64_t b = gw; b < nd; b += nw) {
-    const P1Desc D = d[b];
-    const int q = (XA - (int)(D.seg0 % XA)) % XA;
-    const TX* xb = xs + q * xs_stride + D.seg0 + q;
-    const int nvec = (int)(D.stride / VW);
+    const P1Desc D = N;
+    if (b + nw < nd) N = d[b + nw];
+    const TX* xb = xs + D.seg0;
+    if constexpr (!std::is_same<T, double>::value) {
+      const int q = (XA - (int)(D.seg0 % XA)) % XA;
+      xb += q * xs_stride + q;
+    }
     const T* F = pool + D.off;
-    for (int r = 0; r < D.k; r += NR) {
-      // NR columns r .. r + NR - 1 (those past the rank point at column r and are
-      // neither read, beyond the first two, nor written)
-      const T* fc[NR];
-#pragma unroll
-      for (int j = 0; j < NR; ++j) fc[j] = F + (int64_t)(r + j < D.k ? r + j : r) * D.stride;
-      double sc[NR];
-#pragma unroll
-      for (int j = 0; j < NR; ++j) sc[j] = 0.0;
-      for (int v0 = lane; v0 < nvec; v0 += 32 * U) {
-        typename Tr::R a[NR][U];
-        typename Tr::XV xv[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int v = v0 + 32 * u;
-          if (v < nvec) {
-#pragma unroll
-            for (int j = 0; j < NR; ++j)
-              if (j < 2 || r + j < D.k) a[j][u] = Tr::ld(fc[j] + (int64_t)v * VW);   // no reads past the rank
-            xv[u] = Tr::ldx(xb + (int64_t)v * VW);
-          }
-        }
-        if constexpr (std::is_same<T, double>::value) {
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            if (v0 + 32 * u < nvec) {
-#pragma unroll
-              for (int j = 0; j < NR; ++j) sc[j] = Tr::dot(a[j][u], xv[u], sc[j]);
-            }
-          }
-        } else {
-          // FP32 products and partial sums over the U vectors in flight,
-          // folded into the FP64 sums once per group
-          float fp[NR];
-#pragma unroll
-          for (int j = 0; j < NR; ++j) fp[j] = 0.f;
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            if (v0 + 32 * u < nvec) {
-#pragma unroll
-              for (int j = 0; j < NR; ++j) fp[j] = Tr::dotf(a[j][u], xv[u], fp[j]);
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < NR; ++j) sc[j] += (double)fp[j];
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < NR; ++j) sc[j] = warp_sum(sc[j]);
-      if (lane == 0) {
-#pragma unroll
-        for (int j = 0; j < NR; ++j)
-          if (r + j < D.k) z[D.zoff + r + j] = sc[j];
-      }
+    double* zp = z + D.zoff;
+    for (int left = D.k; left > 0;) {
+      const int ng = (left + 3) / 4, nr = (left + ng - 1) / ng;
+      if (nr == 4) p1_columns<T, 4>(F, D.stride, D.len, xb, zp, lane);
+      else if (nr == 3) p1_columns<T, 3>(F, D.stride, D.len, xb, zp, lane);
+      else if (nr == 2) p1_columns<T, 2>(F, D.stride, D.len, xb, zp, lane);
+      else p1_columns<T, 1>(F, D.stride, D.len, xb, zp, lane);
+      F += (int64_t)nr * D.stride;
+      zp += nr;
+      left -= nr;
     }
   }
 }
@@ -1086,31 +1101,43 @@ __global__ void __launch_bounds__(P2Shape8<SPLIT>::WARPS * 32) mv_phase2_bf16_ke
     if (base + q < (int)W.nrows) y[W.row0 + base + q] += acc[q];
 }
 
+// resident CTAs of phase 1 on the device, asked once per device
+template <typename T>
+static int64_t p1_wave(int device) {
+  static std::atomic<int> known[64];
+  std::atomic<int>* slot = device >= 0 && device < 64 ? &known[device] : nullptr;
+  if (slot && slot->load(std::memory_order_relaxed) > 0) return slot->load(std::memory_order_relaxed);
+  int nsm = 148, per_sm = 0;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mv_phase1_kernel<T>, 256, 0) != cudaSuccess || per_sm < 1)
+    per_sm = 1;
+  if (slot) slot->store(nsm * per_sm, std::memory_order_relaxed);
+  return (int64_t)nsm * per_sm;
+}
+
 template <typename T>
 static int matvec_t(hm_handle* h, const double* d_x, double* d_y, int trans, cudaStream_t st, cudaEvent_t* ev) {
   using TX = typename MvT<T>::X;
   constexpr int XA = 16 / (int)sizeof(TX);
   MvPlan& P = trans ? h->bwd : h->fwd;
   const int64_t stride = pad_to(h->n + 64, 64);
-  HM_TRY(ensure_xs(h, sizeof(TX) * stride * XA));
-  TX* xs = (TX*)h->d_xs;
+  const TX* xs = nullptr;
   if (ev) HM_CUDA_TRY(cudaEventRecord(ev[0], st));
-  {
+  if constexpr (std::is_same<T, double>::value) {
+    xs = d_x;
+  } else {
+    HM_TRY(ensure_xs(h, sizeof(TX) * stride * XA));
     int64_t tot = stride * XA;
     unsigned g = (unsigned)std::min<int64_t>((tot + 255) / 256, 148 * 16);
-    xcopy_kernel<TX><<<g, 256, 0, st>>>(d_x, h->n, xs, stride, XA);
+    xcopy_kernel<TX><<<g, 256, 0, st>>>(d_x, h->n, (TX*)h->d_xs, stride, XA);
+    xs = (const TX*)h->d_xs;
   }
   if (ev) HM_CUDA_TRY(cudaEventRecord(ev[1], st));
   if (P.np1 > 0) {
-    int nsm = 148;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
     // one wave of resident CTAs: the warps stride over equal-sized leaves and
     // finish together (a grid of several partial waves leaves a tail)
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mv_phase1_kernel<T>, 256, 0) != cudaSuccess ||
-        per_sm < 1)
-      per_sm = 1;
-    int64_t blocks = std::min<int64_t>((P.np1 + 7) / 8, (int64_t)nsm * per_sm * std::max(1, h->tune.p1_waves));
+    const int64_t wave = p1_wave<T>(h->device);
+    int64_t blocks = std::min<int64_t>((P.np1 + 7) / 8, wave * std::max(1, h->tune.p1_waves));
     mv_phase1_kernel<T><<<(unsigned)blocks, 256, 0, st>>>(P.d_p1, P.np1, (const T*)h->d_rk, xs, stride, h->d_z);
   }
   if (ev) HM_CUDA_TRY(cudaEventRecord(ev[2], st));
