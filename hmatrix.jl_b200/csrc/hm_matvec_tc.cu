@@ -83,6 +83,7 @@ struct TcPlan {
   int64_t nz2 = 0;
   TcItem2* d_item2 = nullptr;
   int64_t nitem2 = 0;
+  unsigned qmask = 0;      // the shifted copies of X that some segment uses
   bool checked = false;    // `usable` is up to date with the factor pool
   bool usable = false;     // every factor entry is at most 2^100 in magnitude (no NaN)
 };
@@ -325,29 +326,40 @@ __device__ __forceinline__ void tc_mma_role(TcBars* b, uint32_t sbase, uint32_t 
 // KE shifted copies let every segment start on a 16-byte K block; a block of
 // 2*NC rows x 16 bytes is exactly the canonical K-major core-matrix layout.
 // ---------------------------------------------------------------------------
+// A CTA stages its rows of X (read along the columns) in shared memory, split
+// once, and writes every shifted copy that some segment uses (qmask) in
+// 16-byte units.  Bound: the bytes written.  Element by element, with the
+// index arithmetic of each, 64 BF16 columns at n = 2^18 took 1005 us.
 template <typename T, int NC>
-__global__ void tc_xt_kernel(const double* __restrict__ X, int64_t n, int64_t ldx, int ncols, int cb,
-                             typename TcT<T>::Bits* __restrict__ xt, int64_t nkb) {
-  constexpr int KE = TcT<T>::KE;
-  const int64_t blk = 2 * NC * KE;
-  const int64_t per_copy = nkb * blk;
-  const int64_t tot = (int64_t)KE * per_copy;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t q = e / per_copy, r = e - q * per_copy;
-    const int64_t kb = r / blk;
-    int rem = (int)(r - kb * blk);
-    const int part = rem / (NC * KE);
-    rem -= part * NC * KE;
-    const int nn = rem / KE, el = rem - nn * KE;
-    const int64_t t = kb * KE + el - q;
-    const int col = cb * NC + nn;
-    float v = 0.f;
-    if (t >= 0 && t < n && col < ncols) {
-      const float x = (float)X[t + (int64_t)col * ldx];
-      const float h = TcT<T>::hi(x);
-      v = part == 0 ? h : TcT<T>::hi(x - h);
+__global__ void __launch_bounds__(256) tc_xt_kernel(const double* __restrict__ X, int64_t n, int64_t ldx, int ncols,
+                                                    int cb, unsigned qmask, typename TcT<T>::Bits* __restrict__ xt,
+                                                    int64_t nkb) {
+  using Tr = TcT<T>;
+  constexpr int KE = Tr::KE, TK = 64 / KE;               // K blocks of a CTA: 64 rows
+  constexpr int ROWS = 64 + KE, LD = ROWS + 1;
+  __shared__ uint32_t sh[2][NC][LD];                     // hi and lo bits of X[t0 - KE + i][column]
+  const int64_t kb0 = (int64_t)blockIdx.x * TK, t0 = kb0 * KE - KE;
+  for (int e = threadIdx.x; e < NC * ROWS; e += 256) {
+    const int nn = e / ROWS, i = e % ROWS, col = cb * NC + nn;
+    const int64_t t = t0 + i;
+    const float x = (t >= 0 && t < n && col < ncols) ? (float)X[t + (int64_t)col * ldx] : 0.f;
+    const float h = Tr::hi(x);
+    sh[0][nn][i] = (uint32_t)Tr::bits(h);
+    sh[1][nn][i] = (uint32_t)Tr::bits(Tr::hi(x - h));
+  }
+  __syncthreads();
+  for (int q = 0; q < KE; ++q) {
+    if (!(qmask >> q & 1u)) continue;
+    uint4* out = reinterpret_cast<uint4*>(xt + ((int64_t)q * nkb + kb0) * (2 * NC * KE));
+    for (int u = threadIdx.x; u < TK * 2 * NC; u += 256) {
+      const int kb = u / (2 * NC), part = u / NC % 2, nn = u % NC;
+      if (kb0 + kb >= nkb) break;
+      const uint32_t* v = &sh[part][nn][kb * KE - q + KE];
+      uint4 w;
+      if constexpr (KE == 4) w = make_uint4(v[0], v[1], v[2], v[3]);
+      else w = make_uint4(v[0] | v[1] << 16, v[2] | v[3] << 16, v[4] | v[5] << 16, v[6] | v[7] << 16);
+      out[u] = w;
     }
-    xt[e] = TcT<T>::bits(v);
   }
 }
 
@@ -1008,6 +1020,7 @@ static int upload_vec(V** d, const std::vector<V>& v) {
 
 static int build_tc_plan(hm_handle* h, int trans, TcPlan** out) {
   const int eb = elem_bytes(h->storage);
+  const uint32_t KE = 16 / (uint32_t)eb;               // elements of a 16-byte K block (TcT::KE)
   struct Lf { int64_t li; int64_t zoff; };
   // low-rank leaves in pool order with their z offsets
   std::vector<int64_t> order(h->leaves.size());
@@ -1115,6 +1128,7 @@ static int build_tc_plan(hm_handle* h, int trans, TcPlan** out) {
       I.seg0 = (uint32_t)sg.first;
       I.len = (uint32_t)sg.second;
       if (I.len > 0) it1.push_back(I);
+      P->qmask |= 1u << (KE - I.seg0 % KE) % KE;
     }
     i = j;
   }
@@ -1207,9 +1221,7 @@ static int launch_tc(hm_handle* h, TcPlan& P, const double* d_x, double* d_y, in
   }
   const int ncb = (int)((ncols + NC - 1) / NC);
   for (int cb = 0; cb < ncb; ++cb) {
-    const int64_t tot = KE * xt_copy;
-    tc_xt_kernel<T, NC><<<(unsigned)std::min<int64_t>((tot + 255) / 256, (int64_t)nsm * 32), 256, 0, st>>>(
-        d_x, n, n, (int)ncols, cb, xt, nkb);
+    tc_xt_kernel<T, NC><<<(unsigned)((nkb * KE + 63) / 64), 256, 0, st>>>(d_x, n, n, (int)ncols, cb, P.qmask, xt, nkb);
     if (P.nitem1 > 0) {
       P1Args<T, NC> a1{P.d_item1, P.nitem1, P.d_col1, P.d_zpl, (const T*)h->d_rk, xt, xt_copy, zt, h->d_tc_err};
       tc_phase1_kernel<T, NC><<<(unsigned)std::min<int64_t>(nsm, P.nitem1), TC_THREADS, C::BYTES, st>>>(a1);
