@@ -174,15 +174,15 @@ struct Slab {
 
 constexpr int MV_WROWS = 1024;         // rows per phase-2 window (8 warps x 32 lanes x 4 rows)
 
+struct MbCol;              // hm_matvec_multi.cu
+struct MbTile;
+
 struct MvPlan {
   P1Desc* d_p1 = nullptr;
   int64_t np1 = 0;
-  P1Desc* d_p1s = nullptr;         // the same descriptors ordered by input segment (multi-RHS phase 1; built on first use)
-  uint32_t* d_g1s = nullptr;       // groups of d_p1s sharing a segment (ng1 + 1 starts)
-  int64_t ng1 = 0;
-  uint32_t* d_t1s = nullptr;       // segment tasks of d_p1s (nt1 + 1 starts)
-  int64_t nt1 = 0;
-  uint32_t maxlen1 = 0;            // longest segment
+  MbCol* d_mbcol = nullptr;        // multi-RHS phase 1 (built on first use): factor columns by input segment,
+  MbTile* d_mbtile = nullptr;      // tiles of 32 of them (in the allocation of d_mbcol)
+  int64_t nmbtile = 0;
   P2Desc* d_p2 = nullptr;
   int64_t np2 = 0;
   MvWin* d_win = nullptr;
@@ -312,6 +312,8 @@ void lu_describe(const hm_handle* h, int64_t* tiles, int64_t* cap);
 // matvec (hm_matvec.cu)
 int matvec_device(hm_handle* h, const double* d_x, double* d_y, int trans, cudaStream_t st,
                   cudaEvent_t* ev = nullptr);
+// Builds a direction's slab lists on first use; *usable false: they cannot be had.
+int ensure_slabs(hm_handle* h, int trans, bool* usable);
 // Y = H X (trans 0) or H' X (trans 1) for an n x ncols column-major block,
 // factors streamed once per column block (hm_matvec_multi.cu)
 int matvec_multi_device(hm_handle* h, const double* d_x, double* d_y, int64_t ncols, int trans, cudaStream_t st,

@@ -577,9 +577,7 @@ __global__ void __launch_bounds__(SL_WARPS * 32, 2) mv_slab_kernel(const Slab* _
 // ---------------------------------------------------------------------------
 void free_mv_plan(MvPlan& p) {
   if (p.d_p1) cudaFree(p.d_p1);
-  if (p.d_p1s) cudaFree(p.d_p1s);
-  if (p.d_g1s) cudaFree(p.d_g1s);
-  if (p.d_t1s) cudaFree(p.d_t1s);
+  if (p.d_mbcol) cudaFree(p.d_mbcol);
   if (p.d_p2) cudaFree(p.d_p2);
   if (p.d_win) cudaFree(p.d_win);
   if (p.d_p2d) cudaFree(p.d_p2d);
@@ -656,12 +654,14 @@ static void slab_cuts(const hm_handle* h, int64_t most, std::vector<Slab>& out) 
 // The slab size: of 32, 64, .. 224 rows at most, the one whose slabs leave the
 // fewest lanes idle (the larger one on a tie: fewer entries per factor byte),
 // among those that give every SM four slabs; 32 rows for matrices too small
-// for that.
+// for that.  No slab above MaxBlock rows: a row shard is cut at clusters of at
+// most that size, and its slabs are then the whole matrix's.
 static void choose_slabs(const hm_handle* h, std::vector<Slab>& best) {
   slab_cuts(h, 32, best);
   double eff = 0.0;
   std::vector<Slab> v;
   for (int r = 1; r <= SL_RMAX; ++r) {
+    if (r > 1 && h->prm.max_block > 0 && 32 * r > h->prm.max_block) break;
     slab_cuts(h, 32 * r, v);
     if (v.size() < 4 * 148) break;
     int64_t lanes = 0;
@@ -792,7 +792,8 @@ static int build_slab_plan(hm_handle* h, int trans, MvPlan& P) {
 // Builds the slab lists on first use; false: this plan cannot have them (no
 // memory left for them, or an entry field too narrow) and the caller takes
 // the window lists, which every plan has.
-static int ensure_slabs(hm_handle* h, int trans, MvPlan& P, bool* usable) {
+int ensure_slabs(hm_handle* h, int trans, bool* usable) {
+  MvPlan& P = trans ? h->bwd : h->fwd;
   if (!P.d_slab && !P.no_slab) {
     const int s = build_slab_plan(h, trans, P);
     if (s == HM_ERR_OOM || s == HM_ERR_UNSUPPORTED) P.no_slab = true;
@@ -1144,7 +1145,7 @@ static int matvec_t(hm_handle* h, const double* d_x, double* d_y, int trans, cud
   // dense leaves are FP64 with FP64 factors and FP32 otherwise
   using TD = typename std::conditional<std::is_same<T, double>::value, double, float>::type;
   bool slabs = false;
-  if (h->tune.p2_split == 1) HM_TRY(ensure_slabs(h, trans, P, &slabs));
+  if (h->tune.p2_split == 1) HM_TRY(ensure_slabs(h, trans, &slabs));
   if (slabs) {
     mv_slab_kernel<T, TD><<<(unsigned)P.nslab, SL_WARPS * 32, 0, st>>>(
         P.d_slab, P.d_ent, (const T*)h->d_rk, (const TD*)h->d_dense, h->d_z, d_x, d_y);

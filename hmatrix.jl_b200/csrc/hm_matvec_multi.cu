@@ -1,22 +1,25 @@
-// Multi-RHS H-matvec (K5) on the CUDA cores: Y = H X and Y = H' X for an
+// Multi-RHS H-matvec (K5) with FP64 arithmetic: Y = H X and Y = H' X for an
 // n x c block of right-hand sides, the device form of *(Hmat, Matrix)
 // (src/harithm.jl:323-329), which the reference evaluates one column at a
-// time.  Every factor is streamed from HBM once per block of CB columns
-// instead of once per column, in FP64 arithmetic.  This is the path of FP64
-// factors (tcgen05 has no FP64 kind) and of the dense leaves of FP32/BF16
-// handles, whose low-rank part runs on the tensor cores (hm_matvec_tc.cu).
+// time.  Every factor is streamed from HBM once per block of at most 32
+// columns.  This is the path of FP64 factors (tcgen05 has no FP64 kind); the
+// low-rank part of FP32/BF16 handles runs on the tensor cores in FP32
+// (hm_matvec_tc.cu), their dense leaves here (mvm_dense_kernel).
 //
-// Layout: the input is first transposed into XR, n+2 rows of LD = c rounded up
-// to CB doubles (row i holds x[i, 0..c), zero padded), so that a leaf row's CB
-// values are contiguous 16-byte loads.  Phase 1 writes ZR, one row of LD
-// values per low-rank term; phase 2 writes Y column-major directly.
+// Both phases are chains of FP64 tensor-core MMAs (mma.sync m8n8k4, the one
+// FP64 matrix instruction) with the factors read straight from global memory
+// in the operand layout: lane (g, q) = (lane / 4, lane % 4) holds A(g, q),
+// B(q, g) and C(g, 2 q), C(g, 2 q + 1).  An 8 x 4 block of a column-major
+// factor is four runs of 64 bytes (phase 2), its transpose eight runs of 64
+// bytes for two MMAs (phase 1), so no staging in shared memory is needed.
+// Bound: HBM up to 16 columns (an MMA's 256 FMAs take 4 cycles of an SM: 32
+// bytes of factor a cycle against the 23 that HBM delivers), FP64 beyond.
 //
-// Phase 1: one warp per low-rank leaf and column block; a lane owns pairs of
-//          segment rows, accumulates two ranks x CB columns, and the warp
-//          reduces the 2*CB sums with a butterfly reduce-scatter.
-// Phase 2: one CTA per (window half of 512 rows, column block); a thread owns
-//          2 consecutive rows x CB columns; the (leaf, column) entries of the
-//          window are expanded in shared memory with their CB z values.
+// Phase 1: Z = F1' X_seg, a warp per tile of 32 factor columns that share an
+//          input segment (K = segment rows, N = right-hand sides).
+// Phase 2: Y = F2 Z + C X, a CTA per row slab (the slabs of the single-column
+//          phase 2): its warps are groups of 32 rows times a split of the
+//          slab's entries, whose partial sums meet in shared memory.
 #include "hm_internal.h"
 #include "hm_lowrank.cuh"
 
@@ -26,35 +29,341 @@
 
 namespace hm {
 
+// One factor column of F1 and a tile of up to 32 of them (one input segment)
+struct MbCol {
+  uint64_t off;            // pool element offset of the column
+  uint64_t z;              // its row of Z
+};
+struct MbTile {
+  uint32_t col0, ncol, seg0, len;
+};
+
 namespace {
 
-__device__ __forceinline__ float mbf_lo(uint32_t w) { return __uint_as_float(w << 16); }
-__device__ __forceinline__ float mbf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
 
 // two consecutive elements of a factor column as FP64 (the pair starts on an
 // even element; columns are padded to 4 elements and 16 bytes)
-template <typename T> struct Pair;
-template <> struct Pair<double> {
-  __device__ static double2 ld(const double* p) { return __ldcs(reinterpret_cast<const double2*>(p)); }
-  __device__ static double one(const double* p) { return __ldcs(p); }
-};
-template <> struct Pair<float> {
-  __device__ static double2 ld(const float* p) {
-    const float2 v = __ldcs(reinterpret_cast<const float2*>(p));
-    return make_double2(v.x, v.y);
+__device__ __forceinline__ double2 ld_pair(const double* p) { return __ldcs(reinterpret_cast<const double2*>(p)); }
+__device__ __forceinline__ double2 ld_pair(const float* p) {
+  const float2 v = __ldcs(reinterpret_cast<const float2*>(p));
+  return make_double2(v.x, v.y);
+}
+__device__ __forceinline__ double2 ld_pair(const __nv_bfloat16* p) {
+  const uint32_t w = __ldcs(reinterpret_cast<const unsigned int*>(p));
+  return make_double2((double)__uint_as_float(w << 16), (double)__uint_as_float(w & 0xffff0000u));
+}
+__device__ __forceinline__ double ld_one(const double* p) { return __ldcs(p); }
+__device__ __forceinline__ double ld_one(const float* p) { return (double)__ldcs(p); }
+__device__ __forceinline__ double ld_one(const __nv_bfloat16* p) {
+  return (double)__uint_as_float((uint32_t)__ldcs(reinterpret_cast<const unsigned short*>(p)) << 16);
+}
+
+constexpr int MB_MT = 4;                    // M tiles (of 8) a warp owns: 32 factor columns, 32 output rows
+constexpr int MB_WARPS = 8;
+
+// ---------------------------------------------------------------------------
+// phase 1
+// ---------------------------------------------------------------------------
+template <typename T, int NT>
+__global__ void __launch_bounds__(MB_WARPS * 32, NT <= 2 ? 2 : 1)
+    mb_phase1_kernel(const MbTile* __restrict__ tiles, int64_t ntile, const MbCol* __restrict__ cols,
+                     const T* __restrict__ pool, const double* __restrict__ X, int64_t ldx, int ncols, int ncb,
+                     double* __restrict__ Z, int ldz) {
+  constexpr int PD = sizeof(T) == 2 ? 8 : 4;              // columns are padded to PD elements (col_pad_elems)
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const int64_t gw = (int64_t)blockIdx.x * MB_WARPS + (threadIdx.x >> 5);
+  const int64_t nw = (int64_t)gridDim.x * MB_WARPS;
+  for (int64_t w = gw; w < ntile * ncb; w += nw) {
+    const MbTile tl = tiles[w / ncb];
+    const int cb = (int)(w % ncb) * 8 * NT;
+    const T* F[MB_MT];
+#pragma unroll
+    for (int i = 0; i < MB_MT; ++i)
+      F[i] = pool + cols[tl.col0 + min((uint32_t)(8 * i + g), tl.ncol - 1)].off;
+    const int mt = (int)((tl.ncol + 7) / 8);
+    const int len = (int)tl.len, plen = (len + PD - 1) / PD * PD;
+    const double* xb[NT];                                // X's columns of this lane (past the last: the last, into unused columns of Z)
+#pragma unroll
+    for (int j = 0; j < NT; ++j) xb[j] = X + tl.seg0 + (int64_t)min(cb + 8 * j + g, ncols - 1) * ldx;
+    // pairs of X in one load where every column's segment is 16-byte aligned
+    const bool pair = !(len & 1) && !((reinterpret_cast<uintptr_t>(X) >> 3 | tl.seg0 | (uint64_t)ldx) & 1);
+    double acc[MB_MT][NT][2];
+#pragma unroll
+    for (int i = 0; i < MB_MT; ++i)
+#pragma unroll
+      for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    // 16 rows a step (K index 8 h + 2 q + s -> MMA s of half h), the operands
+    // of the next D steps in flight
+    constexpr int D = 1;
+    double2 a[D][MB_MT][2], x[D][NT][2];
+    auto load = [&](int r0, double2 (&A)[MB_MT][2], double2 (&B)[NT][2]) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        // unconditional loads (a branch would put each beside its use): past
+        // the end the last rows are read again and zeros multiplied
+        const int r = r0 + 8 * h + 2 * q;
+#pragma unroll
+        for (int i = 0; i < MB_MT; ++i) {
+          A[i][h] = ld_pair(F[i] + min(r, plen - 2));
+          if (r >= plen) A[i][h] = make_double2(0.0, 0.0);
+        }
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          if (pair) {
+            B[j][h] = __ldg(reinterpret_cast<const double2*>(xb[j] + min(r, len - 2)));
+          } else {
+            B[j][h].x = __ldg(xb[j] + min(r, len - 1));
+            B[j][h].y = __ldg(xb[j] + min(r + 1, len - 1));
+          }
+          if (r >= len) B[j][h].x = 0.0;
+          if (r + 1 >= len) B[j][h].y = 0.0;
+        }
+      }
+    };
+#pragma unroll
+    for (int d = 0; d < D; ++d) load(16 * d, a[d], x[d]);
+    for (int r0 = 0; r0 < len; r0 += 16 * D) {
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        double2 an[MB_MT][2], xn[NT][2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+          for (int i = 0; i < MB_MT; ++i) an[i][h] = a[d][i][h];
+#pragma unroll
+          for (int j = 0; j < NT; ++j) xn[j][h] = x[d][j][h];
+        }
+        load(r0 + 16 * (d + D), a[d], x[d]);             // past the end: zeros
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int i = 0; i < MB_MT; ++i)
+            if (i < mt) {
+#pragma unroll
+              for (int j = 0; j < NT; ++j) {
+                dmma(acc[i][j], an[i][h].x, xn[j][h].x);
+                dmma(acc[i][j], an[i][h].y, xn[j][h].y);
+              }
+            }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < MB_MT; ++i)
+      if ((uint32_t)(8 * i + g) < tl.ncol) {
+        double* zp = Z + cols[tl.col0 + 8 * i + g].z * ldz + cb + 2 * q;
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+          *reinterpret_cast<double2*>(zp + 8 * j) = make_double2(acc[i][j][0], acc[i][j][1]);
+      }
   }
-  __device__ static double one(const float* p) { return (double)__ldcs(p); }
-};
-template <> struct Pair<__nv_bfloat16> {
-  __device__ static double2 ld(const __nv_bfloat16* p) {
-    const uint32_t w = __ldcs(reinterpret_cast<const unsigned int*>(p));
-    return make_double2(mbf_lo(w), mbf_hi(w));
+}
+
+// ---------------------------------------------------------------------------
+// phase 2
+// ---------------------------------------------------------------------------
+// acc += the entries [e0, e1) of one kind: A(row, entry) = the entry's value in
+// the row, B = row zi of V (V(zi, col) at V[zi vr + col vc], columns < vcols).
+// 32 entries (8 steps of K = 4) make a batch; a step's operand registers are
+// refilled from the next batch as soon as the step is consumed.  Batches whose
+// entries all cover this warp's rows (most: leaves end where slabs end) take
+// loads at constant offsets from one pointer; the others clamp and mask.
+template <typename E, int NT>
+__device__ __forceinline__ void mb_entries(const SlabEnt* __restrict__ ents, uint32_t e0, uint32_t e1,
+                                           const E* __restrict__ pool, const double* __restrict__ V, int64_t vr,
+                                           int64_t vc, int vcols, int cb, int row0, int mt, int lane,
+                                           double (&acc)[MB_MT][NT][2]) {
+  if (e0 >= e1) return;
+  const int g = lane >> 2, q = lane & 3;
+  constexpr int D = 8;
+  double a[D][MB_MT], b[D][NT];
+  uint64_t mask = 0;                                     // step d, bits 5 d ..: A values 0 .. 3 and the B row to be zeroed
+  int64_t vo[NT];                                        // columns past the last: the last, into unused columns
+#pragma unroll
+  for (int j = 0; j < NT; ++j) vo[j] = min(cb + 8 * j + g, vcols - 1) * vc;
+  const int nb = (int)((e1 - e0 + 31) / 32);
+  const SlabEnt none{0, 0, 255u | 255u << 8};            // row 255: in no slab
+  auto fetch = [&](int t) {
+    const uint32_t e = e0 + 32 * t + lane;
+    return e < e1 ? ents[e] : none;
+  };
+  // the operands of step d of the batch whose entries the lanes hold in N
+  auto refill = [&](const SlabEnt& N, bool full, int d) {
+    const int src = 4 * d + q;
+    const uint64_t off = __shfl_sync(0xffffffffu, (unsigned long long)(N.off & SLAB_OFF_MASK), src);
+    const uint32_t meta = __shfl_sync(0xffffffffu, N.meta, src), zi = __shfl_sync(0xffffffffu, N.zi, src);
+    const uint32_t lo = meta & 255u, span = (meta >> 8 & 255u) - lo;
+    const E* p = pool + off;
+    const double* v = V + zi * vr;
+#pragma unroll
+    for (int j = 0; j < NT; ++j) b[d][j] = __ldg(v + vo[j]);
+    if (full) {
+      p += row0 + g - (int)lo;
+#pragma unroll
+      for (int i = 0; i < MB_MT; ++i) a[d][i] = ld_one(p + 8 * i);
+    } else {
+      // a row not covered reads the entry's last one (past the entries the
+      // pool's first); its zero replaces the value when the step is consumed
+      // (here it would wait for the load)
+      uint32_t m = lo == 255u ? 16u : 0u;
+#pragma unroll
+      for (int i = 0; i < MB_MT; ++i) {
+        const uint32_t r = (uint32_t)(row0 + 8 * i + g) - lo;
+        if (i < mt) a[d][i] = ld_one(p + min(r, span));
+        m |= (r > span ? 1u : 0u) << i;
+      }
+      mask = (mask & ~((uint64_t)31 << 5 * d)) | (uint64_t)m << 5 * d;
+    }
+  };
+  auto covers = [&](const SlabEnt& N) {
+    return __all_sync(0xffffffffu, (int)(N.meta & 255u) <= row0 &&
+                                       (int)(N.meta >> 8 & 255u) >= row0 + 8 * MB_MT - 1 && (N.meta & 255u) != 255u) != 0;
+  };
+  SlabEnt N = fetch(0);
+  bool was_full = covers(N);                             // of the batch being consumed
+#pragma unroll
+  for (int d = 0; d < D; ++d) refill(N, was_full, d);
+  N = fetch(1);
+  for (int t = 0; t < nb; ++t) {
+    const SlabEnt N2 = fetch(t + 2);
+    const bool full = covers(N), more = t + 1 < nb;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      double an[MB_MT], bn[NT];
+#pragma unroll
+      for (int i = 0; i < MB_MT; ++i) an[i] = a[d][i];
+#pragma unroll
+      for (int j = 0; j < NT; ++j) bn[j] = b[d][j];
+      const uint32_t m = (uint32_t)(mask >> 5 * d) & 31u;
+      if (more) refill(N, full, d);
+      if (!was_full) {
+#pragma unroll
+        for (int i = 0; i < MB_MT; ++i)
+          if (m >> i & 1u) an[i] = 0.0;
+        if (m & 16u) {
+#pragma unroll
+          for (int j = 0; j < NT; ++j) bn[j] = 0.0;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < MB_MT; ++i)
+        if (i < mt) {
+#pragma unroll
+          for (int j = 0; j < NT; ++j) dmma(acc[i][j], an[i], bn[j]);
+        }
+    }
+    N = N2;
+    was_full = full;
   }
-  __device__ static double one(const __nv_bfloat16* p) {
-    const unsigned short u = __ldcs(reinterpret_cast<const unsigned short*>(p));
-    return (double)__uint_as_float((uint32_t)u << 16);
+}
+
+template <typename T, typename TD, int NT>
+__global__ void __launch_bounds__(MB_WARPS * 32, 1)
+    mb_phase2_kernel(const Slab* __restrict__ slabs, const SlabEnt* __restrict__ ents, const T* __restrict__ rk,
+                     const TD* __restrict__ dn, const double* __restrict__ Z, int ldz, const double* __restrict__ X,
+                     int64_t ldx, int ncols, int ncb, double* __restrict__ Y, int64_t ldy) {
+  __shared__ double part[MB_WARPS / 2][32][8 * NT + 1];  // the splits' sums, half the warps' at a time
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const Slab S = slabs[blockIdx.x / ncb];
+  const int cb = (int)(blockIdx.x % ncb) * 8 * NT;
+  // row groups of at most 32 rows (whole M tiles), ks splits of the entries
+  const int ngrp = ((int)S.nrows + 31) / 32;             // at most 7
+  const int ks = ngrp > 4 ? 1 : ngrp > 2 ? 2 : ngrp == 2 ? 4 : 8;
+  const int grp = warp / ks, sp = warp % ks;
+  const int grows = (((int)S.nrows + ngrp - 1) / ngrp + 7) / 8 * 8;
+  const int row0 = grp * grows, mt = grp < ngrp ? min(grows, max(0, (int)S.nrows - row0) + 7) / 8 : 0;
+  double acc[MB_MT][NT][2];
+#pragma unroll
+  for (int i = 0; i < MB_MT; ++i)
+#pragma unroll
+    for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  if (mt > 0) {
+    auto share = [&](uint32_t b, uint32_t e, uint32_t& s0, uint32_t& s1) {
+      const uint32_t n = e - b, per = (n + 4 * ks - 1) / (4 * ks) * 4;
+      s0 = b + min(n, sp * per);
+      s1 = b + min(n, (sp + 1) * per);
+    };
+    uint32_t s0, s1;
+    share(S.begin, S.dense, s0, s1);
+    mb_entries<T, NT>(ents, s0, s1, rk, Z, ldz, 1, ldz, cb, row0, mt, lane, acc);
+    share(S.dense, S.mid, s0, s1);
+    mb_entries<TD, NT>(ents, s0, s1, dn, X, 1, ldx, ncols, cb, row0, mt, lane, acc);
+    // dense leaves read along their rows (H'x): 32 input indices an entry
+    for (uint32_t e = S.mid + sp; e < S.end; e += ks) {
+      const SlabEnt E = ents[e];
+      const uint32_t lo = E.meta & 255u, span = (E.meta >> 8 & 255u) - lo;
+      const int cnt = (int)(E.meta >> 24);
+      const int64_t ld = (int64_t)(E.off >> 40);
+      const TD* p = dn + (E.off & SLAB_OFF_MASK);
+      double a[8][MB_MT], b[8][NT];
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        const int k = 4 * s + q;
+#pragma unroll
+        for (int i = 0; i < MB_MT; ++i) {
+          const uint32_t r = (uint32_t)(row0 + 8 * i + g) - lo;
+          a[s][i] = ld_one(p + min(r, span) * ld + min(k, cnt - 1));
+          if (k >= cnt || r > span) a[s][i] = 0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          b[s][j] = __ldg(X + E.zi + min(k, cnt - 1) + min(cb + 8 * j + g, ncols - 1) * ldx);
+          if (k >= cnt) b[s][j] = 0.0;
+        }
+      }
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+#pragma unroll
+        for (int i = 0; i < MB_MT; ++i)
+          if (i < mt) {
+#pragma unroll
+            for (int j = 0; j < NT; ++j) dmma(acc[i][j], a[s][i], b[s][j]);
+          }
+    }
   }
-};
+  // the splits of a row group, summed pairwise: upper half into the lower half
+  for (int half = ks / 2; half >= 1; half /= 2) {
+    __syncthreads();
+    const int slot = grp * half + (sp >= half ? sp - half : sp);
+    if (mt > 0 && sp >= half && sp < 2 * half) {
+#pragma unroll
+      for (int i = 0; i < MB_MT; ++i)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          part[slot][8 * i + g][8 * j + 2 * q] = acc[i][j][0];
+          part[slot][8 * i + g][8 * j + 2 * q + 1] = acc[i][j][1];
+        }
+    }
+    __syncthreads();
+    if (mt > 0 && sp < half) {
+#pragma unroll
+      for (int i = 0; i < MB_MT; ++i)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          acc[i][j][0] += part[slot][8 * i + g][8 * j + 2 * q];
+          acc[i][j][1] += part[slot][8 * i + g][8 * j + 2 * q + 1];
+        }
+    }
+  }
+  if (mt == 0 || sp != 0) return;
+#pragma unroll
+  for (int i = 0; i < MB_MT; ++i) {
+    const int r = row0 + 8 * i + g;
+    if (i < mt && r < (int)S.nrows) {
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int col = cb + 8 * j + 2 * q + c;
+          if (col < ncols) Y[(int64_t)(S.row0 + r) + col * ldy] = acc[i][j][c];
+        }
+    }
+  }
+}
 
 // XR[i, j] = X[i + j * ldx] (j < ncols, i < n), zero elsewhere, for n + 2 rows
 __global__ void mvm_xr_kernel(const double* __restrict__ X, int64_t n, int64_t ldx, int ncols,
@@ -64,322 +373,6 @@ __global__ void mvm_xr_kernel(const double* __restrict__ X, int64_t n, int64_t l
     const int64_t i = e / ld;
     const int j = (int)(e % ld);
     xr[e] = (i < n && j < ncols) ? X[i + (int64_t)j * ldx] : 0.0;
-  }
-}
-
-// Phase 1 works on groups of up to G1 leaves that share an input segment
-// (descriptors ordered by segment): one x load then feeds G1 leaves x 2 ranks.
-// Lane = (row sub-index rs, column pair cp): a 32-row chunk of the segment is
-// read as RS x IT rows by CP column pairs, so each warp-wide x load is 512
-// contiguous bytes; the factor values of the chunk are loaded once (lane l
-// holds row l) and handed to the lanes that need them by shuffles.
-constexpr int G1 = 4;
-
-template <typename T, int CB>
-__global__ void __launch_bounds__(256) mvm_phase1_kernel(const P1Desc* __restrict__ d, const uint32_t* __restrict__ grp,
-                                                         int64_t ngrp, const T* __restrict__ pool,
-                                                         const double* __restrict__ xr, int ld, int ncb,
-                                                         double* __restrict__ zr) {
-  constexpr int CP = CB / 2, RS = 32 / CP, IT = 32 / RS;
-  const int lane = threadIdx.x & 31;
-  const int cp = lane % CP, rs = lane / CP;
-  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t w = gw; w < ngrp * ncb; w += nw) {
-    const int64_t g = w / ncb;
-    const int cb = (int)(w % ncb);
-    const uint32_t b0 = grp[g], nb = grp[g + 1] - b0;
-    P1Desc D[G1];
-    int kmax = 0;
-#pragma unroll
-    for (int q = 0; q < G1; ++q) {
-      if (q < (int)nb) {
-        D[q] = d[b0 + q];
-        kmax = max(kmax, (int)D[q].k);
-      } else {
-        D[q].k = 0;
-      }
-    }
-    const uint32_t seg0 = D[0].seg0, len = D[0].len;
-    const double* xb = xr + (int64_t)seg0 * ld + cb * CB + 2 * cp;
-    for (int r = 0; r < kmax; r += 2) {
-      double acc[G1][2][2];
-#pragma unroll
-      for (int q = 0; q < G1; ++q)
-#pragma unroll
-        for (int a = 0; a < 2; ++a) acc[q][a][0] = acc[q][a][1] = 0.0;
-      for (uint32_t r0 = 0; r0 < len; r0 += 32) {
-        double2 xv[IT];
-#pragma unroll
-        for (int it = 0; it < IT; ++it) {
-          const uint32_t row = r0 + RS * it + rs;
-          xv[it] = row < len ? __ldg(reinterpret_cast<const double2*>(xb + (int64_t)row * ld)) : make_double2(0.0, 0.0);
-        }
-#pragma unroll
-        for (int q = 0; q < G1; ++q) {
-          if (r < (int)D[q].k) {             // uniform over the warp
-            const T* f0 = pool + D[q].off + (int64_t)r * D[q].stride;
-            const bool two = r + 1 < (int)D[q].k;
-            const uint32_t row = r0 + lane;
-            const double a0 = row < len ? (double)from_store<T>(f0[row]) : 0.0;
-            const double a1 = (two && row < len) ? (double)from_store<T>(f0[D[q].stride + row]) : 0.0;
-#pragma unroll
-            for (int it = 0; it < IT; ++it) {
-              const double u = __shfl_sync(0xffffffffu, a0, RS * it + rs);
-              const double v = __shfl_sync(0xffffffffu, a1, RS * it + rs);
-              acc[q][0][0] = fma(u, xv[it].x, acc[q][0][0]);
-              acc[q][0][1] = fma(u, xv[it].y, acc[q][0][1]);
-              acc[q][1][0] = fma(v, xv[it].x, acc[q][1][0]);
-              acc[q][1][1] = fma(v, xv[it].y, acc[q][1][1]);
-            }
-          }
-        }
-      }
-      // sum over the RS lanes that share a column pair
-#pragma unroll
-      for (int o = CP; o < 32; o <<= 1)
-#pragma unroll
-        for (int q = 0; q < G1; ++q)
-#pragma unroll
-          for (int a = 0; a < 2; ++a) {
-            acc[q][a][0] += __shfl_xor_sync(0xffffffffu, acc[q][a][0], o);
-            acc[q][a][1] += __shfl_xor_sync(0xffffffffu, acc[q][a][1], o);
-          }
-      if (rs == 0) {
-#pragma unroll
-        for (int q = 0; q < G1; ++q)
-#pragma unroll
-          for (int a = 0; a < 2; ++a)
-            if (r + a < (int)D[q].k) {
-              double* zp = zr + (int64_t)(D[q].zoff + r + a) * ld + cb * CB + 2 * cp;
-              *reinterpret_cast<double2*>(zp) = make_double2(acc[q][a][0], acc[q][a][1]);
-            }
-      }
-    }
-  }
-}
-
-// Phase 1, segment tasks: a CTA takes up to S1_LEAVES leaves that share one
-// input segment (descriptors ordered by segment) and stages the segment's rows
-// of X (its CB columns) in shared memory once, rows padded by two doubles so
-// that the 32 rows a warp reads at a time fall in distinct banks.  Each warp
-// runs one leaf at a time, lane = row: its factor values come from its own
-// coalesced loads (a block of S1_ROWS rows prefetched at once), its x row from
-// shared memory, and the 2 x CB sums are reduced over the warp at the end.
-constexpr int S1_LEAVES = 64;
-constexpr int S1_ROWS = 256;                // factor rows prefetched per pass
-
-template <typename T, int CB>
-__global__ void __launch_bounds__(256) mvm_phase1_seg_kernel(const P1Desc* __restrict__ d,
-                                                             const uint32_t* __restrict__ task, int64_t ntask,
-                                                             const T* __restrict__ pool,
-                                                             const double* __restrict__ xr, int ld, int ncb,
-                                                             double* __restrict__ zr) {
-  constexpr int XS = CB + 2;                          // padded row of the staged X
-  constexpr int NV = 2 * CB;
-  extern __shared__ double xs[];                     // len x XS
-  const int64_t tk = blockIdx.x / ncb;
-  const int cb = (int)(blockIdx.x % ncb);
-  const uint32_t b0 = task[tk], b1 = task[tk + 1];
-  const uint32_t seg0 = d[b0].seg0, len = d[b0].len;
-  const double* xb = xr + (int64_t)seg0 * ld + cb * CB;
-  for (uint32_t e = threadIdx.x; e < len * (CB / 2); e += blockDim.x) {
-    const uint32_t row = e / (CB / 2), c2 = e % (CB / 2);
-    *reinterpret_cast<double2*>(xs + row * XS + 2 * c2) =
-        __ldg(reinterpret_cast<const double2*>(xb + (int64_t)row * ld) + c2);
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (uint32_t b = b0 + warp; b < b1; b += blockDim.x / 32) {
-    const P1Desc D = d[b];
-    const T* F = pool + D.off;
-    for (int r = 0; r < D.k; r += 2) {
-      const bool two = r + 1 < D.k;
-      const T* f0 = F + (int64_t)r * D.stride;
-      double v[NV];
-#pragma unroll
-      for (int c = 0; c < NV; ++c) v[c] = 0.0;
-      for (uint32_t base = 0; base < len; base += S1_ROWS) {
-        double u0[S1_ROWS / 32], u1[S1_ROWS / 32];
-#pragma unroll
-        for (int q = 0; q < S1_ROWS / 32; ++q) {
-          const uint32_t row = base + 32 * q + lane;
-          u0[q] = row < len ? (double)from_store<T>(f0[row]) : 0.0;
-          u1[q] = (two && row < len) ? (double)from_store<T>(f0[D.stride + row]) : 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < S1_ROWS / 32; ++q) {
-          const uint32_t row = base + 32 * q + lane;
-          if (base + 32 * q >= len) break;
-          if (row < len) {
-            const double* xrow = xs + row * XS;
-#pragma unroll
-            for (int c = 0; c < CB; c += 2) {
-              const double2 xv = *reinterpret_cast<const double2*>(xrow + c);
-              v[c] = fma(u0[q], xv.x, v[c]);
-              v[c + 1] = fma(u0[q], xv.y, v[c + 1]);
-              v[CB + c] = fma(u1[q], xv.x, v[CB + c]);
-              v[CB + c + 1] = fma(u1[q], xv.y, v[CB + c + 1]);
-            }
-          }
-        }
-      }
-      int idx;
-      const double sum = warp_reduce_scatter<NV>(v, lane, idx);
-      if ((lane & (32 / NV - 1)) == 0) {
-        const int rank = r + idx / CB, col = idx % CB;
-        if (rank < D.k) zr[(int64_t)(D.zoff + rank) * ld + cb * CB + col] = sum;
-      }
-    }
-  }
-}
-
-constexpr int M2_THREADS = 256;             // 2 rows a thread: half a window
-constexpr int M2_NB = 32;                   // descriptors staged per round
-constexpr uint64_t M2_DENSE_FLAG = 1ull << 63;
-
-template <int CB> struct M2Cfg {
-  static constexpr int EMAX = CB >= 16 ? 256 : 512;   // entries per sub-round (z rows in shared memory)
-};
-
-template <typename T, typename TD, int CB>
-__global__ void __launch_bounds__(M2_THREADS) mvm_phase2_kernel(const MvWin* __restrict__ win,
-                                                                const P2Desc* __restrict__ d,
-                                                                const T* __restrict__ rk, const TD* __restrict__ dn,
-                                                                const double* __restrict__ zr,
-                                                                const double* __restrict__ xr, int ld, int ncb,
-                                                                double* __restrict__ Y, int64_t ldy, int ncols) {
-  constexpr int EMAX = M2Cfg<CB>::EMAX;
-  constexpr int U = CB >= 16 ? 4 : 8;         // entries whose factor loads are in flight together
-  __shared__ P2Desc sd[M2_NB];
-  __shared__ int spre[M2_NB + 1];
-  __shared__ uint64_t e_off[EMAX];
-  __shared__ int32_t e_ro[EMAX];
-  __shared__ uint32_t e_m[EMAX];
-  __shared__ uint32_t e_rs[EMAX];
-  __shared__ __align__(16) double e_z[EMAX * CB];
-  const int cb = (int)(blockIdx.x % ncb);
-  const int64_t wh = blockIdx.x / ncb;
-  const MvWin W = win[wh >> 1];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int base = (int)(wh & 1) * (2 * M2_THREADS) + 2 * threadIdx.x;   // first of this thread's 2 rows
-  double acc[2][CB];
-#pragma unroll
-  for (int q = 0; q < 2; ++q)
-#pragma unroll
-    for (int j = 0; j < CB; ++j) acc[q][j] = 0.0;
-  for (uint32_t b0 = W.begin; b0 < W.end; b0 += M2_NB) {
-    const int nb = (int)min((uint32_t)M2_NB, W.end - b0);
-    __syncthreads();
-    if (warp == 0) {
-      int cnt = 0;
-      if (lane < nb) {
-        sd[lane] = d[b0 + lane];
-        // only leaves that cover rows of this half window are expanded
-        const int r0 = sd[lane].row_off, r1 = r0 + (int)sd[lane].m;
-        const int h0 = (int)(wh & 1) * (2 * M2_THREADS);
-        cnt = (r1 > h0 && r0 < h0 + 2 * M2_THREADS) ? (int)sd[lane].cnt : 0;
-      }
-      int incl = cnt;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-      }
-      spre[lane + 1] = incl;
-      if (lane == 0) spre[0] = 0;
-    }
-    __syncthreads();
-    const int total = spre[nb];
-    for (int e0 = 0; e0 < total; e0 += EMAX) {
-      const int ne = min(EMAX, total - e0);
-      if (e0 > 0) __syncthreads();
-      for (int e = threadIdx.x; e < ne; e += blockDim.x) {
-        const int ge = e0 + e;
-        int lo = 0, hi = nb - 1;
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (spre[mid] <= ge) lo = mid; else hi = mid - 1;
-        }
-        const P2Desc& D = sd[lo];
-        const int c = ge - spre[lo];
-        const double* zsrc;
-        if (D.type == P2_RK) {
-          e_off[e] = D.off + (uint64_t)c * D.ld;
-          e_rs[e] = 1;
-          zsrc = zr + (int64_t)(D.aux + c) * ld + cb * CB;
-        } else if (D.type == P2_DENSE) {
-          e_off[e] = (D.off + (uint64_t)c * D.ld) | M2_DENSE_FLAG;
-          e_rs[e] = 1;
-          zsrc = xr + (int64_t)(D.aux + c) * ld + cb * CB;
-        } else {
-          e_off[e] = (D.off + (uint64_t)c) | M2_DENSE_FLAG;
-          e_rs[e] = D.ld;
-          zsrc = xr + (int64_t)(D.aux + c) * ld + cb * CB;
-        }
-#pragma unroll
-        for (int j = 0; j < CB; j += 2)
-          *reinterpret_cast<double2*>(e_z + e * CB + j) = __ldg(reinterpret_cast<const double2*>(zsrc + j));
-        e_ro[e] = D.row_off;
-        e_m[e] = D.m;
-      }
-      __syncthreads();
-      for (int e = 0; e < ne; e += U) {
-        double2 f[U];
-        bool cov = false;                     // some entry of this group covers a row of this thread
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          f[u] = make_double2(0.0, 0.0);
-          const int ee = e + u;
-          if (ee < ne) {
-            const int ro = e_ro[ee];
-            const int mm = (int)e_m[ee];
-            const uint64_t o = e_off[ee];
-            const uint32_t rs = e_rs[ee];
-            const int lr = base - ro;
-            cov = cov || (lr + 1 >= 0 && lr < mm);
-            const bool dense = (o & M2_DENSE_FLAG) != 0;
-            const uint64_t oo = o & ~M2_DENSE_FLAG;
-            if (((ro & 1) == 0) && rs == 1) {
-              if (lr >= 0 && lr < mm) f[u] = dense ? Pair<TD>::ld(dn + oo + lr) : Pair<T>::ld(rk + oo + lr);
-            } else {
-              if (lr >= 0 && lr < mm)
-                f[u].x = dense ? Pair<TD>::one(dn + oo + (uint64_t)lr * rs) : Pair<T>::one(rk + oo + lr);
-              if (lr + 1 >= 0 && lr + 1 < mm)
-                f[u].y = dense ? Pair<TD>::one(dn + oo + (uint64_t)(lr + 1) * rs) : Pair<T>::one(rk + oo + lr + 1);
-            }
-          }
-        }
-        // a warp covers 64 consecutive rows: leaves shorter than the half
-        // window (dense near-field blocks) leave most warps idle here
-        if (!__any_sync(0xffffffffu, cov)) continue;
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (e + u < ne) {
-            const double* zz = e_z + (e + u) * CB;
-#pragma unroll
-            for (int j = 0; j < CB; j += 2) {
-              const double2 zv = *reinterpret_cast<const double2*>(zz + j);
-              acc[0][j] = fma(f[u].x, zv.x, acc[0][j]);
-              acc[0][j + 1] = fma(f[u].x, zv.y, acc[0][j + 1]);
-              acc[1][j] = fma(f[u].y, zv.x, acc[1][j]);
-              acc[1][j + 1] = fma(f[u].y, zv.y, acc[1][j + 1]);
-            }
-          }
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const int r = base + q;
-    if (r < (int)W.nrows) {
-#pragma unroll
-      for (int j = 0; j < CB; ++j) {
-        const int col = cb * CB + j;
-        if (col < ncols) Y[(int64_t)(W.row0 + r) + (int64_t)col * ldy] = acc[q][j];
-      }
-    }
   }
 }
 
@@ -482,111 +475,117 @@ __global__ void __launch_bounds__(128) mvm_dense_kernel(const MvWin* __restrict_
   }
 }
 
-// Phase-1 descriptors ordered by input segment: the warps running at the same
-// time then read the same rows of XR (L1/L2 hits) instead of c x 8 bytes per
-// row from HBM for every leaf.  Stable, so a segment's leaves keep pool order.
-// Groups of at most G1 consecutive sorted descriptors with the same segment:
-// P.d_g1s[g] is the first descriptor of group g, P.d_g1s[ng1] = np1.
-static int ensure_sorted_p1(MvPlan& P) {
-  if (P.d_p1s || P.np1 == 0) return HM_OK;
-  std::vector<P1Desc> v((size_t)P.np1);
-  HM_CUDA_TRY(cudaMemcpy(v.data(), P.d_p1, sizeof(P1Desc) * v.size(), cudaMemcpyDeviceToHost));
-  std::stable_sort(v.begin(), v.end(), [](const P1Desc& a, const P1Desc& b) {
-    return a.seg0 != b.seg0 ? a.seg0 < b.seg0 : a.len < b.len;
-  });
-  std::vector<uint32_t> g;
-  for (size_t i = 0; i < v.size();) {
-    g.push_back((uint32_t)i);
-    size_t j = i + 1;
-    while (j < v.size() && j - i < (size_t)G1 && v[j].seg0 == v[i].seg0 && v[j].len == v[i].len) ++j;
-    i = j;
-  }
-  P.ng1 = (int64_t)g.size();
-  g.push_back((uint32_t)v.size());
-  // segment tasks: runs of equal (seg0, len), cut every S1_LEAVES leaves
-  std::vector<uint32_t> tk;
-  uint32_t maxlen = 0;
-  for (size_t i = 0; i < v.size();) {
-    size_t j = i + 1;
-    while (j < v.size() && j - i < (size_t)S1_LEAVES && v[j].seg0 == v[i].seg0 && v[j].len == v[i].len) ++j;
-    tk.push_back((uint32_t)i);
-    maxlen = std::max(maxlen, v[i].len);
-    i = j;
-  }
-  P.nt1 = (int64_t)tk.size();
-  P.maxlen1 = maxlen;
-  tk.push_back((uint32_t)v.size());
-  HM_CUDA_TRY(cudaMalloc(&P.d_t1s, sizeof(uint32_t) * tk.size()));
-  HM_CUDA_TRY(h2d_sync(P.d_t1s, tk.data(), sizeof(uint32_t) * tk.size()));
-  HM_CUDA_TRY(cudaMalloc(&P.d_p1s, sizeof(P1Desc) * v.size()));
-  HM_CUDA_TRY(h2d_sync(P.d_p1s, v.data(), sizeof(P1Desc) * v.size()));
-  HM_CUDA_TRY(cudaMalloc(&P.d_g1s, sizeof(uint32_t) * g.size()));
-  HM_CUDA_TRY(h2d_sync(P.d_g1s, g.data(), sizeof(uint32_t) * g.size()));
-  return HM_OK;
-}
-
-template <typename T, int CB>
-int launch_multi(hm_handle* h, const double* d_x, double* d_y, int64_t ncols, int trans, cudaStream_t st,
-                 bool dense_only = false) {
-  using TD = typename std::conditional<std::is_same<T, double>::value, double, float>::type;
-  MvPlan& P = trans ? h->bwd : h->fwd;
-  if (!dense_only) HM_TRY(ensure_sorted_p1(P));
-  const int ld = (int)pad_to(ncols, CB);
-  const int ncb = ld / CB;
-  const size_t xr_bytes = sizeof(double) * (size_t)(h->n + 2) * ld;
-  // the dense-only pass needs no phase-1 results
-  const size_t zr_bytes = dense_only ? 0 : sizeof(double) * (size_t)std::max<int64_t>(h->zlen, 1) * ld;
-  if (h->xm_bytes < xr_bytes + zr_bytes) {
+// the block products' scratch in the handle (Z, or the transposed input)
+int block_scratch(hm_handle* h, size_t bytes, double** out) {
+  if (h->xm_bytes < bytes) {
     if (h->d_xm) cudaFree(h->d_xm);
     h->d_xm = nullptr;
     h->xm_bytes = 0;
-    HM_CUDA_TRY(cudaMalloc(&h->d_xm, xr_bytes + zr_bytes));
-    h->xm_bytes = xr_bytes + zr_bytes;
+    HM_CUDA_TRY(cudaMalloc(&h->d_xm, bytes));
+    h->xm_bytes = bytes;
   }
-  double* xr = (double*)h->d_xm;
-  double* zr = (double*)((char*)h->d_xm + xr_bytes);
-  int nsm = 148;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
-  {
-    const int64_t tot = (h->n + 2) * ld;
-    const unsigned g = (unsigned)std::min<int64_t>((tot + 255) / 256, (int64_t)nsm * 16);
-    mvm_xr_kernel<<<g, 256, 0, st>>>(d_x, h->n, h->n, (int)ncols, xr, ld);
+  *out = (double*)h->d_xm;
+  return HM_OK;
+}
+
+// The factor columns of phase 1 by input segment (the clusters' pre-order
+// starts), 32 to a tile; within a segment in pool order.
+int ensure_columns(hm_handle* h, int trans, MvPlan& P) {
+  if (P.d_mbcol || P.np1 == 0) return HM_OK;
+  const int eb = elem_bytes(h->storage);
+  const std::vector<int64_t> order = pool_order(h);
+  const int64_t ncl = (int64_t)h->cl_s.size();
+  std::vector<int64_t> at((size_t)ncl + 1, 0);
+  for (const Leaf& L : h->leaves)
+    if (L.type == T_RK) at[(trans ? L.s : L.t) + 1] += L.k;
+  for (int64_t c = 0; c < ncl; ++c) at[c + 1] += at[c];
+  const int64_t ntot = at[ncl];
+  std::vector<MbCol> col((size_t)ntot);
+  std::vector<MbTile> tile;
+  for (int64_t c = 0; c < ncl; ++c)
+    for (int64_t b = at[c]; b < at[c + 1]; b += 8 * MB_MT)
+      tile.push_back(MbTile{(uint32_t)b, (uint32_t)std::min<int64_t>(8 * MB_MT, at[c + 1] - b), (uint32_t)h->cl_s[c],
+                            (uint32_t)(h->cl_e[c] - h->cl_s[c])});
+  uint64_t z = 0;
+  for (int64_t li : order) {
+    const Leaf& L = h->leaves[li];
+    if (L.type != T_RK) continue;
+    const int64_t npad = col_pad(L.n, eb), mpad = col_pad(L.m, eb);
+    int64_t& next = at[trans ? L.s : L.t];
+    for (int r = 0; r < L.k; ++r)
+      col[next++] = MbCol{(uint64_t)(trans ? L.off + npad * L.k + r * mpad : L.off + r * npad), z++};
   }
-  const int64_t nblk = (int64_t)P.nwin * 2 * ncb;
-  if (nblk > (int64_t)INT32_MAX) return fail(HM_ERR_UNSUPPORTED, "too many phase-2 blocks");
-  if (dense_only) {
-    HM_TRY(split_p2(P));
-    const int64_t ntile = (h->n + 127) / 128;
-    const int64_t blocks = ntile * ncb;
-    if (blocks > (int64_t)INT32_MAX) return fail(HM_ERR_UNSUPPORTED, "too many dense-pass blocks");
-    mvm_dense_kernel<TD, CB><<<(unsigned)blocks, 128, 0, st>>>(P.d_wind, P.d_p2d, (const TD*)h->d_dense, xr, ld, ncb,
-                                                             ntile, d_y, h->n, (int)ncols);
-    HM_CUDA_TRY(cudaGetLastError());
+  const size_t cb = sizeof(MbCol) * col.size();
+  void* d = nullptr;
+  cudaError_t e = cudaMalloc(&d, cb + sizeof(MbTile) * tile.size());
+  if (e != cudaSuccess) return fail(HM_ERR_OOM, std::string("block product columns: ") + cudaGetErrorString(e));
+  P.d_mbcol = (MbCol*)d;                                 // owned by the plan from here on
+  P.d_mbtile = (MbTile*)((char*)d + cb);
+  P.nmbtile = (int64_t)tile.size();
+  HM_CUDA_TRY(h2d_sync(P.d_mbcol, col.data(), cb));
+  HM_CUDA_TRY(h2d_sync(P.d_mbtile, tile.data(), sizeof(MbTile) * tile.size()));
+  return HM_OK;
+}
+
+template <typename T, int NT>
+int launch_multi(hm_handle* h, const double* d_x, double* d_y, int64_t ncols, int trans, cudaStream_t st) {
+  using TD = typename std::conditional<std::is_same<T, double>::value, double, float>::type;
+  MvPlan& P = trans ? h->bwd : h->fwd;
+  bool slabs = false;
+  HM_TRY(ensure_slabs(h, trans, &slabs));
+  if (!slabs) {                                          // no memory for the lists: column by column
+    for (int64_t c = 0; c < ncols; ++c) HM_TRY(matvec_device(h, d_x + c * h->n, d_y + c * h->n, trans, st));
     return HM_OK;
   }
-  const size_t seg_smem = sizeof(double) * (size_t)P.maxlen1 * (CB + 2);
-  if (P.np1 > 0 && seg_smem <= 96 * 1024 && P.nt1 * ncb <= (int64_t)INT32_MAX) {
-    HM_CUDA_TRY(smem_attr((const void*)mvm_phase1_seg_kernel<T, CB>, 96 * 1024));
-    mvm_phase1_seg_kernel<T, CB><<<(unsigned)(P.nt1 * ncb), 256, seg_smem, st>>>(P.d_p1s, P.d_t1s, P.nt1,
-                                                                               (const T*)h->d_rk, xr, ld, ncb, zr);
-  } else if (P.np1 > 0) {                        // segments too long to stage: grouped leaves
-    const int64_t warps = P.ng1 * ncb;
-    const int64_t blocks = std::min<int64_t>((warps + 7) / 8, (int64_t)nsm * 8);
-    mvm_phase1_kernel<T, CB><<<(unsigned)blocks, 256, 0, st>>>(P.d_p1s, P.d_g1s, P.ng1, (const T*)h->d_rk, xr, ld,
-                                                              ncb, zr);
+  HM_TRY(ensure_columns(h, trans, P));
+  const int ld = (int)pad_to(ncols, 8 * NT);
+  const int ncb = ld / (8 * NT);
+  double* z = nullptr;
+  HM_TRY(block_scratch(h, sizeof(double) * (size_t)std::max<int64_t>(h->zlen, 1) * ld, &z));
+  const int64_t nblk = (int64_t)P.nslab * ncb;
+  if (nblk > (int64_t)INT32_MAX) return fail(HM_ERR_UNSUPPORTED, "too many phase-2 blocks");
+  if (P.nmbtile > 0) {
+    const int64_t blocks = std::min<int64_t>((P.nmbtile * ncb + MB_WARPS - 1) / MB_WARPS, 148 * 64);
+    mb_phase1_kernel<T, NT><<<(unsigned)blocks, MB_WARPS * 32, 0, st>>>(
+        P.d_mbtile, P.nmbtile, P.d_mbcol, (const T*)h->d_rk, d_x, h->n, (int)ncols, ncb, z, ld);
   }
-  mvm_phase2_kernel<T, TD, CB><<<(unsigned)nblk, M2_THREADS, 0, st>>>(
-      P.d_win, P.d_p2, (const T*)h->d_rk, (const TD*)h->d_dense, zr, xr, ld, ncb, d_y, h->n, (int)ncols);
+  mb_phase2_kernel<T, TD, NT><<<(unsigned)nblk, MB_WARPS * 32, 0, st>>>(
+      P.d_slab, P.d_ent, (const T*)h->d_rk, (const TD*)h->d_dense, z, ld, d_x, h->n, (int)ncols, ncb, d_y, h->n);
   HM_CUDA_TRY(cudaGetLastError());
   return HM_OK;
 }
 
 template <typename T>
-int multi_t(hm_handle* h, const double* d_x, double* d_y, int64_t ncols, int trans, cudaStream_t st,
-            bool dense_only = false) {
-  if (ncols <= 4) return launch_multi<T, 4>(h, d_x, d_y, ncols, trans, st, dense_only);
-  if (ncols <= 8) return launch_multi<T, 8>(h, d_x, d_y, ncols, trans, st, dense_only);
-  return launch_multi<T, 16>(h, d_x, d_y, ncols, trans, st, dense_only);
+int multi_t(hm_handle* h, const double* d_x, double* d_y, int64_t ncols, int trans, cudaStream_t st) {
+  if (ncols <= 8) return launch_multi<T, 1>(h, d_x, d_y, ncols, trans, st);
+  if (ncols <= 16) return launch_multi<T, 2>(h, d_x, d_y, ncols, trans, st);
+  return launch_multi<T, 4>(h, d_x, d_y, ncols, trans, st);
+}
+
+// the dense leaves (FP32) of a tensor-core call, written into Y
+template <int CB>
+int launch_dense(hm_handle* h, const double* d_x, double* d_y, int64_t ncols, int trans, cudaStream_t st) {
+  MvPlan& P = trans ? h->bwd : h->fwd;
+  HM_TRY(split_p2(P));
+  const int ld = (int)pad_to(ncols, CB);
+  const int ncb = ld / CB;
+  double* xr = nullptr;
+  HM_TRY(block_scratch(h, sizeof(double) * (size_t)(h->n + 2) * ld, &xr));
+  const int64_t tot = (h->n + 2) * ld;
+  mvm_xr_kernel<<<(unsigned)std::min<int64_t>((tot + 255) / 256, 148 * 16), 256, 0, st>>>(d_x, h->n, h->n, (int)ncols,
+                                                                                        xr, ld);
+  const int64_t ntile = (h->n + 127) / 128, blocks = ntile * ncb;
+  if (blocks > (int64_t)INT32_MAX) return fail(HM_ERR_UNSUPPORTED, "too many dense-pass blocks");
+  mvm_dense_kernel<float, CB><<<(unsigned)blocks, 128, 0, st>>>(P.d_wind, P.d_p2d, (const float*)h->d_dense, xr, ld, ncb,
+                                                              ntile, d_y, h->n, (int)ncols);
+  HM_CUDA_TRY(cudaGetLastError());
+  return HM_OK;
+}
+
+int dense_pass(hm_handle* h, const double* d_x, double* d_y, int64_t ncols, int trans, cudaStream_t st) {
+  if (ncols <= 4) return launch_dense<4>(h, d_x, d_y, ncols, trans, st);
+  if (ncols <= 8) return launch_dense<8>(h, d_x, d_y, ncols, trans, st);
+  return launch_dense<16>(h, d_x, d_y, ncols, trans, st);
 }
 
 }  // namespace
@@ -605,14 +604,14 @@ int matvec_multi_device(hm_handle* h, const double* d_x, double* d_y, int64_t nc
       bool tc = false;
       if (!simt) HM_TRY(tc_prepare(h, trans, &tc));
       if (!tc) return multi_t<float>(h, d_x, d_y, ncols, trans, st);
-      HM_TRY(multi_t<float>(h, d_x, d_y, ncols, trans, st, true));
+      HM_TRY(dense_pass(h, d_x, d_y, ncols, trans, st));
       return matvec_multi_tc(h, d_x, d_y, ncols, trans, st);
     }
     default: {
       bool tc = false;
       if (!simt) HM_TRY(tc_prepare(h, trans, &tc));
       if (!tc) return multi_t<__nv_bfloat16>(h, d_x, d_y, ncols, trans, st);
-      HM_TRY(multi_t<__nv_bfloat16>(h, d_x, d_y, ncols, trans, st, true));
+      HM_TRY(dense_pass(h, d_x, d_y, ncols, trans, st));
       return matvec_multi_tc(h, d_x, d_y, ncols, trans, st);
     }
   }
