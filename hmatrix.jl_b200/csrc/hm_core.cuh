@@ -10,7 +10,8 @@ namespace hm {
 // ===========================================================================
 // Recompression core (K3): CGS2 QR of A and B in place, W = R_A R_B^T, one
 // sided Jacobi SVD of W, truncation k = #{s_i/s_1 > eps_trunc}, and
-// A' = Q_A U_k, B' = Q_B V_k S_k.  One CTA per job; smem 3*rmax^2 doubles.
+// A' = Q_A U_k, B' = Q_B V_k S_k.  One CTA per job; smem 3 rmax (rmax + 1)
+// doubles.
 // ===========================================================================
 // Columns [0, j0) are already orthonormal and their block of Rm is set by the
 // caller (cgs2_qr zeroes the rest of Rm first).
@@ -59,6 +60,107 @@ static __device__ void cgs2_qr(TS* X, int len, int ld, int r, TS* Rm /* r x r, c
   }
 }
 
+// Jacobi rotation of a column pair with squared norms al, be and dot product
+// ga != 0: t = tan of the angle, c = cos, s = c t.  t only has to be near the
+// angle that zeroes ga (20 bits: ga shrinks a millionfold instead of vanishing,
+// and the pair is met again), so it comes from the approximate reciprocal and
+// reciprocal square root; c is Newton-refined to full precision, which keeps
+// the rotation orthogonal whatever t is.  Divisions and square roots in full
+// precision made a round of rotations a chain of about 600 cycles.
+__device__ __forceinline__ double rcp_fast(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+__device__ __forceinline__ double rsqrt_fast(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+__device__ __forceinline__ void jacobi_angle(double al, double be, double ga, double& c, double& s) {
+  const double zeta = 0.5 * (be - al) * rcp_fast(ga);
+  const double az = fmin(fabs(zeta), 1e150);               // its square stays finite
+  const double q = fma(az, az, 1.0);
+  double t = rcp_fast(az + q * rsqrt_fast(q));
+  if (zeta < 0.0) t = -t;
+  const double v = fma(t, t, 1.0);                         // in [1, 2]
+  double y = rsqrt_fast(v);
+  y = y * fma(-0.5 * v * y, y, 1.5);                       // Newton for v^(-1/2): 20, 40, full bits
+  y = y * fma(-0.5 * v * y, y, 1.5);
+  c = y;
+  s = y * t;
+}
+__device__ __forceinline__ void jacobi_angle(float al, float be, float ga, float& c, float& s) {
+  const float zeta = (be - al) / (2.f * ga);
+  const float t = (zeta >= 0.f ? 1.f : -1.f) / (fabsf(zeta) + sqrtf(1.f + zeta * zeta));
+  c = 1.f / sqrtf(1.f + t * t);
+  s = c * t;
+}
+
+// One-sided Jacobi on the r <= 16 columns of W (r x r, column stride lw) and
+// of V by ONE warp: 4 lanes a column pair, 4 rows a lane in registers, so that
+// a round is eight pairs at once and needs no block barrier.
+template <typename TS>
+static __device__ void jacobi_warp16(TS* W, TS* V, int r, int lw, TS thr) {
+  const int lane = threadIdx.x & 31, sg = lane >> 2, sl = lane & 3;
+  const int rr = (r + 1) & ~1;
+  const TS thr2 = thr * thr;
+  for (int sweep = 0; sweep < 60; ++sweep) {
+    bool rot = false;
+    for (int round = 0; round < rr - 1; ++round) {
+      auto posv = [&](int q) { return q == 0 ? 0 : 1 + (q - 1 + round) % (rr - 1); };
+      int p = 0, q = 0;
+      bool act = sg < rr / 2;
+      if (act) {
+        p = posv(sg); q = posv(rr - 1 - sg);
+        if (p > q) { const int t = p; p = q; q = t; }
+        act = q < r;
+      }
+      TS *wp = W + p * lw, *wq = W + q * lw, *vp = V + p * lw, *vq = V + q * lw;
+      TS x[4], y[4], u[4], v[4];
+      TS al = 0, be = 0, ga = 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int t = sl + 4 * i;
+        const bool in = act && t < r;
+        x[i] = in ? wp[t] : (TS)0;
+        y[i] = in ? wq[t] : (TS)0;
+        u[i] = in ? vp[t] : (TS)0;
+        v[i] = in ? vq[t] : (TS)0;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        al = fma(x[i], x[i], al);
+        be = fma(y[i], y[i], be);
+        ga = fma(x[i], y[i], ga);
+      }
+#pragma unroll
+      for (int o = 2; o > 0; o >>= 1) {
+        al += __shfl_xor_sync(0xffffffffu, al, o);
+        be += __shfl_xor_sync(0xffffffffu, be, o);
+        ga += __shfl_xor_sync(0xffffffffu, ga, o);
+      }
+      if (act && ga != (TS)0 && ga * ga > thr2 * al * be) {
+        TS c, s;
+        jacobi_angle(al, be, ga, c, s);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int t = sl + 4 * i;
+          if (t < r) {
+            wp[t] = c * x[i] - s * y[i];
+            wq[t] = s * x[i] + c * y[i];
+            vp[t] = c * u[i] - s * v[i];
+            vq[t] = s * u[i] + c * v[i];
+          }
+        }
+        rot = true;
+      }
+      __syncwarp();
+    }
+    if (!__any_sync(0xffffffffu, rot)) break;
+  }
+}
+
 static __device__ void zero_cols(double* X, int len, int64_t ld, int c0, int c1) {
   for (int c = c0; c < c1; ++c)
     for (int i = threadIdx.x; i < len; i += blockDim.x) X[i + (int64_t)c * ld] = 0.0;
@@ -86,8 +188,8 @@ static __device__ void core_body_t(const CoreJob& J, TS* __restrict__ JA, TS* __
   __shared__ int s_k;
   int r = J.r_dev ? *J.r_dev : J.r;
   TS* b0 = sm;                           // R_A, later V (Jacobi right vectors)
-  TS* b1 = sm + rmax * rmax;             // R_B, later U-coefficients
-  TS* b2 = sm + 2 * rmax * rmax;         // W, later V-coefficients
+  TS* b1 = sm + rmax * (rmax + 1);       // R_B, later U-coefficients
+  TS* b2 = sm + 2 * rmax * (rmax + 1);   // W, later V-coefficients
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int pre = J.pre_status ? *J.pre_status : 0;
   if (pre != 0 || r > rmax) {
@@ -135,13 +237,15 @@ static __device__ void core_body_t(const CoreJob& J, TS* __restrict__ JA, TS* __
   }
   cgs2_qr(JA, J.m, J.lda, r, b0, proj, red, ok);
   cgs2_qr(JB, J.n, J.ldb, r, b1, proj, red, ok);
-  // W = R_A R_B^T  (r x r, column-major, ld r)
+  // W = R_A R_B^T  (r x r, column-major; JAC8: an odd column stride, whose
+  // columns start in different banks)
+  const int lw = JAC8 ? r | 1 : r;
   double sabs = 0.0;
   for (int e = threadIdx.x; e < r * r; e += blockDim.x) {
     const int i = e % r, j = e / r;
     TS s = 0;
     for (int q = max(i, j); q < r; ++q) s = fma(b0[i + q * r], b1[j + q * r], s);
-    b2[e] = s;
+    b2[i + j * lw] = s;
     sabs += fabs((double)s);
   }
   sabs = block_sum(sabs, red);
@@ -155,13 +259,17 @@ static __device__ void core_body_t(const CoreJob& J, TS* __restrict__ JA, TS* __
     return;
   }
   // V = I
-  for (int e = threadIdx.x; e < r * r; e += blockDim.x) b0[e] = (e % r == e / r) ? (TS)1 : (TS)0;
+  for (int e = threadIdx.x; e < r * r; e += blockDim.x) b0[e % r + e / r * lw] = (e % r == e / r) ? (TS)1 : (TS)0;
   __syncthreads();
   // one-sided Jacobi on the columns of W, round-robin pairing.  A pair is
   // rotated while its cosine exceeds thr; the truncation only needs the
   // singular values far below eps_trunc, so thr follows it (at least 1e-15)
   const int rr = (r + 1) & ~1;
   const TS thr = (TS)fmax(sizeof(TS) == 8 ? 1e-15 : 1e-7, 1e-3 * eps_trunc);
+  if (JAC8 && r <= 16) {
+    if (w == 0) jacobi_warp16(b2, b0, r, lw, thr);
+    __syncthreads();
+  } else
   for (int sweep = 0; sweep < 60; ++sweep) {
     if (threadIdx.x == 0) s_rot = 0;
     __syncthreads();
@@ -181,8 +289,8 @@ static __device__ void core_body_t(const CoreJob& J, TS* __restrict__ JA, TS* __
             if (p > q) { int t = p; p = q; q = t; }
             act = q < r;
           }
-          TS* wp = b2 + p * r;
-          TS* wq = b2 + q * r;
+          TS* wp = b2 + p * lw;
+          TS* wq = b2 + q * lw;
           TS al = 0, be = 0, ga = 0;
           if (act)
             for (int t = sl; t < r; t += 8) {
@@ -196,12 +304,11 @@ static __device__ void core_body_t(const CoreJob& J, TS* __restrict__ JA, TS* __
             be += __shfl_xor_sync(0xffffffffu, be, o);
             ga += __shfl_xor_sync(0xffffffffu, ga, o);
           }
-          if (act && ga != (TS)0 && fabs(ga) > thr * sqrt(al * be)) {
-            const TS zeta = (be - al) / ((TS)2 * ga);
-            const TS t = (zeta >= (TS)0 ? (TS)1 : (TS)-1) / (fabs(zeta) + sqrt((TS)1 + zeta * zeta));
-            const TS c = (TS)1 / sqrt((TS)1 + t * t), s = c * t;
-            TS* vp = b0 + p * r;
-            TS* vq = b0 + q * r;
+          if (act && ga != (TS)0 && ga * ga > thr * thr * al * be) {
+            TS c, s;
+            jacobi_angle(al, be, ga, c, s);
+            TS* vp = b0 + p * lw;
+            TS* vq = b0 + q * lw;
             for (int t2 = sl; t2 < r; t2 += 8) {
               const TS x = wp[t2], y = wq[t2];
               wp[t2] = c * x - s * y;
@@ -253,7 +360,7 @@ static __device__ void core_body_t(const CoreJob& J, TS* __restrict__ JA, TS* __
   // singular values = column norms of W; sort descending
   for (int j = w; j < r; j += nw) {
     TS s = 0;
-    for (int t = lane; t < r; t += 32) s = fma(b2[t + j * r], b2[t + j * r], s);
+    for (int t = lane; t < r; t += 32) s = fma(b2[t + j * lw], b2[t + j * lw], s);
     s = warp_sum(s);
     if (lane == 0) sig[j] = sqrt(s);
   }
@@ -305,13 +412,13 @@ static __device__ void core_body_t(const CoreJob& J, TS* __restrict__ JA, TS* __
     const int j = e % r, c = e / r;
     const int o = ord[c];
     const TS s = sig[o];
-    b1[e] = s > (TS)0 ? b2[j + o * r] / s : (TS)0;
+    b1[e] = s > (TS)0 ? b2[j + o * lw] / s : (TS)0;
   }
   __syncthreads();
   for (int e = threadIdx.x; e < r * k; e += blockDim.x) {
     const int j = e % r, c = e / r;
     const int o = ord[c];
-    b2[e] = b0[j + o * r] * sig[o];
+    b2[e] = b0[j + o * lw] * sig[o];
   }
   __syncthreads();
   // (column, row) loops without a division per element; the same sums

@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(256) core_recompress_one_kernel(CoreJob J, int
 }
 
 int launch_core_one(const CoreJob& J, double eps_trunc, int* d_flags, cudaStream_t st) {
-  const size_t smem = (size_t)3 * RCORE_MAX * RCORE_MAX * sizeof(double);
+  const size_t smem = (size_t)3 * RCORE_MAX * (RCORE_MAX + 1) * sizeof(double);
   HM_CUDA_TRY(smem_attr((const void*)core_recompress_one_kernel, (int)smem));
   core_recompress_one_kernel<<<1, 256, smem, st>>>(J, RCORE_MAX, eps_trunc, d_flags);
   HM_CUDA_TRY(cudaGetLastError());
@@ -323,9 +323,9 @@ int launch_core_recompress(const CoreJob* d_jobs, int njobs, int rmax, double ep
   if (njobs == 0) return HM_OK;
   if (rmax > RCORE_MAX) return fail(HM_ERR_UNSUPPORTED, "recompression core above " + std::to_string(RCORE_MAX));
   rmax = std::max(rmax, 1);
-  size_t smem = (size_t)3 * rmax * rmax * sizeof(double);
+  size_t smem = (size_t)3 * rmax * (rmax + 1) * sizeof(double);
   const void* kfn = jac8 ? (const void*)core_recompress_kernel<true> : (const void*)core_recompress_kernel<false>;
-  HM_CUDA_TRY(smem_attr(kfn, (int)((size_t)3 * RCORE_MAX * RCORE_MAX * sizeof(double))));
+  HM_CUDA_TRY(smem_attr(kfn, (int)((size_t)3 * RCORE_MAX * (RCORE_MAX + 1) * sizeof(double))));
   // small cores: 2 warps per job, so that many jobs share an SM
   const int nt = rmax <= 32 ? 64 : 256;
   if (jac8) core_recompress_kernel<true><<<njobs, nt, smem, st>>>(d_jobs, rmax, eps_trunc, d_flags);

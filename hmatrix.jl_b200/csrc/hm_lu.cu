@@ -14,6 +14,7 @@
 #include "hm_internal.h"
 #include "hm_lowrank.cuh"
 #include "hm_core.cuh"
+#include "hm_lu_tile.cuh"
 
 
 #include <algorithm>
@@ -426,10 +427,6 @@ struct GatherArgs {
 };
 __device__ void gather_pieces(const GatherArgs& g);
 __global__ void __launch_bounds__(256) lu_gather_pieces_kernel(GatherArgs g) { gather_pieces(g); }
-__global__ void __launch_bounds__(256) lu_gather_pieces_batch_kernel(const GatherArgs* __restrict__ jobs) {
-  gather_pieces(jobs[blockIdx.x]);
-}
-
 __device__ void gather_pieces(const GatherArgs& g) {
   __shared__ int pre[MAX_PIECES + 1];
   if (threadIdx.x == 0) {
@@ -1226,75 +1223,6 @@ static void gemm_batch(Ctx& c, const std::vector<GemmJob>& jobs, bool big = fals
   }
 }
 
-// one low-rank target = truncated sum of its pieces
-struct RcReq {
-  Piece pc[2];
-  int np;
-  double* outA; int64_t ldoa;
-  double* outB; int64_t ldob;
-  int32_t* k;
-  int m, n, kcap;
-};
-
-// size_to_batch: read the largest core size back and launch for it (one host
-// synchronisation); otherwise launch for rmax.
-static void recompress_batch(Ctx& c, const std::vector<RcReq>& reqs, int rmax, bool size_to_batch = true) {
-  if (reqs.empty()) return;
-  rmax = std::min(std::max(rmax, 1), RCORE_MAX);
-  size_t b = 0;
-  while (b < reqs.size()) {
-    size_t e = b, elems = 0;
-    while (e < reqs.size() && (e == b || elems + (size_t)(reqs[e].m + reqs[e].n) * rmax < (size_t)1 << 27)) {
-      elems += (size_t)(reqs[e].m + reqs[e].n) * rmax;
-      ++e;
-    }
-    Blk tmp;
-    tmp.st = c.st;
-    double* scratch = (double*)dmalloc(c, tmp, sizeof(double) * elems);
-    int32_t* rr = (int32_t*)dmalloc(c, tmp, sizeof(int32_t) * (e - b));
-    std::vector<GatherArgs> ga(e - b);
-    std::vector<CoreJob> cj(e - b);
-    size_t off = 0;
-    for (size_t q = b; q < e; ++q) {
-      const RcReq& R = reqs[q];
-      GatherArgs& g = ga[q - b];
-      g = GatherArgs{};
-      for (int p = 0; p < R.np; ++p) g.pc[p] = R.pc[p];
-      g.np = R.np;
-      g.SA = scratch + off;
-      g.SB = scratch + off + (size_t)R.m * rmax;
-      g.M = R.m; g.N = R.n; g.rmax = rmax; g.r_out = rr + (q - b); g.flags = c.flags;
-      CoreJob& J = cj[q - b];
-      J = CoreJob{};
-      J.A = g.SA; J.B = g.SB; J.outA = R.outA; J.outB = R.outB;
-      J.m = R.m; J.n = R.n; J.lda = std::max(R.m, 1); J.ldb = std::max(R.n, 1);
-      J.ldoa = (int32_t)R.ldoa; J.ldob = (int32_t)R.ldob; J.kcap = R.kcap;
-      J.zero_test = 1; J.rank = R.k; J.r_dev = g.r_out; J.zero_fill = 1;
-      off += (size_t)(R.m + R.n) * rmax;
-    }
-    GatherArgs* dg = upload_jobs(c, tmp, ga);
-    CoreJob* dc = upload_jobs(c, tmp, cj);
-    lu_gather_pieces_batch_kernel<<<(unsigned)(e - b), 256, 0, c.st>>>(dg);
-    LU_LAUNCH_CHECK();
-    // size the core launch to the largest core of this batch (ranks are on
-    // the device: one small read-back per batch)
-    int rlaunch = rmax;
-    if (size_to_batch) {
-      int32_t* dmax = (int32_t*)dmalloc(c, tmp, sizeof(int32_t));
-      lu_max_int_kernel<<<1, 256, 0, c.st>>>(rr, (int)(e - b), dmax);
-      LU_LAUNCH_CHECK();
-      int32_t hmax = 0;
-      if (cudaMemcpyAsync(&hmax, dmax, sizeof(int32_t), cudaMemcpyDeviceToHost, c.st) != cudaSuccess ||
-          cudaStreamSynchronize(c.st) != cudaSuccess)
-        throw LuError(HM_ERR_CUDA, "core size read-back");
-      rlaunch = std::min(rmax, std::max(8, (hmax + 7) / 8 * 8));
-    }
-    int s = launch_core_recompress(dc, (int)(e - b), rlaunch, c.eps_trunc, c.flags, c.st, true);
-    if (s != HM_OK) throw LuError(s, "batched recompression launch");
-    b = e;
-  }
-}
-
 // The off-diagonal part of step k's trailing update, generated on the device:
 // for every pair i != j of trailing tiles, A_ij B_ij' - Q_ij B_kj' is gathered
 // into one [A | -Q] [B | B_kj] pair and recompressed (Q_ij = A_ik W_kj, the
@@ -1375,46 +1303,20 @@ __global__ void __launch_bounds__(256) lu_tile_gather_kernel(TileJobArgs a) {
   gather_pieces(g);
 }
 
-// H_tile += s * A B' for an H-structured diagonal tile, as jobs: dense leaves
-// get a product, low-rank leaves a recompression (hmat_add! of H += Rk splits
-// the low-rank term over the children, src/harithm.jl:129-142)
-static void tile_add_lowrank(const Blk& H, int r0, int c0, const double* A, int64_t lda, const double* B,
-                             int64_t ldb, const int32_t* k, int cap, double s, std::vector<GemmJob>& gj,
-                             std::vector<RcReq>& rj) {
-  if (H.type == T_DENSE) {
-    GemmJob g{};
-    g.A = View{const_cast<double*>(A) + r0, 1, lda, H.m, cap};
-    g.B = vtr(View{const_cast<double*>(B) + c0, 1, ldb, H.n, cap});
-    g.C = H.Cv();
-    g.alpha = s;
-    g.beta = 1.0;
-    gj.push_back(g);
-  } else if (H.type == T_RK) {
-    RcReq R{};
-    R.pc[0] = Piece{H.A, H.lda, H.B, H.ldb, H.k, H.m, H.n, 0, 0, 1.0};
-    R.pc[1] = Piece{A + r0, lda, B + c0, ldb, k, H.m, H.n, 0, 0, s};
-    R.np = 2;
-    R.outA = H.A; R.ldoa = H.lda; R.outB = H.B; R.ldob = H.ldb; R.k = H.k;
-    R.m = H.m; R.n = H.n; R.kcap = H.cap;
-    rj.push_back(R);
-  } else {
-    const int m = H.ch[0]->m, n = H.ch[0]->n;
-    tile_add_lowrank(*H.ch[0], r0, c0, A, lda, B, ldb, k, cap, s, gj, rj);
-    tile_add_lowrank(*H.ch[1], r0, c0 + n, A, lda, B, ldb, k, cap, s, gj, rj);
-    tile_add_lowrank(*H.ch[2], r0 + m, c0, A, lda, B, ldb, k, cap, s, gj, rj);
-    tile_add_lowrank(*H.ch[3], r0 + m, c0 + n, A, lda, B, ldb, k, cap, s, gj, rj);
-  }
-}
-
 // ---------------------------------------------------------------------------
 // tile LU.  When every leaf outside the diagonal tiles (row group x column
 // group blocks) is one low-rank block covering its whole tile -- the
 // partition of the aca2 route with the identity adjacency -- the recursion of
 // lu! is carried out tile by tile (right-looking), which performs the same
-// operations with leaf-local pivoting but batches them: per step k the
-// diagonal tile is factorised by the recursion above, the whole row panel
-// (A factors of tiles (k, j>k)) and column panel (B factors of tiles (i>k, k))
-// are solved as one wide triangular solve each, every core B_ik' A_kj comes
+// operations with leaf-local pivoting but batches them.  The diagonal tiles
+// are held dense: their low-rank blocks (a few per cent of the matrix) are
+// expanded at load, so a step's update of a tile is one rank-k product instead
+// of a recompression per block, and its LU one kernel instead of a recursion of
+// about a hundred launches (8 leaves of 32 rows: 3.2 ms, now 0.1 ms); the
+// result is the same LU without the truncations inside the tile.  Per step k
+// the diagonal tile is factorised, the whole row panel (A factors of tiles
+// (k, j>k)) and column panel (B factors of tiles (i>k, k)) are solved as one
+// wide triangular solve each, every core B_ik' A_kj comes
 // out of one GEMM, and all updates of the trailing tiles run as one batched
 // product + one batched recompression.  Updates are truncated per step (the
 // recursion sums some products before truncating); both stay within
@@ -1423,7 +1325,7 @@ static void tile_add_lowrank(const Blk& H, int r0, int c0, const double* A, int6
 struct TileLU {
   int T = 0;
   std::vector<int64_t> start, size;      // tile ranges
-  std::vector<BP> diag;                  // diagonal tiles (H or dense)
+  std::vector<BP> diag;                  // diagonal tiles, dense
   std::vector<double*> Ap, Bp;           // row panels (m_i x T*cap), column panels (n_j x T*cap)
   int32_t* kmat = nullptr;               // ranks of the off-diagonal tiles, T x T
   BP hold;                               // owns the panel memory
@@ -1543,7 +1445,7 @@ __global__ void __launch_bounds__(128) lu_tile_core_kernel(TileJobArgs a, int rl
     if (threadIdx.x == 0) atomicOr(a.flags, 1);
     r = rl;
   }
-  TS* XA = sm + 3 * rl * rl;
+  TS* XA = sm + 3 * rl * (rl + 1);
   TS* XB = XA + (int64_t)smax * rl;
   for (int q = 0; q < r; ++q)
     for (int t = threadIdx.x; t < mi; t += blockDim.x)
@@ -1622,7 +1524,7 @@ static void recompress_tile_pairs(Ctx& c, const TileLU& TL, int k, int64_t R, co
     // fused path: the pairs' factors staged in shared memory, in FP32 when the
     // truncation tolerance is loose (>= 1e-6, the mixed-precision scheme)
     const bool f32 = c.eps_trunc >= MIXED_CORE_EPS;
-    const size_t smem = (f32 ? sizeof(float) : sizeof(double)) * ((size_t)3 * rl * rl + (size_t)2 * smax * rl);
+    const size_t smem = (f32 ? sizeof(float) : sizeof(double)) * ((size_t)3 * rl * (rl + 1) + (size_t)2 * smax * rl);
     if (smem <= 200 * 1024) {
       const void* kfn = f32 ? (const void*)lu_tile_core_kernel<float> : (const void*)lu_tile_core_kernel<double>;
       if (smem_attr(kfn, 200 * 1024) != cudaSuccess) throw LuError(HM_ERR_CUDA, "tile core smem");
@@ -1734,9 +1636,94 @@ static void tile_factor(Ctx& c, const hm_handle* h, TileLU& TL, const std::vecto
   if (cudaMemcpyAsync(TL.kmat, kh.data(), sizeof(int32_t) * T * T, cudaMemcpyHostToDevice, c.st) != cudaSuccess)
     throw LuError(HM_ERR_CUDA, "rank upload");
   cudaStreamSynchronize(c.st);       // kh leaves scope before the async copy otherwise
-  TL.diag.resize(T);
-  for (int i = 0; i < T; ++i) TL.diag[i] = build_tree(c, h, dnode[i], ld);
   ld.flush(c);
+  // the diagonal tiles: every leaf expanded into the dense tile, and the row
+  // ranges of the diagonal leaves (the pivots stay inside them)
+  TL.diag.resize(T);
+  std::vector<int32_t> leaf;                       // tile by tile: leaf starts, then the size
+  std::vector<int> leaf0(T), nleaf(T);
+  int mmax = 1, smax = 1;
+  {
+    const int deb = dense_elem_bytes(h->storage), dt = h->storage == HM_F64 ? HM_F64 : HM_F32;
+    std::vector<DiagLoad> jobs;
+    std::vector<std::pair<int64_t, int>> cuts;     // (first row, rows) of a tile's diagonal leaves
+    for (int i = 0; i < T; ++i) {
+      const int S = (int)TL.size[i];
+      smax = std::max(smax, S);
+      TL.diag[i] = new_dense(c, S, S, gcl[i], gcl[i]);
+      TL.diag[i]->row0 = TL.start[i];
+      cuts.clear();
+      std::vector<int32_t> todo(1, dnode[i]);
+      while (!todo.empty()) {
+        const Node& nd = h->nodes[todo.back()];
+        todo.pop_back();
+        if (nd.type == T_H) {
+          for (int q = 0; q < 4; ++q) todo.push_back(nd.child[q]);
+          continue;
+        }
+        const Leaf& L = h->leaves[nd.leaf];
+        DiagLoad J{};
+        J.m = L.m; J.n = L.n; J.k = L.k; J.dense = nd.type == T_DENSE; J.ctype = dt; J.rtype = h->storage;
+        J.dst = TL.diag[i]->C + (L.row0 - TL.start[i]) + (L.col0 - TL.start[i]) * (int64_t)S;
+        J.ldd = S;
+        if (J.dense) {
+          J.C = (const char*)h->d_dense + L.off * deb;
+          J.ldc = col_pad(L.m, deb);
+        } else {
+          const int64_t npad = col_pad(L.n, eb), mpad = col_pad(L.m, eb);
+          J.B = base + L.off * eb;
+          J.ldb = npad;
+          J.A = base + (L.off + npad * L.k) * eb;
+          J.lda = mpad;
+        }
+        jobs.push_back(J);
+        if (nd.s == nd.t) {
+          if (!J.dense || L.m != L.n) throw LuError(HM_ERR_UNSUPPORTED, "H should not be a low-rank matrix");
+          cuts.push_back({L.row0 - TL.start[i], L.m});
+          mmax = std::max(mmax, L.m);
+        }
+      }
+      std::sort(cuts.begin(), cuts.end());
+      leaf0[i] = (int)leaf.size();
+      nleaf[i] = (int)cuts.size();
+      int64_t next = 0;
+      for (auto& q : cuts) {
+        if (q.first != next) throw LuError(HM_ERR_UNSUPPORTED, "diagonal leaves do not cover their tile");
+        leaf.push_back((int32_t)q.first);
+        next += q.second;
+      }
+      if (next != S) throw LuError(HM_ERR_UNSUPPORTED, "diagonal leaves do not cover their tile");
+      leaf.push_back(S);
+    }
+    if (mmax > 150) throw LuError(HM_ERR_UNSUPPORTED, "diagonal leaf above 150 rows (MinBlock too large)");
+    for (size_t b = 0; b < jobs.size(); b += (size_t)1 << 30) {
+      const size_t nb = std::min<size_t>((size_t)1 << 30, jobs.size() - b);
+      Blk tmp;
+      tmp.st = c.st;
+      std::vector<DiagLoad> part(jobs.begin() + b, jobs.begin() + b + nb);
+      lu_diag_load_kernel<<<dim3((unsigned)nb, 4), 256, 0, c.st>>>(upload_jobs(c, tmp, part));
+      LU_LAUNCH_CHECK();
+    }
+  }
+  int32_t* d_leaf = (int32_t*)dmalloc(c, *TL.hold, sizeof(int32_t) * leaf.size());
+  double** d_D = (double**)dmalloc(c, *TL.hold, sizeof(void*) * T);
+  {
+    std::vector<double*> D(T);
+    for (int i = 0; i < T; ++i) D[i] = TL.diag[i]->C;
+    if (cudaMemcpyAsync(d_leaf, leaf.data(), sizeof(int32_t) * leaf.size(), cudaMemcpyHostToDevice, c.st) != cudaSuccess ||
+        cudaMemcpyAsync(d_D, D.data(), sizeof(void*) * T, cudaMemcpyHostToDevice, c.st) != cudaSuccess ||
+        cudaStreamSynchronize(c.st) != cudaSuccess)
+      throw LuError(HM_ERR_CUDA, "diagonal tile tables");
+  }
+  // the LU kernel by the largest leaf
+  const void* diag_fn = mmax <= 32 ? (const void*)lu_diag_kernel<32> : mmax <= 64 ? (const void*)lu_diag_kernel<64>
+                                                                                : (const void*)lu_diag_kernel<160>;
+  const int M = mmax <= 32 ? 32 : mmax <= 64 ? 64 : 160;
+  const size_t diag_smem = M == 32 ? diag_lu_smem<32>() : M == 64 ? diag_lu_smem<64>() : diag_lu_smem<160>();
+  const bool panel_sm = tp_smem(smax) <= 220 * 1024;     // a panel's columns fit in shared memory
+  if (smem_attr(diag_fn, (int)diag_smem) != cudaSuccess ||
+      (panel_sm && smem_attr((const void*)lu_panel_kernel, 220 * 1024) != cudaSuccess))
+    throw LuError(HM_ERR_CUDA, "tile kernels smem");
 
   // Step k: the diagonal tile's LU and the panels (x: the stream they run on),
   // then the trailing update.  With a look-ahead stream, the LU and panels of
@@ -1745,14 +1732,24 @@ static void tile_factor(Ctx& c, const hm_handle* h, TileLU& TL, const std::vecto
   auto panels = [&](Ctx& x, int k, StepQ& out) {
     const int mk = (int)TL.size[k];
     const int R = (T - k - 1) * cap;
-    lu_rec(x, *TL.diag[k]);
+    DiagLu dl{TL.diag[k]->C, mk, nleaf[k], d_leaf + leaf0[k], x.P, TL.start[k], x.flags};
+    if (M == 32) lu_diag_kernel<32><<<DL_CTAS, 32 * DL_WARPS, diag_smem, x.st>>>(dl);
+    else if (M == 64) lu_diag_kernel<64><<<DL_CTAS, 32 * DL_WARPS, diag_smem, x.st>>>(dl);
+    else lu_diag_kernel<160><<<DL_CTAS, 32 * DL_WARPS, diag_smem, x.st>>>(dl);
+    LU_LAUNCH_CHECK();
     if (k > 0) laswp(x, View{TL.Ap[k], 1, mk, mk, k * cap}, TL.start[k]);
     if (R == 0) return;
     View Ua{TL.Ai(k, k + 1, cap), 1, mk, mk, R};          // A factors of tiles (k, j>k)
     View Lb{TL.Bj(k + 1, k, cap), 1, mk, mk, R};          // B factors of tiles (i>k, k)
-    laswp(x, Ua, TL.start[k]);
-    mfs(x, *TL.diag[k], Ua, true, true);                  // L_kk^{-1} P_k A_kj
-    mfs(x, *TL.diag[k], vtr(Lb), false, false);           // B_ik' U_kk^{-1}
+    if (panel_sm) {                                       // L_kk^{-1} P_k A_kj and B_ik' U_kk^{-1}
+      PanelArgs pa{TL.diag[k]->C, mk, T, k, cap, x.P, TL.start[k], TL.Ap[k], TL.Bp[k], TL.kmat};
+      lu_panel_kernel<<<dim3((T - k - 1 + TP_TILES - 1) / TP_TILES, 2), 256, tp_smem(mk), x.st>>>(pa);
+      LU_LAUNCH_CHECK();
+    } else {
+      laswp(x, Ua, TL.start[k]);
+      mfs(x, *TL.diag[k], Ua, true, true);
+      mfs(x, *TL.diag[k], vtr(Lb), false, false);
+    }
     out.hold = std::make_shared<Blk>();
     out.hold->st = c.st;                                  // freed after the main stream used it
     Blk& hold = *out.hold;
@@ -1786,17 +1783,12 @@ static void tile_factor(Ctx& c, const hm_handle* h, TileLU& TL, const std::vecto
     for (auto& g : gq) big_tiles += (int64_t)((g.C.rows + GB_T - 1) / GB_T) * ((g.C.cols + GB_T - 1) / GB_T);
     gemm_batch(x, gq, macs >= 4.0e6 && big_tiles >= 148);
   };
-  // updates of the trailing diagonal tiles i in [i0, i1) (H-structured targets)
-  auto diag_updates = [&](int k, const StepQ& sq, int i0, int i1) {
-    std::vector<RcReq> rj;
-    std::vector<GemmJob> gd;
-    for (int i = i0; i < i1; ++i) {
-      const int mi = (int)TL.size[i];
-      const double* Qii = sq.Q[i] + (int64_t)(i - k - 1) * cap * mi;
-      tile_add_lowrank(*TL.diag[i], 0, 0, Qii, mi, TL.Bj(k, i, cap), mi, TL.kmat + k * T + i, cap, -1.0, gd, rj);
-    }
-    gemm_batch(c, gd);
-    recompress_batch(c, rj, 2 * cap, false);              // no read-back: keeps the host ahead
+  // updates of the trailing diagonal tiles i in [i0, i1)
+  auto diag_updates = [&](int k, int i0, int i1) {
+    if (i1 <= i0) return;
+    DiagUpdate du{TL.d_Ap, TL.d_Bp, d_D, TL.d_size, TL.kmat, T, cap, k, i0};
+    lu_diag_update_kernel<<<dim3((smax + 31) / 32, i1 - i0), 256, sizeof(double) * (cap * cap + 32 * cap), c.st>>>(du);
+    LU_LAUNCH_CHECK();
   };
   Ctx cl = c;
   cl.st = look;
@@ -1821,17 +1813,17 @@ static void tile_factor(Ctx& c, const hm_handle* h, TileLU& TL, const std::vecto
     const int rl = tile_rank_bound(c, TL, k, 2 * cap);
     StepQ next;
     if (look) {
-      diag_updates(k, cur, k + 1, k + 2);
+      diag_updates(k, k + 1, k + 2);
       recompress_tile_pairs(c, TL, k, R, cur.qbase, 2 * cap, 1, rl);   // tile row and column k+1
       if (cudaEventRecord(ev_up, c.st) != cudaSuccess || cudaStreamWaitEvent(look, ev_up, 0) != cudaSuccess)
         throw LuError(HM_ERR_CUDA, "look-ahead wait");
       panels(cl, k + 1, next);
       if (cudaEventRecord(ev_dn, look) != cudaSuccess) throw LuError(HM_ERR_CUDA, "look-ahead record");
       recompress_tile_pairs(c, TL, k, R, cur.qbase, 2 * cap, 2, rl);   // the rest
-      diag_updates(k, cur, k + 2, T);
+      diag_updates(k, k + 2, T);
       if (cudaStreamWaitEvent(c.st, ev_dn, 0) != cudaSuccess) throw LuError(HM_ERR_CUDA, "look-ahead join");
     } else {
-      diag_updates(k, cur, k + 1, T);
+      diag_updates(k, k + 1, T);
       recompress_tile_pairs(c, TL, k, R, cur.qbase, 2 * cap, 0, rl);
       panels(c, k + 1, next);
     }
@@ -2009,48 +2001,8 @@ __global__ void __launch_bounds__(SW_THREADS, 2) lu_sweep_kernel(SweepTab t, dou
   }
 }
 
-// dense copy of the factored diagonal tiles' leaves (dense or low-rank)
-struct DensJob {
-  double* dst;
-  int64_t ldd;
-  const double* C;
-  int64_t ldc;
-  const double* A;
-  int64_t lda;
-  const double* B;
-  int64_t ldb;
-  const int32_t* k;
-  int m, n, type;
-};
-__global__ void lu_densify_batch_kernel(const DensJob* __restrict__ jobs) {
-  const DensJob J = jobs[blockIdx.x];
-  const int k = J.type == T_RK ? *J.k : 0;
-  for (int64_t e = threadIdx.x; e < (int64_t)J.m * J.n; e += blockDim.x) {
-    const int i = (int)(e % J.m), j = (int)(e / J.m);
-    double v;
-    if (J.type == T_DENSE) {
-      v = J.C[i + (int64_t)j * J.ldc];
-    } else {
-      v = 0.0;
-      for (int q = 0; q < k; ++q) v = fma(J.A[i + (int64_t)q * J.lda], J.B[j + (int64_t)q * J.ldb], v);
-    }
-    J.dst[i + (int64_t)j * J.ldd] = v;
-  }
-}
-
-static void densify_jobs(const Blk& H, double* dst, int64_t ldd, std::vector<DensJob>& out) {
-  if (H.type == T_H) {
-    const int m = H.ch[0]->m, n = H.ch[0]->n;
-    densify_jobs(*H.ch[0], dst, ldd, out);
-    densify_jobs(*H.ch[1], dst + (int64_t)n * ldd, ldd, out);
-    densify_jobs(*H.ch[2], dst + m, ldd, out);
-    densify_jobs(*H.ch[3], dst + m + (int64_t)n * ldd, ldd, out);
-    return;
-  }
-  out.push_back(DensJob{dst, ldd, H.C, H.ldc, H.A, H.lda, H.B, H.ldb, H.k, H.m, H.n, H.type});
-}
-
-// Inverses of the unit-lower L (upper = 0) or the upper U (upper = 1) of the
+// The same inverses for tiles whose columns do not fit in shared memory, of the
+// unit-lower L (upper = 0) or the upper U (upper = 1) of the
 // packed S x S tiles D (column-major), one thread per column of the inverse,
 // written row-major to W (W[i*S + j] = inverse(i, j)) and column-major to Wc.
 // All threads of a tile run the same substitution, so the reads of D are
@@ -2099,20 +2051,11 @@ static void ensure_sweep(Ctx& c, TileLU& TL) {
   int smax = 0;
   std::vector<double*> D(T);
   std::vector<const double*> inv[4];         // Lc, Uc, Ur, Lr: the matrices of which = 0..3
-  std::vector<DensJob> jobs;
   for (int k = 0; k < T; ++k) {
     const int S = (int)TL.size[k];
     smax = std::max(smax, S);
-    D[k] = (double*)dmalloc(c, tmp, sizeof(double) * (size_t)S * S);
+    D[k] = TL.diag[k]->C;
     for (int w = 0; w < 4; ++w) inv[w].push_back((double*)dmalloc(c, *hold, sizeof(double) * (size_t)S * S));
-    densify_jobs(*TL.diag[k], D[k], S, jobs);
-  }
-  for (size_t b = 0; b < jobs.size(); b += 65535) {
-    const size_t nb = std::min<size_t>(65535, jobs.size() - b);
-    std::vector<DensJob> part(jobs.begin() + b, jobs.begin() + b + nb);
-    DensJob* dj = upload_jobs(c, tmp, part);
-    lu_densify_batch_kernel<<<(unsigned)nb, 256, 0, c.st>>>(dj);
-    LU_LAUNCH_CHECK();
   }
   std::vector<int32_t> sz(T);
   for (int k = 0; k < T; ++k) sz[k] = (int32_t)TL.size[k];
@@ -2133,14 +2076,28 @@ static void ensure_sweep(Ctx& c, TileLU& TL) {
     TL.d_size = (int32_t*)up(sz.data(), sizeof(int32_t) * T);
   }
   for (int w = 0; w < 4; ++w) TL.d_inv[w] = (const double**)up(inv[w].data(), sizeof(void*) * T);
-  const dim3 g((smax + 127) / 128, T);
   // L^-1: row-major (which 3) and column-major (which 0); U^-1: row-major (2), column-major (1)
-  lu_tri_inverse_kernel<<<g, 128, 0, c.st>>>(dD, (double* const*)TL.d_inv[3], (double* const*)TL.d_inv[0],
-                                             TL.d_size, 0);
-  LU_LAUNCH_CHECK();
-  lu_tri_inverse_kernel<<<g, 128, 0, c.st>>>(dD, (double* const*)TL.d_inv[2], (double* const*)TL.d_inv[1],
-                                             TL.d_size, 1);
-  LU_LAUNCH_CHECK();
+  if (tp_smem(smax) <= 220 * 1024) {
+    if (smem_attr((const void*)lu_inverse_kernel, 220 * 1024) != cudaSuccess) throw LuError(HM_ERR_CUDA, "inverse smem");
+    InverseArgs ia{dD, {(double* const*)TL.d_inv[0], (double* const*)TL.d_inv[1]},
+                   {(double* const*)TL.d_inv[3], (double* const*)TL.d_inv[2]}, TL.d_size};
+    for (int t = 0; t < T; t += 65535) {       // grid.y
+      InverseArgs b = ia;
+      for (int w = 0; w < 2; ++w) { b.C[w] += t; b.R[w] += t; }
+      b.D += t;
+      b.size += t;
+      lu_inverse_kernel<<<dim3((smax + TP_COLS - 1) / TP_COLS, std::min(65535, T - t), 2), 256, tp_smem(smax), c.st>>>(b);
+      LU_LAUNCH_CHECK();
+    }
+  } else {
+    const dim3 g((smax + 127) / 128, T);
+    lu_tri_inverse_kernel<<<g, 128, 0, c.st>>>(dD, (double* const*)TL.d_inv[3], (double* const*)TL.d_inv[0],
+                                               TL.d_size, 0);
+    LU_LAUNCH_CHECK();
+    lu_tri_inverse_kernel<<<g, 128, 0, c.st>>>(dD, (double* const*)TL.d_inv[2], (double* const*)TL.d_inv[1],
+                                               TL.d_size, 1);
+    LU_LAUNCH_CHECK();
+  }
   if (cudaStreamSynchronize(c.st) != cudaSuccess) throw LuError(HM_ERR_CUDA, "sweep set-up");
   TL.sweep_hold = hold;
 }
