@@ -13,16 +13,13 @@ namespace hm {
 // A' = Q_A U_k, B' = Q_B V_k S_k.  One CTA per job; smem 3 rmax (rmax + 1)
 // doubles.
 // ===========================================================================
-// Columns [0, j0) are already orthonormal and their block of Rm is set by the
-// caller (cgs2_qr zeroes the rest of Rm first).
 template <typename TS>
 static __device__ void cgs2_qr(TS* X, int len, int ld, int r, TS* Rm /* r x r, col-major */,
-                        TS* proj /* r */, double* red, int j0 = 0) {
-  for (int e = threadIdx.x; e < r * r; e += blockDim.x)
-    if (!(e % r < j0 && e / r < j0)) Rm[e] = 0.0;
+                        TS* proj /* r */, double* red) {
+  for (int e = threadIdx.x; e < r * r; e += blockDim.x) Rm[e] = 0.0;
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int j = j0; j < r; ++j) {
+  for (int j = 0; j < r; ++j) {
     TS* xj = X + (int64_t)j * ld;
     for (int pass = 0; pass < 2; ++pass) {
       for (int i = w; i < j; i += nw) {
@@ -99,49 +96,63 @@ __device__ __forceinline__ void jacobi_angle(float al, float be, float ga, float
 
 // One-sided Jacobi on the r <= 16 columns of W (r x r, column stride lw) and
 // of V by ONE warp: 4 lanes a column pair, 4 rows a lane in registers, so that
-// a round is eight pairs at once and needs no block barrier.
+// a round is eight pairs at once and needs no block barrier.  A pair is rotated
+// while its cosine exceeds thr, unless one of its columns is below neg times
+// the largest column of W: what that column holds is truncated and moves the
+// singular values by less than neg.  (A core has about as many such columns as
+// it keeps, rounding noise that takes twice the sweeps to put in order.)  Ends
+// when a whole sweep's rounds in a row rotated nothing.
 template <typename TS>
-static __device__ void jacobi_warp16(TS* W, TS* V, int r, int lw, TS thr) {
+static __device__ void jacobi_warp16(TS* W, TS* V, int r, int lw, TS thr, TS neg) {
   const int lane = threadIdx.x & 31, sg = lane >> 2, sl = lane & 3;
-  const int rr = (r + 1) & ~1;
+  const int rr = (r + 1) & ~1, np = rr - 1;              // columns (even), rounds of a sweep
   const TS thr2 = thr * thr;
-  for (int sweep = 0; sweep < 60; ++sweep) {
-    bool rot = false;
-    for (int round = 0; round < rr - 1; ++round) {
-      auto posv = [&](int q) { return q == 0 ? 0 : 1 + (q - 1 + round) % (rr - 1); };
-      int p = 0, q = 0;
-      bool act = sg < rr / 2;
-      if (act) {
-        p = posv(sg); q = posv(rr - 1 - sg);
-        if (p > q) { const int t = p; p = q; q = t; }
-        act = q < r;
-      }
-      TS *wp = W + p * lw, *wq = W + q * lw, *vp = V + p * lw, *vq = V + q * lw;
-      TS x[4], y[4], u[4], v[4];
-      TS al = 0, be = 0, ga = 0;
+  TS big = 0;                                            // the largest squared column norm, times neg^2
+  if (lane < r)
+    for (int t = 0; t < r; ++t) big = fma(W[t + lane * lw], W[t + lane * lw], big);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int t = sl + 4 * i;
-        const bool in = act && t < r;
-        x[i] = in ? wp[t] : (TS)0;
-        y[i] = in ? wq[t] : (TS)0;
-        u[i] = in ? vp[t] : (TS)0;
-        v[i] = in ? vq[t] : (TS)0;
-      }
+  for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
+  big *= neg * neg;
+  // tournament pairing: place 0 stays, the others move one on every round
+  int a = sg, b = np - sg;
+  const bool in_play = sg < rr / 2;
+  for (int round = 0, quiet = 0; round < 60 * np && quiet < np; ++round) {
+    const int p = min(a, b), q = max(a, b);
+    const bool act = in_play && q < r;
+    TS *wp = W + p * lw, *wq = W + q * lw;
+    TS x[4], y[4];
+    TS al = 0, be = 0, ga = 0;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        al = fma(x[i], x[i], al);
-        be = fma(y[i], y[i], be);
-        ga = fma(x[i], y[i], ga);
-      }
+    for (int i = 0; i < 4; ++i) {
+      const int t = sl + 4 * i;
+      const bool in = act && t < r;
+      x[i] = in ? wp[t] : (TS)0;
+      y[i] = in ? wq[t] : (TS)0;
+    }
 #pragma unroll
-      for (int o = 2; o > 0; o >>= 1) {
-        al += __shfl_xor_sync(0xffffffffu, al, o);
-        be += __shfl_xor_sync(0xffffffffu, be, o);
-        ga += __shfl_xor_sync(0xffffffffu, ga, o);
-      }
-      if (act && ga != (TS)0 && ga * ga > thr2 * al * be) {
-        TS c, s;
+    for (int i = 0; i < 4; ++i) {
+      al = fma(x[i], x[i], al);
+      be = fma(y[i], y[i], be);
+      ga = fma(x[i], y[i], ga);
+    }
+#pragma unroll
+    for (int o = 2; o > 0; o >>= 1) {
+      al += __shfl_xor_sync(0xffffffffu, al, o);
+      be += __shfl_xor_sync(0xffffffffu, be, o);
+      ga += __shfl_xor_sync(0xffffffffu, ga, o);
+    }
+    const bool rot = act && fmin(al, be) > big && ga * ga > thr2 * al * be;
+    if (__any_sync(0xffffffffu, rot)) {
+      quiet = 0;
+      if (rot) {
+        TS *vp = V + p * lw, *vq = V + q * lw;
+        TS u[4], v[4], c, s;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int t = min(sl + 4 * i, r - 1);
+          u[i] = vp[t];
+          v[i] = vq[t];
+        }
         jacobi_angle(al, be, ga, c, s);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -153,11 +164,13 @@ static __device__ void jacobi_warp16(TS* W, TS* V, int r, int lw, TS thr) {
             vq[t] = s * u[i] + c * v[i];
           }
         }
-        rot = true;
       }
       __syncwarp();
+    } else {
+      ++quiet;
     }
-    if (!__any_sync(0xffffffffu, rot)) break;
+    if (a != 0) a = a == np ? 1 : a + 1;
+    b = b == np ? 1 : b + 1;
   }
 }
 
@@ -211,32 +224,8 @@ static __device__ void core_body_t(const CoreJob& J, TS* __restrict__ JA, TS* __
     if (threadIdx.x == 0) *J.rank = 0;
     return;
   }
-  const int ok = min(J.ortho_k, r);
-  if (ok > 0) {
-    // A's leading columns are orthonormal: R_A = I there.  B's are orthogonal:
-    // normalise them, R_B = diag(norms).
-    for (int e = threadIdx.x; e < ok * ok; e += blockDim.x) {
-      const int i = e % ok, j = e / ok;
-      b0[i + j * r] = (i == j) ? 1.0 : 0.0;
-      b1[i + j * r] = 0.0;
-    }
-    for (int j = w; j < ok; j += nw) {
-      TS s = 0;
-      for (int t = lane; t < J.n; t += 32) s = fma(JB[t + (int64_t)j * J.ldb], JB[t + (int64_t)j * J.ldb], s);
-      s = warp_sum(s);
-      if (lane == 0) proj[j] = sqrt(s);
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < J.n * ok; e += blockDim.x) {
-      const int t = e % J.n, j = e / J.n;
-      const TS nj = proj[j];
-      JB[t + (int64_t)j * J.ldb] = nj > (TS)0 ? JB[t + (int64_t)j * J.ldb] / nj : (TS)0;
-    }
-    if (threadIdx.x < ok) b1[threadIdx.x + threadIdx.x * r] = proj[threadIdx.x];
-    __syncthreads();
-  }
-  cgs2_qr(JA, J.m, J.lda, r, b0, proj, red, ok);
-  cgs2_qr(JB, J.n, J.ldb, r, b1, proj, red, ok);
+  cgs2_qr(JA, J.m, J.lda, r, b0, proj, red);
+  cgs2_qr(JB, J.n, J.ldb, r, b1, proj, red);
   // W = R_A R_B^T  (r x r, column-major; JAC8: an odd column stride, whose
   // columns start in different banks)
   const int lw = JAC8 ? r | 1 : r;
@@ -267,7 +256,7 @@ static __device__ void core_body_t(const CoreJob& J, TS* __restrict__ JA, TS* __
   const int rr = (r + 1) & ~1;
   const TS thr = (TS)fmax(sizeof(TS) == 8 ? 1e-15 : 1e-7, 1e-3 * eps_trunc);
   if (JAC8 && r <= 16) {
-    if (w == 0) jacobi_warp16(b2, b0, r, lw, thr);
+    if (w == 0) jacobi_warp16(b2, b0, r, lw, thr, (TS)(1e-3 * eps_trunc));
     __syncthreads();
   } else
   for (int sweep = 0; sweep < 60; ++sweep) {

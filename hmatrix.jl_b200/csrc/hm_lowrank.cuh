@@ -120,8 +120,6 @@ struct CoreJob {
   int32_t zero_fill;       // zero the output columns [k, kcap)
   int32_t known_zero;      // the output's columns [zero_from, kcap) are zero already:
   int32_t zero_from;       // zero_fill stops there (writes only what changes)
-  int32_t ortho_k;         // the first ortho_k columns of A are orthonormal and those of B
-                           // mutually orthogonal (a previous core's output): no QR for them
 };
 
 // Fully pivoted ACA job (deps/src/ACA_FullyPivoted.cpp:9-151).  rel_mode: the

@@ -15,6 +15,7 @@
 #include "hm_lowrank.cuh"
 #include "hm_core.cuh"
 #include "hm_lu_tile.cuh"
+#include "hm_lu_pair.cuh"
 
 
 #include <algorithm>
@@ -192,13 +193,6 @@ __device__ __forceinline__ void gemm_big_tile(const View& A, const View& B, cons
 __global__ void __launch_bounds__(256) lu_gemm_big_kernel(View A, View B, View C, double alpha, double beta) {
   gemm_big_tile(A, B, C, alpha, beta, blockIdx.y * GB_T, blockIdx.x * GB_T);
 }
-__global__ void __launch_bounds__(256) lu_gemm_big_batch_kernel(const GemmJob* __restrict__ jobs) {
-  const GemmJob& J = jobs[blockIdx.z];
-  const int i0 = blockIdx.y * GB_T, j0 = blockIdx.x * GB_T;
-  if (i0 >= J.C.rows || j0 >= J.C.cols) return;
-  gemm_big_tile(J.A, J.B, J.C, J.alpha, J.beta, i0, j0);
-}
-
 // Y = alpha * X + beta * Y (beta == 0: Y is not read)
 __global__ void lu_axpby_kernel(View Y, View X, double alpha, double beta) {
   const int64_t tot = (int64_t)Y.rows * Y.cols;
@@ -460,18 +454,6 @@ __device__ void gather_pieces(const GatherArgs& g) {
 
 __global__ void lu_copy_int_kernel(int32_t* dst, const int32_t* src) { *dst = *src; }
 
-__global__ void lu_max_int_kernel(const int32_t* __restrict__ v, int n, int32_t* __restrict__ out) {
-  __shared__ int32_t red[256];
-  int32_t m = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) m = max(m, v[i]);
-  red[threadIdx.x] = m;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) red[threadIdx.x] = max(red[threadIdx.x], red[threadIdx.x + s]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *out = red[0];
-}
 __global__ void lu_set_int_kernel(int32_t* dst, int v) { *dst = v; }
 
 template <typename T>
@@ -1202,106 +1184,26 @@ struct Loader {
 static BP build_tree(Ctx& c, const hm_handle* h, int32_t node, Loader& ld);
 static BP build_from_handle(Ctx& c, const hm_handle* h, int32_t node);
 
-// independent products in one launch; big = true: 128 x 128 tiles
-static void gemm_batch(Ctx& c, const std::vector<GemmJob>& jobs, bool big = false) {
+// independent products in one launch
+static void gemm_batch(Ctx& c, const std::vector<GemmJob>& jobs) {
   if (jobs.empty()) return;
-  const int t = big ? GB_T : 32;
   int gx = 1, gy = 1;
   for (auto& j : jobs) {
-    gx = std::max(gx, (j.C.cols + t - 1) / t);
-    gy = std::max(gy, (j.C.rows + t - 1) / t);
+    gx = std::max(gx, (j.C.cols + 31) / 32);
+    gy = std::max(gy, (j.C.rows + 31) / 32);
   }
   for (size_t b = 0; b < jobs.size(); b += 65535) {
     const size_t nb = std::min<size_t>(65535, jobs.size() - b);
     Blk tmp;
     tmp.st = c.st;
     std::vector<GemmJob> part(jobs.begin() + b, jobs.begin() + b + nb);
-    GemmJob* d = upload_jobs(c, tmp, part);
-    if (big) lu_gemm_big_batch_kernel<<<dim3(gx, gy, (unsigned)nb), 256, 0, c.st>>>(d);
-    else lu_gemm_batch_kernel<<<dim3(gx, gy, (unsigned)nb), 256, 0, c.st>>>(d);
+    lu_gemm_batch_kernel<<<dim3(gx, gy, (unsigned)nb), 256, 0, c.st>>>(upload_jobs(c, tmp, part));
     LU_LAUNCH_CHECK();
   }
 }
 
-// The off-diagonal part of step k's trailing update, generated on the device:
-// for every pair i != j of trailing tiles, A_ij B_ij' - Q_ij B_kj' is gathered
-// into one [A | -Q] [B | B_kj] pair and recompressed (Q_ij = A_ik W_kj, the
-// panel product of step k).  Job q of the batch is pair (ii, jj) of the
-// trailing tiles with the diagonal skipped; its scratch is a fixed stride.
-// Pair q of the trailing update of step k: mode 0 every pair i != j of the
-// tiles (k, T); mode 1 the pairs of tile row and tile column k+1; mode 2 the
-// pairs among the tiles (k+1, T).
-__device__ __forceinline__ void tile_pair(int T, int k, int mode, int64_t gq, int& i, int& j) {
-  if (mode == 1) {
-    const int n1 = T - k - 2;
-    if (gq < n1) { i = k + 1; j = k + 2 + (int)gq; }
-    else { i = k + 2 + (int)(gq - n1); j = k + 1; }
-    return;
-  }
-  const int base = mode == 2 ? k + 2 : k + 1;
-  const int Tr = T - base;
-  const int ii = (int)(gq / (Tr - 1));
-  int jj = (int)(gq % (Tr - 1));
-  if (jj >= ii) ++jj;
-  i = base + ii;
-  j = base + jj;
-}
-static int64_t tile_pair_count(int T, int k, int mode) {
-  const int64_t Tr = T - k - 1;
-  if (mode == 0) return Tr * (Tr - 1);
-  if (mode == 1) return Tr >= 2 ? 2 * (Tr - 1) : 0;
-  return Tr >= 2 ? (Tr - 1) * (Tr - 2) : 0;
-}
-
 // truncation tolerance from which the tile recompressions run in FP32
 constexpr double MIXED_CORE_EPS = 1e-6;
-
-struct TileJobArgs {
-  const double* const* Ap;
-  const double* const* Bp;
-  const int64_t* start;
-  const int32_t* size;
-  int32_t* kmat;
-  int T, cap, k, rmax;
-  int64_t R;                 // (T-k-1) cap: columns of a Q panel row
-  const double* qbase;       // Q_i = qbase + (start[i] - start[k+1]) R
-  double* scratch;
-  int64_t stride;            // scratch doubles per job
-  int32_t* rr;               // gathered rank per job
-  int* flags;
-  CoreJob* cj;
-  int64_t q0;                // first job of this batch
-  int mode;                  // which pairs (tile_pair)
-};
-__global__ void __launch_bounds__(256) lu_tile_gather_kernel(TileJobArgs a) {
-  const int64_t q = blockIdx.x;
-  const int64_t gq = a.q0 + q;
-  int i, j;
-  tile_pair(a.T, a.k, a.mode, gq, i, j);
-  const int mi = a.size[i], nj = a.size[j];
-  const double* Qi = a.qbase + (a.start[i] - a.start[a.k + 1]) * a.R;
-  double* Aij = const_cast<double*>(a.Ap[i]) + (int64_t)j * a.cap * mi;
-  double* Bij = const_cast<double*>(a.Bp[j]) + (int64_t)i * a.cap * nj;
-  GatherArgs g{};
-  g.pc[0] = Piece{Aij, mi, Bij, nj, a.kmat + i * a.T + j, mi, nj, 0, 0, 1.0};
-  g.pc[1] = Piece{Qi + (int64_t)(j - a.k - 1) * a.cap * mi, mi, a.Bp[j] + (int64_t)a.k * a.cap * nj, nj,
-                  a.kmat + a.k * a.T + j, mi, nj, 0, 0, -1.0};
-  g.np = 2;
-  g.SA = a.scratch + q * a.stride;
-  g.SB = g.SA + (int64_t)mi * a.rmax;
-  g.M = mi; g.N = nj; g.rmax = a.rmax;
-  g.r_out = a.rr + q;
-  g.flags = a.flags;
-  if (threadIdx.x == 0) {
-    CoreJob J{};
-    J.A = g.SA; J.B = g.SB; J.outA = Aij; J.outB = Bij;
-    J.m = mi; J.n = nj; J.lda = max(mi, 1); J.ldb = max(nj, 1);
-    J.ldoa = mi; J.ldob = nj; J.kcap = a.cap;
-    J.zero_test = 1; J.rank = a.kmat + i * a.T + j; J.r_dev = g.r_out; J.zero_fill = 1;
-    a.cj[q] = J;
-  }
-  gather_pieces(g);
-}
 
 // ---------------------------------------------------------------------------
 // tile LU.  When every leaf outside the diagonal tiles (row group x column
@@ -1316,9 +1218,8 @@ __global__ void __launch_bounds__(256) lu_tile_gather_kernel(TileJobArgs a) {
 // result is the same LU without the truncations inside the tile.  Per step k
 // the diagonal tile is factorised, the whole row panel (A factors of tiles
 // (k, j>k)) and column panel (B factors of tiles (i>k, k)) are solved as one
-// wide triangular solve each, every core B_ik' A_kj comes
-// out of one GEMM, and all updates of the trailing tiles run as one batched
-// product + one batched recompression.  Updates are truncated per step (the
+// wide triangular solve each, and every pair of trailing tiles is updated and
+// recompressed by one CTA that forms its core B_ik' A_kj itself.  Updates are truncated per step (the
 // recursion sums some products before truncating); both stay within
 // eps_trunc of the exact Schur complement.
 // ---------------------------------------------------------------------------
@@ -1421,157 +1322,72 @@ static bool tile_structure(const hm_handle* h, std::vector<int32_t>& gcl, std::v
   return false;
 }
 
-// The same update with the gather fused into the recompression: the CTA
-// loads [A_ij | -Q_ij] and [B_ij | B_kj] into shared memory (rl columns at
-// most, smax rows) and runs the QR + SVD core there.
-// TS: the precision of the staged factors and of the QR + SVD core (FP32 when
-// the truncation tolerance is loose: the mixed-precision factorisation)
+// The recompressions of step k's pairs (tile_pair's mode), every launch sized
+// without knowing a rank: first all pairs by the register kernel, whose pairs
+// of larger rank go on a list for the next kernel, to the last one, which
+// takes any rank the capacity allows.  ws: the lists and their counts.
+struct PairLists {
+  int32_t* list[3];          // [T (T - 1)] each
+  int* count;                // [8]
+  void* scratch;             // of the last kernel: blocks x 2 smax rl
+  int smax, blocks;
+};
 template <typename TS>
-__global__ void __launch_bounds__(128) lu_tile_core_kernel(TileJobArgs a, int rl, int smax, double eps_trunc) {
-  extern __shared__ double sm_raw[];
-  TS* sm = reinterpret_cast<TS*>(sm_raw);
-  const int64_t gq = a.q0 + blockIdx.x;
-  int i, j;
-  tile_pair(a.T, a.k, a.mode, gq, i, j);
-  const int mi = a.size[i], nj = a.size[j];
-  const double* Qij = a.qbase + (a.start[i] - a.start[a.k + 1]) * a.R + (int64_t)(j - a.k - 1) * a.cap * mi;
-  double* Aij = const_cast<double*>(a.Ap[i]) + (int64_t)j * a.cap * mi;
-  double* Bij = const_cast<double*>(a.Bp[j]) + (int64_t)i * a.cap * nj;
-  const double* Bkj = a.Bp[j] + (int64_t)a.k * a.cap * nj;
-  int32_t* kij = a.kmat + i * a.T + j;
-  const int k1 = *kij, k2 = a.kmat[a.k * a.T + j];
-  int r = k1 + k2;
-  if (r > rl) {                      // cannot happen: rl bounds every pair of the step
-    if (threadIdx.x == 0) atomicOr(a.flags, 1);
-    r = rl;
-  }
-  TS* XA = sm + 3 * rl * (rl + 1);
-  TS* XB = XA + (int64_t)smax * rl;
-  for (int q = 0; q < r; ++q)
-    for (int t = threadIdx.x; t < mi; t += blockDim.x)
-      XA[t + q * mi] = (TS)(q < k1 ? Aij[t + (int64_t)q * mi] : -Qij[t + (int64_t)(q - k1) * mi]);
-  for (int q = 0; q < r; ++q)
-    for (int t = threadIdx.x; t < nj; t += blockDim.x)
-      XB[t + q * nj] = (TS)(q < k1 ? Bij[t + (int64_t)q * nj] : Bkj[t + (int64_t)(q - k1) * nj]);
-  __syncthreads();
-  CoreJob J{};
-  J.outA = Aij; J.outB = Bij;
-  J.m = mi; J.n = nj; J.r = r; J.lda = max(mi, 1); J.ldb = max(nj, 1);
-  J.ldoa = mi; J.ldob = nj; J.kcap = a.cap;
-  J.zero_test = 1; J.rank = kij; J.zero_fill = 1;
-  // the tile's columns at and beyond its previous rank k1 are zero: only the
-  // columns [k, k1) a smaller new rank frees need zeros
-  J.known_zero = 1; J.zero_from = k1;
-  // from step 1 on, every trailing tile (and tile (k, j)) is a previous step's
-  // core output: A_ij orthonormal, B_ij and B_kj with orthogonal columns
-  J.ortho_k = a.k >= 1 ? k1 : 0;
-  core_body_t<TS, true>(J, XA, XB, rl, eps_trunc, a.flags);
-}
-
-// an upper bound of rank(A_ij) + rank(B_kj) over the trailing pairs of step k
-__global__ void lu_tile_rank_bound_kernel(const int32_t* __restrict__ kmat, int T, int k, int32_t* out) {
-  __shared__ int32_t red[256];
-  int32_t m1 = 0, m2 = 0;
-  const int Tr = T - k - 1;
-  for (int e = threadIdx.x; e < Tr * Tr; e += blockDim.x) {
-    const int i = k + 1 + e / Tr, j = k + 1 + e % Tr;
-    if (i != j) m1 = max(m1, kmat[i * T + j]);
-  }
-  for (int j = k + 1 + threadIdx.x; j < T; j += blockDim.x) m2 = max(m2, kmat[k * T + j]);
-  red[threadIdx.x] = m1;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) red[threadIdx.x] = max(red[threadIdx.x], red[threadIdx.x + s]);
-    __syncthreads();
-  }
-  const int32_t a1 = red[0];
-  __syncthreads();
-  red[threadIdx.x] = m2;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) red[threadIdx.x] = max(red[threadIdx.x], red[threadIdx.x + s]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *out = a1 + red[0];
-}
-
-// the launch size of step k's recompression cores: a bound of rank(A_ij) +
-// rank(B_kj) over its pairs, read back once per step
-static int tile_rank_bound(Ctx& c, const TileLU& TL, int k, int rmax) {
-  Blk tmp;
-  tmp.st = c.st;
-  int32_t* dmax = (int32_t*)dmalloc(c, tmp, sizeof(int32_t));
-  lu_tile_rank_bound_kernel<<<1, 256, 0, c.st>>>(TL.kmat, TL.T, k, dmax);
-  LU_LAUNCH_CHECK();
-  int32_t hb = 0;
-  if (cudaMemcpyAsync(&hb, dmax, sizeof(int32_t), cudaMemcpyDeviceToHost, c.st) != cudaSuccess ||
-      cudaStreamSynchronize(c.st) != cudaSuccess)
-    throw LuError(HM_ERR_CUDA, "rank bound read-back");
-  return std::min(std::min(std::max(rmax, 1), RCORE_MAX), std::max(8, (hb + 7) / 8 * 8));
-}
-
-static void recompress_tile_pairs(Ctx& c, const TileLU& TL, int k, int64_t R, const double* qbase, int rmax,
-                                  int mode, int rl) {
+static void recompress_pairs_t(Ctx& c, const TileLU& TL, const PairLists& W, int k, int mode) {
   const int T = TL.T;
   const int64_t njobs = tile_pair_count(T, k, mode);
   if (njobs <= 0) return;
-  rmax = std::min(std::max(rmax, 1), RCORE_MAX);
-  int64_t smax = 1;
-  for (int i = k + 1; i < T; ++i) smax = std::max<int64_t>(smax, TL.size[i]);
-  Blk tmp;
-  tmp.st = c.st;
-  {
-    // fused path: the pairs' factors staged in shared memory, in FP32 when the
-    // truncation tolerance is loose (>= 1e-6, the mixed-precision scheme)
-    const bool f32 = c.eps_trunc >= MIXED_CORE_EPS;
-    const size_t smem = (f32 ? sizeof(float) : sizeof(double)) * ((size_t)3 * rl * (rl + 1) + (size_t)2 * smax * rl);
-    if (smem <= 200 * 1024) {
-      const void* kfn = f32 ? (const void*)lu_tile_core_kernel<float> : (const void*)lu_tile_core_kernel<double>;
-      if (smem_attr(kfn, 200 * 1024) != cudaSuccess) throw LuError(HM_ERR_CUDA, "tile core smem");
-      for (int64_t q0 = 0; q0 < njobs; q0 += INT32_MAX) {
-        const int64_t nb = std::min<int64_t>(INT32_MAX, njobs - q0);
-        TileJobArgs a{TL.d_Ap, TL.d_Bp, TL.d_start, TL.d_size, TL.kmat, T, c.cap, k, rmax, R, qbase, nullptr, 0,
-                      nullptr, c.flags, nullptr, q0, mode};
-        if (f32) lu_tile_core_kernel<float><<<(unsigned)nb, 128, smem, c.st>>>(a, rl, (int)smax, c.eps_trunc);
-        else lu_tile_core_kernel<double><<<(unsigned)nb, 128, smem, c.st>>>(a, rl, (int)smax, c.eps_trunc);
-        LU_LAUNCH_CHECK();
-      }
-      return;
-    }
+  if (njobs > INT32_MAX) throw LuError(HM_ERR_UNSUPPORTED, "too many tile pairs");
+  HM_LU_CUDA(cudaMemsetAsync(W.count, 0, 8 * sizeof(int), c.st));
+  PairArgs a{};
+  a.Ap = (double* const*)TL.d_Ap; a.Bp = (double* const*)TL.d_Bp; a.size = TL.d_size; a.kmat = TL.kmat;
+  a.T = T; a.cap = c.cap; a.k = k; a.mode = mode; a.eps = c.eps_trunc; a.flags = c.flags;
+  a.out = W.list[0]; a.nout = W.count;
+  auto next = [&](int i) {             // the list just written becomes the input
+    a.in = W.list[i]; a.nin = W.count + i;
+    a.out = i < 2 ? W.list[i + 1] : nullptr; a.nout = i < 2 ? W.count + i + 1 : nullptr;
+  };
+  const unsigned pers = (unsigned)std::min<int64_t>(njobs, 148 * 4);
+  if (W.smax <= 256) {
+    lu_pair_kernel<TS, 1, 8><<<(unsigned)njobs, 64, 0, c.st>>>(a);
+    LU_LAUNCH_CHECK();
+    next(0);
+    lu_pair_kernel<TS, 1, 12><<<pers, 64, 0, c.st>>>(a);
+  } else {
+    lu_pair_kernel<TS, 2, 8><<<(unsigned)njobs, 128, 0, c.st>>>(a);
+    LU_LAUNCH_CHECK();
+    next(0);
+    lu_pair_kernel<TS, 2, 12><<<pers, 128, 0, c.st>>>(a);
   }
-  const int64_t stride = 2 * smax * rmax;
-  const int64_t per = std::max<int64_t>(1, std::min<int64_t>(((int64_t)1 << 28) / stride, 65535));
-  const int64_t nb0 = std::min(per, njobs);
-  double* scratch = (double*)dmalloc(c, tmp, sizeof(double) * (size_t)(nb0 * stride));
-  int32_t* rr = (int32_t*)dmalloc(c, tmp, sizeof(int32_t) * (size_t)nb0);
-  CoreJob* cj = (CoreJob*)dmalloc(c, tmp, sizeof(CoreJob) * (size_t)nb0);
-  int32_t* dmax = (int32_t*)dmalloc(c, tmp, sizeof(int32_t));
-  for (int64_t q0 = 0; q0 < njobs; q0 += per) {
-    const int64_t nb = std::min(per, njobs - q0);
-    TileJobArgs a{TL.d_Ap, TL.d_Bp, TL.d_start, TL.d_size, TL.kmat, T, c.cap, k, rmax, R, qbase, scratch, stride,
-                  rr, c.flags, cj, q0, mode};
-    lu_tile_gather_kernel<<<(unsigned)nb, 256, 0, c.st>>>(a);
+  LU_LAUNCH_CHECK();
+  next(1);
+  // up to 24 columns of 256 rows, or what else fits twice on an SM, staged in
+  // shared memory; the rest in scratch
+  const int rl = (int)std::min<size_t>(24, (104 * 1024 / sizeof(TS) - c.cap * c.cap) / (2 * W.smax + 3 * 25));
+  const int rmax = std::min(2 * c.cap, RCORE_MAX);
+  auto smem = [&](int q, bool staged) {
+    return sizeof(TS) * ((size_t)3 * q * (q + 1) + (staged ? (size_t)2 * W.smax * q + c.cap * c.cap : 0));
+  };
+  if (smem_attr((const void*)lu_tile_core_kernel<TS>, (int)sizeof(double) * 3 * RCORE_MAX * (RCORE_MAX + 1)) != cudaSuccess)
+    throw LuError(HM_ERR_CUDA, "tile core smem");
+  if (rl > 12) {
+    lu_tile_core_kernel<TS><<<std::min<unsigned>(pers, 148 * 2), 128, smem(rl, true), c.st>>>(a, rl, W.smax, (TS*)nullptr);
     LU_LAUNCH_CHECK();
-    lu_max_int_kernel<<<1, 256, 0, c.st>>>(rr, (int)nb, dmax);
+    next(2);
+  } else {
+    a.out = nullptr;
+  }
+  if (rmax > std::max(rl, 12)) {
+    lu_tile_core_kernel<TS><<<std::min<unsigned>(pers, (unsigned)W.blocks), 128, smem(rmax, false), c.st>>>(
+        a, rmax, W.smax, (TS*)W.scratch);
     LU_LAUNCH_CHECK();
-    int32_t hmax = 0;
-    if (cudaMemcpyAsync(&hmax, dmax, sizeof(int32_t), cudaMemcpyDeviceToHost, c.st) != cudaSuccess ||
-        cudaStreamSynchronize(c.st) != cudaSuccess)
-      throw LuError(HM_ERR_CUDA, "core size read-back");
-    const int rlaunch = std::min(rmax, std::max(8, (hmax + 7) / 8 * 8));
-    int st = launch_core_recompress(cj, (int)nb, rlaunch, c.eps_trunc, c.flags, c.st, true);
-    if (st != HM_OK) throw LuError(st, "batched recompression launch");
   }
 }
-
-// Step k's products for the trailing update, kept until the update has run:
-// W = B_ik' A_kj for the whole panels and Q_i = A_ik W for every trailing tile
-// row (freed on the main stream).
-struct StepQ {
-  std::shared_ptr<Blk> hold;
-  double* qbase = nullptr;
-  std::vector<double*> Q;
-};
+static void recompress_pairs(Ctx& c, const TileLU& TL, const PairLists& W, int k, int mode) {
+  // FP32 when the truncation tolerance is loose (>= 1e-6, the mixed-precision scheme)
+  if (c.eps_trunc >= MIXED_CORE_EPS) recompress_pairs_t<float>(c, TL, W, k, mode);
+  else recompress_pairs_t<double>(c, TL, W, k, mode);
+}
 
 static void tile_factor(Ctx& c, const hm_handle* h, TileLU& TL, const std::vector<int32_t>& gcl,
                         const std::vector<int32_t>& dnode, cudaStream_t look) {
@@ -1729,7 +1545,7 @@ static void tile_factor(Ctx& c, const hm_handle* h, TileLU& TL, const std::vecto
   // then the trailing update.  With a look-ahead stream, the LU and panels of
   // tile k+1 run there as soon as step k has updated tile row and column k+1,
   // overlapping the rest of step k's update on the main stream.
-  auto panels = [&](Ctx& x, int k, StepQ& out) {
+  auto panels = [&](Ctx& x, int k) {
     const int mk = (int)TL.size[k];
     const int R = (T - k - 1) * cap;
     DiagLu dl{TL.diag[k]->C, mk, nleaf[k], d_leaf + leaf0[k], x.P, TL.start[k], x.flags};
@@ -1750,38 +1566,6 @@ static void tile_factor(Ctx& c, const hm_handle* h, TileLU& TL, const std::vecto
       mfs(x, *TL.diag[k], Ua, true, true);
       mfs(x, *TL.diag[k], vtr(Lb), false, false);
     }
-    out.hold = std::make_shared<Blk>();
-    out.hold->st = c.st;                                  // freed after the main stream used it
-    Blk& hold = *out.hold;
-    double* W = (double*)dmalloc(x, hold, sizeof(double) * (size_t)R * R);
-    View Wv{W, 1, R, R, R};
-    gemm(x, Wv, vtr(Lb), Ua, 1.0, 0.0);                   // W_ij = B_ik' A_kj
-    // Q_i = A_ik W_i,:   (m_i x R) for every trailing tile row i
-    std::vector<double*>& Q = out.Q;
-    Q.assign(T, nullptr);
-    int64_t qtot = 0;
-    for (int i = k + 1; i < T; ++i) qtot += TL.size[i] * (int64_t)R;
-    out.qbase = (double*)dmalloc(x, hold, sizeof(double) * (size_t)qtot);
-    int64_t qo = 0;
-    for (int i = k + 1; i < T; ++i) { Q[i] = out.qbase + qo; qo += TL.size[i] * (int64_t)R; }
-    // Q_i = A_ik W_i,: for every trailing tile row: one batched launch, with
-    // 128 x 128 tiles once the products are large
-    std::vector<GemmJob> gq;
-    double macs = 0.0;
-    for (int i = k + 1; i < T; ++i) {
-      const int mi = (int)TL.size[i];
-      GemmJob g{};
-      g.A = View{TL.Ai(i, k, cap), 1, mi, mi, cap};
-      g.B = vsub(Wv, (i - k - 1) * cap, 0, cap, R);
-      g.C = View{Q[i], 1, mi, mi, R};
-      g.alpha = 1.0; g.beta = 0.0;
-      gq.push_back(g);
-      macs += (double)mi * R * cap;
-    }
-    // 128 x 128 tiles when the batch fills the GPU with them
-    int64_t big_tiles = 0;
-    for (auto& g : gq) big_tiles += (int64_t)((g.C.rows + GB_T - 1) / GB_T) * ((g.C.cols + GB_T - 1) / GB_T);
-    gemm_batch(x, gq, macs >= 4.0e6 && big_tiles >= 148);
   };
   // updates of the trailing diagonal tiles i in [i0, i1)
   auto diag_updates = [&](int k, int i0, int i1) {
@@ -1805,29 +1589,34 @@ static void tile_factor(Ctx& c, const hm_handle* h, TileLU& TL, const std::vecto
       if (b) cudaEventDestroy(b);
     }
   } evg{ev_up, ev_dn, look};
-  StepQ cur;
-  panels(c, 0, cur);
-  for (int k = 0; k < T; ++k) {
-    const int R = (T - k - 1) * cap;
-    if (R == 0) break;
-    const int rl = tile_rank_bound(c, TL, k, 2 * cap);
-    StepQ next;
+  // lists of the pairs each recompression kernel leaves to the next, and the
+  // last one's scratch
+  Blk wsb;
+  wsb.st = c.st;
+  PairLists ws{};
+  ws.smax = smax;
+  const size_t per = sizeof(double) * ((size_t)2 * smax * std::min(2 * cap, RCORE_MAX) + cap * cap);
+  ws.blocks = (int)std::max<size_t>(16, std::min<size_t>(148 * 2, ((size_t)256 << 20) / per));
+  for (auto& l : ws.list) l = (int32_t*)dmalloc(c, wsb, sizeof(int32_t) * (size_t)T * T);
+  ws.count = (int*)dmalloc(c, wsb, 8 * sizeof(int));
+  ws.scratch = dmalloc(c, wsb, per * ws.blocks);
+  panels(c, 0);
+  for (int k = 0; k + 1 < T; ++k) {
     if (look) {
       diag_updates(k, k + 1, k + 2);
-      recompress_tile_pairs(c, TL, k, R, cur.qbase, 2 * cap, 1, rl);   // tile row and column k+1
+      recompress_pairs(c, TL, ws, k, 1);                  // tile row and column k+1
       if (cudaEventRecord(ev_up, c.st) != cudaSuccess || cudaStreamWaitEvent(look, ev_up, 0) != cudaSuccess)
         throw LuError(HM_ERR_CUDA, "look-ahead wait");
-      panels(cl, k + 1, next);
+      panels(cl, k + 1);
       if (cudaEventRecord(ev_dn, look) != cudaSuccess) throw LuError(HM_ERR_CUDA, "look-ahead record");
-      recompress_tile_pairs(c, TL, k, R, cur.qbase, 2 * cap, 2, rl);   // the rest
+      recompress_pairs(c, TL, ws, k, 2);                  // the rest
       diag_updates(k, k + 2, T);
       if (cudaStreamWaitEvent(c.st, ev_dn, 0) != cudaSuccess) throw LuError(HM_ERR_CUDA, "look-ahead join");
     } else {
       diag_updates(k, k + 1, T);
-      recompress_tile_pairs(c, TL, k, R, cur.qbase, 2 * cap, 0, rl);
-      panels(c, k + 1, next);
+      recompress_pairs(c, TL, ws, k, 0);
+      panels(c, k + 1);
     }
-    cur = std::move(next);
   }
 }
 
