@@ -1679,6 +1679,40 @@ __device__ void sweep_z(const SweepTab& t, const double* F, int64_t ldy, int nc,
   __syncthreads();
 }
 
+// Each step's launch may start while the previous one runs (programmatic
+// dependent launch): what does not depend on it -- the inverse's rows, the
+// factor columns of the first dot products -- is loaded before the wait, so a
+// step costs one round of dependent loads instead of a launch and four.
+__device__ __forceinline__ void sweep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void sweep_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// this warp's first factor column of Q (rows lane + 32 j), and its dot product
+// with y_s; later columns and rows past SW_QREG loads go the plain way
+constexpr int SW_QREG = 12;
+__device__ __forceinline__ void sweep_q_prefetch(const double* Q, int r, int Ss, int warp, int lane, double (&qreg)[SW_QREG]) {
+#pragma unroll
+  for (int j = 0; j < SW_QREG; ++j) {
+    const int row = lane + 32 * j;
+    qreg[j] = warp < r && row < Ss ? __ldg(Q + row + (int64_t)warp * Ss) : 0.0;
+  }
+}
+// one column of z = Q' y_s into zsh (no barrier); yreg: y_s at this lane's rows
+__device__ __forceinline__ void sweep_z1(const double* Q, const double* ys, int r, int Ss, int warp, int lane,
+                                         const double (&qreg)[SW_QREG], const double (&yreg)[SW_QREG], double* zsh) {
+  for (int q = warp; q < r; q += SW_THREADS / 32) {
+    double acc = 0.0;
+#pragma unroll
+    for (int j = 0; j < SW_QREG; ++j) {
+      const int row = lane + 32 * j;
+      const double v = q == warp ? qreg[j] : (row < Ss ? __ldg(Q + row + (int64_t)q * Ss) : 0.0);
+      acc = fma(v, yreg[j], acc);
+    }
+    for (int row = lane + 32 * SW_QREG; row < Ss; row += 32) acc = fma(__ldg(Q + row + (int64_t)q * Ss), ys[row], acc);
+    acc = warp_sum(acc);
+    if (lane == 0) zsh[q] = acc;
+  }
+}
+
 // A_i -= P (Q' y_s): the finished tile s applied to the pending tile i
 __device__ void sweep_update(const SweepTab& t, double* A, const double* F, int64_t ldy, int nc, int i, int s,
                              bool trans, double* zsh) {
@@ -1686,10 +1720,39 @@ __device__ void sweep_update(const SweepTab& t, double* A, const double* F, int6
   const double* Q;
   int r;
   sweep_factors(t, i, s, trans, P, Q, r);
+  const int Si = t.size[i], Ss = t.size[s], warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double qreg[SW_QREG];
+  sweep_q_prefetch(Q, r, Ss, warp, lane, qreg);
+  sweep_wait();
   if (r <= 0) return;
-  sweep_z(t, F, ldy, nc, s, Q, r, zsh);
-  const int Si = t.size[i];
   double* yi = A + t.start[i];
+  const double* ys = F + t.start[s];
+  if (nc == 1) {
+    double yreg[SW_QREG], preg[8];
+#pragma unroll
+    for (int j = 0; j < SW_QREG; ++j) yreg[j] = lane + 32 * j < Ss ? ys[lane + 32 * j] : 0.0;
+    const int row = threadIdx.x;                          // this thread's first row
+    const double y0 = row < Si ? yi[row] : 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) preg[q] = q < r && row < Si ? __ldg(P + row + (int64_t)q * Si) : 0.0;
+    sweep_z1(Q, ys, r, Ss, warp, lane, qreg, yreg, zsh);
+    __syncthreads();
+    if (row < Si) {
+      double acc = 0.0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (q < r) acc = fma(preg[q], zsh[q], acc);
+      for (int q = 8; q < r; ++q) acc = fma(__ldg(P + row + (int64_t)q * Si), zsh[q], acc);
+      yi[row] = y0 - acc;
+    }
+    for (int e = row + SW_THREADS; e < Si; e += SW_THREADS) {
+      double acc = 0.0;
+      for (int q = 0; q < r; ++q) acc = fma(__ldg(P + e + (int64_t)q * Si), zsh[q], acc);
+      yi[e] -= acc;
+    }
+    return;
+  }
+  sweep_z(t, F, ldy, nc, s, Q, r, zsh);
   for (int e = threadIdx.x; e < Si * nc; e += SW_THREADS) {
     const int row = e % Si, cc = e / Si;
     double acc = 0.0;
@@ -1699,45 +1762,93 @@ __device__ void sweep_update(const SweepTab& t, double* A, const double* F, int6
   }
 }
 
-// Finisher f of tile k: rows [f rpf, f rpf + rpf) (rpf <= 32) of
-// M (A_k - P (Q' y_s)) written to F, where M = Inv[which][k] (M[q*S + r] =
-// M(r, q); which 0 and 2 lower, 1 and 3 upper).  Lane = row, warp = segment
-// of the columns q the rows need: each thread loads its part of M into
-// registers first (those loads wait for nothing), then the update of tile k
-// from the finished tile s (if any) is recomputed for the rows q needed, and
-// the 8 segment sums of a row are added in shared memory.
-constexpr int SW_MREG = 32;
+// Finisher f of tile k: SW_ROWS rows from f SW_ROWS on of M (A_k - P (Q' y_s))
+// written to F, where M = Inv[which][k] (M[q*S + r] = M(r, q); which 0 and 2
+// lower, 1 and 3 upper).  A half warp per segment of the columns q the rows
+// need, a lane per row: each thread loads its part of M into registers before
+// the wait, then the update of tile k from the finished tile s (if any) is
+// recomputed for the rows q needed, and the 16 segment sums of a row are added
+// in shared memory.
+constexpr int SW_MREG = 24;
+constexpr int SW_ROWS = 16;
+constexpr int SW_SEGS = SW_THREADS / SW_ROWS;
 __device__ void sweep_finish(const SweepTab& t, const double* A, double* F, int64_t ldy, int nc, int k, int s,
-                             bool has_src, bool trans, int which, int f, int rpf, int chunk, double* sh) {
-  constexpr int NW = SW_THREADS / 32;
+                             bool has_src, bool trans, int which, int f, int chunk, double* sh) {
   const int S = t.size[k];
-  const int r0 = f * rpf, r1 = min(S, r0 + rpf), nr = r1 - r0;
-  if (nr <= 0) return;
+  const int r0 = f * SW_ROWS, r1 = min(S, r0 + SW_ROWS), nr = r1 - r0;
   const bool lower = which == 0 || which == 2;
   const int qa = lower ? 0 : r0, qb = lower ? r1 : S, span = qb - qa;
-  const int segl = (span + NW - 1) / NW;
+  const int segl = (span + SW_SEGS - 1) / SW_SEGS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool row_ok = lane < nr;
-  const int qs = qa + warp * segl;                    // this thread's columns [qs, qs + segl)
+  const int rl = lane % SW_ROWS, seg = threadIdx.x / SW_ROWS;
+  const bool row_ok = rl < nr;
+  const int qs = qa + seg * segl;                     // this thread's columns [qs, qs + segl)
   const double* const* inv = which == 0 ? t.Inv0 : which == 1 ? t.Inv1 : which == 2 ? t.Inv2 : t.Inv3;
-  const double* M = inv[k] + r0 + lane;               // M(r0 + lane, q) = M[q*S]
+  const double* M = inv[k] + r0 + rl;                 // M(r0 + rl, q) = M[q*S]
   double mreg[SW_MREG];
-  const bool in_reg = segl <= SW_MREG;
-  if (in_reg) {
 #pragma unroll
-    for (int j = 0; j < SW_MREG; ++j)
-      mreg[j] = (row_ok && j < segl && qs + j < qb) ? __ldg(M + (int64_t)(qs + j) * S) : 0.0;
-  }
+  for (int j = 0; j < SW_MREG; ++j)
+    mreg[j] = (row_ok && j < segl && qs + j < qb) ? __ldg(M + (int64_t)(qs + j) * S) : 0.0;
   double* ysh = sh;                                   // span x chunk
-  double* part = ysh + (size_t)S * chunk;             // NW x 32 x chunk
-  double* zsh = part + (size_t)NW * 32 * chunk;       // cap x nc
+  double* part = ysh + (size_t)S * chunk;             // SW_SEGS x SW_ROWS x chunk
+  double* zsh = part + (size_t)SW_THREADS * chunk;    // cap x nc
   const double* P = nullptr;
   const double* Q = nullptr;
   int r = 0;
   if (has_src) sweep_factors(t, k, s, trans, P, Q, r);
-  if (r > 0) sweep_z(t, F, ldy, nc, s, Q, r, zsh);
+  const int Ss = has_src ? t.size[s] : 0;
+  const double* ys = F + (has_src ? t.start[s] : 0);
   const double* yk = A + t.start[k];
   double* out = F + t.start[k];
+  double qreg[SW_QREG];
+  sweep_q_prefetch(Q, r, Ss, warp, lane, qreg);
+  sweep_wait();
+  if (nr <= 0) return;
+  auto times_m = [&](const double* yv) {              // this thread's part of its row of M yv
+    double acc = 0.0;
+#pragma unroll
+    for (int j = 0; j < SW_MREG; ++j)
+      if (j < segl && qs + j < qb) acc = fma(mreg[j], yv[qs + j], acc);
+    if (row_ok)                                       // segments longer than the registers hold
+#pragma unroll 8
+      for (int q = qs + SW_MREG; q < min(qs + segl, qb); ++q) acc = fma(__ldg(M + (int64_t)q * S), yv[q], acc);
+    return acc;
+  };
+  if (nc == 1) {
+    double yreg[SW_QREG], preg[8];
+#pragma unroll
+    for (int j = 0; j < SW_QREG; ++j) yreg[j] = r > 0 && lane + 32 * j < Ss ? ys[lane + 32 * j] : 0.0;
+    const int q0 = threadIdx.x;
+    const double y0 = q0 < span ? yk[qa + q0] : 0.0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) preg[j] = j < r && q0 < span ? __ldg(P + qa + q0 + (int64_t)j * S) : 0.0;
+    if (r > 0) sweep_z1(Q, ys, r, Ss, warp, lane, qreg, yreg, zsh);
+    __syncthreads();
+    if (q0 < span) {
+      double v = y0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (j < r) v = fma(-preg[j], zsh[j], v);
+      for (int j = 8; j < r; ++j) v = fma(-__ldg(P + qa + q0 + (int64_t)j * S), zsh[j], v);
+      ysh[q0] = v;
+    }
+    for (int q = q0 + SW_THREADS; q < span; q += SW_THREADS) {
+      double v = yk[qa + q];
+      for (int j = 0; j < r; ++j) v = fma(-__ldg(P + qa + q + (int64_t)j * S), zsh[j], v);
+      ysh[q] = v;
+    }
+    __syncthreads();
+    part[threadIdx.x] = times_m(ysh - qa);
+    __syncthreads();
+    if (threadIdx.x < nr) {
+      double acc = 0.0;
+#pragma unroll
+      for (int w = 0; w < SW_SEGS; ++w) acc += part[w * SW_ROWS + threadIdx.x];
+      out[r0 + threadIdx.x] = acc;
+    }
+    return;
+  }
+  if (r > 0) sweep_z(t, F, ldy, nc, s, Q, r, zsh);
   for (int c0 = 0; c0 < nc; c0 += chunk) {
     const int ncc = min(chunk, nc - c0);
     __syncthreads();                                  // ysh and part free
@@ -1749,24 +1860,13 @@ __device__ void sweep_finish(const SweepTab& t, const double* A, double* F, int6
       ysh[q + cc * span] = v;
     }
     __syncthreads();
-    for (int cc = 0; cc < ncc; ++cc) {
-      const double* yv = ysh + cc * span - qa;        // yv[q], q in [qa, qb)
-      double acc = 0.0;
-      if (in_reg) {
-#pragma unroll
-        for (int j = 0; j < SW_MREG; ++j)
-          if (j < segl && qs + j < qb) acc = fma(mreg[j], yv[qs + j], acc);
-      } else if (row_ok) {
-        for (int q = qs; q < min(qs + segl, qb); ++q) acc = fma(__ldg(M + (int64_t)q * S), yv[q], acc);
-      }
-      part[(cc * NW + warp) * 32 + lane] = acc;
-    }
+    for (int cc = 0; cc < ncc; ++cc) part[cc * SW_THREADS + threadIdx.x] = times_m(ysh + cc * span - qa);
     __syncthreads();
     for (int e = threadIdx.x; e < nr * ncc; e += SW_THREADS) {
       const int ii = e % nr, cc = e / nr;
       double acc = 0.0;
 #pragma unroll
-      for (int w = 0; w < NW; ++w) acc += part[(cc * NW + w) * 32 + ii];
+      for (int w = 0; w < SW_SEGS; ++w) acc += part[cc * SW_THREADS + w * SW_ROWS + ii];
       out[r0 + ii + (int64_t)(c0 + cc) * ldy] = acc;
     }
   }
@@ -1775,19 +1875,20 @@ __device__ void sweep_finish(const SweepTab& t, const double* A, double* F, int6
 // Step k of a sweep (dir +1 forward, -1 backward; which: 0 L, 1 U, 2 U', 3 L').
 // A holds the pending right-hand sides, F receives the finished tiles; the
 // finished tile s = k - dir is applied to tile k by the nf finisher CTAs and
-// to every later tile of the sweep by one CTA each.
+// to every later tile of the sweep by one CTA each.  Bound: the latency of the
+// chain of steps (grid completion, y_s, two barriers, 24 FMAs a thread).  64
+// tiles of 312 rows, one column: 13.4 us a step with plain launches and a warp
+// per row of M, 4.9 us so; a solve at n = 65536 (256 tiles) 1.7 ms, was 6.7.
 __global__ void __launch_bounds__(SW_THREADS, 2) lu_sweep_kernel(SweepTab t, double* A, double* F, int64_t ldy,
-                                                              int nc, int k, int dir, int which, int nf, int rpf,
-                                                              int chunk) {
+                                                              int nc, int k, int dir, int which, int nf, int chunk) {
   extern __shared__ double sh[];
+  sweep_release();
   const bool trans = which >= 2;
   const int s = k - dir;
   const bool has_src = s >= 0 && s < t.T;
-  if ((int)blockIdx.x < nf) {
-    sweep_finish(t, A, F, ldy, nc, k, s, has_src, trans, which, blockIdx.x, rpf, chunk, sh);
-  } else if (has_src) {
-    sweep_update(t, A, F, ldy, nc, k + dir * ((int)blockIdx.x - nf + 1), s, trans, sh);
-  }
+  if ((int)blockIdx.x < nf) sweep_finish(t, A, F, ldy, nc, k, s, has_src, trans, which, blockIdx.x, chunk, sh);
+  else if (has_src) sweep_update(t, A, F, ldy, nc, k + dir * ((int)blockIdx.x - nf + 1), s, trans, sh);
+  else sweep_wait();
 }
 
 // The same inverses for tiles whose columns do not fit in shared memory, of the
@@ -1901,7 +2002,6 @@ static void tile_sweeps(Ctx& c, const TileLU& TL, View X, bool trans) {
   const int T = TL.T, nc = X.cols;
   int smax = 1;
   for (int k = 0; k < T; ++k) smax = std::max<int>(smax, (int)TL.size[k]);
-  const int rpf = 32;                                              // rows of a finisher (a lane each)
   const int chunk = std::min(nc, 8);                               // columns staged per pass
   const size_t smem = sizeof(double) * ((size_t)smax * chunk + (size_t)SW_THREADS * chunk + (size_t)c.cap * nc);
   if (smem > 200 * 1024 || X.rs != 1) {
@@ -1914,18 +2014,24 @@ static void tile_sweeps(Ctx& c, const TileLU& TL, View X, bool trans) {
   double* W = (double*)dmalloc(c, tmp, sizeof(double) * (size_t)X.cs * nc);
   SweepTab t{TL.d_Ap, TL.d_Bp, TL.d_inv[0], TL.d_inv[1], TL.d_inv[2], TL.d_inv[3], TL.d_start, TL.d_size,
              TL.kmat, T, c.cap};
-  for (int k = 0; k < T; ++k) {
-    const int nf = ((int)TL.size[k] + rpf - 1) / rpf;
-    const int nu = k > 0 ? T - 1 - k : 0;
-    lu_sweep_kernel<<<nf + nu, SW_THREADS, smem, c.st>>>(t, X.p, W, X.cs, nc, k, 1, trans ? 2 : 0, nf, rpf, chunk);
-    LU_LAUNCH_CHECK();
-  }
-  for (int k = T - 1; k >= 0; --k) {
-    const int nf = ((int)TL.size[k] + rpf - 1) / rpf;
-    const int nu = k < T - 1 ? k : 0;
-    lu_sweep_kernel<<<nf + nu, SW_THREADS, smem, c.st>>>(t, W, X.p, X.cs, nc, k, -1, trans ? 3 : 1, nf, rpf, chunk);
-    LU_LAUNCH_CHECK();
-  }
+  // the first launch is a plain one: what it loads early is then complete
+  auto step = [&](double* A, double* F, int k, int dir, int which, bool overlap) {
+    const int nf = ((int)TL.size[k] + SW_ROWS - 1) / SW_ROWS;
+    const int nu = dir > 0 ? (k > 0 ? T - 1 - k : 0) : (k < T - 1 ? k : 0);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(nf + nu));
+    cfg.blockDim = dim3(SW_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c.st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = overlap ? 1 : 0;
+    HM_LU_CUDA(cudaLaunchKernelEx(&cfg, lu_sweep_kernel, t, A, F, X.cs, nc, k, dir, which, nf, chunk));
+  };
+  for (int k = 0; k < T; ++k) step(X.p, W, k, 1, trans ? 2 : 0, k > 0);
+  for (int k = T - 1; k >= 0; --k) step(W, X.p, k, -1, trans ? 3 : 1, true);
 }
 
 // y = P b, forward (unit L), backward (U) tile by tile; trans: U' then L'

@@ -46,3 +46,26 @@ def test_tiles_from_reduced_storage(storage):
     assert L.info().lu_tiles >= 2
     x, it, rr = L.solve_refined(y, tol=1e-12, max_iter=10)
     assert rr <= 1e-12
+
+
+# a sweep step keeps the first 384 rows of a tile's dot products and the first
+# 24 columns of each row segment in registers and loads the rest later: tiles
+# on both sides, ragged ones, and the one-column path against the many-column
+# one.  The same factors, so only rounding separates the two: the condition
+# number (|H| < n, shift 1) times 2^-53 times a growth of 100.
+@pytest.mark.parametrize("n,maxb", [(700, 128), (1537, 384), (1999, 512), (4100, 1024), (3000, 100)])
+def test_sweep_columns(n, maxb):
+    import hmatrix as hm
+    rng = np.random.default_rng(n)
+    _, H = hm.NewHmat(hm.Params(LuMode="tiles", Geom=np.sort(rng.uniform(0, 10, n)), Kernel=hm.Cauchy(1.0), MaxBlock=maxb,
+                                MinBlock=32, MaxRank=16, ConsMethod="aca2", εComp=1e-10, Tree="bisect", Shift=1.0))
+    L = hm.lu(H)
+    assert L.info().lu_tiles >= 2
+    tol = n * 2.0 ** -53 * 100
+    Y = rng.standard_normal((n, 64))
+    for trans in (False, True):
+        one = np.stack([L.solve(Y[:, j], trans=trans) for j in range(64)], axis=1)
+        for nc in (2, 8, 9, 64):
+            X = L.solve(Y[:, :nc], trans=trans)
+            assert np.linalg.norm(X - one[:, :nc]) <= tol * np.linalg.norm(X)
+        assert np.array_equal(one[:, 0], L.solve(Y[:, 0], trans=trans))
