@@ -7,28 +7,32 @@
 //   share one input segment are cut into 128-column M-tiles; one tcgen05 MMA
 //   chain per tile computes Z_tile = F1_tile' X_seg (K = segment points,
 //   N = right-hand-side columns) into a TMEM accumulator.
-// Phase 2 (Y += F2 Z): an output window of 512 rows keeps its Z slots (the k
-//   values of every leaf that touches the window) contiguous; one MMA chain
-//   per 128-row tile of a window runs K over the window's slots.  The dense
+// Phase 2 (Y += F2 Z): one MMA chain per tile of 128 output rows, K = the Z
+//   slots of the leaves with rows in the tile.  Each z is stored once, in the
+//   order of the output clusters; a tile lists the 16-byte K blocks of slots
+//   it takes, 16 to a stage, and its Z tile is gathered block by block.  (Z
+//   slots copied per window of 512 rows cost phase 1 a serial chain of copies
+//   for each long column, and phase 2 every small leaf of the window in all
+//   four of its tiles: n = 2^18, 64 columns, BF16: phases 1 + 2 669 + 631 us, now 272 + 333; n = 200000,
+//   16 columns, FP32: 484 + 1190 us, now 418 + 545.)  The dense
 //   leaves are added by the CUDA-core block kernel first.
 //
 // Data movement.  Factor columns are contiguous in the pool, so a pipeline
-// stage takes one contiguous piece of each factor column it needs (phase 1:
-// KC values = 256 bytes of each of the tile's 128 columns; phase 2: the
-// tile's rows of each of KC columns) into a raw shared-memory stage, by
-// 16-byte cp.async gathers of four producer warps (16 lanes per 256-byte
-// piece, so every warp instruction reads whole 128-byte lines) whose
-// completion arrives on the stage's mbarrier without blocking the producers
-// (cp.async.mbarrier.arrive.noinc).  A 1-D bulk copy per factor column would
-// be simpler, but each lane's bulk copy issues separately (about 80 cycles a
-// copy measured), which capped a single producer warp near 1 TB/s.  The X / Z
-// tile of the stage, one contiguous block pre-tiled in the MMA's K-major
-// core-matrix layout, arrives by one bulk copy of the TMA engine.  Converter warps read the
-// raw stage row by row (one TMEM lane per thread), split FP32 values into TF32
-// hi and lo parts, and write the A operand straight into tensor memory
-// (tcgen05.st); the MMA reads A from TMEM and B from shared memory.  Shared
-// memory thus carries each factor byte twice (bulk-copy write, converter read)
-// instead of five times when hi/lo operand tiles are staged in shared memory.
+// stage takes one contiguous piece of each factor column it needs into a raw
+// shared-memory stage.  Phase 1: KC values = 256 bytes of each of the tile's
+// 128 columns, by 16-byte cp.async gathers (16 lanes per piece) whose
+// completion arrives on the stage's mbarrier without blocking the producers.
+// Phase 2: the tile's rows of each of KC columns (up to 512 bytes), a bulk copy
+// each: a lane's copy issues in about 80 cycles, so eight warps share them
+// (cp.async pieces were issued at 35 cycles per 512 bytes and SM, 624 us against
+// 572 for FP32, n = 200000, 16 columns).  The X / Z tile of the stage, pre-tiled
+// as the MMA's core matrices, arrives by bulk copies too (one, or one per run of
+// K blocks).  Converter warps read the raw stage row by row (one TMEM lane per
+// thread), split FP32 values into TF32 hi and lo parts, and write the A operand
+// straight into tensor memory (tcgen05.st); the MMA reads A from TMEM and B from
+// shared memory.  Shared memory thus carries each factor byte twice (copy,
+// converter read) instead of five times when hi/lo operand tiles are staged in
+// shared memory.
 //
 // Accuracy.  FP32 factors use three TF32 products per term (F_hi X_hi +
 // F_hi X_lo + F_lo X_hi, the split of Ootomo & Yokota 2022), BF16 factors
@@ -37,11 +41,11 @@
 // Both splits round to nearest and leave exact values of the narrow format,
 // so the hardware's own input conversion does not matter.
 //
-// Roles per CTA (persistent, one per SM, 13 warps): warps 8-11 produce stages;
-// warps 0-7 convert them into two TMEM A buffers (warp w: TMEM lanes
-// 32 (w % 4) .., the K half w / 4 of each stage, two converter warps per SM
-// sub-partition) and drain the accumulator of the previous tile (tcgen05.ld)
-// once its MMAs are known to be done; warp 12 issues the MMAs (one thread).
+// Roles per CTA (persistent, one per SM): warps 0-7 convert raw stages into the
+// TMEM A buffers (warp w: TMEM lanes 32 (w % 4) .., the K half w / 4 of each
+// stage) and drain the accumulator of the previous tile (tcgen05.ld) once its
+// MMAs are known to be done; then the producer warps; the last warp issues the
+// MMAs (one elected thread).
 // The two TMEM accumulators alternate between tiles.  mbarriers link
 // the roles; every wait is bounded, and a timeout sets an error word and ends
 // the kernel cleanly once the copies and MMAs in flight have finished.
@@ -55,21 +59,19 @@ namespace hm {
 
 struct TcCol1 {            // phase-1 M row: one factor column of F1
   uint64_t off;            // pool element offset of the column's first entry
-  uint32_t zp0, zp1;       // its Z slots: zpl[zp0 .. zp1)
+  uint32_t zp, pad;        // its Z slot
 };
 struct TcItem1 {           // one tile of up to 128 columns of one input segment
   uint32_t col0, ncol;     // columns [col0, col0 + ncol) of the column table
   uint32_t seg0, len;      // input index range of the segment
 };
-struct TcZ2 {              // phase-2 K column (a Z slot) inside its window
-  int64_t a_off;           // pool element offset of F2 at window row rlo
-  int32_t rlo, rhi;        // rows [rlo, rhi) of the window it covers
+struct TcZ2 {              // phase-2 K column (a Z slot): one column of F2
+  int64_t a_off;           // pool element offset of its row rlo
+  uint32_t rlo, rhi;       // output rows [rlo, rhi); empty for the padding slots
 };
-struct TcItem2 {           // one tile of up to 128 rows of an output window
+struct TcItem2 {           // one tile of up to 128 output rows
   uint32_t row0, nrows;    // first output row of the tile, its rows
-  uint32_t zb, ze;         // the window's Z slots [zb, ze)
-  uint32_t toff;           // row offset of the tile inside its window
-  uint32_t pad;
+  uint32_t sb, nk;         // its stages: 16 K blocks each, blk[16 sb ..]
 };
 
 struct TcPlan {
@@ -77,10 +79,9 @@ struct TcPlan {
   int64_t ncol1 = 0;
   TcItem1* d_item1 = nullptr;
   int64_t nitem1 = 0;
-  uint32_t* d_zpl = nullptr;
-  int64_t nzpl = 0;
   TcZ2* d_z2 = nullptr;
-  int64_t nz2 = 0;
+  int64_t nz2 = 0;         // Z slots; the block of slots after them is zero
+  uint32_t* d_blk = nullptr;   // K blocks (KE slots) of the phase-2 stages
   TcItem2* d_item2 = nullptr;
   int64_t nitem2 = 0;
   unsigned qmask = 0;      // the shifted copies of X that some segment uses
@@ -90,17 +91,29 @@ struct TcPlan {
 
 namespace {
 
-constexpr int TC_WR = 512;           // rows of a phase-2 window
-constexpr int TC_PW = 4;                          // producer warps
-constexpr int TC_MMA_WARP = 8 + TC_PW;             // warps 0-7 convert + drain, 8 .. produce, then MMA
-constexpr int TC_THREADS = 32 * (TC_MMA_WARP + 1);
-constexpr int TC_PROD0 = 256;                      // first producer thread
-constexpr int TC_NPROD = 32 * TC_PW;
+constexpr int TC_ROWS = 128;         // output rows of a phase-2 tile
+constexpr int TC_KB = 16;            // K blocks of a stage
+// warps of a CTA: converters (they drain too), then producers, then the MMA issuer
+template <int CW_, int PW_>
+struct TcRoles {
+  static constexpr int CW = CW_, PW = PW_;            // converter (a multiple of 4) and producer warps
+  static constexpr int MMA = CW + PW;
+  static constexpr int THREADS = 32 * (MMA + 1);
+  static constexpr int PROD0 = 32 * CW;               // first producer thread
+  static constexpr int NPROD = 32 * PW;
+  static constexpr int NH = CW / 4;                   // converters per TMEM lane: shares of a stage's columns
+};
+// phase 1: 8 producer warps take FP32 at n = 200000, 16 columns from 456 to 418
+// us; BF16 at n = 2^18, 64 columns, is faster with 4 (272 against 384 us)
+template <typename T> using TcR1 = TcRoles<8, sizeof(T) == 4 ? 8 : 4>;
+// phase 2: 4 producer warps 660 us and 16 converter warps 597 us against 545
+// (FP32, n = 200000, 16 columns)
+using TcR2 = TcRoles<8, 8>;
 constexpr int TC_NA_MAX = 4;         // TMEM A buffers, at most
 constexpr int TC_TMEM_COLS = 512;    // one CTA per SM (shared memory), so all of TMEM
 constexpr uint32_t TC_WAIT = 1u << 22;   // polls of a bounded mbarrier wait
 // Phase 2 adds its FP32 accumulator into the FP64 Y every NC / 2 stages
-// (32 NC Z slots for FP32 factors, 64 NC for BF16): a window's K runs over
+// (32 NC Z slots for FP32 factors, 64 NC for BF16): a tile's K runs over
 // every leaf that touches it (thousands of terms at n = 2^20), and one FP32 sum
 // over all of them would lose accuracy as n grows.  The segment grows with the
 // column block so that the Y traffic of the adds (16 NC bytes a tile row) stays
@@ -117,6 +130,7 @@ template <> struct TcT<float> {
   static constexpr int FMT = tc::FMT_TF32;
   static constexpr bool SPLIT = true;               // A = A_hi + A_lo
   static constexpr int SIG = 11;                    // significant bits of the narrow format
+  static constexpr int Z_MN = 0;                    // Z blocks K-major: [2 NC columns][KE slots]
   static constexpr int SHIFT = 0;                   // its bits: the FP32 pattern >> SHIFT
   using Bits = uint32_t;
   __device__ static float hi(float x) { return tc::tf32_rn(x); }
@@ -131,7 +145,10 @@ template <> struct TcT<__nv_bfloat16> {
   static constexpr int FMT = tc::FMT_BF16;
   static constexpr bool SPLIT = false;              // BF16 factors are exact
   static constexpr int SIG = 8;
-  static constexpr int SHIFT = 16;
+  // Z blocks as 8 x 8 core matrices [slot][column]: a phase-1 row (one slot)
+  // writes 16 bytes for 8 columns instead of 8 scattered 2-byte pieces
+  static constexpr int Z_MN = 1;
+  static constexpr int SHIFT = 16;                  // (BF16 pieces are packed with byte permutes)
   using Bits = uint16_t;
   __device__ static float hi(float x) { return tc::bf16_rn(x); }
   __device__ static Bits bits(float x) { return (uint16_t)(__float_as_uint(x) >> 16); }
@@ -171,17 +188,17 @@ struct TcCfg {
   static_assert(BYTES <= 227 * 1024, "stages exceed the shared memory of a CTA");
   static_assert(ACC0 + 2 * ACCW <= TC_TMEM_COLS, "A buffers and accumulators exceed TMEM");
   static_assert(RS1 % 16 == 0 && RS2 % 16 == 0 && B_BYTES % 16 == 0, "bulk copies move 16-byte units");
-  static_assert(KC % TC_PW == 0 && KC % Tr::KM == 0, "a stage is whole MMAs and whole producer warps");
+  static_assert(KC % TcR1<T>::PW == 0 && KC % TcR2::PW == 0 && KC % Tr::KM == 0, "a stage is whole MMAs and whole producer warps");
 };
 
 struct TcBars {
   uint64_t full[5];        // raw stage landed (the producers' cp.async arrivals)
   uint64_t bfull[5];       // the stage's B tile landed (bulk-copy bytes + one arrival)
   uint64_t empty[5];       // the MMAs that read the stage's B tile finished (tcgen05.commit)
-  uint64_t afull[TC_NA_MAX];   // A buffer written (256 converter threads)
+  uint64_t afull[TC_NA_MAX];   // A buffer written (an arrival per converter warp)
   uint64_t aempty[TC_NA_MAX];  // the MMAs that read the A buffer finished
   uint64_t accfull[2];     // accumulator complete (commit after a tile's last MMA)
-  uint64_t accempty[2];    // accumulator drained (256 converter threads)
+  uint64_t accempty[2];    // accumulator drained (an arrival per converter warp)
   uint64_t done;           // the MMA issuer's last commit: every MMA finished
   uint32_t tmem;
   int abort;
@@ -189,6 +206,9 @@ struct TcBars {
 static_assert(sizeof(TcBars) <= 512, "barrier block");
 static_assert((TcT<float>::KE & (TcT<float>::KE - 1)) == 0 && (TcT<__nv_bfloat16>::KE & (TcT<__nv_bfloat16>::KE - 1)) == 0,
               "K blocks of a power-of-two size");
+static_assert(TcT<__nv_bfloat16>::KE == 8, "core matrices of 8 slots x 8 columns");
+static_assert(TcT<float>::KC == TC_KB * TcT<float>::KE && TcT<__nv_bfloat16>::KC == TC_KB * TcT<__nv_bfloat16>::KE,
+              "a stage is TC_KB K blocks");
 static_assert(TcT<float>::KC * 4 == 256 && TcT<__nv_bfloat16>::KC * 2 == 256, "phase-1 pieces are 16 x 16 bytes");
 
 __device__ __forceinline__ void tc_fail(int* err, TcBars* b, int code) {
@@ -213,9 +233,15 @@ __device__ __forceinline__ bool tc_wait_warp(TcBars* b, uint64_t* bar, uint32_t 
   return __all_sync(0xffffffffu, ok) != 0;
 }
 
+// one arrival for a whole warp, after every lane's work
+__device__ __forceinline__ void tc_warp_arrive(uint64_t* bar, int lane) {
+  __syncwarp();
+  if (lane == 0) tc::mbar_arrive(bar);
+}
+
 // barriers, TMEM; called by all threads.  full_count: arrivals that complete
-// a raw stage.
-__device__ __forceinline__ uint32_t tc_setup(TcBars* b, int warp, int nstage, uint32_t full_count) {
+// a raw stage; conv: converter warps.
+__device__ __forceinline__ uint32_t tc_setup(TcBars* b, int warp, int nstage, uint32_t full_count, uint32_t conv) {
   if (threadIdx.x == 0) {
     for (int s = 0; s < nstage; ++s) {
       tc::mbar_init(&b->full[s], full_count);
@@ -223,12 +249,12 @@ __device__ __forceinline__ uint32_t tc_setup(TcBars* b, int warp, int nstage, ui
       tc::mbar_init(&b->empty[s], 1);
     }
     for (int q = 0; q < TC_NA_MAX; ++q) {
-      tc::mbar_init(&b->afull[q], 256);
+      tc::mbar_init(&b->afull[q], conv);
       tc::mbar_init(&b->aempty[q], 1);
     }
     for (int q = 0; q < 2; ++q) {
       tc::mbar_init(&b->accfull[q], 1);
-      tc::mbar_init(&b->accempty[q], 256);
+      tc::mbar_init(&b->accempty[q], conv);
     }
     tc::mbar_init(&b->done, 1);
     b->abort = 0;
@@ -251,73 +277,83 @@ __device__ __forceinline__ void tc_teardown(TcBars* b, int warp, uint32_t tmem) 
   }
 }
 
-// The B-tile producer's last step: every bulk copy it issued has landed.  The
-// wait ignores an abort (shared memory must not be released under copies in
-// flight) but stays bounded.  `it` stages were issued, stage s last by the
-// largest iteration below `it` that is s mod nstage.
-__device__ __forceinline__ void tc_copies_drain(TcBars* b, uint32_t it, int nstage, int* err) {
+// A producer's last step: every bulk copy it issued has landed.  The wait
+// ignores an abort (shared memory must not be released under copies in
+// flight) but stays bounded.  `it` stages were issued on the barriers `bar`,
+// stage s last by the largest iteration below `it` that is s mod nstage.
+__device__ __forceinline__ void tc_copies_drain(TcBars* b, uint64_t* bar, uint32_t it, int nstage, int* err) {
   for (int s = 0; s < nstage && (uint32_t)s < it; ++s) {
     const uint32_t last = it - 1 - ((it - 1 - (uint32_t)s) % (uint32_t)nstage);
-    if (!tc::mbar_wait(&b->bfull[s], (last / (uint32_t)nstage) & 1u, TC_WAIT)) tc_fail(err, b, 32);
+    if (!tc::mbar_wait(&bar[s], (last / (uint32_t)nstage) & 1u, TC_WAIT)) tc_fail(err, b, 32);
   }
 }
 
-// MMA issuer (one thread): per tile, K stages of A (TMEM) x B (shared
-// memory); nk_of(w) gives tile w's stages.  Every kseg stages of a tile form
+// MMA issuer (one warp in uniform control flow, one elected thread issues: its
+// operands stay in uniform registers, which the MMA takes): per tile, K stages of A (TMEM) x B (shared
+// memory, K-major or with B_MN the columns of a core matrix contiguous); nk_of(w) gives tile w's stages.  Every kseg stages of a tile form
 // one accumulation segment: a fresh accumulator (q = segment parity) that the
 // converters drain when it completes.
-template <typename T, int NC, typename NkOf>
+template <typename T, int NC, int B_MN, typename NkOf>
 __device__ __forceinline__ void tc_mma_role(TcBars* b, uint32_t sbase, uint32_t tmem, int64_t nitems, NkOf nk_of,
                                             int kseg, int* err) {
   using Tr = TcT<T>;
   using C = TcCfg<T, NC>;
   constexpr uint32_t LBO_B = 2 * NC * 16, SBO_B = 128;        // K-major [hi | lo] B tiles
-  const uint32_t id_full = tc::idesc(Tr::FMT, 2 * NC, 0, 0);
-  const uint32_t id_half = tc::idesc(Tr::FMT, NC, 0, 0);
+  const uint32_t id_full = tc::idesc(Tr::FMT, 2 * NC, 0, B_MN);
+  const uint32_t id_half = tc::idesc(Tr::FMT, NC, 0, B_MN);
+  const bool leader = tc::elect_one();
+  tmem = __shfl_sync(0xffffffffu, tmem, 0);
   uint32_t it = 0, j = 0;                                      // stages, segments
   bool ok = true;
   int nk = blockIdx.x < nitems ? nk_of(blockIdx.x) : 0;
   for (int64_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
     const int nk_next = w + gridDim.x < nitems ? nk_of(w + gridDim.x) : 0;   // loaded ahead of its use
+    nk = __shfl_sync(0xffffffffu, nk, 0);
     for (int k0 = 0; k0 < nk && ok; k0 += kseg, ++j) {
       const int k1 = min(nk, k0 + kseg);
       const uint32_t q = j & 1u;
-      if (!tc_wait(b, &b->accempty[q], ((j >> 1) & 1u) ^ 1u, err, 2)) { ok = false; break; }
-      tc::tc_fence_after();
+      if (!tc_wait_warp(b, &b->accempty[q], ((j >> 1) & 1u) ^ 1u, err, 2)) { ok = false; break; }
       const uint32_t dacc = tmem + (uint32_t)C::ACC0 + q * C::ACCW;
       for (int kc = k0; kc < k1; ++kc, ++it) {
-        const int s = (int)(it % C::S), a = (int)(it % C::NA);
-        if (!tc_wait(b, &b->bfull[s], (it / C::S) & 1u, err, 4)) { ok = false; break; }
-        if (!tc_wait(b, &b->afull[a], (it / C::NA) & 1u, err, 4)) { ok = false; break; }
+        const uint32_t s = it % C::S, a = it % C::NA;
+        if (!tc_wait_warp(b, &b->bfull[s], (it / C::S) & 1u, err, 4)) { ok = false; break; }
+        if (!tc_wait_warp(b, &b->afull[a], (it / C::NA) & 1u, err, 4)) { ok = false; break; }
         tc::tc_fence_after();
-        const uint32_t bbase = sbase + (uint32_t)(s * C::STAGE);
-        const uint32_t abuf = tmem + (uint32_t)(a * Tr::ACOLS);
+        const uint64_t bd0 = tc::smem_desc(sbase + s * (uint32_t)C::STAGE, LBO_B, SBO_B);
+        const uint32_t abuf = tmem + a * (uint32_t)Tr::ACOLS;
+        if (leader) {
 #pragma unroll
-        for (int ks = 0; ks < Tr::KC / Tr::KM; ++ks) {
-          const uint64_t bd = tc::smem_desc(bbase + ks * 2 * LBO_B, LBO_B, SBO_B);
-          if constexpr (Tr::SPLIT) {
-            // hi products into chain 0, lo products into chain 1 (or chain 0)
-            tc::mma_ts<Tr::KIND>(dacc, abuf + ks * 8, bd, id_full, (kc > k0 || ks > 0) ? 1u : 0u);
-            if constexpr (C::NCH == 2)
-              tc::mma_ts<Tr::KIND>(dacc + 2 * NC, abuf + Tr::KC + ks * 8, bd, id_half, (kc > k0 || ks > 0) ? 1u : 0u);
-            else
-              tc::mma_ts<Tr::KIND>(dacc, abuf + Tr::KC + ks * 8, bd, id_half, 1u);
-          } else {
-            // K steps alternate between the chains
-            const uint32_t ch = C::NCH == 2 ? (uint32_t)(ks & 1) : 0u;
-            tc::mma_ts<Tr::KIND>(dacc + ch * 2 * NC, abuf + ks * 8, bd, id_full,
-                                 (kc > k0 || ks >= C::NCH) ? 1u : 0u);
+          for (int ks = 0; ks < Tr::KC / Tr::KM; ++ks) {
+            const uint64_t bd = bd0 + (uint64_t)((ks * 2 * LBO_B) >> 4);   // the address field alone moves
+            if constexpr (Tr::SPLIT) {
+              // hi products into chain 0, lo products into chain 1 (or chain 0)
+              tc::mma_ts<Tr::KIND>(dacc, abuf + ks * 8, bd, id_full, (kc > k0 || ks > 0) ? 1u : 0u);
+              if constexpr (C::NCH == 2)
+                tc::mma_ts<Tr::KIND>(dacc + 2 * NC, abuf + Tr::KC + ks * 8, bd, id_half, (kc > k0 || ks > 0) ? 1u : 0u);
+              else
+                tc::mma_ts<Tr::KIND>(dacc, abuf + Tr::KC + ks * 8, bd, id_half, 1u);
+            } else {
+              // K steps alternate between the chains
+              const uint32_t ch = C::NCH == 2 ? (uint32_t)(ks & 1) : 0u;
+              tc::mma_ts<Tr::KIND>(dacc + ch * 2 * NC, abuf + ks * 8, bd, id_full,
+                                   (kc > k0 || ks >= C::NCH) ? 1u : 0u);
+            }
           }
+          tc::mma_commit(&b->empty[s]);
+          tc::mma_commit(&b->aempty[a]);
         }
-        tc::mma_commit(&b->empty[s]);
-        tc::mma_commit(&b->aempty[a]);
+        __syncwarp();
       }
-      if (ok) tc::mma_commit(&b->accfull[q]);
+      if (ok && leader) tc::mma_commit(&b->accfull[q]);
+      __syncwarp();
     }
     nk = nk_next;
   }
-  tc::mma_commit(&b->done);
-  if (!tc::mbar_wait(&b->done, 0u, TC_WAIT)) tc_fail(err, b, 16);
+  if (leader) {
+    tc::mma_commit(&b->done);
+    if (!tc::mbar_wait(&b->done, 0u, TC_WAIT)) tc_fail(err, b, 16);
+  }
+  __syncwarp();
 }
 
 // ---------------------------------------------------------------------------
@@ -469,10 +505,11 @@ __device__ __forceinline__ uint32_t slot_val(const uint8_t* rb, const int4* meta
   const uint32_t v = reinterpret_cast<const uint16_t*>(rb)[md.z + m];
   return (uint32_t)(m - md.x) < (uint32_t)md.y ? v : 0u;
 }
+template <int NH>
 __device__ __forceinline__ void conv2(const uint8_t* rb, const int4* meta, int m, uint32_t ta, int h, float* tag) {
-  constexpr int KC = TcT<float>::KC;
+  constexpr int KC = TcT<float>::KC, W = KC / NH;
 #pragma unroll 1
-  for (int c0 = 32 * h; c0 < 32 * h + 32; c0 += 16) {
+  for (int c0 = W * h; c0 < W * h + W; c0 += 16) {
     float x[16];
     uint32_t hi[16], lo[16];
 #pragma unroll
@@ -482,10 +519,12 @@ __device__ __forceinline__ void conv2(const uint8_t* rb, const int4* meta, int m
     tc::tmem_st16(ta + KC + c0, lo);
   }
 }
+template <int NH>
 __device__ __forceinline__ void conv2(const uint8_t* rb, const int4* meta, int m, uint32_t ta, int h,
                                       __nv_bfloat16* tag) {
+  constexpr int W = TcT<__nv_bfloat16>::KC / 2 / NH;
 #pragma unroll 1
-  for (int c0 = 32 * h; c0 < 32 * h + 32; c0 += 16) {
+  for (int c0 = W * h; c0 < W * h + W; c0 += 16) {
     uint32_t wv[16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
@@ -504,7 +543,6 @@ struct P1Args {
   const TcItem1* items;
   int64_t nitems;
   const TcCol1* cols;
-  const uint32_t* zpl;
   const T* pool;
   const typename TcT<T>::Bits* xt;   // XT of this column block
   int64_t xt_copy;                   // elements of one shifted copy
@@ -513,25 +551,26 @@ struct P1Args {
 };
 
 template <typename T, int NC>
-__global__ void __launch_bounds__(TC_THREADS, 1) tc_phase1_kernel(P1Args<T, NC> a) {
+__global__ void __launch_bounds__(TcR1<T>::THREADS, 1) tc_phase1_kernel(P1Args<T, NC> a) {
   using Tr = TcT<T>;
   using C = TcCfg<T, NC>;
+  using R = TcR1<T>;
   constexpr int KE = Tr::KE, KC = Tr::KC;
   extern __shared__ __align__(1024) uint8_t smem[];
   TcBars* bars = reinterpret_cast<TcBars*>(smem + C::BAR_OFF);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t tmem = tc_setup(bars, warp, C::S, TC_NPROD);    // the producers' cp.async arrivals
+  const uint32_t tmem = tc_setup(bars, warp, C::S, R::NPROD, R::CW);    // the producers' cp.async arrivals
   const uint32_t sbase = tc::smem_u32(smem);
   auto nk_of = [&](int64_t w) { return (int)((a.items[w].len + KC - 1) / KC); };
 
-  if (warp >= 8 && warp < TC_MMA_WARP) {
+  if (warp >= R::CW && warp < R::MMA) {
     // ---------------- producers: the X tile (one bulk copy) and 256 bytes of each column ----------------
-    // thread pt copies 16-byte piece q of the columns cg, cg + CG, .., (CG = 2 TC_PW column groups)
+    // thread pt copies 16-byte piece q of the columns cg, cg + CG, .., (CG = NPROD / 16 column groups)
     // (the tile's column offsets are loaded into registers once per tile:
     // re-reading them every stage put a load latency in front of each stage's
     // copies; the first stage's wait is covered by the stages already queued)
-    constexpr int CG = TC_NPROD / 16, CPT = 128 / CG;      // column groups, columns per thread
-    const int pt = threadIdx.x - TC_PROD0;
+    constexpr int CG = R::NPROD / 16, CPT = 128 / CG;      // column groups, columns per thread
+    const int pt = threadIdx.x - R::PROD0;
     const int q = pt & 15, cg = pt >> 4;
     uint32_t it = 0;
     int64_t w = blockIdx.x;
@@ -566,9 +605,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_phase1_kernel(P1Args<T, NC> 
 #pragma unroll
         for (int j = 0; j < CPT; ++j) {
           const uint32_t c = (uint32_t)(cg + CG * j);
-          const bool ok = in && c < I.ncol;
-          tc::cp_async16(dst + c * C::RS1, ok ? (const void*)(a.pool + coff[j] + el) : (const void*)a.pool,
-                         ok ? 16u : 0u);
+          if (in && c < I.ncol) tc::cp_async16(dst + c * C::RS1, a.pool + coff[j] + el, 16u);
         }
         tc::cp_async_mbar_arrive(&bars->full[s]);
         ++it;
@@ -585,20 +622,22 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_phase1_kernel(P1Args<T, NC> 
       I = I2;
     }
     tc::cp_async_wait_all();
-    if (pt == 0) tc_copies_drain(bars, it, C::S, a.err);
-  } else if (warp == TC_MMA_WARP) {
+    if (pt == 0) tc_copies_drain(bars, bars->bfull, it, C::S, a.err);
+  } else if (warp == R::MMA) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) tc_mma_role<T, NC>(bars, sbase, tmem, a.nitems, nk_of, 1 << 30, a.err);   // one segment a tile
-  } else if (warp < 8) {
+    tc_mma_role<T, NC, 0>(bars, sbase, tmem, a.nitems, nk_of, 1 << 30, a.err);   // one segment a tile
+  } else if (warp < R::CW) {
     // ---------------- converters (thread = TMEM lane m = tile row = factor column m) + drain ----------------
     const int m = 32 * (warp & 3) + lane, h = warp >> 2;
     const uint32_t lb = (uint32_t)(32 * (warp & 3)) << 16;
-    // drain of tile jj: Z slots of row m, accumulator columns [h NC / 2, h NC / 2 + NC / 2)
+    // drain of tile jj: the Z slot of row m, accumulator columns [h NC / 2, h NC / 2 + NC / 2)
     auto drain = [&](const TcItem1& J, uint32_t jj) -> bool {
       const uint32_t q = jj & 1u;
       const bool valid = (uint32_t)m < J.ncol;
       TcCol1 Cc{};
       if (valid) Cc = a.cols[J.col0 + m];
+      typename Tr::Bits* zb =
+          a.zt + (int64_t)(Cc.zp / KE) * (2 * NC * KE) + (Cc.zp % KE) * (Tr::Z_MN ? 8 : 1);
       if (!tc_wait_warp(bars, &bars->accfull[q], (jj >> 1) & 1u, a.err, 8)) return false;
       tc::tc_fence_after();
 #pragma unroll 1
@@ -608,9 +647,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_phase1_kernel(P1Args<T, NC> 
         if (valid) {
           uint32_t zh[8], zl[8];
           tc::split_n<Tr::SIG>(zz, zh, zl);
-          for (uint32_t zi = Cc.zp0; zi < Cc.zp1; ++zi) {
-            const uint32_t zp = a.zpl[zi];
-            typename Tr::Bits* zb = a.zt + (int64_t)(zp / KE) * (2 * NC * KE) + (zp % KE);
+          if constexpr (Tr::Z_MN) {
+            auto pack = [](const uint32_t (&v)[8]) {
+              return make_uint4(__byte_perm(v[0], v[1], 0x7632), __byte_perm(v[2], v[3], 0x7632),
+                                __byte_perm(v[4], v[5], 0x7632), __byte_perm(v[6], v[7], 0x7632));
+            };
+            *reinterpret_cast<uint4*>(zb + j0 * 8) = pack(zh);
+            *reinterpret_cast<uint4*>(zb + (NC + j0) * 8) = pack(zl);
+          } else {
 #pragma unroll
             for (int jj2 = 0; jj2 < 8; ++jj2) {
               zb[(j0 + jj2) * KE] = (typename Tr::Bits)(zh[jj2] >> Tr::SHIFT);
@@ -620,7 +664,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_phase1_kernel(P1Args<T, NC> 
         }
       }
       tc::tc_fence_before();
-      tc::mbar_arrive(&bars->accempty[q]);
+      tc_warp_arrive(&bars->accempty[q], lane);
       return true;
     };
     uint32_t it = 0, j = 0;
@@ -642,10 +686,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_phase1_kernel(P1Args<T, NC> 
         tc::tc_fence_after();
         const uint8_t* raw = smem + s * C::STAGE + C::B_BYTES + m * C::RS1;
         const int kl = row ? (int)min((int64_t)KC, (int64_t)I.len - (int64_t)kc * KC) : 0;
-        conv1(raw, kl, tmem + lb + (uint32_t)(ab * Tr::ACOLS), h, (T*)nullptr);
-        tc::tmem_wait_st();
+        // a warp without a column leaves its A rows as they are: they reach
+        // only its own accumulator rows, which nobody reads
+        if (32u * (warp & 3) < I.ncol) {
+          conv1(raw, kl, tmem + lb + (uint32_t)(ab * Tr::ACOLS), h, (T*)nullptr);
+          tc::tmem_wait_st();
+        }
         tc::tc_fence_before();
-        tc::mbar_arrive(&bars->afull[ab]);
+        tc_warp_arrive(&bars->afull[ab], lane);
         if (pend && kc == kd) {
           pend = false;
           if (!drain(Ip, j - 1)) { stop = true; break; }
@@ -668,6 +716,7 @@ struct P2Args {
   const TcItem2* items;
   int64_t nitems;
   const TcZ2* z2;
+  const uint32_t* blk;
   const T* pool;
   const typename TcT<T>::Bits* zt;
   double* Y;
@@ -677,118 +726,121 @@ struct P2Args {
 };
 
 template <typename T, int NC>
-__global__ void __launch_bounds__(TC_THREADS, 1) tc_phase2_kernel(P2Args<T, NC> a) {
+__global__ void __launch_bounds__(TcR2::THREADS, 1) tc_phase2_kernel(P2Args<T, NC> a) {
   using Tr = TcT<T>;
   using C = TcCfg<T, NC>;
+  using R = TcR2;
   constexpr int KE = Tr::KE, KC = Tr::KC, ES = C::ES;
   extern __shared__ __align__(1024) uint8_t smem[];
   TcBars* bars = reinterpret_cast<TcBars*>(smem + C::BAR_OFF);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t tmem = tc_setup(bars, warp, C::S, TC_NPROD + TC_PW);   // cp.async arrivals + slot-table arrivals
+  const uint32_t tmem = tc_setup(bars, warp, C::S, R::PW, R::CW);   // a producer warp's slot table and bytes
   const uint32_t sbase = tc::smem_u32(smem);
-  auto nk_of = [&](int64_t w) {
-    const TcItem2 I = a.items[w];
-    return (int)((I.ze - (I.zb / KE) * KE + KC - 1) / KC);
-  };
+  auto nk_of = [&](int64_t w) { return (int)a.items[w].nk; };
 
-  if (warp >= 8 && warp < TC_MMA_WARP) {
-    // ---------------- producers: the Z tile (one bulk copy) and each slot's rows of the tile ----------------
+  if (warp >= R::CW && warp < R::MMA) {
+    // ---------------- producers: the Z tile (a bulk copy per K block) and each slot's rows of the tile ----------------
     // warp pw handles slots SPW pw .. SPW pw + SPW - 1 of a stage; lane i
-    // (< SPW) holds slot SPW pw + i's descriptor, loaded one stage ahead; per
-    // slot the warp copies the rows lane by lane (16 bytes a lane) and lane 0
-    // writes the slot table entry
-    constexpr int SPW = KC / TC_PW;
+    // (< SPW) holds slot SPW pw + i's descriptor, loaded one stage ahead, and
+    // its K block of the stage after that; per slot the warp copies the rows
+    // lane by lane (16 bytes a lane)
+    constexpr int SPW = KC / R::PW;
     static_assert(SPW <= 32, "one descriptor per lane");
-    const int pw = warp - 8;
+    const int pw = warp - R::CW;
     uint32_t it = 0;
-    auto load_desc = [&](const TcItem2& J, int kc) {
-      const int64_t zp = (int64_t)(J.zb / KE) * KE + (int64_t)kc * KC + SPW * pw + (lane % SPW);
-      return (lane < SPW && zp >= (int64_t)J.zb && zp < (int64_t)J.ze) ? a.z2[zp] : TcZ2{0, 0, 0};
+    // a cursor over this CTA's stages
+    struct Cur { int64_t w; int kc; TcItem2 I, In; };
+    auto item = [&](int64_t w) { return w < a.nitems ? a.items[w] : TcItem2{0, 0, 0, 0}; };
+    auto step = [&](Cur& c) {
+      if (++c.kc < (int)c.I.nk) return;
+      c.w += gridDim.x;
+      c.kc = 0;
+      c.I = c.In;
+      c.In = item(c.w + gridDim.x);
     };
-    int64_t w = blockIdx.x;
-    TcItem2 I = w < a.nitems ? a.items[w] : TcItem2{};
-    int nk = w < a.nitems ? nk_of(w) : 0;
-    TcItem2 In = w + gridDim.x < a.nitems ? a.items[w + gridDim.x] : TcItem2{};
-    TcZ2 cur = w < a.nitems ? load_desc(I, 0) : TcZ2{0, 0, 0};
-    int kc = 0;
-    while (w < a.nitems) {
-      // the next stage's cursor and descriptors
-      int64_t w2 = w;
-      int kc2 = kc + 1, nk2 = nk;
-      TcItem2 I2 = I;
-      if (kc2 == nk) {
-        w2 = w + gridDim.x;
-        kc2 = 0;
-        I2 = In;
-        nk2 = w2 < a.nitems ? (int)((I2.ze - (I2.zb / KE) * KE + KC - 1) / KC) : 0;
-      }
-      const TcZ2 nxt = w2 < a.nitems ? load_desc(I2, kc2) : TcZ2{0, 0, 0};
-      {
-        // the descriptors of the stage after that into L2 (one 128-byte line
-        // holds 8 of them)
-        const int64_t zq = (int64_t)(I2.zb / KE) * KE + (int64_t)(kc2 + 1) * KC + SPW * pw + 8 * lane;
-        if (w2 < a.nitems && 8 * lane < SPW && zq < (int64_t)I2.ze)
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(a.z2 + zq));
-      }
+    const int kbl = (SPW * pw + lane % SPW) / KE;          // this lane's K block of a stage
+    auto load_blk = [&](const Cur& c) { return c.w < a.nitems ? __ldg(a.blk + (int64_t)(c.I.sb + c.kc) * TC_KB + kbl) : 0u; };
+    auto load_bz = [&](const Cur& c) {                     // the K block whose Z values lane copies (warp 0)
+      return c.w < a.nitems ? __ldg(a.blk + (int64_t)(c.I.sb + c.kc) * TC_KB + lane % TC_KB) : 0u;
+    };
+    auto load_desc = [&](uint32_t b) { return a.z2[(int64_t)b * KE + (SPW * pw + lane % SPW) % KE]; };
+    Cur c0{(int64_t)blockIdx.x, 0, item(blockIdx.x), item((int64_t)blockIdx.x + gridDim.x)};
+    Cur c2 = c0;
+    TcZ2 cur = load_desc(load_blk(c0));
+    uint32_t bz = load_bz(c0);
+    step(c2);
+    uint32_t b1 = load_blk(c2), bz1 = load_bz(c2);
+    while (c0.w < a.nitems) {
+      // the next stage's descriptors, the K blocks of the one after it
+      const TcZ2 nxt = load_desc(b1);
+      step(c2);
+      const uint32_t b2 = load_blk(c2), bz2 = load_bz(c2);
+      const TcItem2 I = c0.I;
       // this stage
       const int s = (int)(it % C::S);
       if (!tc_wait_warp(bars, &bars->empty[s], ((it / C::S) & 1u) ^ 1u, a.err, 1)) break;
       const uint32_t st = sbase + (uint32_t)(s * C::STAGE);
       int4* meta = reinterpret_cast<int4*>(smem + s * C::STAGE + C::B_BYTES + C::RAW2);
-      const int64_t zc = (int64_t)(I.zb / KE) * KE + (int64_t)kc * KC;
-      if (pw == 0 && lane == 0) {
-        tc::mbar_arrive_expect_tx(&bars->bfull[s], (uint32_t)C::B_BYTES);
-        tc::bulk_g2s(st, a.zt + (zc / KE) * (2 * NC * KE), C::B_BYTES, &bars->bfull[s]);
+      if (pw == 0) {
+        // a bulk copy per run of consecutive K blocks (each costs the warp
+        // about 80 cycles; a cluster's slots are one run)
+        const uint32_t prev = __shfl_up_sync(0xffffffffu, bz, 1);
+        const bool first = lane < TC_KB && (lane == 0 || bz != prev + 1);
+        const unsigned starts = __ballot_sync(0xffffffffu, first);
+        if (lane == 0) tc::mbar_arrive_expect_tx(&bars->bfull[s], (uint32_t)C::B_BYTES);
+        __syncwarp();
+        if (first) {
+          const unsigned later = starts & ~((2u << lane) - 1u);
+          const int len = (later ? __ffs(later) - 1 : TC_KB) - lane;
+          tc::bulk_g2s(st + lane * (C::B_BYTES / TC_KB), a.zt + (int64_t)bz * (2 * NC * KE),
+                       (uint32_t)(len * (C::B_BYTES / TC_KB)), &bars->bfull[s]);
+        }
       }
       // lane i (< SPW): slot SPW pw + i's copy and table entry
-      const int toff = (int)I.toff;
       int64_t src = 0;
       uint32_t dsto = 0, nb = 0;
       if (lane < SPW) {
         const int k = SPW * pw + lane;
-        const int r0 = max(cur.rlo, toff), r1 = min(cur.rhi, toff + 128);
+        // the tile's first row and the slot's rows of the tile, from the tile's first
+        const int64_t toff = I.row0;
+        const int64_t r0 = max((int64_t)cur.rlo, toff), r1 = min((int64_t)cur.rhi, toff + TC_ROWS);
         int4 md = make_int4(0, 0, 0, 0);
         if (r0 < r1) {
-          // element offset of window row i: g(i) = a_off + i - rlo; the raw row
+          // element offset of output row i: g(i) = a_off + i - rlo; the raw row
           // holds g(toff) - sh .. in 16-byte units (sh = g(toff) mod KE)
-          const int64_t gt = cur.a_off + (toff - cur.rlo);
+          const int64_t gt = cur.a_off + (toff - (int64_t)cur.rlo);
           const int shl = (int)(gt & (KE - 1));                 // KE is a power of two
-          const int64_t g0 = cur.a_off + (r0 - cur.rlo), g1 = cur.a_off + (r1 - cur.rlo);
+          const int64_t g0 = cur.a_off + (r0 - (int64_t)cur.rlo), g1 = cur.a_off + (r1 - (int64_t)cur.rlo);
           const int64_t slo = g0 & ~(int64_t)(KE - 1);
           const int64_t shi = (g1 + KE - 1) & ~(int64_t)(KE - 1);
           src = slo;
           dsto = (uint32_t)(C::B_BYTES + k * C::RS2 + (slo - (gt - shl)) * ES);
           nb = (uint32_t)((shi - slo) * ES);
-          md = make_int4(r0 - toff, r1 - r0, k * (C::RS2 / ES) + shl, 0);
+          md = make_int4((int)(r0 - toff), (int)(r1 - r0), k * (C::RS2 / ES) + shl, 0);
         }
         meta[k] = md;
       }
-      // the copies, slot by slot, 16 bytes a lane (whole 128-byte lines per instruction)
-#pragma unroll 4
-      for (int i = 0; i < SPW; ++i) {
-        const uint32_t nbi = __shfl_sync(0xffffffffu, nb, i);
-        const int64_t srci = (int64_t)__shfl_sync(0xffffffffu, (long long)src, i);
-        const uint32_t dsti = __shfl_sync(0xffffffffu, dsto, i);
-        if ((uint32_t)lane * 16u < nbi) tc::cp_async16(st + dsti + lane * 16, a.pool + srci + lane * KE, 16u);
-        if (lane == 0 && nbi > 512u) tc::cp_async16(st + dsti + 512, a.pool + srci + 32 * KE, 16u);
-      }
-      __threadfence_block();                                  // the table entries before lane 0's release
+      // a bulk copy per slot, after the slot table and the warp's bytes are announced
+      const uint32_t tot = __reduce_add_sync(0xffffffffu, nb);
       __syncwarp();
-      tc::cp_async_mbar_arrive(&bars->full[s]);
-      if (lane == 0) tc::mbar_arrive(&bars->full[s]);        // the slot table (release)
+      if (lane == 0) tc::mbar_arrive_expect_tx(&bars->full[s], tot);
+      __syncwarp();
+      if (nb) tc::bulk_g2s(st + dsto, a.pool + src, nb, &bars->full[s]);
       ++it;
-      if (w2 != w) In = w2 + gridDim.x < a.nitems ? a.items[w2 + gridDim.x] : TcItem2{};
-      w = w2;
-      kc = kc2;
-      nk = nk2;
-      I = I2;
+      step(c0);
       cur = nxt;
+      bz = bz1;
+      b1 = b2;
+      bz1 = bz2;
     }
-    tc::cp_async_wait_all();
-    if (pw == 0 && lane == 0) tc_copies_drain(bars, it, C::S, a.err);
-  } else if (warp == TC_MMA_WARP) {
-    if (lane == 0) tc_mma_role<T, NC>(bars, sbase, tmem, a.nitems, nk_of, tc_kseg2<NC>(), a.err);
-  } else if (warp < 8) {
+    if (lane == 0) {
+      tc_copies_drain(bars, bars->full, it, C::S, a.err);
+      if (pw == 0) tc_copies_drain(bars, bars->bfull, it, C::S, a.err);
+    }
+    __syncwarp();
+  } else if (warp == R::MMA) {
+    tc_mma_role<T, NC, TcT<T>::Z_MN>(bars, sbase, tmem, a.nitems, nk_of, tc_kseg2<NC>(), a.err);
+  } else if (warp < R::CW) {
     // ---------------- converters (thread = TMEM lane m = tile row m) + drain ----------------
     const int m = 32 * (warp & 3) + lane, h = warp >> 2;
     const uint32_t lb = (uint32_t)(32 * (warp & 3)) << 16;
@@ -800,19 +852,23 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_phase2_kernel(P2Args<T, NC> 
       const bool valid = (uint32_t)m < J.nrows;
       double* yr = a.Y + (int64_t)J.row0 + m;
 #pragma unroll 1
-      for (int j0 = h * (NC / 2); j0 < (h + 1) * (NC / 2); j0 += 8) {
+      for (int j0 = 8 * h; j0 < NC; j0 += 8 * R::NH) {
         float dd[8];
         acc_load8<T, NC>(tmem + lb + (uint32_t)(C::ACC0 + q * C::ACCW + j0), dd);
         if (valid) {
+          double* yc = yr + (int64_t)(a.cb * NC + j0) * a.ldy;
+          const int nc8 = a.ncols - (a.cb * NC + j0);
+          double y8[8];
 #pragma unroll
-          for (int jj2 = 0; jj2 < 8; ++jj2) {
-            const int col = a.cb * NC + j0 + jj2;
-            if (col < a.ncols) yr[(int64_t)col * a.ldy] += (double)dd[jj2];
-          }
+          for (int jj2 = 0; jj2 < 8; ++jj2)                // all in flight before the first store
+            y8[jj2] = jj2 < nc8 ? yc[(int64_t)jj2 * a.ldy] : 0.0;
+#pragma unroll
+          for (int jj2 = 0; jj2 < 8; ++jj2)
+            if (jj2 < nc8) yc[(int64_t)jj2 * a.ldy] = y8[jj2] + (double)dd[jj2];
         }
       }
       tc::tc_fence_before();
-      tc::mbar_arrive(&bars->accempty[q]);
+      tc_warp_arrive(&bars->accempty[q], lane);
       return true;
     };
     uint32_t it = 0, j = 0;                              // stages, accumulation segments
@@ -821,7 +877,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_phase2_kernel(P2Args<T, NC> 
     TcItem2 I = blockIdx.x < a.nitems ? a.items[blockIdx.x] : TcItem2{};
     for (int64_t w = blockIdx.x; w < a.nitems && !stop; w += gridDim.x) {
       const TcItem2 I2 = w + gridDim.x < a.nitems ? a.items[w + gridDim.x] : TcItem2{};
-      const int nk = (int)((I.ze - (I.zb / KE) * KE + KC - 1) / KC);
+      const int nk = (int)I.nk;
       for (int k0 = 0; k0 < nk && !stop; k0 += tc_kseg2<NC>(), ++j) {
         const int k1 = min(nk, k0 + tc_kseg2<NC>());
         const int kd = k0 + min(C::NA - 1, k1 - k0 - 1);  // as in phase 1, per segment
@@ -831,11 +887,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_phase2_kernel(P2Args<T, NC> 
           if (!tc_wait_warp(bars, &bars->aempty[ab], ((it / C::NA) & 1u) ^ 1u, a.err, 64)) { stop = true; break; }
           tc::tc_fence_after();
           const uint8_t* rb = smem + s * C::STAGE + C::B_BYTES;
-          conv2(rb, reinterpret_cast<const int4*>(rb + C::RAW2), m, tmem + lb + (uint32_t)(ab * Tr::ACOLS), h,
+          conv2<R::NH>(rb, reinterpret_cast<const int4*>(rb + C::RAW2), m, tmem + lb + (uint32_t)(ab * Tr::ACOLS), h,
                 (T*)nullptr);
           tc::tmem_wait_st();
           tc::tc_fence_before();
-          tc::mbar_arrive(&bars->afull[ab]);
+          tc_warp_arrive(&bars->afull[ab], lane);
           if (pend && kc == kd) {
             pend = false;
             if (!drain(Ip, j - 1)) { stop = true; break; }
@@ -1001,8 +1057,8 @@ void free_tc_plan(TcPlan*& p) {
   if (!p) return;
   if (p->d_col1) cudaFree(p->d_col1);
   if (p->d_item1) cudaFree(p->d_item1);
-  if (p->d_zpl) cudaFree(p->d_zpl);
   if (p->d_z2) cudaFree(p->d_z2);
+  if (p->d_blk) cudaFree(p->d_blk);
   if (p->d_item2) cudaFree(p->d_item2);
   delete p;
   p = nullptr;
@@ -1021,79 +1077,74 @@ static int upload_vec(V** d, const std::vector<V>& v) {
 static int build_tc_plan(hm_handle* h, int trans, TcPlan** out) {
   const int eb = elem_bytes(h->storage);
   const uint32_t KE = 16 / (uint32_t)eb;               // elements of a 16-byte K block (TcT::KE)
+  // Z slots: the low-rank leaves by output cluster (the clusters are in
+  // pre-order, so a tile's leaves lie in few runs), within one in pool order;
+  // each z is stored once.
+  const std::vector<int64_t> order = pool_order(h);
+  const int64_t n = h->n, ncl = (int64_t)h->cl_s.size();
+  std::vector<int64_t> at((size_t)ncl + 1, 0);
+  for (const Leaf& L : h->leaves)
+    if (L.type == T_RK) at[(trans ? L.t : L.s) + 1] += L.k;
+  for (int64_t c = 0; c < ncl; ++c) at[c + 1] += at[c];
+  const int64_t nz = at[ncl];
+  if (nz > (int64_t)(UINT32_MAX / 2)) return fail(HM_ERR_UNSUPPORTED, "too many low-rank terms for the tensor-core plan");
   struct Lf { int64_t li; int64_t zoff; };
-  // low-rank leaves in pool order with their z offsets
-  std::vector<int64_t> order(h->leaves.size());
-  for (size_t i = 0; i < order.size(); ++i) order[i] = (int64_t)i;
-  std::stable_sort(order.begin(), order.end(), [&](int64_t x, int64_t y) {
-    return h->leaves[x].off < h->leaves[y].off;
-  });
   std::vector<Lf> rk;
-  int64_t z = 0;
-  for (int64_t li : order) {
-    const Leaf& L = h->leaves[li];
-    if (L.type != T_RK || L.k == 0) continue;
-    rk.push_back({li, z});
-    z += L.k;
-  }
-  const int64_t zlen = z;
-  TcPlan* P = new TcPlan();
-  // ---- phase 2: windows of TC_WR output rows; Z slots window by window,
-  // items = the 128-row tiles of a window that some slot covers
-  const int64_t n = h->n;
-  const int64_t nwin = (n + TC_WR - 1) / TC_WR;
-  std::vector<std::vector<int32_t>> per(nwin);      // rk indices touching each window
-  for (size_t i = 0; i < rk.size(); ++i) {
-    const Leaf& L = h->leaves[rk[i].li];
-    const int64_t o0 = trans ? L.col0 : L.row0, o1 = o0 + (trans ? L.n : L.m);
-    for (int64_t w = o0 / TC_WR; w * TC_WR < o1; ++w) per[w].push_back((int32_t)i);
-  }
-  std::vector<TcZ2> z2;
-  std::vector<TcItem2> it2;
-  std::vector<uint32_t> zp_count(zlen + 1, 0);        // Z slots of each z, then prefix
-  for (int64_t w = 0; w < nwin; ++w)
-    for (int32_t i : per[w]) {
-      const Leaf& L = h->leaves[rk[i].li];
-      for (int r = 0; r < L.k; ++r) zp_count[rk[i].zoff + r + 1]++;
+  {
+    std::vector<int64_t> next(at.begin(), at.end() - 1);
+    for (int64_t li : order) {
+      const Leaf& L = h->leaves[li];
+      if (L.type != T_RK || L.k == 0) continue;
+      int64_t& z = next[trans ? L.t : L.s];
+      rk.push_back({li, z});
+      z += L.k;
     }
-  for (int64_t q = 0; q < zlen; ++q) zp_count[q + 1] += zp_count[q];
-  std::vector<uint32_t> zpl(zp_count[zlen]), fillpos(zp_count.begin(), zp_count.end() - 1);
-  for (int64_t w = 0; w < nwin; ++w) {
-    if (per[w].empty()) continue;
-    const uint32_t zb = (uint32_t)z2.size();
-    const int64_t wrows = std::min<int64_t>(TC_WR, n - w * TC_WR);
-    bool tile_used[TC_WR / 128] = {false, false, false, false};
-    for (int32_t i : per[w]) {
-      const Leaf& L = h->leaves[rk[i].li];
-      const int64_t npad = col_pad(L.n, eb), mpad = col_pad(L.m, eb);
-      const int64_t o0 = trans ? L.col0 : L.row0, o1 = o0 + (trans ? L.n : L.m);
-      const int64_t lo = std::max<int64_t>(o0, w * TC_WR), hi = std::min<int64_t>(o1, (w + 1) * TC_WR);
-      for (int64_t t = (lo - w * TC_WR) / 128; t * 128 < hi - w * TC_WR; ++t) tile_used[t] = true;
-      for (int r = 0; r < L.k; ++r) {
-        // F2: A (m x k, stride mpad) for H*x, B (n x k, stride npad) for H'*x
-        const int64_t col = trans ? L.off + (int64_t)r * npad : L.off + npad * L.k + (int64_t)r * mpad;
-        TcZ2 Z{};
-        Z.a_off = col + (lo - o0);
-        Z.rlo = (int32_t)(lo - w * TC_WR);
-        Z.rhi = (int32_t)(hi - w * TC_WR);
-        zpl[fillpos[rk[i].zoff + r]++] = (uint32_t)z2.size();
-        z2.push_back(Z);
+  }
+  TcPlan* P = new TcPlan();
+  // ---- phase 2: a 128-row tile takes the K blocks (KE consecutive slots)
+  // that hold a slot of a cluster with rows in the tile, each once; whole
+  // stages, filled with the zero block
+  const uint32_t zero = (uint32_t)((nz + KE - 1) / KE);
+  std::vector<TcZ2> z2((size_t)(zero + 1) * KE, TcZ2{0, 0, 0});
+  for (const Lf& f : rk) {
+    const Leaf& L = h->leaves[f.li];
+    const int64_t npad = col_pad(L.n, eb), mpad = col_pad(L.m, eb);
+    const int64_t o0 = trans ? L.col0 : L.row0, o1 = o0 + (trans ? L.n : L.m);
+    for (int r = 0; r < L.k; ++r)
+      // F2: A (m x k, stride mpad) for H*x, B (n x k, stride npad) for H'*x
+      z2[f.zoff + r] = TcZ2{trans ? L.off + (int64_t)r * npad : L.off + npad * L.k + (int64_t)r * mpad, (uint32_t)o0,
+                            (uint32_t)o1};
+  }
+  const int64_t ntile = (n + TC_ROWS - 1) / TC_ROWS;
+  std::vector<int64_t> tb((size_t)ntile + 1, 0);
+  std::vector<uint32_t> last((size_t)ntile, UINT32_MAX), blk;
+  std::vector<int64_t> fill;
+  for (int pass = 0; pass < 2; ++pass) {               // count, then write
+    for (int64_t c = 0; c < ncl; ++c) {
+      if (at[c] == at[c + 1] || h->cl_s[c] >= h->cl_e[c]) continue;
+      const uint32_t b0 = (uint32_t)(at[c] / KE), b1 = (uint32_t)((at[c + 1] - 1) / KE);
+      for (int64_t t = h->cl_s[c] / TC_ROWS; t * TC_ROWS < h->cl_e[c]; ++t) {
+        const uint32_t f = b0 + (last[t] == b0 ? 1 : 0);   // a block shared with the tile's previous cluster
+        if (f > b1) continue;
+        last[t] = b1;
+        if (pass == 0) tb[t + 1] += b1 - f + 1;
+        else
+          for (uint32_t b = f; b <= b1; ++b) blk[fill[t]++] = b;
       }
     }
-    const uint32_t ze = (uint32_t)z2.size();
-    for (int t = 0; t < TC_WR / 128 && t * 128 < wrows; ++t) {
-      if (!tile_used[t]) continue;
-      TcItem2 I{};
-      I.row0 = (uint32_t)(w * TC_WR + t * 128);
-      I.nrows = (uint32_t)std::min<int64_t>(128, wrows - t * 128);
-      I.zb = zb;
-      I.ze = ze;
-      I.toff = (uint32_t)(t * 128);
-      it2.push_back(I);
+    if (pass == 0) {
+      for (int64_t t = 0; t < ntile; ++t) tb[t + 1] = tb[t] + (tb[t + 1] + TC_KB - 1) / TC_KB * TC_KB;
+      if (tb[ntile] / TC_KB > (int64_t)(UINT32_MAX / 2)) { delete P; return fail(HM_ERR_UNSUPPORTED, "too many low-rank terms for the tensor-core plan"); }
+      blk.assign((size_t)tb[ntile], zero);
+      fill.assign(tb.begin(), tb.end() - 1);
+      std::fill(last.begin(), last.end(), UINT32_MAX);
     }
-    std::vector<int32_t>().swap(per[w]);
   }
-  if (z2.size() > (size_t)UINT32_MAX / 2) { delete P; return fail(HM_ERR_UNSUPPORTED, "too many low-rank terms for the tensor-core plan"); }
+  std::vector<TcItem2> it2;
+  for (int64_t t = 0; t < ntile; ++t)
+    if (tb[t] < tb[t + 1])
+      it2.push_back(TcItem2{(uint32_t)(t * TC_ROWS), (uint32_t)std::min<int64_t>(TC_ROWS, n - t * TC_ROWS),
+                            (uint32_t)(tb[t] / TC_KB), (uint32_t)((tb[t + 1] - tb[t]) / TC_KB)});
   // ---- phase 1: factor columns of F1 grouped by input segment, 128 per tile
   std::vector<int32_t> ord1(rk.size());
   for (size_t i = 0; i < rk.size(); ++i) ord1[i] = (int32_t)i;
@@ -1114,8 +1165,7 @@ static int build_tc_plan(hm_handle* h, int trans, TcPlan** out) {
       for (int r = 0; r < L.k; ++r) {
         TcCol1 Cc{};
         Cc.off = trans ? (uint64_t)(L.off + npad * L.k + (int64_t)r * mpad) : (uint64_t)(L.off + (int64_t)r * npad);
-        Cc.zp0 = zp_count[rk[ord1[j]].zoff + r];
-        Cc.zp1 = zp_count[rk[ord1[j]].zoff + r + 1];
+        Cc.zp = (uint32_t)(rk[ord1[j]].zoff + r);
         col1.push_back(Cc);
       }
       ++j;
@@ -1134,14 +1184,13 @@ static int build_tc_plan(hm_handle* h, int trans, TcPlan** out) {
   }
   P->ncol1 = (int64_t)col1.size();
   P->nitem1 = (int64_t)it1.size();
-  P->nzpl = (int64_t)zpl.size();
-  P->nz2 = (int64_t)z2.size();
+  P->nz2 = nz;
   P->nitem2 = (int64_t)it2.size();
   int s = HM_OK;
   if (s == HM_OK) s = upload_vec(&P->d_col1, col1);
   if (s == HM_OK) s = upload_vec(&P->d_item1, it1);
-  if (s == HM_OK) s = upload_vec(&P->d_zpl, zpl);
   if (s == HM_OK) s = upload_vec(&P->d_z2, z2);
+  if (s == HM_OK) s = upload_vec(&P->d_blk, blk);
   if (s == HM_OK) s = upload_vec(&P->d_item2, it2);
   if (s != HM_OK) { free_tc_plan(P); return s; }
   *out = P;
@@ -1190,7 +1239,7 @@ static int launch_tc(hm_handle* h, TcPlan& P, const double* d_x, double* d_y, in
   const int64_t n = h->n;
   const int64_t nkb = (n + KE + KC) / KE + 2;                   // XT blocks per shifted copy
   const int64_t xt_copy = nkb * 2 * NC * KE;
-  const int64_t zkb = (P.nz2 + KC) / KE + 2;                    // Z blocks (with zero padding)
+  const int64_t zkb = (P.nz2 + KE - 1) / KE + 1;                    // Z blocks (with zero padding)
   const size_t xt_bytes = sizeof(Bits) * (size_t)(KE * xt_copy);
   const size_t zt_bytes = sizeof(Bits) * (size_t)(zkb * 2 * NC * KE);
   const size_t need = (xt_bytes + 255) / 256 * 256 + zt_bytes;
@@ -1223,12 +1272,12 @@ static int launch_tc(hm_handle* h, TcPlan& P, const double* d_x, double* d_y, in
   for (int cb = 0; cb < ncb; ++cb) {
     tc_xt_kernel<T, NC><<<(unsigned)((nkb * KE + 63) / 64), 256, 0, st>>>(d_x, n, n, (int)ncols, cb, P.qmask, xt, nkb);
     if (P.nitem1 > 0) {
-      P1Args<T, NC> a1{P.d_item1, P.nitem1, P.d_col1, P.d_zpl, (const T*)h->d_rk, xt, xt_copy, zt, h->d_tc_err};
-      tc_phase1_kernel<T, NC><<<(unsigned)std::min<int64_t>(nsm, P.nitem1), TC_THREADS, C::BYTES, st>>>(a1);
+      P1Args<T, NC> a1{P.d_item1, P.nitem1, P.d_col1, (const T*)h->d_rk, xt, xt_copy, zt, h->d_tc_err};
+      tc_phase1_kernel<T, NC><<<(unsigned)std::min<int64_t>(nsm, P.nitem1), TcR1<T>::THREADS, C::BYTES, st>>>(a1);
     }
     if (P.nitem2 > 0) {
-      P2Args<T, NC> a2{P.d_item2, P.nitem2, P.d_z2, (const T*)h->d_rk, zt, d_y, n, (int)ncols, cb, h->d_tc_err};
-      tc_phase2_kernel<T, NC><<<(unsigned)std::min<int64_t>(nsm, P.nitem2), TC_THREADS, C::BYTES, st>>>(a2);
+      P2Args<T, NC> a2{P.d_item2, P.nitem2, P.d_z2, P.d_blk, (const T*)h->d_rk, zt, d_y, n, (int)ncols, cb, h->d_tc_err};
+      tc_phase2_kernel<T, NC><<<(unsigned)std::min<int64_t>(nsm, P.nitem2), TcR2::THREADS, C::BYTES, st>>>(a2);
     }
   }
   HM_CUDA_TRY(cudaGetLastError());
