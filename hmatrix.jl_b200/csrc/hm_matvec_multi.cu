@@ -365,112 +365,122 @@ __global__ void __launch_bounds__(MB_WARPS * 32, 1)
   }
 }
 
-// XR[i, j] = X[i + j * ldx] (j < ncols, i < n), zero elsewhere, for n + 2 rows
-__global__ void mvm_xr_kernel(const double* __restrict__ X, int64_t n, int64_t ldx, int ncols,
-                              double* __restrict__ xr, int ld) {
-  const int64_t tot = (n + 2) * ld;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = e / ld;
-    const int j = (int)(e % ld);
-    xr[e] = (i < n && j < ncols) ? X[i + (int64_t)j * ldx] : 0.0;
-  }
-}
-
 // The dense leaves' part of Y = H X alone (the tensor-core kernels add the
-// low-rank part afterwards).  One CTA per 128 output rows and column block,
-// a warp per 32 rows.  Warp 0 collects the window's dense leaves that cover
-// the tile; for each, the CTA stages the X rows of its input segment in shared
-// memory (DX_ROWS at a time, coalesced) and every warp whose rows it covers
-// streams the leaf column by column (32 consecutive rows a load, eight
-// columns in flight) against those rows.  Each warp writes its rows of Y once.
-constexpr int DX_ROWS = 64;
+// low-rank part afterwards): a warp per 32 output rows and block of 8 NT
+// columns walks its window's dense leaves, 4 x NT MMAs for every four input
+// indices, with A (the leaf) and B (X) read straight from global memory, the
+// next batch of D steps in flight while one is consumed.  Bound: FP64 from 16
+// columns on (a warp's step of 4 + NT loads feeds 4 NT MMAs), the loads'
+// latency below.  One FMA per row and column with X staged in shared memory
+// (a 16-byte shared load for two FMAs) took, with the transposed copy of X it
+// needed, 853 us against 239 (n = 2^18, 64 columns; n = 200000, 16
+// columns: 194 against 79).
+template <int NT>
+struct DensePass {
+  static constexpr int D = NT >= 8 ? 1 : NT >= 4 ? 2 : 4;       // steps of a batch
+  static constexpr int CTAS = NT >= 8 ? 2 : NT >= 4 ? 3 : 4;
+};
 
-template <typename TD, int CB>
-__global__ void __launch_bounds__(128) mvm_dense_kernel(const MvWin* __restrict__ win, const P2Desc* __restrict__ d,
-                                                        const TD* __restrict__ dn, const double* __restrict__ xr,
-                                                        int ld, int ncb, int64_t ntile, double* __restrict__ Y,
-                                                        int64_t ldy, int ncols) {
-  __shared__ P2Desc sd[32];
-  __shared__ int s_cnt;
-  __shared__ __align__(16) double xs[DX_ROWS * CB];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int cb = (int)(blockIdx.x % ncb);
-  const int64_t grow = (int64_t)(blockIdx.x / ncb) * 128;      // first output row of the tile
+template <typename TD, int NT>
+__global__ void __launch_bounds__(128, DensePass<NT>::CTAS)
+    mvm_dense_kernel(const MvWin* __restrict__ win, const P2Desc* __restrict__ d, const TD* __restrict__ dn,
+                     const double* __restrict__ X, int64_t n, int64_t ldx, int ncols, int ncb, double* __restrict__ Y,
+                     int64_t ldy) {
+  constexpr int D = DensePass<NT>::D;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const int cb = (int)(blockIdx.x % ncb) * 8 * NT;
+  const int64_t grow = ((int64_t)(blockIdx.x / ncb) * 4 + warp) * 32;   // the warp's first output row
+  if (grow >= n) return;
   const MvWin W = win[grow / MV_WROWS];
-  const int t0 = (int)(grow - W.row0);                         // tile rows [t0, t0 + 128) of the window
-  const int w0 = t0 + 32 * warp;                               // this warp's rows [w0, w0 + 32)
-  const int r = w0 + lane;
-  double acc[CB];
+  const int w0 = (int)(grow - W.row0);
+  int64_t xc[NT];                                        // this lane's columns of X (a repeated one past the last)
 #pragma unroll
-  for (int j = 0; j < CB; ++j) acc[j] = 0.0;
+  for (int j = 0; j < NT; ++j) xc[j] = (int64_t)min(cb + 8 * j + g, ncols - 1) * ldx;
+  double acc[4][NT][2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
   for (uint32_t b0 = W.begin; b0 < W.end; b0 += 32) {
-    __syncthreads();
-    if (warp == 0) {
-      const uint32_t nb = min(32u, W.end - b0);
-      P2Desc D{};
-      bool cov = false;
-      if ((uint32_t)lane < nb) {
-        D = d[b0 + lane];
-        cov = D.row_off < t0 + 128 && D.row_off + (int)D.m > t0;
+    P2Desc E{};
+    if (b0 + lane < W.end) E = d[b0 + lane];
+    unsigned todo = __ballot_sync(0xffffffffu, E.cnt > 0 && E.row_off < w0 + 32 && E.row_off + (int)E.m > w0);
+    while (todo) {
+      const int src = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const uint64_t off = __shfl_sync(0xffffffffu, (unsigned long long)E.off, src);
+      const int ro = __shfl_sync(0xffffffffu, E.row_off, src), m = (int)__shfl_sync(0xffffffffu, E.m, src);
+      const int ld = (int)__shfl_sync(0xffffffffu, E.ld, src), cnt = (int)__shfl_sync(0xffffffffu, E.cnt, src);
+      const uint32_t in0 = __shfl_sync(0xffffffffu, E.aux, src);
+      const bool tr = __shfl_sync(0xffffffffu, (int)E.type, src) == P2_DENSE_T;
+      const int64_t rs = tr ? ld : 1, cs = tr ? 1 : ld;   // strides of a row and of an input index
+      const TD* ap[4];
+      unsigned in = 0;                                    // bit i: row w0 + 8 i + g belongs to the leaf
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int lr = w0 + 8 * i + g - ro;
+        in |= (lr >= 0 && lr < m ? 1u : 0u) << i;
+        ap[i] = dn + off + min(max(lr, 0), m - 1) * rs;
       }
-      const unsigned bal = __ballot_sync(0xffffffffu, cov);
-      if (cov) sd[__popc(bal & ((1u << lane) - 1u))] = D;
-      if (lane == 0) s_cnt = __popc(bal);
-    }
-    __syncthreads();
-    const int cnt = s_cnt;
-    for (int li = 0; li < cnt; ++li) {
-      const P2Desc L = sd[li];
-      const bool wcov = L.row_off < w0 + 32 && L.row_off + (int)L.m > w0;   // uniform per warp
-      const int lr = r - L.row_off;
-      const bool mine = lr >= 0 && lr < (int)L.m;
-      const bool tr = L.type == P2_DENSE_T;
-      const TD* col = dn + L.off + (mine ? (tr ? (int64_t)lr * L.ld : (int64_t)lr) : 0);
-      const int64_t cs = tr ? 1 : (int64_t)L.ld;                // distance between the leaf's input columns
-      for (uint32_t c0 = 0; c0 < L.cnt; c0 += DX_ROWS) {
-        const int nr = (int)min((uint32_t)DX_ROWS, L.cnt - c0);
-        __syncthreads();                                         // the previous rows are consumed
-        for (int e = threadIdx.x; e < nr * (CB / 2); e += blockDim.x) {
-          const int rr = e / (CB / 2), jj = e % (CB / 2);
-          reinterpret_cast<double2*>(xs)[e] =
-              __ldg(reinterpret_cast<const double2*>(xr + (int64_t)(L.aux + c0 + rr) * ld + cb * CB) + jj);
+      const double* xp = X + in0;
+      const bool rows = __all_sync(0xffffffffu, in == 15u);
+      float an[D][4];
+      double bn[D][NT];
+      // loads are always in range (clamped); what lies outside is masked when used
+      auto fetch = [&](int c, float (&a)[D][4], double (&b)[D][NT]) {
+#pragma unroll
+        for (int e = 0; e < D; ++e) {
+          const int k = min(c + 4 * e + q, cnt - 1);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) a[e][i] = (float)__ldg(ap[i] + k * cs);
+#pragma unroll
+          for (int j = 0; j < NT; ++j) b[e][j] = __ldg(xp + k + xc[j]);
         }
-        __syncthreads();
-        if (!wcov) continue;
-        int c = 0;
-        for (; c + 8 <= nr; c += 8) {
-          double v[8];
+      };
+      fetch(0, an, bn);
+      for (int c = 0; c < cnt; c += 4 * D) {
+        float a[D][4];
+        double b[D][NT];
 #pragma unroll
-          for (int u = 0; u < 8; ++u) v[u] = mine ? (double)__ldcs(col + (int64_t)(c0 + c + u) * cs) : 0.0;
+        for (int e = 0; e < D; ++e) {
 #pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const double* xx = xs + (c + u) * CB;
+          for (int i = 0; i < 4; ++i) a[e][i] = an[e][i];
 #pragma unroll
-            for (int j = 0; j < CB; j += 2) {
-              const double2 x = *reinterpret_cast<const double2*>(xx + j);
-              acc[j] = fma(v[u], x.x, acc[j]);
-              acc[j + 1] = fma(v[u], x.y, acc[j + 1]);
-            }
+          for (int j = 0; j < NT; ++j) b[e][j] = bn[e][j];
+        }
+        fetch(c + 4 * D, an, bn);
+        if (!rows || c + 4 * D > cnt) {
+#pragma unroll
+          for (int e = 0; e < D; ++e) {
+            const bool k = c + 4 * e + q < cnt;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[e][i] = k && (in >> i & 1u) ? a[e][i] : 0.f;
+#pragma unroll
+            for (int j = 0; j < NT; ++j) b[e][j] = k ? b[e][j] : 0.0;
           }
         }
-        for (; c < nr; ++c) {
-          const double v = mine ? (double)__ldcs(col + (int64_t)(c0 + c) * cs) : 0.0;
-          const double* xx = xs + c * CB;
 #pragma unroll
-          for (int j = 0; j < CB; j += 2) {
-            const double2 x = *reinterpret_cast<const double2*>(xx + j);
-            acc[j] = fma(v, x.x, acc[j]);
-            acc[j + 1] = fma(v, x.y, acc[j + 1]);
+        for (int e = 0; e < D; ++e)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const double av = (double)a[e][i];
+#pragma unroll
+            for (int j = 0; j < NT; ++j) dmma(acc[i][j], av, b[e][j]);
           }
-        }
       }
     }
   }
-  if (r < (int)W.nrows) {
 #pragma unroll
-    for (int j = 0; j < CB; ++j) {
-      const int cl = cb * CB + j;
-      if (cl < ncols) Y[(int64_t)(W.row0 + r) + (int64_t)cl * ldy] = acc[j];
+  for (int i = 0; i < 4; ++i) {
+    const int64_t r = grow + 8 * i + g;
+    if (r < n) {
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int col = cb + 8 * j + 2 * q + c;
+          if (col < ncols) Y[r + col * ldy] = acc[i][j][c];
+        }
     }
   }
 }
@@ -563,29 +573,25 @@ int multi_t(hm_handle* h, const double* d_x, double* d_y, int64_t ncols, int tra
 }
 
 // the dense leaves (FP32) of a tensor-core call, written into Y
-template <int CB>
+template <int NT>
 int launch_dense(hm_handle* h, const double* d_x, double* d_y, int64_t ncols, int trans, cudaStream_t st) {
   MvPlan& P = trans ? h->bwd : h->fwd;
   HM_TRY(split_p2(P));
-  const int ld = (int)pad_to(ncols, CB);
-  const int ncb = ld / CB;
-  double* xr = nullptr;
-  HM_TRY(block_scratch(h, sizeof(double) * (size_t)(h->n + 2) * ld, &xr));
-  const int64_t tot = (h->n + 2) * ld;
-  mvm_xr_kernel<<<(unsigned)std::min<int64_t>((tot + 255) / 256, 148 * 16), 256, 0, st>>>(d_x, h->n, h->n, (int)ncols,
-                                                                                        xr, ld);
-  const int64_t ntile = (h->n + 127) / 128, blocks = ntile * ncb;
+  const int64_t ncb = (ncols + 8 * NT - 1) / (8 * NT), blocks = (h->n + 127) / 128 * ncb;
   if (blocks > (int64_t)INT32_MAX) return fail(HM_ERR_UNSUPPORTED, "too many dense-pass blocks");
-  mvm_dense_kernel<float, CB><<<(unsigned)blocks, 128, 0, st>>>(P.d_wind, P.d_p2d, (const float*)h->d_dense, xr, ld, ncb,
-                                                              ntile, d_y, h->n, (int)ncols);
+  mvm_dense_kernel<float, NT><<<(unsigned)blocks, 128, 0, st>>>(P.d_wind, P.d_p2d, (const float*)h->d_dense, d_x, h->n,
+                                                              h->n, (int)ncols, (int)ncb, d_y, h->n);
   HM_CUDA_TRY(cudaGetLastError());
   return HM_OK;
 }
 
+// the narrowest column block that holds the columns: a step's loads of the leaf
+// serve the whole block, and MMAs on columns that are not there cost as much
 int dense_pass(hm_handle* h, const double* d_x, double* d_y, int64_t ncols, int trans, cudaStream_t st) {
-  if (ncols <= 4) return launch_dense<4>(h, d_x, d_y, ncols, trans, st);
-  if (ncols <= 8) return launch_dense<8>(h, d_x, d_y, ncols, trans, st);
-  return launch_dense<16>(h, d_x, d_y, ncols, trans, st);
+  if (ncols <= 8) return launch_dense<1>(h, d_x, d_y, ncols, trans, st);
+  if (ncols <= 16) return launch_dense<2>(h, d_x, d_y, ncols, trans, st);
+  if (ncols <= 32) return launch_dense<4>(h, d_x, d_y, ncols, trans, st);
+  return launch_dense<8>(h, d_x, d_y, ncols, trans, st);
 }
 
 }  // namespace

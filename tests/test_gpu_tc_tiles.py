@@ -27,3 +27,19 @@ def test_tile_lists(storage, n, minb, rank):
             R = np.stack([H.matvec(X[:, j], trans=trans) for j in range(nc)], 1)
             assert np.linalg.norm(Y - R) <= TOL[storage] * np.linalg.norm(R), (nc, trans)
             assert np.abs(Y - R).max() <= 40 * TOL[storage] * np.abs(R).max(), (nc, trans)
+
+
+# the dense leaves alone (one leaf is the whole matrix, or every leaf is full
+# rank): FP64 sums of exact products of the stored FP32 entries
+@pytest.mark.parametrize("n,minb", [(5, 8), (33, 64), (64, 64), (100, 128), (301, 301)])
+def test_dense_leaves(n, minb):
+    import hmatrix as hm
+    rng = np.random.default_rng(n)
+    _, H = hm.NewHmat(hm.Params(Geom=np.sort(rng.uniform(0, 10, n)), Kernel=hm.Cauchy(1.0), MaxBlock=minb, MinBlock=minb,
+                                MaxRank=8, ConsMethod="aca2", εComp=1e-9, Tree="bisect", Storage=hm.F32))
+    D = H.to_dense()
+    for nc in (2, 7, 9, 16, 31, 64, 65):
+        X = rng.standard_normal((n, nc))
+        for A, trans in ((D, False), (D.T, True)):
+            Y = H.matvec(X, trans=trans)
+            assert np.abs(Y - A @ X).max() <= 8 * n * 2.0 ** -53 * (np.abs(A) @ np.abs(X)).max()
