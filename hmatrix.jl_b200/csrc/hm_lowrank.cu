@@ -6,11 +6,13 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 namespace hm {
 
 // ===========================================================================
-// aca2 (src/hlu.jl:59-111), one warp per block.  Deterministic pivots: the
+// aca2 (src/hlu.jl:59-111), W threads per block: a warp or a CTA of ACA_W.
+// Deterministic pivots: the
 // first row, then the arg-max of |a_r| over unused rows (the reference draws
 // a random unused row inside its "patience" loop, hlu.jl:72-85).  Up to R
 // terms; stops after the first term with |a_r||b_r|/(|a_1||b_1|) <= eps
@@ -20,6 +22,7 @@ struct AcaJob {
   int64_t row0, col0;
   int32_t m, n;
   int64_t off;      // element offset of the leaf in the low-rank pool
+  int64_t id;       // its place among the low-rank leaves (ranks, pivots)
 };
 
 // Pivots: piv (2 R entries a job: row tau_r, column sigma_r of step r) is
@@ -27,22 +30,94 @@ struct AcaJob {
 // only) takes the recorded rows and columns and runs exactly ranks[job]
 // steps with no stopping test, so that the factors of a nearby kernel come
 // from the same cross approximation and vary smoothly with its parameter.
-template <typename T>
-__global__ void __launch_bounds__(128) aca2_kernel(
+//
+// Bound: FP64 arithmetic (the kernel's and the pivot's divisions) and, below
+// it, the latency of a step.  Step r reads the r earlier columns of A and B
+// again from the block's scratch; with a warp per block some 4700 blocks were in
+// flight and their scratch (100 KB at rank 15) left L2.  50000 points in 2-D,
+// blocks of 390 x 390, both passes: 6.8 ms by warps, 4.8 by CTAs of 128 threads
+// (64: 5.4, 256: 5.3, 512: 7.8).  Blocks of at most ACA_SMALL rows and columns
+// leave a CTA's threads idle and stay with warps.
+constexpr int ACA_W = 128;
+constexpr int ACA_SMALL = 128;
+constexpr int ACA_COEF = 64;         // the largest MaxRank: factors that the entries of a step share
+
+template <int W>
+struct AcaShared {
+  double coef[W > 32 ? ACA_COEF : 1];
+  double a[2][W / 32], v[2][W / 32], s[2][W / 32];   // alternating, so that a reduction needs one barrier
+  int i[2][W / 32];
+};
+
+// arg-max (smallest index on ties) and sum over the job's W threads
+template <int W>
+__device__ __forceinline__ void aca_reduce(AcaShared<W>& sh, int par, double& best, int64_t& idx, double& val, double& sum) {
+  warp_argmax(best, idx, val);
+  sum = warp_sum(sum);
+  if constexpr (W == 32) {
+    __syncwarp();
+  } else {
+    const int w = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) {
+      sh.a[par][w] = best;
+      sh.v[par][w] = val;
+      sh.s[par][w] = sum;
+      sh.i[par][w] = idx == INT64_MAX ? INT32_MAX : (int)idx;
+    }
+    __syncthreads();
+    best = sh.a[par][0];
+    val = sh.v[par][0];
+    sum = sh.s[par][0];
+    int bi = sh.i[par][0];
+#pragma unroll
+    for (int q = 1; q < W / 32; ++q) {
+      const double a = sh.a[par][q];
+      const int i = sh.i[par][q];
+      if (a > best || (a == best && i < bi)) { best = a; val = sh.v[par][q]; bi = i; }
+      sum += sh.s[par][q];
+    }
+    idx = bi == INT32_MAX ? INT64_MAX : (int64_t)bi;
+  }
+}
+
+template <typename T, int W>
+__global__ void __launch_bounds__(W == 32 ? 128 : W, W == 32 ? 1 : 1024 / W) aca2_kernel(
     KernelDesc kd, const double* __restrict__ geom, int64_t ng, const AcaJob* __restrict__ jobs,
     int64_t njobs, int R, double eps_comp, double* __restrict__ scratch, int mcap, int ncap,
     int32_t* __restrict__ ranks, T* __restrict__ pool, int write, int32_t* __restrict__ piv, int pmode) {
-  const int lane = threadIdx.x & 31;
-  const int64_t gwarp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  double* SA = scratch + gwarp * (int64_t)R * (mcap + ncap);   // A: R columns of mcap
+  __shared__ AcaShared<W> shared[W == 32 ? 4 : 1];
+  AcaShared<W>& sh = shared[W == 32 ? threadIdx.x >> 5 : 0];
+  const int lane = threadIdx.x % W;                            // of the job's threads
+  const int64_t first = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / W;
+  const int64_t ngroup = ((int64_t)gridDim.x * blockDim.x) / W;
+  double* SA = scratch + first * (int64_t)R * (mcap + ncap);   // A: R columns of mcap
   double* SB = SA + (int64_t)R * mcap;                         // B: R columns of ncap
+  auto sync = [] { if constexpr (W == 32) __syncwarp(); else __syncthreads(); };
+  // sum_{q < r} S[q cap] F[q fcap], F's entries shared by the job's threads (the
+  // reduction before it is the barrier that ends their last use)
+  auto share = [&](const double* F, int64_t fcap, int r) {
+    if constexpr (W > 32) {
+      if (lane < r) sh.coef[lane] = F[lane * fcap];
+      __syncthreads();
+    }
+  };
+  auto dot = [&](const double* S, int64_t cap, const double* F, int64_t fcap, int r) {
+    double s = 0.0;
+    if constexpr (W > 32) {
+#pragma unroll 8
+      for (int q = 0; q < r; ++q) s = fma(S[q * cap], sh.coef[q], s);
+    } else {
+      for (int q = 0; q < r; ++q) s = fma(S[q * cap], F[q * fcap], s);
+    }
+    return s;
+  };
 
-  for (int64_t job = gwarp; job < njobs; job += nwarps) {
-    const AcaJob J = jobs[job];
+  for (int64_t jn = first; jn < njobs; jn += ngroup) {
+    const AcaJob J = jobs[jn];
+    const int64_t job = J.id;
     const int m = J.m, n = J.n;
     int tau = 0;
-    uint64_t used = 0;          // bit q of lane l: row l + 32q is used
+    uint64_t used = 0;          // bit q of thread l: row l + W q is used
     double na0 = 1.0, nb0 = 1.0;
     int rank = R;
     int32_t* jp = piv ? piv + job * 2 * (int64_t)R : nullptr;
@@ -53,48 +128,37 @@ __global__ void __launch_bounds__(128) aca2_kernel(
       // residual row tau (src/hlu.jl:73-77)
       double best = -1.0, bval = 0.0, nB = 0.0;
       int64_t bidx = INT64_MAX;
-      for (int j = lane; j < n; j += 32) {
+      share(SA + tau, mcap, r);
+      for (int j = lane; j < n; j += W) {
         double v = kernel_eval(kd, geom, ng, J.row0 + tau, J.col0 + j);
-        if (r > 0) {
-          double s = 0.0;
-          for (int q = 0; q < r; ++q) s = fma(SB[(int64_t)q * ncap + j], SA[(int64_t)q * mcap + tau], s);
-          v = v - s;
-        }
+        if (r > 0) v = v - dot(SB + j, ncap, SA + tau, mcap, r);
         SB[(int64_t)r * ncap + j] = v;
         nB = fma(v, v, nB);
         double a = fabs(v);
         if (a > best) { best = a; bidx = j; bval = v; }
       }
-      warp_argmax(best, bidx, bval);
-      nB = warp_sum(nB);
-      __syncwarp();
+      aca_reduce<W>(sh, 0, best, bidx, bval, nB);
       const int sigma = pmode == 2 ? jp[2 * r + 1] : (int)bidx;
       const double delta = pmode == 2 ? SB[(int64_t)r * ncap + sigma] : bval;
       if (!(delta != 0.0)) { rank = r; break; }      // delta == 0 (src/hlu.jl:87-89)
       if (pmode == 1 && lane == 0) { jp[2 * r] = tau; jp[2 * r + 1] = sigma; }
-      if ((tau & 31) == lane) used |= 1ull << (tau >> 5);
-      __syncwarp();
+      if (tau % W == lane) used |= 1ull << (tau / W);
       // residual column sigma, new a_r (src/hlu.jl:93-98)
       double nA = 0.0, best2 = -1.0, v2 = 0.0;
       int64_t idx2 = INT64_MAX;
-      for (int i = lane; i < m; i += 32) {
+      share(SB + sigma, ncap, r);
+      for (int i = lane; i < m; i += W) {
         double v = kernel_eval(kd, geom, ng, J.row0 + i, J.col0 + sigma);
-        if (r > 0) {
-          double s = 0.0;
-          for (int q = 0; q < r; ++q) s = fma(SA[(int64_t)q * mcap + i], SB[(int64_t)q * ncap + sigma], s);
-          v = v - s;
-        }
+        if (r > 0) v = v - dot(SA + i, mcap, SB + sigma, ncap, r);
         v = v / delta;
         SA[(int64_t)r * mcap + i] = v;
         nA = fma(v, v, nA);
-        if (!((used >> (i >> 5)) & 1ull)) {
+        if (!((used >> (i / W)) & 1ull)) {
           double a = fabs(v);
           if (a > best2) { best2 = a; idx2 = i; v2 = v; }
         }
       }
-      warp_argmax(best2, idx2, v2);
-      nA = warp_sum(nA);
-      __syncwarp();
+      aca_reduce<W>(sh, 1, best2, idx2, v2, nA);
       const double na = sqrt(nA), nb = sqrt(nB);
       if (r == 0) { na0 = na; nb0 = nb; }
       if (pmode == 2) continue;                          // replay: the recorded steps, no stopping test
@@ -111,12 +175,12 @@ __global__ void __launch_bounds__(128) aca2_kernel(
       T* Bout = pool + J.off;
       T* Aout = Bout + npad * rank;
       for (int q = 0; q < rank; ++q) {
-        for (int j = lane; j < npad; j += 32) Bout[q * npad + j] = to_store<T>(j < n ? SB[(int64_t)q * ncap + j] : 0.0);
-        for (int i = lane; i < mpad; i += 32) Aout[q * mpad + i] = to_store<T>(i < m ? SA[(int64_t)q * mcap + i] : 0.0);
+        for (int j = lane; j < npad; j += W) Bout[q * npad + j] = to_store<T>(j < n ? SB[(int64_t)q * ncap + j] : 0.0);
+        for (int i = lane; i < mpad; i += W) Aout[q * mpad + i] = to_store<T>(i < m ? SA[(int64_t)q * mcap + i] : 0.0);
       }
       if (lane == 0 && ranks[job] != rank) ranks[job] = -1 - rank;   // must match the rank pass
     }
-    __syncwarp();
+    sync();
   }
 }
 
@@ -124,27 +188,41 @@ static int aca2_launch(hm_handle* h, const std::vector<int64_t>& rk_leaf, int wr
                        std::vector<int32_t>* ranks_out, int pmode) {
   const int64_t nj = (int64_t)rk_leaf.size();
   if (nj == 0) { if (ranks_out) ranks_out->clear(); return HM_OK; }
+  // small blocks first (a warp each), then the others (a CTA each)
   std::vector<AcaJob> jobs(nj);
-  int mcap = 1, ncap = 1;
+  int mcap[2] = {1, 1}, ncap[2] = {1, 1};
+  int64_t nsmall = 0;
+  auto small = [&](const Leaf& L) { return std::max(L.m, L.n) <= ACA_SMALL; };
+  for (int64_t i = 0; i < nj; ++i) nsmall += small(h->leaves[rk_leaf[i]]);
+  int64_t at[2] = {0, nsmall};
   for (int64_t i = 0; i < nj; ++i) {
     const Leaf& L = h->leaves[rk_leaf[i]];
-    jobs[i] = AcaJob{L.row0, L.col0, L.m, L.n, L.off};
-    mcap = std::max(mcap, L.m);
-    ncap = std::max(ncap, L.n);
+    const int c = small(L) ? 0 : 1;
+    jobs[at[c]++] = AcaJob{L.row0, L.col0, L.m, L.n, L.off, i};
+    mcap[c] = std::max(mcap[c], L.m);
+    ncap[c] = std::max(ncap[c], L.n);
   }
-  if (mcap > ACA_MAX_EXTENT || ncap > ACA_MAX_EXTENT)
+  if (std::max(mcap[0], mcap[1]) > ACA_MAX_EXTENT || std::max(ncap[0], ncap[1]) > ACA_MAX_EXTENT)
     return fail(HM_ERR_UNSUPPORTED, "aca2 block larger than " + std::to_string(ACA_MAX_EXTENT));
   const int R = std::max(1, h->prm.max_rank);   // aca2(..., MaxRank-1): up to MaxRank terms
+  if (R > ACA_COEF) return fail(HM_ERR_UNSUPPORTED, "aca2 rank above " + std::to_string(ACA_COEF));
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
-  int64_t per_warp = (int64_t)R * (mcap + ncap) * 8;
-  int64_t nwarps = std::min<int64_t>((int64_t)nsm * 32, std::max<int64_t>(4, (int64_t)(1ll << 30) / per_warp));
-  nwarps = std::min<int64_t>(nwarps, (nj + 3) / 4 * 4);
-  nwarps = std::max<int64_t>(4, nwarps / 4 * 4);
+  // groups in flight: as many as run at once, within 1 GB of scratch; the two
+  // launches follow each other and share it
+  const int64_t count[2] = {nsmall, nj - nsmall};
+  int64_t per[2], groups[2], need = 0;
+  for (int c = 0; c < 2; ++c) {
+    per[c] = (int64_t)R * (mcap[c] + ncap[c]) * 8;
+    const int64_t most = c == 0 ? (int64_t)nsm * 32 : (int64_t)nsm * (1024 / ACA_W), q = c == 0 ? 4 : 1;
+    groups[c] = std::min(most, std::max<int64_t>(q, (int64_t)(1ll << 30) / per[c]));
+    groups[c] = std::min(groups[c], (count[c] + q - 1) / q * q) / q * q;
+    need = std::max(need, per[c] * groups[c]);
+  }
   double* scratch = nullptr;
   AcaJob* dj = nullptr;
   int32_t* dr = nullptr;
-  HM_CUDA_TRY(cudaMalloc(&scratch, per_warp * nwarps));
+  HM_CUDA_TRY(cudaMalloc(&scratch, need));
   HM_CUDA_TRY(cudaMalloc(&dj, sizeof(AcaJob) * nj));
   HM_CUDA_TRY(cudaMalloc(&dr, sizeof(int32_t) * nj));
   HM_CUDA_TRY(cudaMemcpyAsync(dj, jobs.data(), sizeof(AcaJob) * nj, cudaMemcpyHostToDevice, h->stream));
@@ -153,20 +231,21 @@ static int aca2_launch(hm_handle* h, const std::vector<int64_t>& rk_leaf, int wr
     for (int64_t i = 0; i < nj; ++i) kk[i] = h->leaves[rk_leaf[i]].k;
     HM_CUDA_TRY(cudaMemcpyAsync(dr, kk.data(), sizeof(int32_t) * nj, cudaMemcpyHostToDevice, h->stream));
   }
-  unsigned grid = (unsigned)(nwarps / 4);
+  auto run = [&](auto* pool) {
+    using T = std::remove_pointer_t<decltype(pool)>;
+    if (groups[0] > 0)
+      aca2_kernel<T, 32><<<(unsigned)(groups[0] / 4), 128, 0, h->stream>>>(
+          h->kd, h->d_geom, h->n, dj, count[0], R, h->prm.eps_comp, scratch, mcap[0], ncap[0], dr, pool, write,
+          h->d_piv, pmode);
+    if (groups[1] > 0)
+      aca2_kernel<T, ACA_W><<<(unsigned)groups[1], ACA_W, 0, h->stream>>>(
+          h->kd, h->d_geom, h->n, dj + nsmall, count[1], R, h->prm.eps_comp, scratch, mcap[1], ncap[1], dr, pool,
+          write, h->d_piv, pmode);
+  };
   switch (write ? h->storage : HM_F64) {
-    case HM_F64:
-      aca2_kernel<double><<<grid, 128, 0, h->stream>>>(h->kd, h->d_geom, h->n, dj, nj, R, h->prm.eps_comp,
-                                                      scratch, mcap, ncap, dr, (double*)h->d_rk, write, h->d_piv, pmode);
-      break;
-    case HM_F32:
-      aca2_kernel<float><<<grid, 128, 0, h->stream>>>(h->kd, h->d_geom, h->n, dj, nj, R, h->prm.eps_comp,
-                                                     scratch, mcap, ncap, dr, (float*)h->d_rk, write, h->d_piv, pmode);
-      break;
-    default:
-      aca2_kernel<__nv_bfloat16><<<grid, 128, 0, h->stream>>>(h->kd, h->d_geom, h->n, dj, nj, R,
-                                                             h->prm.eps_comp, scratch, mcap, ncap, dr,
-                                                             (__nv_bfloat16*)h->d_rk, write, h->d_piv, pmode);
+    case HM_F64: run((double*)h->d_rk); break;
+    case HM_F32: run((float*)h->d_rk); break;
+    default: run((__nv_bfloat16*)h->d_rk);
   }
   HM_CUDA_TRY(cudaGetLastError());
   std::vector<int32_t> ranks(nj);
