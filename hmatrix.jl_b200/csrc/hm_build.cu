@@ -522,6 +522,8 @@ void free_handle_data(hm_handle* h) {
   fr(h->d_tc);
   fr(h->d_tc_err);
   fr(h->d_piv);
+  fr(h->d_aca);
+  h->d_aca = nullptr;
   fr(h->d_dd);
   h->d_dd = nullptr;
   h->dd_bytes = 0;

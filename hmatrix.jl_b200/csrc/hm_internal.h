@@ -178,6 +178,8 @@ struct MbCol;              // hm_matvec_multi.cu
 struct MbTile;
 
 struct MvPlan {
+  void* d_desc = nullptr;          // the allocation of d_p1, d_p2 and d_win
+  size_t desc_bytes = 0;
   P1Desc* d_p1 = nullptr;
   int64_t np1 = 0;
   MbCol* d_mbcol = nullptr;        // multi-RHS phase 1 (built on first use): factor columns by input segment,
@@ -248,6 +250,7 @@ struct hm_handle {
   int* d_tc_err = nullptr;         // error word of their bounded waits
   void* d_dd = nullptr;            // compensated residual: z as hi + lo
   size_t dd_bytes = 0;
+  void* d_aca = nullptr;           // aca2 scratch, from the rank pass to the write pass
   int32_t* d_piv = nullptr;        // aca2 pivots (row, column) of every step, when kept
   int64_t piv_count = 0;
 

@@ -219,12 +219,16 @@ static int aca2_launch(hm_handle* h, const std::vector<int64_t>& rk_leaf, int wr
     groups[c] = std::min(groups[c], (count[c] + q - 1) / q * q) / q * q;
     need = std::max(need, per[c] * groups[c]);
   }
-  double* scratch = nullptr;
-  AcaJob* dj = nullptr;
-  int32_t* dr = nullptr;
-  HM_CUDA_TRY(cudaMalloc(&scratch, need));
-  HM_CUDA_TRY(cudaMalloc(&dj, sizeof(AcaJob) * nj));
-  HM_CUDA_TRY(cudaMalloc(&dr, sizeof(int32_t) * nj));
+  // one allocation, made by the rank pass and given back by the write pass (a
+  // handful made and freed twice took 3 of 17 ms at 50000 points in 2-D)
+  const size_t so = pad_to(need, 256), jo = pad_to((int64_t)(sizeof(AcaJob) * nj), 256);
+  if (!h->d_aca) {
+    cudaError_t e = cudaMalloc(&h->d_aca, so + jo + sizeof(int32_t) * nj);
+    if (e != cudaSuccess) return fail(HM_ERR_OOM, std::string("aca2 scratch: ") + cudaGetErrorString(e));
+  }
+  double* scratch = (double*)h->d_aca;
+  AcaJob* dj = (AcaJob*)((char*)h->d_aca + so);
+  int32_t* dr = (int32_t*)((char*)h->d_aca + so + jo);
   HM_CUDA_TRY(cudaMemcpyAsync(dj, jobs.data(), sizeof(AcaJob) * nj, cudaMemcpyHostToDevice, h->stream));
   if (write) {
     std::vector<int32_t> kk(nj);
@@ -251,10 +255,9 @@ static int aca2_launch(hm_handle* h, const std::vector<int64_t>& rk_leaf, int wr
   std::vector<int32_t> ranks(nj);
   HM_CUDA_TRY(cudaMemcpyAsync(ranks.data(), dr, sizeof(int32_t) * nj, cudaMemcpyDeviceToHost, h->stream));
   HM_CUDA_TRY(cudaStreamSynchronize(h->stream));
-  cudaFree(scratch);
-  cudaFree(dj);
-  cudaFree(dr);
   if (write) {
+    cudaFree(h->d_aca);
+    h->d_aca = nullptr;
     for (int64_t i = 0; i < nj; ++i)
       if (ranks[i] < 0) return fail(HM_ERR_CUDA, "aca2 write pass disagrees with the rank pass");
   } else {

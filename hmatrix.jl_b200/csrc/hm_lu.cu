@@ -505,6 +505,8 @@ struct Blk {
   int cap = 0;
   BP ch[4];
   std::vector<void*> own;
+  char* part = nullptr;               // the rest of a reserved allocation (dmalloc takes from it first)
+  size_t left = 0;
   cudaStream_t st = nullptr;
   ~Blk() {
     for (void* p : own) cudaFreeAsync(p, st);
@@ -528,10 +530,29 @@ static void* dmalloc(Ctx& c, Blk& b, size_t bytes) {
   }
   tape_note_temporary(bytes);
   void* p = nullptr;
+  const size_t r = arena_round(bytes);
+  if (r <= b.left) {
+    p = b.part;
+    b.part += r;
+    b.left -= r;
+    return p;
+  }
   cudaError_t e = cudaMallocAsync(&p, std::max<size_t>(bytes, 8), c.st);
   if (e != cudaSuccess) throw LuError(HM_ERR_OOM, std::string("H-LU temporary: ") + cudaGetErrorString(e));
   b.own.push_back(p);
   return p;
+}
+
+// One allocation for the next dmalloc calls on b, `bytes` of them in whole
+// arena_round units.  The factorisations of a batch allocate at the same time
+// and wait for one another in the allocator, up to half a millisecond a call:
+// 16 problems of 1024 to 8192 points, factorised and solved, 95.7 ms with an
+// allocation per panel and inverse, 78.4 ms so.
+static void reserve(Ctx& c, Blk& b, size_t bytes) {
+  if (c.ar || bytes == 0) return;
+  b.left = 0;
+  b.part = (char*)dmalloc(c, b, bytes);
+  b.left = bytes;
 }
 
 static BP new_dense(Ctx& c, int m, int n, int32_t s, int32_t t) {
@@ -1403,6 +1424,13 @@ static void tile_factor(Ctx& c, const hm_handle* h, TileLU& TL, const std::vecto
   TL.hold->st = c.st;
   TL.Ap.resize(T);
   TL.Bp.resize(T);
+  {
+    size_t tot = arena_round(sizeof(int32_t) * T * T) + 2 * arena_round(sizeof(void*) * T) +
+                 arena_round(sizeof(int64_t) * T) + arena_round(sizeof(int32_t) * T);
+    for (int i = 0; i < T; ++i)
+      tot += 2 * arena_round(sizeof(double) * TL.size[i] * T * cap) + arena_round(sizeof(double) * TL.size[i] * TL.size[i]);
+    reserve(c, *TL.hold, tot);
+  }
   for (int i = 0; i < T; ++i) {
     TL.Ap[i] = (double*)dmalloc(c, *TL.hold, sizeof(double) * TL.size[i] * T * cap);
     TL.Bp[i] = (double*)dmalloc(c, *TL.hold, sizeof(double) * TL.size[i] * T * cap);
@@ -1466,7 +1494,13 @@ static void tile_factor(Ctx& c, const hm_handle* h, TileLU& TL, const std::vecto
     for (int i = 0; i < T; ++i) {
       const int S = (int)TL.size[i];
       smax = std::max(smax, S);
-      TL.diag[i] = new_dense(c, S, S, gcl[i], gcl[i]);
+      TL.diag[i] = std::make_shared<Blk>();             // its array is TL.hold's
+      TL.diag[i]->st = c.st;
+      TL.diag[i]->type = T_DENSE;
+      TL.diag[i]->m = TL.diag[i]->n = S;
+      TL.diag[i]->s = TL.diag[i]->t = gcl[i];
+      TL.diag[i]->C = (double*)dmalloc(c, *TL.hold, sizeof(double) * (size_t)S * S);
+      TL.diag[i]->ldc = std::max(S, 1);
       TL.diag[i]->row0 = TL.start[i];
       cuts.clear();
       std::vector<int32_t> todo(1, dnode[i]);
@@ -1597,6 +1631,8 @@ static void tile_factor(Ctx& c, const hm_handle* h, TileLU& TL, const std::vecto
   ws.smax = smax;
   const size_t per = sizeof(double) * ((size_t)2 * smax * std::min(2 * cap, RCORE_MAX) + cap * cap);
   ws.blocks = (int)std::max<size_t>(16, std::min<size_t>(148 * 2, ((size_t)256 << 20) / per));
+  reserve(c, wsb, std::size(ws.list) * arena_round(sizeof(int32_t) * (size_t)T * T) + arena_round(8 * sizeof(int)) +
+                      arena_round(per * ws.blocks));
   for (auto& l : ws.list) l = (int32_t*)dmalloc(c, wsb, sizeof(int32_t) * (size_t)T * T);
   ws.count = (int*)dmalloc(c, wsb, 8 * sizeof(int));
   ws.scratch = dmalloc(c, wsb, per * ws.blocks);
@@ -1941,6 +1977,11 @@ static void ensure_sweep(Ctx& c, TileLU& TL) {
   int smax = 0;
   std::vector<double*> D(T);
   std::vector<const double*> inv[4];         // Lc, Uc, Ur, Lr: the matrices of which = 0..3
+  {
+    size_t tot = 4 * arena_round(sizeof(void*) * T);
+    for (int k = 0; k < T; ++k) tot += 4 * arena_round(sizeof(double) * (size_t)TL.size[k] * TL.size[k]);
+    reserve(c, *hold, tot);
+  }
   for (int k = 0; k < T; ++k) {
     const int S = (int)TL.size[k];
     smax = std::max(smax, S);

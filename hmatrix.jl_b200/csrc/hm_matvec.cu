@@ -576,10 +576,8 @@ __global__ void __launch_bounds__(SL_WARPS * 32, 2) mv_slab_kernel(const Slab* _
 // plan construction
 // ---------------------------------------------------------------------------
 void free_mv_plan(MvPlan& p) {
-  if (p.d_p1) cudaFree(p.d_p1);
+  if (p.d_desc) cudaFree(p.d_desc);
   if (p.d_mbcol) cudaFree(p.d_mbcol);
-  if (p.d_p2) cudaFree(p.d_p2);
-  if (p.d_win) cudaFree(p.d_win);
   if (p.d_p2d) cudaFree(p.d_p2d);
   if (p.d_wind) cudaFree(p.d_wind);
   if (p.d_p2r) cudaFree(p.d_p2r);
@@ -835,7 +833,20 @@ int build_mv_descriptors(hm_handle* h, const std::vector<int64_t>& order, int tr
     p1.push_back(D);
   }
   const int64_t nwin = (n + MV_WROWS - 1) / MV_WROWS;
-  std::vector<std::vector<P2Desc>> per(nwin);
+  // the windows' descriptors in pool order: count, then place
+  std::vector<int64_t> at((size_t)nwin + 1, 0);
+  for (const Leaf& L : h->leaves) {
+    if (L.type == T_RK && L.k == 0) continue;
+    const int64_t o0 = trans ? L.col0 : L.row0, oe = o0 + (trans ? L.n : L.m);
+    for (int64_t w = o0 / MV_WROWS; w * MV_WROWS < oe; ++w) ++at[w + 1];
+  }
+  for (int64_t w = 0; w < nwin; ++w) at[w + 1] += at[w];
+  if (at[nwin] > (int64_t)UINT32_MAX) return fail(HM_ERR_UNSUPPORTED, "too many matvec descriptors");
+  std::vector<MvWin> wins(nwin);
+  for (int64_t w = 0; w < nwin; ++w)
+    wins[w] = MvWin{(uint32_t)(w * MV_WROWS), (uint32_t)std::min<int64_t>(MV_WROWS, n - w * MV_WROWS), (uint32_t)at[w],
+                    (uint32_t)at[w + 1]};
+  std::vector<P2Desc> p2((size_t)at[nwin]);
   for (int64_t li : order) {
     const Leaf& L = h->leaves[li];
     if (L.type == T_RK && L.k == 0) continue;
@@ -861,33 +872,23 @@ int build_mv_descriptors(hm_handle* h, const std::vector<int64_t>& order, int tr
     for (int64_t w = o0 / MV_WROWS; w * MV_WROWS < oe; ++w) {
       P2Desc E = D;
       E.row_off = (int32_t)(o0 - w * MV_WROWS);
-      per[w].push_back(E);
+      p2[at[w]++] = E;
     }
   }
-  std::vector<P2Desc> p2;
-  std::vector<MvWin> wins(nwin);
-  for (int64_t w = 0; w < nwin; ++w) {
-    wins[w].row0 = (uint32_t)(w * MV_WROWS);
-    wins[w].nrows = (uint32_t)std::min<int64_t>(MV_WROWS, n - w * MV_WROWS);
-    wins[w].begin = (uint32_t)p2.size();
-    p2.insert(p2.end(), per[w].begin(), per[w].end());
-    wins[w].end = (uint32_t)p2.size();
-    std::vector<P2Desc>().swap(per[w]);
-  }
-  if (p2.size() > (size_t)UINT32_MAX) return fail(HM_ERR_UNSUPPORTED, "too many matvec descriptors");
   P.np1 = (int64_t)p1.size();
   P.np2 = (int64_t)p2.size();
   P.nwin = (int32_t)nwin;
-  if (!p1.empty()) {
-    HM_CUDA_TRY(cudaMalloc(&P.d_p1, sizeof(P1Desc) * p1.size()));
-    HM_CUDA_TRY(h2d_sync(P.d_p1, p1.data(), sizeof(P1Desc) * p1.size()));
-  }
-  if (!p2.empty()) {
-    HM_CUDA_TRY(cudaMalloc(&P.d_p2, sizeof(P2Desc) * p2.size()));
-    HM_CUDA_TRY(h2d_sync(P.d_p2, p2.data(), sizeof(P2Desc) * p2.size()));
-  }
-  HM_CUDA_TRY(cudaMalloc(&P.d_win, sizeof(MvWin) * nwin));
-  HM_CUDA_TRY(h2d_sync(P.d_win, wins.data(), sizeof(MvWin) * nwin));
+  // one allocation for the three lists: each takes a third of a millisecond, and
+  // as long again to free
+  const size_t b1 = sizeof(P1Desc) * p1.size(), b2 = sizeof(P2Desc) * p2.size(), bw = sizeof(MvWin) * nwin;
+  HM_CUDA_TRY(cudaMalloc(&P.d_desc, b1 + b2 + bw));
+  P.desc_bytes = b1 + b2 + bw;
+  P.d_p1 = (P1Desc*)P.d_desc;
+  P.d_p2 = (P2Desc*)((char*)P.d_desc + b1);
+  P.d_win = (MvWin*)((char*)P.d_desc + b1 + b2);
+  if (b1) HM_CUDA_TRY(h2d_sync(P.d_p1, p1.data(), b1));
+  if (b2) HM_CUDA_TRY(h2d_sync(P.d_p2, p2.data(), b2));
+  HM_CUDA_TRY(h2d_sync(P.d_win, wins.data(), bw));
   return HM_OK;
 }
 
@@ -1581,9 +1582,13 @@ int copy_handle(const hm_handle* h, hm_handle** out) {
     const MvPlan& a = t ? h->bwd : h->fwd;
     MvPlan& b = t ? c->bwd : c->fwd;
     b.np1 = a.np1; b.np2 = a.np2; b.nwin = a.nwin;
-    chk(dup((void**)&b.d_p1, a.d_p1, sizeof(P1Desc) * a.np1));
-    chk(dup((void**)&b.d_p2, a.d_p2, sizeof(P2Desc) * a.np2));
-    chk(dup((void**)&b.d_win, a.d_win, sizeof(MvWin) * a.nwin));
+    chk(dup(&b.d_desc, a.d_desc, a.desc_bytes));
+    if (s == HM_OK && b.d_desc) {
+      b.desc_bytes = a.desc_bytes;
+      b.d_p1 = (P1Desc*)b.d_desc;
+      b.d_p2 = (P2Desc*)((char*)b.d_desc + sizeof(P1Desc) * a.np1);
+      b.d_win = (MvWin*)((char*)b.d_desc + sizeof(P1Desc) * a.np1 + sizeof(P2Desc) * a.np2);
+    }
   }
   if (s == HM_OK && h->lu) s = lu_copy(h, c);
   c->factorized = h->factorized;

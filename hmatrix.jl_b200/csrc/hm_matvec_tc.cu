@@ -131,7 +131,6 @@ template <> struct TcT<float> {
   static constexpr bool SPLIT = true;               // A = A_hi + A_lo
   static constexpr int SIG = 11;                    // significant bits of the narrow format
   static constexpr int Z_MN = 0;                    // Z blocks K-major: [2 NC columns][KE slots]
-  static constexpr int SHIFT = 0;                   // its bits: the FP32 pattern >> SHIFT
   using Bits = uint32_t;
   __device__ static float hi(float x) { return tc::tf32_rn(x); }
   __device__ static Bits bits(float x) { return __float_as_uint(x); }
@@ -148,7 +147,6 @@ template <> struct TcT<__nv_bfloat16> {
   // Z blocks as 8 x 8 core matrices [slot][column]: a phase-1 row (one slot)
   // writes 16 bytes for 8 columns instead of 8 scattered 2-byte pieces
   static constexpr int Z_MN = 1;
-  static constexpr int SHIFT = 16;                  // (BF16 pieces are packed with byte permutes)
   using Bits = uint16_t;
   __device__ static float hi(float x) { return tc::bf16_rn(x); }
   __device__ static Bits bits(float x) { return (uint16_t)(__float_as_uint(x) >> 16); }
@@ -555,6 +553,7 @@ __global__ void __launch_bounds__(TcR1<T>::THREADS, 1) tc_phase1_kernel(P1Args<T
   using Tr = TcT<T>;
   using C = TcCfg<T, NC>;
   using R = TcR1<T>;
+  static_assert(R::NH == 2, "conv1 takes half of a stage");
   constexpr int KE = Tr::KE, KC = Tr::KC;
   extern __shared__ __align__(1024) uint8_t smem[];
   TcBars* bars = reinterpret_cast<TcBars*>(smem + C::BAR_OFF);
@@ -657,8 +656,8 @@ __global__ void __launch_bounds__(TcR1<T>::THREADS, 1) tc_phase1_kernel(P1Args<T
           } else {
 #pragma unroll
             for (int jj2 = 0; jj2 < 8; ++jj2) {
-              zb[(j0 + jj2) * KE] = (typename Tr::Bits)(zh[jj2] >> Tr::SHIFT);
-              zb[NC * KE + (j0 + jj2) * KE] = (typename Tr::Bits)(zl[jj2] >> Tr::SHIFT);
+              zb[(j0 + jj2) * KE] = (typename Tr::Bits)zh[jj2];
+              zb[NC * KE + (j0 + jj2) * KE] = (typename Tr::Bits)zl[jj2];
             }
           }
         }
