@@ -494,7 +494,7 @@ int hm_set_tune(hm_handle* h, int32_t p2_split, int32_t p1_waves) {
     return fail(HM_ERR_ARG, "phase-2 shape must be 1, 2, 4 or 8");
   if (p1_waves != 1 && p1_waves != 2 && p1_waves != 4) return fail(HM_ERR_ARG, "phase-1 waves must be 1, 2 or 4");
   if (p2_split == 1 && h->storage == HM_BF16)
-    return fail(HM_ERR_UNSUPPORTED, "phase 2 by tree clusters needs FP64 or FP32 factors");
+    return fail(HM_ERR_UNSUPPORTED, "phase 2 by row slabs is set by hand for FP64 or FP32 factors only");
   h->tune.p2_split = p2_split;
   h->tune.p1_waves = p1_waves;
   return HM_OK;

@@ -754,11 +754,17 @@ static int build_slab_plan(hm_handle* h, int trans, MvPlan& P) {
   const size_t sb = sizeof(Slab) * slab.size(), so = pad_to((int64_t)sb, 256);
   void* keep = nullptr;                                  // slabs and entries
   void* tmp = nullptr;
-  if (cudaMalloc(&keep, so + sizeof(SlabEnt) * std::max<size_t>(tot, 1)) != cudaSuccess) {
+  // small leaf lists stay behind the entries: an allocation of their own costs
+  // a small matrix's first product more than the product
+  const size_t ent_bytes = pad_to((int64_t)(sizeof(SlabEnt) * std::max<size_t>(tot, 1)), 256);
+  const bool behind = lb + pb <= (size_t)1 << 20;
+  if (cudaMalloc(&keep, so + ent_bytes + (behind ? lb + pb : 0)) != cudaSuccess) {
     cudaGetLastError();
     return HM_ERR_OOM;
   }
-  if (cudaMallocAsync(&tmp, std::max<size_t>(lb + pb, 8), h->stream) != cudaSuccess) {
+  if (behind) {
+    tmp = (char*)keep + so + ent_bytes;
+  } else if (cudaMallocAsync(&tmp, lb + pb, h->stream) != cudaSuccess) {
     cudaGetLastError();
     cudaFree(keep);
     return HM_ERR_OOM;
@@ -775,7 +781,7 @@ static int build_slab_plan(hm_handle* h, int trans, MvPlan& P) {
       e = cudaGetLastError();
     }
   }
-  cudaFreeAsync(tmp, h->stream);
+  if (!behind) cudaFreeAsync(tmp, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);   // the caller's stream reads the entries next
   if (e != cudaSuccess) {
     cudaFree(keep);

@@ -498,8 +498,24 @@ int block_scratch(hm_handle* h, size_t bytes, double** out) {
   return HM_OK;
 }
 
+// A leaf's factor columns in the table: columns [at, at + k), column r at pool
+// element off + r stride, row z + r of Z
+struct MbLeaf {
+  uint64_t off, z;
+  uint32_t at, stride, k, pad;
+};
+__global__ void __launch_bounds__(256) mb_column_kernel(const MbLeaf* __restrict__ leaf, int64_t nleaf,
+                                                        MbCol* __restrict__ col) {
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 8;   // eight threads a leaf
+  if (i >= nleaf) return;
+  const MbLeaf L = leaf[i];
+  for (uint32_t r = threadIdx.x % 8; r < L.k; r += 8)
+    col[(uint64_t)L.at + r] = MbCol{L.off + (uint64_t)r * L.stride, L.z + r};
+}
+
 // The factor columns of phase 1 by input segment (the clusters' pre-order
-// starts), 32 to a tile; within a segment in pool order.
+// starts), 32 to a tile; within a segment in pool order.  The device writes the
+// table from the leaves: made on the host it took 3 of a first call's 9.5 ms (n = 2^17).
 int ensure_columns(hm_handle* h, int trans, MvPlan& P) {
   if (P.d_mbcol || P.np1 == 0) return HM_OK;
   const int eb = elem_bytes(h->storage);
@@ -510,30 +526,60 @@ int ensure_columns(hm_handle* h, int trans, MvPlan& P) {
     if (L.type == T_RK) at[(trans ? L.s : L.t) + 1] += L.k;
   for (int64_t c = 0; c < ncl; ++c) at[c + 1] += at[c];
   const int64_t ntot = at[ncl];
-  std::vector<MbCol> col((size_t)ntot);
+  if (ntot > (int64_t)UINT32_MAX) return fail(HM_ERR_UNSUPPORTED, "too many factor columns");
   std::vector<MbTile> tile;
   for (int64_t c = 0; c < ncl; ++c)
     for (int64_t b = at[c]; b < at[c + 1]; b += 8 * MB_MT)
       tile.push_back(MbTile{(uint32_t)b, (uint32_t)std::min<int64_t>(8 * MB_MT, at[c + 1] - b), (uint32_t)h->cl_s[c],
                             (uint32_t)(h->cl_e[c] - h->cl_s[c])});
   uint64_t z = 0;
+  std::vector<MbLeaf> leaf;
+  leaf.reserve(order.size());
   for (int64_t li : order) {
     const Leaf& L = h->leaves[li];
-    if (L.type != T_RK) continue;
+    if (L.type != T_RK || L.k == 0) continue;
     const int64_t npad = col_pad(L.n, eb), mpad = col_pad(L.m, eb);
     int64_t& next = at[trans ? L.s : L.t];
-    for (int r = 0; r < L.k; ++r)
-      col[next++] = MbCol{(uint64_t)(trans ? L.off + npad * L.k + r * mpad : L.off + r * npad), z++};
+    leaf.push_back(MbLeaf{(uint64_t)(trans ? L.off + npad * L.k : L.off), z, (uint32_t)next,
+                          (uint32_t)(trans ? mpad : npad), (uint32_t)L.k, 0});
+    next += L.k;
+    z += (uint64_t)L.k;
   }
-  const size_t cb = sizeof(MbCol) * col.size();
+  const size_t cb = sizeof(MbCol) * (size_t)ntot, lb = sizeof(MbLeaf) * leaf.size();
   void* d = nullptr;
-  cudaError_t e = cudaMalloc(&d, cb + sizeof(MbTile) * tile.size());
-  if (e != cudaSuccess) return fail(HM_ERR_OOM, std::string("block product columns: ") + cudaGetErrorString(e));
-  P.d_mbcol = (MbCol*)d;                                 // owned by the plan from here on
+  void* tmp = nullptr;
+  const size_t tl = pad_to((int64_t)(sizeof(MbTile) * tile.size()), 256);
+  const bool behind = lb <= (size_t)1 << 20;             // a small leaf list stays behind the tables
+  cudaError_t e = cudaMalloc(&d, cb + tl + (behind ? lb : 0));
+  if (e == cudaSuccess && behind) {
+    tmp = (char*)d + cb + tl;
+  } else if (e == cudaSuccess && cudaMallocAsync(&tmp, lb, h->stream) != cudaSuccess) {
+    cudaFree(d);
+    e = cudaErrorMemoryAllocation;
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(HM_ERR_OOM, std::string("block product columns: ") + cudaGetErrorString(e));
+  }
+  if (lb) {
+    e = cudaMemcpyAsync(tmp, leaf.data(), lb, cudaMemcpyHostToDevice, h->stream);
+    if (e == cudaSuccess) {
+      mb_column_kernel<<<(unsigned)((leaf.size() + 31) / 32), 256, 0, h->stream>>>((const MbLeaf*)tmp,
+                                                                                  (int64_t)leaf.size(), (MbCol*)d);
+      e = cudaGetLastError();
+    }
+  }
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync((char*)d + cb, tile.data(), sizeof(MbTile) * tile.size(), cudaMemcpyHostToDevice, h->stream);
+  if (!behind) cudaFreeAsync(tmp, h->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);   // the caller's stream reads the table next
+  if (e != cudaSuccess) {
+    cudaFree(d);
+    return fail(HM_ERR_CUDA, std::string("block product columns: ") + cudaGetErrorString(e));
+  }
+  P.d_mbcol = (MbCol*)d;
   P.d_mbtile = (MbTile*)((char*)d + cb);
   P.nmbtile = (int64_t)tile.size();
-  HM_CUDA_TRY(h2d_sync(P.d_mbcol, col.data(), cb));
-  HM_CUDA_TRY(h2d_sync(P.d_mbtile, tile.data(), sizeof(MbTile) * tile.size()));
   return HM_OK;
 }
 
@@ -597,9 +643,9 @@ int dense_pass(hm_handle* h, const double* d_x, double* d_y, int64_t ncols, int 
 }  // namespace
 
 // FP64 factors (no tensor-core kind for FP64), simt, or factors beyond the
-// tensor-core path's range (2^100): the CUDA-core block kernels for the whole
-// product.  FP32/BF16 factors: the dense leaves on the CUDA cores (they write
-// every row of Y), then the low-rank part on the tensor cores (added into Y).
+// tensor-core path's range (2^100): the FP64 block kernels for the whole
+// product.  FP32/BF16 factors: the dense leaves in FP64 (written into every
+// row of Y), then the low-rank part on the tensor cores (added into Y).
 int matvec_multi_device(hm_handle* h, const double* d_x, double* d_y, int64_t ncols, int trans, cudaStream_t st,
                         bool simt) {
   if (ncols <= 0) return HM_OK;

@@ -13,9 +13,9 @@
 //   it takes, 16 to a stage, and its Z tile is gathered block by block.  (Z
 //   slots copied per window of 512 rows cost phase 1 a serial chain of copies
 //   for each long column, and phase 2 every small leaf of the window in all
-//   four of its tiles: n = 2^18, 64 columns, BF16: phases 1 + 2 669 + 631 us, now 272 + 333; n = 200000,
-//   16 columns, FP32: 484 + 1190 us, now 418 + 545.)  The dense
-//   leaves are added by the CUDA-core block kernel first.
+//   four of its tiles.  Phases 1 and 2, n = 2^18, 64 columns, BF16: 669 and 631
+//   us so, now 272 and 333; n = 200000, 16 columns, FP32: 484 and 1190 us, now
+//   418 and 545.)  The dense leaves are written by mvm_dense_kernel first.
 //
 // Data movement.  Factor columns are contiguous in the pool, so a pipeline
 // stage takes one contiguous piece of each factor column it needs into a raw
@@ -1297,7 +1297,7 @@ static int tc_dispatch(hm_handle* h, TcPlan& P, const double* d_x, double* d_y, 
 
 // Builds the plan of a direction on first use and reports whether the
 // tensor-core path applies (FP32/BF16 factors, all of them at most 2^100 in
-// magnitude); otherwise the caller takes the CUDA-core block kernels.
+// magnitude); otherwise the caller takes the FP64 block kernels.
 int tc_prepare(hm_handle* h, int trans, bool* usable) {
   *usable = false;
   if (h->storage != HM_F32 && h->storage != HM_BF16) return HM_OK;
