@@ -68,7 +68,7 @@ extern "C" {
 #define HM_FLAG_DEVICE_PTRS 1u
 #define HM_FLAG_TRANS       2u   /* hm_solve / hm_solve_refined: solve with H' */
 #define HM_FLAG_MV_SIMT     4u   /* hm_matvec, several columns, FP32/BF16 factors:
-                                    the CUDA-core block kernels instead of the
+                                    the FP64 block kernels instead of the
                                     tensor cores                                */
 
 /* Mirror of the reference's global Params (src/utils.jl:8-24) restricted
