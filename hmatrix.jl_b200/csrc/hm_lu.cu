@@ -1697,7 +1697,9 @@ __device__ __forceinline__ void sweep_factors(const SweepTab& t, int i, int s, b
   }
 }
 
-// zsh[q + c r] = (Q' y_s)[q, c], y_s = the finished tile s in F
+// zsh[q + c r] = (Q' y_s)[q, c], y_s = the finished tile s in F.  Plain loads
+// of y_s: the step that writes it may still run when this one starts (dependent
+// launches), and the non-coherent load asks for data nobody writes meanwhile.
 __device__ void sweep_z(const SweepTab& t, const double* F, int64_t ldy, int nc, int s, const double* Q, int r,
                         double* zsh) {
   const int Ss = t.size[s];
@@ -1708,7 +1710,7 @@ __device__ void sweep_z(const SweepTab& t, const double* F, int64_t ldy, int nc,
     double acc = 0.0;
 #pragma unroll 8
     for (int row = lane; row < Ss; row += 32)
-      acc = fma(__ldg(Q + row + (int64_t)q * Ss), __ldg(ys + row + cc * ldy), acc);
+      acc = fma(__ldg(Q + row + (int64_t)q * Ss), ys[row + cc * ldy], acc);
     acc = warp_sum(acc);
     if (lane == 0) zsh[q + cc * r] = acc;
   }
