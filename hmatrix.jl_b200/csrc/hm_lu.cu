@@ -1368,37 +1368,46 @@ static void recompress_pairs_t(Ctx& c, const TileLU& TL, const PairLists& W, int
     a.in = W.list[i]; a.nin = W.count + i;
     a.out = i < 2 ? W.list[i + 1] : nullptr; a.nout = i < 2 ? W.count + i + 1 : nullptr;
   };
+  // what the later kernels take: up to 24 columns of 256 rows, or what else fits
+  // twice on an SM, staged in shared memory; the rest in scratch.  Each follows
+  // where some pair is left to it: the register kernels hold 12 columns, but only
+  // of tiles of up to 512 rows.
+  const int rl = (int)std::min<size_t>(24, (104 * 1024 / sizeof(TS) - c.cap * c.cap) / (2 * W.smax + 3 * 25));
+  const int rmax = std::min(2 * c.cap, RCORE_MAX);
+  const int taken = W.smax <= 512 ? 12 : 0;
+  const bool staged = rl > taken && rmax > taken, scratch = rmax > std::max(rl, taken);
+  auto smem = [&](int q, bool st) {
+    return sizeof(TS) * ((size_t)3 * q * (q + 1) + (st ? (size_t)2 * W.smax * q + c.cap * c.cap : 0));
+  };
   const unsigned pers = (unsigned)std::min<int64_t>(njobs, 148 * 4);
+  // the second register kernel; with nothing behind it a pair it cannot take is an error
+  auto second = [&] {
+    next(0);
+    if (!staged && !scratch) a.out = nullptr;
+  };
   if (W.smax <= 256) {
     lu_pair_kernel<TS, 1, 8><<<(unsigned)njobs, 64, 0, c.st>>>(a);
     LU_LAUNCH_CHECK();
-    next(0);
+    second();
     lu_pair_kernel<TS, 1, 12><<<pers, 64, 0, c.st>>>(a);
   } else {
     lu_pair_kernel<TS, 2, 8><<<(unsigned)njobs, 128, 0, c.st>>>(a);
     LU_LAUNCH_CHECK();
-    next(0);
+    second();
     lu_pair_kernel<TS, 2, 12><<<pers, 128, 0, c.st>>>(a);
   }
   LU_LAUNCH_CHECK();
-  next(1);
-  // up to 24 columns of 256 rows, or what else fits twice on an SM, staged in
-  // shared memory; the rest in scratch
-  const int rl = (int)std::min<size_t>(24, (104 * 1024 / sizeof(TS) - c.cap * c.cap) / (2 * W.smax + 3 * 25));
-  const int rmax = std::min(2 * c.cap, RCORE_MAX);
-  auto smem = [&](int q, bool staged) {
-    return sizeof(TS) * ((size_t)3 * q * (q + 1) + (staged ? (size_t)2 * W.smax * q + c.cap * c.cap : 0));
-  };
   if (smem_attr((const void*)lu_tile_core_kernel<TS>, (int)sizeof(double) * 3 * RCORE_MAX * (RCORE_MAX + 1)) != cudaSuccess)
     throw LuError(HM_ERR_CUDA, "tile core smem");
-  if (rl > 12) {
+  if (staged) {
+    next(1);
+    if (!scratch) a.out = nullptr;
     lu_tile_core_kernel<TS><<<std::min<unsigned>(pers, 148 * 2), 128, smem(rl, true), c.st>>>(a, rl, W.smax, (TS*)nullptr);
     LU_LAUNCH_CHECK();
-    next(2);
-  } else {
-    a.out = nullptr;
   }
-  if (rmax > std::max(rl, 12)) {
+  if (scratch) {
+    next(staged ? 2 : 1);
+    a.out = nullptr;
     lu_tile_core_kernel<TS><<<std::min<unsigned>(pers, (unsigned)W.blocks), 128, smem(rmax, false), c.st>>>(
         a, rmax, W.smax, (TS*)W.scratch);
     LU_LAUNCH_CHECK();

@@ -139,7 +139,10 @@ __global__ void __launch_bounds__(64 * WPS) lu_pair_kernel(PairArgs a) {
       continue;
     }
     if (r > RMAX || max(max(v.m, v.n), v.s) > 32 * WPS * ROWS) {
-      if (threadIdx.x == 0) a.out[atomicAdd(a.nout, 1)] = (int32_t)pq;
+      if (threadIdx.x == 0) {
+        if (a.out) a.out[atomicAdd(a.nout, 1)] = (int32_t)pq;
+        else atomicOr(a.flags, 1);     // nobody is left to take it (the host launches a kernel for every size)
+      }
       continue;
     }
     __syncthreads();                   // the previous pair's shared memory
@@ -359,7 +362,7 @@ __global__ void __launch_bounds__(128) lu_tile_core_kernel(PairArgs a, int rl, i
     if (r > rl) {
       if (threadIdx.x == 0) {
         if (a.out) a.out[atomicAdd(a.nout, 1)] = a.in[b];
-        else atomicOr(a.flags, 1);     // cannot happen: the last kernel takes 2 cap columns
+        else atomicOr(a.flags, 1);     // nobody is left to take it (the last kernel holds 2 cap columns)
       }
       continue;
     }
