@@ -628,6 +628,14 @@ static void trsm_lower(Ctx& c, View L, View X, bool unit) {
   LU_LAUNCH_CHECK();
 }
 
+// rows of a diagonal leaf at most, of the recursion (the leaf and its pivots in
+// 200 KB) and of the tiles (lu_diag_kernel<160>)
+constexpr int LU_LEAF_MAX = 159;
+static_assert(sizeof(double) * LU_LEAF_MAX * LU_LEAF_MAX + sizeof(int) * LU_LEAF_MAX <= 200 * 1024, "leaf in shared memory");
+[[noreturn]] static void leaf_too_large() {
+  throw LuError(HM_ERR_UNSUPPORTED, "diagonal leaf above " + std::to_string(LU_LEAF_MAX) + " rows (MinBlock too large)");
+}
+
 static void getrf(Ctx& c, View C, int64_t goff) {
   const int m = C.rows;
   if (m != C.cols) throw LuError(HM_ERR_UNSUPPORTED, "non-square diagonal leaf");
@@ -636,8 +644,8 @@ static void getrf(Ctx& c, View C, int64_t goff) {
     LU_LAUNCH_CHECK();
     return;
   }
+  if (m > LU_LEAF_MAX) leaf_too_large();
   const size_t smem = sizeof(double) * (size_t)m * m + sizeof(int) * m;
-  if (smem > 200 * 1024) throw LuError(HM_ERR_UNSUPPORTED, "diagonal leaf above 150 rows (MinBlock too large)");
   if (smem_attr((const void*)lu_getrf_kernel, 200 * 1024) != cudaSuccess)
     throw LuError(HM_ERR_CUDA, "getrf smem attribute");
   lu_getrf_kernel<<<1, 256, smem, c.st>>>(C, c.P, goff, c.flags);
@@ -1554,7 +1562,7 @@ static void tile_factor(Ctx& c, const hm_handle* h, TileLU& TL, const std::vecto
       if (next != S) throw LuError(HM_ERR_UNSUPPORTED, "diagonal leaves do not cover their tile");
       leaf.push_back(S);
     }
-    if (mmax > 150) throw LuError(HM_ERR_UNSUPPORTED, "diagonal leaf above 150 rows (MinBlock too large)");
+    if (mmax > LU_LEAF_MAX) leaf_too_large();
     for (size_t b = 0; b < jobs.size(); b += (size_t)1 << 30) {
       const size_t nb = std::min<size_t>((size_t)1 << 30, jobs.size() - b);
       Blk tmp;
