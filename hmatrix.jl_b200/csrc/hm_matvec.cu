@@ -426,8 +426,7 @@ __global__ void __launch_bounds__(P2Shape<SPLIT>::WARPS * 32) mv_phase2_kernel(c
 constexpr int SL_WARPS = 8;
 constexpr int SL_RMAX = 7;                     // rows a lane at most
 
-// one element of a factor or dense leaf: how it is loaded and its value in the
-// kernel's arithmetic (FP64 factors: FP64, the others FP32 products)
+// one element of a factor or dense leaf: how it is loaded and its value
 template <typename E> struct SlT {
   using Raw = E;
   __device__ static Raw ld(const E* p) { return __ldcs(p); }
@@ -482,7 +481,7 @@ __device__ __forceinline__ void slab_sum(const SlabEnt* __restrict__ ents, uint3
 #pragma unroll
         for (int q = 0; q < R; ++q)
           if (first[u] + 32 * q <= span[u]) {            // rows not covered: an infinite z stays out
-            if constexpr (std::is_same<A, double>::value) acc[q] = fma(SlT<E>::val(raw[u][q]), zz, acc[q]);
+            if constexpr (std::is_same<A, double>::value) acc[q] = fma((A)SlT<E>::val(raw[u][q]), zz, acc[q]);
             else part[q] = fmaf(SlT<E>::val(raw[u][q]), zz, part[q]);
           }
         // FP32 products and partial sums over 8 entries, folded into the FP64
@@ -506,12 +505,15 @@ template <typename T, typename TD, int R>
 __device__ __forceinline__ void slab_rows(const Slab& S, const SlabEnt* __restrict__ ents, const T* __restrict__ rk,
                                           const TD* __restrict__ dn, const double* __restrict__ z,
                                           const double* __restrict__ x, double* __restrict__ part_sh, int warp, int lane) {
+  // the dense leaves of BF16 factors (near field, FP32) are FP64 products, as
+  // they are in every other shape and direction
   using A = typename std::conditional<std::is_same<T, double>::value, double, float>::type;
+  using AD = typename std::conditional<std::is_same<T, float>::value, float, double>::type;
   double acc[R];
 #pragma unroll
   for (int q = 0; q < R; ++q) acc[q] = 0.0;
   slab_sum<T, A, R>(ents, S.begin, S.dense - S.begin, rk, z, warp, lane, acc);
-  slab_sum<TD, A, R>(ents, S.dense, S.mid - S.dense, dn, x, warp, lane, acc);
+  slab_sum<TD, AD, R>(ents, S.dense, S.mid - S.dense, dn, x, warp, lane, acc);
   // dense leaves read along their rows (H'x): an entry is 32 input indices of
   // one leaf; lane = input index (coalesced), 16 rows at a time, whose sums
   // over the lanes a reduce-scatter leaves in lanes 2 i and 2 i + 1
