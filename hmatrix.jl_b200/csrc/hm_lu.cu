@@ -1380,12 +1380,14 @@ static void recompress_pairs_t(Ctx& c, const TileLU& TL, const PairLists& W, int
   // twice on an SM, staged in shared memory; the rest in scratch.  Each follows
   // where some pair is left to it: the register kernels hold 12 columns, but only
   // of tiles of up to 512 rows.
-  const int rl = (int)std::min<size_t>(24, (104 * 1024 / sizeof(TS) - c.cap * c.cap) / (2 * W.smax + 3 * 25));
+  const int rl =
+      (int)std::min<size_t>(24, (104 * 1024 - sizeof(double) * c.cap * c.cap) / (sizeof(TS) * (2 * W.smax + 3 * 25)));
   const int rmax = std::min(2 * c.cap, RCORE_MAX);
   const int taken = W.smax <= 512 ? 12 : 0;
   const bool staged = rl > taken && rmax > taken, scratch = rmax > std::max(rl, taken);
   auto smem = [&](int q, bool st) {
-    return sizeof(TS) * ((size_t)3 * q * (q + 1) + (st ? (size_t)2 * W.smax * q + c.cap * c.cap : 0));
+    return sizeof(TS) * ((size_t)3 * q * (q + 1) + (st ? (size_t)2 * W.smax * q : 0)) +
+           (st ? sizeof(double) * c.cap * c.cap : 0);
   };
   const unsigned pers = (unsigned)std::min<int64_t>(njobs, 148 * 4);
   // the second register kernel; with nothing behind it a pair it cannot take is an error

@@ -85,13 +85,13 @@ __device__ __forceinline__ PairView pair_view(const PairArgs& a, int64_t q) {
 // columns a pair took 71,000 cycles with three pairs an SM (15,000 of them
 // reading A_ik W from memory, 23,000 in block-wide Gram-Schmidt, 19,000 in the
 // SVD).  Ranks here are 3 to 5 at n = 65536 (eps 1e-10).
-template <typename TS, int WPS>
+template <int WPS>
 struct SideSum {                       // sums over a side's threads
-  TS (*red)[WPS][16];                  // [parity][warp][value]
+  double (*red)[WPS][16];              // [parity][warp][value]
   int side, warp, lane, par;
   // the values [from, to)
-  template <int NV>
-  __device__ __forceinline__ void operator()(TS (&v)[NV], int from, int to) {
+  template <typename V, int NV>
+  __device__ __forceinline__ void operator()(V (&v)[NV], int from, int to) {
 #pragma unroll
     for (int i = 0; i < NV; ++i)
       if (i >= from && i < to) {
@@ -106,9 +106,9 @@ struct SideSum {                       // sums over a side's threads
 #pragma unroll
       for (int i = 0; i < NV; ++i)
         if (i >= from && i < to) {
-          TS s = red[par][0][i];
+          V s = (V)red[par][0][i];
 #pragma unroll
-          for (int w = 1; w < WPS; ++w) s += red[par][w][i];
+          for (int w = 1; w < WPS; ++w) s += (V)red[par][w][i];
           v[i] = s;
         }
       par ^= 1;
@@ -119,10 +119,17 @@ struct SideSum {                       // sums over a side's threads
 template <typename TS, int WPS, int RMAX>
 __global__ void __launch_bounds__(64 * WPS) lu_pair_kernel(PairArgs a) {
   constexpr int ROWS = 8, CAPW = 48;   // rows a lane; rank capacity (RCORE_MAX / 2)
-  __shared__ TS sW[CAPW * RMAX];       // W, ka x kb
+  // W and A_ik W are FP64 sums of FP64 factors whatever TS is: what is subtracted
+  // from A_ij must not carry the core's rounding.  FP64 cores form them in x's
+  // registers, FP32 ones WC columns at a time in registers of their own (2: 180
+  // to 226 registers, 4: 252 to 255).  In FP32 the factors of a mixed LU were 22 %
+  // further from the FP64 ones (8 tiles of 250 rows, l = 40: 2.4e-6 against 2.0e-6
+  // of the norm) and no faster (n = 8192 14.6 ms, now 14.4; 65536 200 and 211).
+  constexpr int WC = sizeof(TS) == 8 ? RMAX : 2;
+  __shared__ double sW[CAPW * RMAX];   // W, ka x kb
   __shared__ TS sR[2][RMAX * RMAX];    // R of either side, then the coefficients of either output
   __shared__ TS sC[RMAX * (RMAX | 1)], sV[RMAX * (RMAX | 1)];
-  __shared__ TS sred[2][2][WPS][16];
+  __shared__ double sred[2][2][WPS][16];
   __shared__ TS sig[RMAX];
   __shared__ int ord[RMAX], s_k;
   const int side = threadIdx.x / (32 * WPS), st = threadIdx.x % (32 * WPS), lane = threadIdx.x & 31;
@@ -146,14 +153,14 @@ __global__ void __launch_bounds__(64 * WPS) lu_pair_kernel(PairArgs a) {
       continue;
     }
     __syncthreads();                   // the previous pair's shared memory
-    SideSum<TS, WPS> sum{sred[side], side, st >> 5, lane, 0};
+    SideSum<WPS> sum{sred[side], side, st >> 5, lane, 0};
     TS x[RMAX][ROWS];
     const int len = side ? v.n : v.m;
-    auto load = [&](const double* p, int rows, TS (&c)[ROWS]) {
+    auto load = [&](const double* p, int rows, auto (&c)[ROWS]) {
 #pragma unroll
       for (int u = 0; u < ROWS; ++u) {
         const int t = st + 32 * WPS * u;
-        c[u] = t < rows ? (TS)p[t] : (TS)0;
+        c[u] = t < rows ? p[t] : 0.0;
       }
     };
     if (side == 0) {
@@ -165,27 +172,39 @@ __global__ void __launch_bounds__(64 * WPS) lu_pair_kernel(PairArgs a) {
           for (int u = 0; u < ROWS; ++u) x[c][u] = (TS)0;
       }
     } else {
-      // W[l][c] = B_ik(:, l) . A_kj(:, c)
+      // W[l][c] = B_ik(:, l) . A_kj(:, c), NC columns from c0 on, which y holds
+      auto dots = [&](auto& y, int c0) {
+        constexpr int NC = (int)(sizeof(y) / sizeof(y[0]));
 #pragma unroll
-      for (int c = 0; c < RMAX; ++c)
-        if (c < v.kb) load(v.Akj + (int64_t)c * v.s, v.s, x[c]);
+        for (int c = 0; c < NC; ++c)
+          if (c0 + c < v.kb) load(v.Akj + (int64_t)(c0 + c) * v.s, v.s, y[c]);
 #pragma unroll 1
-      for (int l = 0; l < ka; ++l) {
-        TS t[ROWS], d[RMAX];
-        load(v.Bik + (int64_t)l * v.s, v.s, t);
+        for (int l = 0; l < ka; ++l) {
+          double t[ROWS], d[NC];
+          load(v.Bik + (int64_t)l * v.s, v.s, t);
 #pragma unroll
-        for (int c = 0; c < RMAX; ++c) {
-          d[c] = (TS)0;
-          if (c < v.kb) {
+          for (int c = 0; c < NC; ++c) {
+            d[c] = 0.0;
+            if (c0 + c < v.kb) {
 #pragma unroll
-            for (int u = 0; u < ROWS; ++u) d[c] = fma(t[u], x[c][u], d[c]);
+              for (int u = 0; u < ROWS; ++u) d[c] = fma(t[u], y[c][u], d[c]);
+            }
+          }
+          sum(d, 0, v.kb - c0);
+          if (st == 0) {
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+              if (c0 + c < v.kb) sW[l * RMAX + c0 + c] = d[c];
           }
         }
-        sum(d, 0, v.kb);
-        if (st == 0) {
-#pragma unroll
-          for (int c = 0; c < RMAX; ++c)
-            if (c < v.kb) sW[l * RMAX + c] = d[c];
+      };
+      if constexpr (WC == RMAX) {
+        dots(x, 0);
+      } else {
+#pragma unroll 1
+        for (int c0 = 0; c0 < v.kb; c0 += WC) {
+          double y[WC][ROWS];
+          dots(y, c0);
         }
       }
 #pragma unroll
@@ -195,17 +214,47 @@ __global__ void __launch_bounds__(64 * WPS) lu_pair_kernel(PairArgs a) {
     __syncthreads();
     if (side == 0) {
       // columns k1 .. r - 1: -A_ik W
+      if constexpr (WC == RMAX) {
 #pragma unroll 1
-      for (int l = 0; l < ka; ++l) {
-        TS t[ROWS];
-        load(v.Aik + (int64_t)l * v.m, v.m, t);
+        for (int l = 0; l < ka; ++l) {
+          double t[ROWS];
+          load(v.Aik + (int64_t)l * v.m, v.m, t);
 #pragma unroll
-        for (int c = 0; c < RMAX; ++c)
-          if (c >= k1 && c < r) {
-            const TS w = -sW[l * RMAX + c - k1];
+          for (int c = 0; c < RMAX; ++c)
+            if (c >= k1 && c < r) {
+              const double w = -sW[l * RMAX + c - k1];
 #pragma unroll
-            for (int u = 0; u < ROWS; ++u) x[c][u] = fma(t[u], w, x[c][u]);
+              for (int u = 0; u < ROWS; ++u) x[c][u] = fma(t[u], w, x[c][u]);
+            }
+        }
+      } else {
+#pragma unroll 1
+        for (int c0 = 0; c0 < v.kb; c0 += WC) {
+          double y[WC][ROWS];
+#pragma unroll
+          for (int c = 0; c < WC; ++c)
+#pragma unroll
+            for (int u = 0; u < ROWS; ++u) y[c][u] = 0.0;
+#pragma unroll 1
+          for (int l = 0; l < ka; ++l) {
+            double t[ROWS];
+            load(v.Aik + (int64_t)l * v.m, v.m, t);
+#pragma unroll
+            for (int c = 0; c < WC; ++c) {
+              const double w = c0 + c < v.kb ? -sW[l * RMAX + c0 + c] : 0.0;
+#pragma unroll
+              for (int u = 0; u < ROWS; ++u) y[c][u] = fma(t[u], w, y[c][u]);
+            }
           }
+#pragma unroll
+          for (int c = 0; c < RMAX; ++c)
+#pragma unroll
+            for (int q = 0; q < WC; ++q)
+              if (c == k1 + c0 + q && c < r) {
+#pragma unroll
+                for (int u = 0; u < ROWS; ++u) x[c][u] = (TS)y[q][u];
+              }
+        }
       }
     }
     // Gram-Schmidt, twice per column; once for the columns of A_ij and B_ij,
@@ -351,9 +400,12 @@ template <typename TS>
 __global__ void __launch_bounds__(128) lu_tile_core_kernel(PairArgs a, int rl, int smax, TS* scratch) {
   extern __shared__ double sm_raw[];
   TS* sm = reinterpret_cast<TS*>(sm_raw);
-  TS* XA = scratch ? scratch + (int64_t)blockIdx.x * (2 * smax * rl + a.cap * a.cap) : sm + 3 * rl * (rl + 1);
+  // W (cap x cap, FP64 as in the register kernel), then the factors
+  const int64_t cw = (int64_t)a.cap * a.cap * (8 / sizeof(TS));
+  TS* base = scratch ? scratch + (int64_t)blockIdx.x * (2 * smax * rl + cw) : sm + 3 * rl * (rl + 1);   // both even
+  double* sw = reinterpret_cast<double*>(base);
+  TS* XA = base + cw;
   TS* XB = XA + (int64_t)smax * rl;
-  TS* sw = XB + (int64_t)smax * rl;    // W, cap x cap
   const int nin = *a.nin;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int b = blockIdx.x; b < nin; b += gridDim.x) {
@@ -373,16 +425,16 @@ __global__ void __launch_bounds__(128) lu_tile_core_kernel(PairArgs a, int rl, i
 #pragma unroll 4
       for (int t = lane; t < v.s; t += 32) s = fma(x[t], y[t], s);
       s = warp_sum(s);
-      if (lane == 0) sw[e] = (TS)s;
+      if (lane == 0) sw[e] = s;
     }
     __syncthreads();
     for (int q = 0; q < r; ++q)
       for (int t = threadIdx.x; t < v.m; t += blockDim.x) {
-        TS s = (TS)0;
-        if (q < k1) s = (TS)v.A[t + (int64_t)q * v.m];
+        double s = 0.0;
+        if (q < k1) s = v.A[t + (int64_t)q * v.m];
         else
-          for (int l = 0; l < ka; ++l) s = fma((TS)v.Aik[t + (int64_t)l * v.m], -sw[l + (q - k1) * ka], s);
-        XA[t + q * v.m] = s;
+          for (int l = 0; l < ka; ++l) s = fma(v.Aik[t + (int64_t)l * v.m], -sw[l + (q - k1) * ka], s);
+        XA[t + q * v.m] = (TS)s;
       }
     for (int q = 0; q < r; ++q)
       for (int t = threadIdx.x; t < v.n; t += blockDim.x)
