@@ -204,29 +204,23 @@ __global__ void lu_axpby_kernel(View Y, View X, double alpha, double beta) {
   }
 }
 
-// X <- L^{-1} X, L (m x m) lower triangular (strided: upper/transposed/reversed
-// triangles are views of this one), one thread per column of X.
+// X <- L^{-1} X, L (m x m, m <= 96) lower triangular (strided: upper/transposed/
+// reversed triangles are views of this one), one thread per column of X.
 __global__ void __launch_bounds__(128) lu_trsm_lower_kernel(View L, View X, int unit) {
   extern __shared__ double Ls[];
   const int m = L.rows;
-  const bool sm = m <= 96;
-  if (sm) {
-    for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
-      const int i = e % m, j = e / m;
-      Ls[e] = (j <= i) ? L.p[(int64_t)i * L.rs + (int64_t)j * L.cs] : 0.0;
-    }
-    __syncthreads();
+  for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
+    const int i = e % m, j = e / m;
+    Ls[e] = (j <= i) ? L.p[(int64_t)i * L.rs + (int64_t)j * L.cs] : 0.0;
   }
+  __syncthreads();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= X.cols) return;
   double* x = X.p + (int64_t)j * X.cs;
   for (int i = 0; i < m; ++i) {
     double s = x[(int64_t)i * X.rs];
-    for (int l = 0; l < i; ++l) {
-      const double lil = sm ? Ls[i + l * m] : L.p[(int64_t)i * L.rs + (int64_t)l * L.cs];
-      s = fma(-lil, x[(int64_t)l * X.rs], s);
-    }
-    if (!unit) s = s / (sm ? Ls[i + i * m] : L.p[(int64_t)i * L.rs + (int64_t)i * L.cs]);
+    for (int l = 0; l < i; ++l) s = fma(-Ls[i + l * m], x[(int64_t)l * X.rs], s);
+    if (!unit) s = s / Ls[i + i * m];
     x[(int64_t)i * X.rs] = s;
   }
 }
@@ -609,6 +603,31 @@ static void axpby(Ctx& c, View Y, View X, double alpha, double beta) {
   LU_LAUNCH_CHECK();
 }
 
+// X <- L^-1 X for triangles of 97 to TRSM_ROWS rows, 32 columns a CTA, staged in
+// shared memory.  Larger ones are halved, with a product by all SMs between the
+// halves (trsm_lower).  One thread a column with the triangle read from L2 was a
+// chain of rows^2 / 2 dependent steps: 100 right-hand sides at n = 8192, 32 tiles
+// of 256 rows, 165 ms so, 11 now; 8 tiles of 1024 rows 730 and 11 ms; the LU of the
+// latter, whose panels take this way too, 544 and 33 ms.  Pieces of up to 512 rows:
+// 12 ms and 37 ms.
+constexpr int TRSM_ROWS = 256;
+__global__ void __launch_bounds__(256) lu_trsm_block_kernel(View L, View X, int unit) {
+  extern __shared__ double sm[];
+  const int S = L.rows, ldx = tp_ldx(S), c0 = (int)blockIdx.x * TP_COLS, nc = min(TP_COLS, X.cols - c0);
+  double* xg = X.p + (int64_t)c0 * X.cs;
+  double* tri = sm + TP_COLS * ldx;                      // 32 x 33, then the 32 reciprocals
+  for (int e = threadIdx.x; e < TP_COLS * S; e += blockDim.x) {
+    const int cc = e / S, i = e % S;
+    sm[cc * ldx + i] = cc < nc ? xg[(int64_t)cc * X.cs + (int64_t)i * X.rs] : 0.0;
+  }
+  __syncthreads();
+  tile_trsm(L.p, L.rs, L.cs, S, unit != 0, sm, ldx, nc, 0, tri, tri + 32 * 33);
+  for (int e = threadIdx.x; e < nc * S; e += blockDim.x) {
+    const int cc = e / S, i = e % S;
+    xg[(int64_t)cc * X.cs + (int64_t)i * X.rs] = sm[cc * ldx + i];
+  }
+}
+
 static void trsm_lower(Ctx& c, View L, View X, bool unit) {
   if (X.cols == 0 || L.rows == 0) return;
   if (L.rows <= 32) {
@@ -621,10 +640,27 @@ static void trsm_lower(Ctx& c, View L, View X, bool unit) {
     LU_LAUNCH_CHECK();
     return;
   }
-  if (smem_attr((const void*)lu_trsm_lower_kernel, 96 * 96 * (int)sizeof(double)) != cudaSuccess)
+  if (L.rows <= 96) {
+    if (smem_attr((const void*)lu_trsm_lower_kernel, 96 * 96 * (int)sizeof(double)) != cudaSuccess)
+      throw LuError(HM_ERR_CUDA, "trsm smem attribute");
+    const size_t smem = sizeof(double) * (size_t)L.rows * L.rows;
+    lu_trsm_lower_kernel<<<(X.cols + 127) / 128, 128, smem, c.st>>>(L, X, unit ? 1 : 0);
+    LU_LAUNCH_CHECK();
+    return;
+  }
+  // dense diagonal tiles (solves of many columns, panels of large tiles) and the
+  // largest leaves: halves of at most TRSM_ROWS rows with a product between them
+  if (L.rows > TRSM_ROWS) {
+    const int m = (L.rows / 2 + 31) / 32 * 32, r = L.rows - m;
+    const View X1 = vsub(X, 0, 0, m, X.cols), X2 = vsub(X, m, 0, r, X.cols);
+    trsm_lower(c, vsub(L, 0, 0, m, m), X1, unit);
+    gemm(c, X2, vsub(L, m, 0, r, m), X1, -1.0, 1.0);
+    trsm_lower(c, vsub(L, m, m, r, r), X2, unit);
+    return;
+  }
+  if (smem_attr((const void*)lu_trsm_block_kernel, (int)tp_smem(TRSM_ROWS)) != cudaSuccess)
     throw LuError(HM_ERR_CUDA, "trsm smem attribute");
-  const size_t smem = L.rows <= 96 ? sizeof(double) * (size_t)L.rows * L.rows : 0;
-  lu_trsm_lower_kernel<<<(X.cols + 127) / 128, 128, smem, c.st>>>(L, X, unit ? 1 : 0);
+  lu_trsm_block_kernel<<<(X.cols + TP_COLS - 1) / TP_COLS, 256, tp_smem(L.rows), c.st>>>(L, X, unit ? 1 : 0);
   LU_LAUNCH_CHECK();
 }
 

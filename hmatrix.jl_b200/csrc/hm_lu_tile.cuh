@@ -566,7 +566,7 @@ static __device__ void tile_trsm(const double* __restrict__ T, int64_t rs, int64
     // the block's triangle, column-major with stride 33
     for (int e = threadIdx.x; e < 1024; e += blockDim.x) {
       int i, l;
-      if (rs == 1) { i = e & 31; l = e >> 5; } else { l = e & 31; i = e >> 5; }
+      if (rs == 1 || rs == -1) { i = e & 31; l = e >> 5; } else { l = e & 31; i = e >> 5; }
       // skewed: row l + d of column l at d + 32 l, zeros past the end
       if (l <= i) {
         const double v = i < nr ? __ldg(T + (r0 + i) * rs + (r0 + l) * cs) : 0.0;
