@@ -1351,24 +1351,46 @@ static bool tile_check(const hm_handle* h, const std::vector<int32_t>& gcl, std:
 // Otherwise the shallowest depth whose clusters form a valid tiling (a median
 // bisection of an n that is not a power of two mixes cluster sizes on both
 // sides of MaxBlock on one level, so the admissible blocks start one level
-// lower on part of it).
+// lower on part of it).  Tiles of at most TILE_MAX rows where there is a tiling
+// of such, the leaves above that taken in parts: a diagonal tile is dense, and
+// its LU, S^3 on the eight SMs of a cluster, is the longer the larger it is.
+// H-LU, n = 16384 (bbfmm), tiles of 4096 rows 410 ms, cut into tiles of 2048 150;
+// as block trees 302 and 238 ms.
+constexpr int64_t TILE_MAX = 2048;
+
 static bool tile_structure(const hm_handle* h, std::vector<int32_t>& gcl, std::vector<int32_t>& diag_node) {
   const int64_t ncl = (int64_t)h->cl_s.size();
   auto by_start = [&](int32_t a, int32_t b) { return h->cl_s[a] < h->cl_s[b]; };
-  {
-    std::vector<char> is_row(ncl, 0), covered(ncl, 0);
-    for (auto& L : h->leaves) is_row[L.s] = 1;
+  auto rows = [&](int64_t c) { return h->cl_e[c] - h->cl_s[c]; };
+  auto largest = [&] {
+    int64_t m = 0;
+    for (int32_t c : gcl) m = std::max(m, rows(c));
+    return m;
+  };
+  std::vector<char> is_row(ncl, 0);
+  for (auto& L : h->leaves) is_row[L.s] = 1;
+  // the highest clusters of at most `most` rows that are a leaf's row cluster or lie below one
+  auto highest = [&](int64_t most) {
+    std::vector<char> covered(ncl, 0), below(ncl, 0);
     gcl.clear();
     for (int64_t c = 0; c < ncl; ++c) {
-      if (!covered[c] && is_row[c]) gcl.push_back((int32_t)c);
-      if (h->cl_left[c] >= 0) {
-        const char cv = covered[c] || is_row[c];
-        covered[h->cl_left[c]] = cv;
-        covered[h->cl_right[c]] = cv;
-      }
+      const bool row = is_row[c] || below[c];
+      const bool take = !covered[c] && row && (rows(c) <= most || h->cl_left[c] < 0);
+      if (take) gcl.push_back((int32_t)c);
+      if (h->cl_left[c] >= 0)
+        for (int64_t ch : {h->cl_left[c], h->cl_right[c]}) {
+          covered[ch] = covered[c] || take;
+          below[ch] = row;
+        }
     }
     std::sort(gcl.begin(), gcl.end(), by_start);
-    if (tile_check(h, gcl, diag_node)) return true;
+    return tile_check(h, gcl, diag_node);
+  };
+  if (highest(TILE_MAX)) return true;
+  std::vector<int32_t> first, first_node;       // a tiling with a larger tile
+  if (highest(INT64_MAX)) {
+    first = gcl;
+    first_node = diag_node;
   }
   int maxd = 0;
   for (int64_t c = 0; c < ncl; ++c) maxd = std::max(maxd, (int)h->cl_depth[c]);
@@ -1378,13 +1400,20 @@ static bool tile_structure(const hm_handle* h, std::vector<int32_t>& gcl, std::v
     for (int64_t c = 0; c < ncl; ++c)
       if (h->cl_depth[c] == d) {
         gcl.push_back((int32_t)c);
-        cover += h->cl_e[c] - h->cl_s[c];
+        cover += rows(c);
       }
-    if (cover != h->n) return false;            // a cluster leaf above depth d: no deeper level covers
+    if (cover != h->n) break;                   // a cluster leaf above depth d: no deeper level covers
     std::sort(gcl.begin(), gcl.end(), by_start);
-    if (tile_check(h, gcl, diag_node)) return true;
+    if (!tile_check(h, gcl, diag_node)) continue;
+    if (largest() <= TILE_MAX) return true;
+    if (first.empty()) {
+      first = gcl;
+      first_node = diag_node;
+    }
   }
-  return false;
+  gcl.swap(first);
+  diag_node.swap(first_node);
+  return !gcl.empty();
 }
 
 // The recompressions of step k's pairs (tile_pair's mode), every launch sized
