@@ -447,7 +447,6 @@ int hm_autotune(hm_handle* h, int64_t ncols, int32_t calls, double* times) {
   // single right-hand side: phase-2 split x phase-1 waves
   float best = -1.f;
   hm_handle::Tune keep = h->tune;
-  const bool slabs = keep.p2_split == 1;
   const int splits[3] = {2, 4, 8}, waves[3] = {1, 2, 4};
   if (times)
     for (int i = 0; i < 15; ++i) times[i] = -1.0;
@@ -462,9 +461,8 @@ int hm_autotune(hm_handle* h, int64_t ncols, int32_t calls, double* times) {
   };
   for (int a = 0; a < 3; ++a)
     for (int b = 0; b < 3; ++b) HM_TRY(try_shape(splits[a], b, 3 * a + b));
-  // phase 2 by row slabs (BF16 factors: where it is the default, on trees off the 64-row grid)
-  if (h->storage != HM_BF16 || slabs)
-    for (int b = 0; b < 3; ++b) HM_TRY(try_shape(1, b, 12 + b));
+  // phase 2 by row slabs
+  for (int b = 0; b < 3; ++b) HM_TRY(try_shape(1, b, 12 + b));
   h->tune = keep;
   // several columns on the tensor cores: the column block
   if (ncols > 1 && (h->storage == HM_F32 || h->storage == HM_BF16)) {
@@ -494,7 +492,9 @@ int hm_set_tune(hm_handle* h, int32_t p2_split, int32_t p1_waves) {
     return fail(HM_ERR_ARG, "phase-2 shape must be 1, 2, 4 or 8");
   if (p1_waves != 1 && p1_waves != 2 && p1_waves != 4) return fail(HM_ERR_ARG, "phase-1 waves must be 1, 2 or 4");
   if (p2_split == 1 && h->storage == HM_BF16)
-    return fail(HM_ERR_UNSUPPORTED, "phase 2 by row slabs is set by hand for FP64 or FP32 factors only");
+    return fail(HM_ERR_UNSUPPORTED,
+                "phase 2 by row slabs is set by hand for FP64 or FP32 factors only (BF16: the default of a new "
+                "handle, and hm_autotune's choice)");
   h->tune.p2_split = p2_split;
   h->tune.p1_waves = p1_waves;
   return HM_OK;

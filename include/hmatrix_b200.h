@@ -213,10 +213,9 @@ int hm_matvec(hm_handle* h, const double* X, double* Y, int64_t ncols,
 
 /* Autotuner of the matvec launch shapes on this handle's own data: times
  * `calls` matvecs (CUDA events, after two untimed ones) for every phase-2
- * shape (2, 4, 8 CTAs per 1024-row window, or, with FP64/FP32 factors and
- * where it is the default, one CTA per slab of at most 224 rows) and phase-1
- * grid (1, 2, 4 resident waves) and keeps the fastest; with ncols > 1
- * and FP32/BF16 factors, also the tensor-core column block (16, 32, 64) for
+ * shape (2, 4, 8 CTAs per 1024-row window, or one CTA per slab of at most 224
+ * rows) and phase-1 grid (1, 2, 4 resident waves) and keeps the fastest; with
+ * ncols > 1 and FP32/BF16 factors, also the tensor-core column block (16, 32, 64) for
  * that many columns.  The choice stays with the handle (hm_info reports it).
  * The window shapes give bit-identical results; the slab shape sums the
  * same products in another order.  times (may be NULL) receives 15 mean
@@ -228,8 +227,9 @@ int hm_autotune(hm_handle* h, int64_t ncols, int32_t calls, double* times);
 /* Sets the single-column matvec launch shapes by hand (a choice hm_autotune
  * made earlier on the same data, say): p2_split 2, 4 or 8 CTAs per phase-2
  * window, or 1 for phase 2 by row slabs (not with BF16 factors:
- * HM_ERR_UNSUPPORTED); p1_waves 1, 2 or 4.  Other values: HM_ERR_ARG.  No
- * counterpart in the reference. */
+ * HM_ERR_UNSUPPORTED; slabs are their default up to n = 2^18 and off the 64-row
+ * grid, and hm_autotune goes back to them where they are the fastest); p1_waves
+ * 1, 2 or 4.  Other values: HM_ERR_ARG.  No counterpart in the reference. */
 int hm_set_tune(hm_handle* h, int32_t p2_split, int32_t p1_waves);
 
 /* Waits for `stream` (NULL: the handle's stream) and reports, once, whether a
