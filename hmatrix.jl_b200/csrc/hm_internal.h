@@ -315,8 +315,9 @@ void lu_describe(const hm_handle* h, int64_t* tiles, int64_t* cap);
 // matvec (hm_matvec.cu)
 int matvec_device(hm_handle* h, const double* d_x, double* d_y, int trans, cudaStream_t st,
                   cudaEvent_t* ev = nullptr);
-// Builds a direction's slab lists on first use; *usable false: they cannot be had.
-int ensure_slabs(hm_handle* h, int trans, bool* usable);
+// Builds a direction's slab lists on first use; *usable false: they cannot be
+// had, or not now (st is being captured).
+int ensure_slabs(hm_handle* h, int trans, cudaStream_t st, bool* usable);
 // Y = H X (trans 0) or H' X (trans 1) for an n x ncols column-major block,
 // factors streamed once per column block (hm_matvec_multi.cu)
 int matvec_multi_device(hm_handle* h, const double* d_x, double* d_y, int64_t ncols, int trans, cudaStream_t st,

@@ -796,11 +796,18 @@ static int build_slab_plan(hm_handle* h, int trans, MvPlan& P) {
 }
 
 // Builds the slab lists on first use; false: this plan cannot have them (no
-// memory left for them, or an entry field too narrow) and the caller takes
-// the window lists, which every plan has.
-int ensure_slabs(hm_handle* h, int trans, bool* usable) {
+// memory left for them, or an entry field too narrow), or not now (st is being
+// captured, which forbids allocations), and the caller takes the window lists,
+// which every plan has.
+int ensure_slabs(hm_handle* h, int trans, cudaStream_t st, bool* usable) {
   MvPlan& P = trans ? h->bwd : h->fwd;
   if (!P.d_slab && !P.no_slab) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();   // the legacy stream beside a capture
+    else if (cap != cudaStreamCaptureStatusNone) {
+      *usable = false;
+      return HM_OK;
+    }
     const int s = build_slab_plan(h, trans, P);
     if (s == HM_ERR_OOM || s == HM_ERR_UNSUPPORTED) P.no_slab = true;
     else if (s != HM_OK) return s;
@@ -1154,7 +1161,7 @@ static int matvec_t(hm_handle* h, const double* d_x, double* d_y, int trans, cud
   // dense leaves are FP64 with FP64 factors and FP32 otherwise
   using TD = typename std::conditional<std::is_same<T, double>::value, double, float>::type;
   bool slabs = false;
-  if (h->tune.p2_split == 1) HM_TRY(ensure_slabs(h, trans, &slabs));
+  if (h->tune.p2_split == 1) HM_TRY(ensure_slabs(h, trans, st, &slabs));
   if (slabs) {
     mv_slab_kernel<T, TD><<<(unsigned)P.nslab, SL_WARPS * 32, 0, st>>>(
         P.d_slab, P.d_ent, (const T*)h->d_rk, (const TD*)h->d_dense, h->d_z, d_x, d_y);

@@ -588,8 +588,8 @@ int launch_multi(hm_handle* h, const double* d_x, double* d_y, int64_t ncols, in
   using TD = typename std::conditional<std::is_same<T, double>::value, double, float>::type;
   MvPlan& P = trans ? h->bwd : h->fwd;
   bool slabs = false;
-  HM_TRY(ensure_slabs(h, trans, &slabs));
-  if (!slabs) {                                          // no memory for the lists: column by column
+  HM_TRY(ensure_slabs(h, trans, st, &slabs));
+  if (!slabs) {                                          // no lists: column by column
     for (int64_t c = 0; c < ncols; ++c) HM_TRY(matvec_device(h, d_x + c * h->n, d_y + c * h->n, trans, st));
     return HM_OK;
   }
