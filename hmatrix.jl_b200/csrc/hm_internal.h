@@ -195,7 +195,7 @@ struct MvPlan {
   MvWin* d_winr = nullptr;         // windows over d_p2r
   // phase 2 by row slabs (phase-2 shape 1; built on first use)
   Slab* d_slab = nullptr;          // nslab slabs
-  SlabEnt* d_ent = nullptr;        // (in the allocation of d_slab)
+  SlabEnt* d_ent = nullptr;
   int32_t nslab = 0;
   bool no_slab = false;            // the lists could not be had
 };

@@ -585,45 +585,125 @@ void free_mv_plan(MvPlan& p) {
   if (p.d_p2r) cudaFree(p.d_p2r);
   if (p.d_winr) cudaFree(p.d_winr);
   if (p.d_slab) cudaFree(p.d_slab);
+  if (p.d_ent) cudaFree(p.d_ent);
   p = MvPlan{};
 }
 
-// One leaf of a slab plan: its factor (low-rank) or block (dense) over the
-// output rows [row0, row0 + m), which are (part of) the slabs [w0, w1]; slot:
-// index of its first (leaf, slab) pair
-struct SlabLeaf {
-  int64_t off;
-  uint32_t row0, m, ld, zi, cnt, slot, w0, w1;
-  uint16_t type;
+// The entries of the slabs, from the window lists that every plan has on the
+// device: a warp per slab walks the leaves of its one or two windows (a leaf that
+// reaches back before the second one was met in the first) and counts, or writes,
+// an entry per column of those with rows in the slab; low-rank leaves first, those
+// read along their rows (dense, H'x) last, each kind in list order.  Made by the
+// host from the leaves, a first product waited 3.2 ms for the lists at n = 131072
+// (70912 leaves), most of it in the host's caches, and for their upload.
+struct SlabTotal {
+  unsigned long long entries;
+  unsigned long long narrow;             // a row stride too large for its field
 };
-// entries of one leaf, a warp per leaf: pos[slot + w - w0] is its first entry
-// in slab w
-__global__ void __launch_bounds__(256) slab_fill_kernel(const SlabLeaf* __restrict__ leaf, int64_t nleaf,
-                                                        const uint32_t* __restrict__ pos,
-                                                        const Slab* __restrict__ slabs, SlabEnt* __restrict__ ent) {
+template <bool FILL>
+__global__ void __launch_bounds__(256) slab_lists_kernel(Slab* __restrict__ slabs, int64_t nslab,
+                                                         const MvWin* __restrict__ win, const P2Desc* __restrict__ d,
+                                                         SlabEnt* __restrict__ ent, SlabTotal* __restrict__ total) {
   const int lane = threadIdx.x & 31;
-  const int64_t li = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (li >= nleaf) return;
-  const SlabLeaf L = leaf[li];
-  const uint32_t ne = L.type == P2_DENSE_T ? (L.cnt + 31) / 32 : L.cnt;
-  for (uint32_t w = L.w0; w <= L.w1; ++w) {
-    const uint32_t s0 = slabs[w].row0, s1 = s0 + slabs[w].nrows;
-    const uint32_t a = max(L.row0, s0), b = min(L.row0 + L.m, s1);
-    const uint32_t p = pos[L.slot + (w - L.w0)];
-    for (uint32_t c = lane; c < ne; c += 32) {
-      SlabEnt E;
-      E.meta = (a - s0) | (b - 1 - s0) << 8 | (uint32_t)L.type << 16;
-      if (L.type == P2_DENSE_T) {
-        E.off = (uint64_t)(L.off + (int64_t)(a - L.row0) * L.ld + 32 * c) | (uint64_t)L.ld << 40;
-        E.zi = L.zi + 32 * c;
-        E.meta |= min(32u, L.cnt - 32 * c) << 24;
+  const int64_t sl = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (sl >= nslab) return;
+  const Slab S = slabs[sl];
+  const int64_t s0 = S.row0, s1 = s0 + S.nrows;
+  // next entry (FILL), or this lane's counts: low-rank, dense, along rows
+  uint32_t at[3] = {FILL ? S.begin : 0u, FILL ? S.dense : 0u, FILL ? S.mid : 0u};
+  bool narrow = false;
+  const int64_t w0 = s0 / MV_WROWS, w1 = (s1 - 1) / MV_WROWS;
+  for (int64_t w = w0; w <= w1; ++w) {
+    const MvWin W = win[w];
+    for (uint32_t b0 = W.begin; b0 < W.end; b0 += 32) {
+      P2Desc D{};
+      if (b0 + lane < W.end) D = d[b0 + lane];
+      const int64_t o0 = w * MV_WROWS + D.row_off;
+      const bool in = D.m > 0 && o0 < s1 && o0 + D.m > s0 && (w == w0 || D.row_off >= 0);
+      const uint32_t ne = D.type == P2_DENSE_T ? (D.cnt + 31) / 32 : D.cnt;
+      if constexpr (!FILL) {
+        if (in) {
+#pragma unroll
+          for (int k = 0; k < 3; ++k)
+            if ((D.type == P2_RK ? 0 : D.type == P2_DENSE ? 1 : 2) == k) at[k] += ne;
+          narrow = narrow || (D.type == P2_DENSE_T && D.ld >= 1u << 24);
+        }
       } else {
-        E.off = (uint64_t)(L.off + (int64_t)c * L.ld + (a - L.row0));
-        E.zi = L.zi + c;
+        for (unsigned todo = __ballot_sync(0xffffffffu, in); todo; todo &= todo - 1) {
+          const int src = __ffs(todo) - 1;
+          const uint64_t off = __shfl_sync(0xffffffffu, (unsigned long long)D.off, src);
+          const int64_t r0 = __shfl_sync(0xffffffffu, (long long)o0, src);
+          const int64_t r1 = r0 + __shfl_sync(0xffffffffu, D.m, src);
+          const uint32_t ld = __shfl_sync(0xffffffffu, D.ld, src), zi = __shfl_sync(0xffffffffu, D.aux, src);
+          const uint32_t cnt = __shfl_sync(0xffffffffu, D.cnt, src), n = __shfl_sync(0xffffffffu, ne, src);
+          const uint32_t type = __shfl_sync(0xffffffffu, (uint32_t)D.type, src);
+          const int64_t a = r0 > s0 ? r0 : s0, b = r1 < s1 ? r1 : s1;
+          const uint32_t meta = (uint32_t)(a - s0) | (uint32_t)(b - 1 - s0) << 8 | type << 16;
+          uint32_t& p = type == P2_RK ? at[0] : type == P2_DENSE ? at[1] : at[2];
+          for (uint32_t c = lane; c < n; c += 32) {
+            SlabEnt E;
+            if (type == P2_DENSE_T) {
+              E.off = (off + (uint64_t)(a - r0) * ld + 32 * c) | (uint64_t)ld << 40;
+              E.zi = zi + 32 * c;
+              E.meta = meta | min(32u, cnt - 32 * c) << 24;
+            } else {
+              E.off = off + (uint64_t)c * ld + (uint64_t)(a - r0);
+              E.zi = zi + c;
+              E.meta = meta;
+            }
+            ent[p + c] = E;
+          }
+          p += n;
+        }
       }
-      ent[p + c] = E;
     }
   }
+  if constexpr (!FILL) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) at[k] = __reduce_add_sync(0xffffffffu, at[k]);
+    if (lane == 0) {
+      slabs[sl].begin = at[0];
+      slabs[sl].dense = at[1];
+      slabs[sl].mid = at[2];
+    }
+    if (narrow) atomicOr(&total->narrow, 1ull);
+  }
+}
+
+// counts -> entry ranges, slab after slab, by one CTA
+__global__ void __launch_bounds__(1024) slab_scan_kernel(Slab* __restrict__ slabs, int64_t nslab,
+                                                         SlabTotal* __restrict__ total) {
+  __shared__ unsigned long long sum[32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  unsigned long long base = 0;
+  for (int64_t b = 0; b < nslab; b += 1024) {
+    const int64_t i = b + threadIdx.x;
+    Slab S{};
+    if (i < nslab) S = slabs[i];
+    const unsigned long long own = (unsigned long long)S.begin + S.dense + S.mid;
+    unsigned long long incl = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    __syncthreads();                                     // the last round's sums
+    if (lane == 31) sum[warp] = incl;
+    __syncthreads();
+    unsigned long long first = base + incl - own;
+    for (int q = 0; q < 32; ++q) {
+      if (q < warp) first += sum[q];
+      base += sum[q];
+    }
+    if (i < nslab) {
+      S.end = (uint32_t)(first + own);
+      S.mid = (uint32_t)(first + S.begin + S.dense);
+      S.dense = (uint32_t)(first + S.begin);
+      S.begin = (uint32_t)first;
+      slabs[i] = S;
+    }
+  }
+  if (threadIdx.x == 0) total->entries = base;
 }
 
 // The slab boundaries for slabs of at most `most` rows: the highest clusters
@@ -674,124 +754,42 @@ static void choose_slabs(const hm_handle* h, std::vector<Slab>& best) {
   }
 }
 
-// The slab lists of one direction.  z offsets follow the pool order of the
-// low-rank leaves, as in build_mv_descriptors; a slab lists its leaves in pool
-// order, low-rank ones first, those read along their rows (dense, H'x) last.
-static int build_slab_plan(hm_handle* h, int trans, MvPlan& P) {
-  const int eb = elem_bytes(h->storage), deb = dense_elem_bytes(h->storage);
+// The slab lists of one direction.
+static int build_slab_plan(hm_handle* h, MvPlan& P) {
   std::vector<Slab> slab;
   choose_slabs(h, slab);
   const int64_t nslab = (int64_t)slab.size();
-  auto slab_of = [&](int64_t row) {
-    return (uint32_t)(std::upper_bound(slab.begin(), slab.end(), row,
-                                       [](int64_t r, const Slab& S) { return r < (int64_t)S.row0; }) - slab.begin() - 1);
-  };
-  // per cluster: leaves of one cluster share its slabs
-  const int64_t ncl = (int64_t)h->cl_s.size();
-  std::vector<uint32_t> c0((size_t)ncl), c1((size_t)ncl);
-  for (int64_t c = 0; c < ncl; ++c) {
-    c0[c] = slab_of(h->cl_s[c]);
-    c1[c] = slab_of(h->cl_e[c] - 1);
-  }
-  const std::vector<int64_t> order = pool_order(h);
-  std::vector<SlabLeaf> leaf;
-  leaf.reserve(order.size());
-  std::vector<uint64_t> cnt[3];                          // entries per slab: low-rank, dense, along rows
-  for (auto& v : cnt) v.assign((size_t)nslab, 0);
-  auto section = [](uint16_t type) { return type == P2_RK ? 0 : type == P2_DENSE ? 1 : 2; };
-  uint64_t slots = 0, z = 0;
-  for (int64_t li : order) {
-    const Leaf& L = h->leaves[li];
-    const int64_t npad = col_pad(L.n, eb), mpad = col_pad(L.m, eb);
-    SlabLeaf D{};
-    D.row0 = (uint32_t)(trans ? L.col0 : L.row0);
-    D.m = (uint32_t)(trans ? L.n : L.m);
-    if (L.type == T_RK) {
-      D.type = P2_RK;
-      D.off = trans ? L.off : L.off + npad * L.k;
-      D.ld = (uint32_t)(trans ? npad : mpad);
-      D.zi = (uint32_t)z;
-      D.cnt = (uint32_t)L.k;
-      z += (uint64_t)L.k;
-      if (L.k == 0) continue;
-    } else {
-      const int64_t ldc = col_pad(L.m, deb);
-      D.type = trans ? P2_DENSE_T : P2_DENSE;
-      D.off = L.off;
-      D.ld = (uint32_t)ldc;
-      D.zi = (uint32_t)(trans ? L.row0 : L.col0);
-      D.cnt = (uint32_t)(trans ? L.m : L.n);
-      if (trans && ldc >= (int64_t)1 << 24) return HM_ERR_UNSUPPORTED;   // the entry's stride field
-    }
-    D.slot = (uint32_t)slots;
-    D.w0 = c0[trans ? L.t : L.s];
-    D.w1 = c1[trans ? L.t : L.s];
-    slots += (uint64_t)(D.w1 - D.w0 + 1);
-    for (uint32_t w = D.w0; w <= D.w1; ++w) cnt[section(D.type)][w] += D.type == P2_DENSE_T ? (D.cnt + 31) / 32 : D.cnt;
-    leaf.push_back(D);
-  }
-  uint64_t tot = 0;
-  for (int64_t w = 0; w < nslab; ++w) {
-    Slab& S = slab[w];
-    uint32_t* at[3] = {&S.dense, &S.mid, &S.end};
-    S.begin = (uint32_t)tot;
-    for (int k = 0; k < 3; ++k) {
-      const uint64_t first = tot;
-      tot += cnt[k][w];
-      *at[k] = (uint32_t)tot;
-      cnt[k][w] = first;                                 // from here on: next free entry
-    }
-  }
-  if (tot > (uint64_t)UINT32_MAX || slots > (uint64_t)UINT32_MAX) return HM_ERR_UNSUPPORTED;
-  std::vector<uint32_t> pos((size_t)slots);
-  for (const SlabLeaf& D : leaf) {
-    for (uint32_t w = D.w0; w <= D.w1; ++w) {
-      uint64_t& next = cnt[section(D.type)][w];
-      pos[D.slot + (w - D.w0)] = (uint32_t)next;
-      next += D.type == P2_DENSE_T ? (D.cnt + 31) / 32 : D.cnt;
-    }
-  }
-  // one upload: leaves, first entries, slabs; the entries are written by the device
-  const size_t lb = sizeof(SlabLeaf) * leaf.size(), pb = sizeof(uint32_t) * pos.size();
+  if (nslab > INT32_MAX) return HM_ERR_UNSUPPORTED;
   const size_t sb = sizeof(Slab) * slab.size(), so = pad_to((int64_t)sb, 256);
-  void* keep = nullptr;                                  // slabs and entries
-  void* tmp = nullptr;
-  // small leaf lists stay behind the entries: an allocation of their own costs
-  // a small matrix's first product more than the product
-  const size_t ent_bytes = pad_to((int64_t)(sizeof(SlabEnt) * std::max<size_t>(tot, 1)), 256);
-  const bool behind = lb + pb <= (size_t)1 << 20;
-  if (cudaMalloc(&keep, so + ent_bytes + (behind ? lb + pb : 0)) != cudaSuccess) {
+  struct Mem {                                           // given back unless the plan takes it
+    void* p = nullptr;
+    ~Mem() { if (p) cudaFree(p); }
+  } lists, ents;
+  auto no_memory = [] {
     cudaGetLastError();
     return HM_ERR_OOM;
-  }
-  if (behind) {
-    tmp = (char*)keep + so + ent_bytes;
-  } else if (cudaMallocAsync(&tmp, lb + pb, h->stream) != cudaSuccess) {
-    cudaGetLastError();
-    cudaFree(keep);
-    return HM_ERR_OOM;
-  }
-  cudaError_t e = cudaMemcpyAsync(keep, slab.data(), sb, cudaMemcpyHostToDevice, h->stream);
-  if (!leaf.empty()) {
-    if (e == cudaSuccess) e = cudaMemcpyAsync(tmp, leaf.data(), lb, cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync((char*)tmp + lb, pos.data(), pb, cudaMemcpyHostToDevice, h->stream);
-    const int64_t nl = (int64_t)leaf.size();
-    if (e == cudaSuccess) {
-      slab_fill_kernel<<<(unsigned)((nl + 7) / 8), 256, 0, h->stream>>>(
-          (const SlabLeaf*)tmp, nl, (const uint32_t*)((char*)tmp + lb), (const Slab*)keep,
-          (SlabEnt*)((char*)keep + so));
-      e = cudaGetLastError();
-    }
-  }
-  if (!behind) cudaFreeAsync(tmp, h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);   // the caller's stream reads the entries next
-  if (e != cudaSuccess) {
-    cudaFree(keep);
-    return fail(HM_ERR_CUDA, std::string("row slabs: ") + cudaGetErrorString(e));
-  }
-  P.d_slab = (Slab*)keep;
-  P.d_ent = (SlabEnt*)((char*)keep + so);
+  };
+  if (cudaMalloc(&lists.p, so + sizeof(SlabTotal)) != cudaSuccess) return no_memory();
+  Slab* d_slab = (Slab*)lists.p;
+  SlabTotal* d_total = (SlabTotal*)((char*)lists.p + so);
+  SlabTotal total{};
+  const unsigned grid = (unsigned)((nslab + 7) / 8);
+  HM_CUDA_TRY(cudaMemcpyAsync(d_slab, slab.data(), sb, cudaMemcpyHostToDevice, h->stream));
+  HM_CUDA_TRY(cudaMemsetAsync(d_total, 0, sizeof(SlabTotal), h->stream));
+  slab_lists_kernel<false><<<grid, 256, 0, h->stream>>>(d_slab, nslab, P.d_win, P.d_p2, nullptr, d_total);
+  slab_scan_kernel<<<1, 1024, 0, h->stream>>>(d_slab, nslab, d_total);
+  HM_CUDA_TRY(cudaGetLastError());
+  HM_CUDA_TRY(cudaMemcpyAsync(&total, d_total, sizeof(SlabTotal), cudaMemcpyDeviceToHost, h->stream));
+  HM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+  if (total.narrow || total.entries > (unsigned long long)UINT32_MAX) return HM_ERR_UNSUPPORTED;
+  if (cudaMalloc(&ents.p, sizeof(SlabEnt) * std::max<size_t>(total.entries, 1)) != cudaSuccess) return no_memory();
+  slab_lists_kernel<true><<<grid, 256, 0, h->stream>>>(d_slab, nslab, P.d_win, P.d_p2, (SlabEnt*)ents.p, d_total);
+  HM_CUDA_TRY(cudaGetLastError());
+  HM_CUDA_TRY(cudaStreamSynchronize(h->stream));         // the caller's stream reads the entries next
+  P.d_slab = d_slab;
+  P.d_ent = (SlabEnt*)ents.p;
   P.nslab = (int32_t)nslab;
+  lists.p = ents.p = nullptr;
   return HM_OK;
 }
 
@@ -808,7 +806,7 @@ int ensure_slabs(hm_handle* h, int trans, cudaStream_t st, bool* usable) {
       *usable = false;
       return HM_OK;
     }
-    const int s = build_slab_plan(h, trans, P);
+    const int s = build_slab_plan(h, P);
     if (s == HM_ERR_OOM || s == HM_ERR_UNSUPPORTED) P.no_slab = true;
     else if (s != HM_OK) return s;
   }
