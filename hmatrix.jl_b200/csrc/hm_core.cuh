@@ -183,11 +183,10 @@ static __device__ void zero_cols(double* X, int len, int64_t ld, int c0, int c1)
 // FP32 Gram-Schmidt and Jacobi keep far more accuracy than the truncation
 // discards).  A, B: the tall factors (in TS), J's other fields as for
 // core_body; the new factors are written in FP64.
-// JAC8 (the H-LU tile kernel): Jacobi rounds with 8 lanes per column pair, so
-// a round's pairs run at once instead of one after another per warp, and the
-// singular values ordered by a parallel rank count instead of one thread's
-// selection sort.  The rotations and the order are the same; only the order
-// of the sums in the dot products differs.
+// JAC8 (the H-LU tile kernel): cores of up to 16 columns by jacobi_warp16, larger
+// ones in Jacobi rounds with 8 lanes per column pair, so that a round's pairs run
+// at once instead of one after another per warp, and the singular values ordered
+// by a parallel rank count instead of one thread's selection sort.
 template <typename TS, bool JAC8 = false>
 static __device__ void core_body_t(const CoreJob& J, TS* __restrict__ JA, TS* __restrict__ JB, int rmax,
                                    double eps_trunc, int* __restrict__ flags) {

@@ -53,6 +53,14 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
   return s;
 }
 
+// one FP64 matrix instruction: C(8 x 8) += A(8 x 4) B(4 x 8); lane (g, q) =
+// (lane / 4, lane % 4) holds A(g, q), B(q, g), C(g, 2 q) and C(g, 2 q + 1)
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+
 // Sums NV values over the warp.  Each round halves the values a lane keeps
 // (it sends the other half to the partner lane), so 2*CB sums cost NV-1
 // shuffles instead of 5*NV.  On return the lane holds the total of value idx;
@@ -138,8 +146,7 @@ int launch_aca_fp(const AcaFpJob* d_jobs, int njobs, cudaStream_t st);   // one 
 int launch_core_one(const CoreJob& J, double eps_trunc, int* d_flags, cudaStream_t st);
 // launch the batched recompression; status of rank overflow/nonfinite is
 // OR-ed into *d_flags (bit 0: rank > kcap, bit 1: non-finite).
-// jac8: the Jacobi rounds and ordering of the H-LU's recompressions (core_body_t)
 int launch_core_recompress(const CoreJob* d_jobs, int njobs, int rmax, double eps_trunc,
-                           int* d_flags, cudaStream_t st, bool jac8 = false);
+                           int* d_flags, cudaStream_t st);
 
 }  // namespace hm

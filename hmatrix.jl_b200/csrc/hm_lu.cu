@@ -1284,9 +1284,9 @@ constexpr double MIXED_CORE_EPS = 1e-6;
 // the diagonal tile is factorised, the whole row panel (A factors of tiles
 // (k, j>k)) and column panel (B factors of tiles (i>k, k)) are solved as one
 // wide triangular solve each, and every pair of trailing tiles is updated and
-// recompressed by one CTA that forms its core B_ik' A_kj itself.  Updates are truncated per step (the
-// recursion sums some products before truncating); both stay within
-// eps_trunc of the exact Schur complement.
+// recompressed by one CTA that forms its core B_ik' A_kj itself.  Updates are
+// truncated per step (the recursion sums some products before truncating); both
+// stay within eps_trunc of the exact Schur complement.
 // ---------------------------------------------------------------------------
 struct TileLU {
   int T = 0;

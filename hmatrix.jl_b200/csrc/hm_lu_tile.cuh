@@ -9,14 +9,6 @@
 
 namespace hm {
 
-// one FP64 matrix instruction: C(8 x 8) += A(8 x 4) B(4 x 8); lane (g, q) =
-// (lane / 4, lane % 4) holds A(g, q), B(q, g), C(g, 2 q) and C(g, 2 q + 1)
-__device__ __forceinline__ void tile_dmma(double (&c)[2], double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-      : "+d"(c[0]), "+d"(c[1])
-      : "d"(a), "d"(b));
-}
-
 // ---------------------------------------------------------------------------
 // diagonal tiles: load
 // ---------------------------------------------------------------------------
@@ -454,7 +446,7 @@ __global__ void __cluster_dims__(DL_CTAS, 1, 1) __launch_bounds__(32 * DL_WARPS,
 #pragma unroll
           for (int s = 0; s < 8; ++s) {
             const bool in = k + 4 * s + q < m;
-            tile_dmma(acc, in ? -x[s] : 0.0, in ? y[s] : 0.0);
+            dmma(acc, in ? -x[s] : 0.0, in ? y[s] : 0.0);
           }
         }
 #pragma unroll
@@ -508,7 +500,7 @@ __global__ void __cluster_dims__(DL_CTAS, 1, 1) __launch_bounds__(32 * DL_WARPS,
 #pragma unroll
               for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) tile_dmma(acc[i][j], x[i], y[j]);
+                for (int j = 0; j < 4; ++j) dmma(acc[i][j], x[i], y[j]);
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i)
@@ -583,8 +575,8 @@ static __device__ void tile_trsm(const double* __restrict__ T, int64_t rs, int64
 #pragma unroll 8
     for (int k = b0; k < r0; k += 4) {
       const double t = __ldg(tp + (k + q) * cs);
-      tile_dmma(acc[0], t, x0[k + q]);
-      tile_dmma(acc[1], t, x1[k + q]);
+      dmma(acc[0], t, x0[k + q]);
+      dmma(acc[1], t, x1[k + q]);
     }
     if (8 * mt + g < nr) {
 #pragma unroll

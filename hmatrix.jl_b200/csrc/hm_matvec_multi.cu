@@ -40,12 +40,6 @@ struct MbTile {
 
 namespace {
 
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-      : "+d"(c[0]), "+d"(c[1])
-      : "d"(a), "d"(b));
-}
-
 // two consecutive elements of a factor column as FP64 (the pair starts on an
 // even element; columns are padded to 4 elements and 16 bytes)
 __device__ __forceinline__ double2 ld_pair(const double* p) { return __ldcs(reinterpret_cast<const double2*>(p)); }

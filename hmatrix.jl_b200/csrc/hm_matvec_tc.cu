@@ -287,8 +287,9 @@ __device__ __forceinline__ void tc_copies_drain(TcBars* b, uint64_t* bar, uint32
 }
 
 // MMA issuer (one warp in uniform control flow, one elected thread issues: its
-// operands stay in uniform registers, which the MMA takes): per tile, K stages of A (TMEM) x B (shared
-// memory, K-major or with B_MN the columns of a core matrix contiguous); nk_of(w) gives tile w's stages.  Every kseg stages of a tile form
+// operands stay in uniform registers, which the MMA takes): per tile, K stages of
+// A (TMEM) x B (shared memory, K-major or with B_MN the columns of a core matrix
+// contiguous); nk_of(w) gives tile w's stages.  Every kseg stages of a tile form
 // one accumulation segment: a fresh accumulator (q = segment parity) that the
 // converters drain when it completes.
 template <typename T, int NC, int B_MN, typename NkOf>
