@@ -137,7 +137,7 @@ struct __align__(16) P1Desc {          // 32 bytes
   uint32_t zoff;           // offset of this leaf's k values in z
   uint16_t k;
   uint16_t pad0;
-  uint32_t pad1;
+  uint32_t cl;             // input cluster
 };
 static_assert(sizeof(P1Desc) == 32, "P1Desc must stay 32 bytes");
 

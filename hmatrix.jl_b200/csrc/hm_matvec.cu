@@ -843,6 +843,7 @@ int build_mv_descriptors(hm_handle* h, const std::vector<int64_t>& order, int tr
     else { D.off = L.off + npad * L.k; D.seg0 = (uint32_t)L.row0; D.len = L.m; D.stride = (uint32_t)mpad; }
     D.zoff = zoff[li];
     D.k = (uint16_t)L.k;
+    D.cl = (uint32_t)(trans ? L.s : L.t);
     p1.push_back(D);
   }
   const int64_t nwin = (n + MV_WROWS - 1) / MV_WROWS;

@@ -492,62 +492,89 @@ int block_scratch(hm_handle* h, size_t bytes, double** out) {
   return HM_OK;
 }
 
-// A leaf's factor columns in the table: columns [at, at + k), column r at pool
-// element off + r stride, row z + r of Z
-struct MbLeaf {
-  uint64_t off, z;
-  uint32_t at, stride, k, pad;
+// The factor columns of phase 1 by input segment (one per cluster), 32 to a tile,
+// from the descriptors of the single-column phase 1: columns counted per cluster,
+// the clusters' ranges and tiles by one CTA, then each leaf's columns put in its
+// cluster's range.  Which of a cluster's leaves comes first is left to the atomics:
+// every column's sums are its own.  Made on the host from the leaves the table took
+// 2.1 ms of a first product's 4.7 (n = 2^17).
+struct MbSeg {
+  uint32_t seg0, len, cnt, next;         // columns; next free one
 };
-__global__ void __launch_bounds__(256) mb_column_kernel(const MbLeaf* __restrict__ leaf, int64_t nleaf,
+__global__ void __launch_bounds__(256) mb_count_kernel(const P1Desc* __restrict__ d, int64_t nd, MbSeg* __restrict__ seg) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nd) return;
+  const P1Desc D = d[i];
+  seg[D.cl].seg0 = D.seg0;               // the same value from every leaf of the cluster
+  seg[D.cl].len = D.len;
+  atomicAdd(&seg[D.cl].cnt, (uint32_t)D.k);
+}
+__global__ void __launch_bounds__(1024) mb_tiles_kernel(MbSeg* __restrict__ seg, int64_t ncl, MbTile* __restrict__ tile,
+                                                        uint32_t* __restrict__ ntile) {
+  __shared__ uint32_t sum[2][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t base[2] = {0, 0};             // columns, tiles
+  for (int64_t b = 0; b < ncl; b += 1024) {
+    const int64_t i = b + threadIdx.x;
+    MbSeg S{};
+    if (i < ncl) S = seg[i];
+    const uint32_t own[2] = {S.cnt, (S.cnt + 8 * MB_MT - 1) / (8 * MB_MT)};
+    uint32_t at[2];
+    __syncthreads();                     // the last round's sums
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      uint32_t incl = own[q];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+      }
+      if (lane == 31) sum[q][warp] = incl;
+      at[q] = base[q] + incl - own[q];
+    }
+    __syncthreads();
+    for (int w = 0; w < 32; ++w)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        if (w < warp) at[q] += sum[q][w];
+        base[q] += sum[q][w];
+      }
+    if (i < ncl && S.cnt > 0) {
+      seg[i].next = at[0];
+      for (uint32_t c = 0, t = at[1]; c < S.cnt; c += 8 * MB_MT, ++t)
+        tile[t] = MbTile{at[0] + c, min(8u * MB_MT, S.cnt - c), S.seg0, S.len};
+    }
+  }
+  if (threadIdx.x == 0) *ntile = base[1];
+}
+__global__ void __launch_bounds__(256) mb_column_kernel(const P1Desc* __restrict__ d, int64_t nd, MbSeg* __restrict__ seg,
                                                         MbCol* __restrict__ col) {
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 8;   // eight threads a leaf
-  if (i >= nleaf) return;
-  const MbLeaf L = leaf[i];
-  for (uint32_t r = threadIdx.x % 8; r < L.k; r += 8)
-    col[(uint64_t)L.at + r] = MbCol{L.off + (uint64_t)r * L.stride, L.z + r};
+  P1Desc D{};
+  uint32_t at = 0;
+  if (i < nd) {
+    D = d[i];
+    if (threadIdx.x % 8 == 0) at = atomicAdd(&seg[D.cl].next, (uint32_t)D.k);
+  }
+  at = __shfl_sync(0xffffffffu, at, threadIdx.x & 24);
+  for (uint32_t r = threadIdx.x % 8; r < D.k; r += 8)
+    col[(uint64_t)at + r] = MbCol{D.off + (uint64_t)r * D.stride, (uint64_t)D.zoff + r};
 }
 
-// The factor columns of phase 1 by input segment (the clusters' pre-order
-// starts), 32 to a tile; within a segment in pool order.  The device writes the
-// table from the leaves: made on the host it took 3 of a first call's 9.5 ms (n = 2^17).
-int ensure_columns(hm_handle* h, int trans, MvPlan& P) {
+int ensure_columns(hm_handle* h, MvPlan& P) {
   if (P.d_mbcol || P.np1 == 0) return HM_OK;
-  const int eb = elem_bytes(h->storage);
-  const std::vector<int64_t> order = pool_order(h);
   const int64_t ncl = (int64_t)h->cl_s.size();
-  std::vector<int64_t> at((size_t)ncl + 1, 0);
-  for (const Leaf& L : h->leaves)
-    if (L.type == T_RK) at[(trans ? L.s : L.t) + 1] += L.k;
-  for (int64_t c = 0; c < ncl; ++c) at[c + 1] += at[c];
-  const int64_t ntot = at[ncl];
-  if (ntot > (int64_t)UINT32_MAX) return fail(HM_ERR_UNSUPPORTED, "too many factor columns");
-  std::vector<MbTile> tile;
-  for (int64_t c = 0; c < ncl; ++c)
-    for (int64_t b = at[c]; b < at[c + 1]; b += 8 * MB_MT)
-      tile.push_back(MbTile{(uint32_t)b, (uint32_t)std::min<int64_t>(8 * MB_MT, at[c + 1] - b), (uint32_t)h->cl_s[c],
-                            (uint32_t)(h->cl_e[c] - h->cl_s[c])});
-  uint64_t z = 0;
-  std::vector<MbLeaf> leaf;
-  leaf.reserve(order.size());
-  for (int64_t li : order) {
-    const Leaf& L = h->leaves[li];
-    if (L.type != T_RK || L.k == 0) continue;
-    const int64_t npad = col_pad(L.n, eb), mpad = col_pad(L.m, eb);
-    int64_t& next = at[trans ? L.s : L.t];
-    leaf.push_back(MbLeaf{(uint64_t)(trans ? L.off + npad * L.k : L.off), z, (uint32_t)next,
-                          (uint32_t)(trans ? mpad : npad), (uint32_t)L.k, 0});
-    next += L.k;
-    z += (uint64_t)L.k;
-  }
-  const size_t cb = sizeof(MbCol) * (size_t)ntot, lb = sizeof(MbLeaf) * leaf.size();
-  void* d = nullptr;
-  void* tmp = nullptr;
-  const size_t tl = pad_to((int64_t)(sizeof(MbTile) * tile.size()), 256);
-  const bool behind = lb <= (size_t)1 << 20;             // a small leaf list stays behind the tables
-  cudaError_t e = cudaMalloc(&d, cb + tl + (behind ? lb : 0));
+  const size_t cb = pad_to((int64_t)sizeof(MbCol) * h->zlen, 256);
+  const size_t tb = pad_to((int64_t)sizeof(MbTile) * (h->zlen / (8 * MB_MT) + std::min(ncl, P.np1)), 256);
+  // the segments, needed to make the table only, behind it if they are small
+  const size_t gb = sizeof(MbSeg) * (size_t)ncl + 16;
+  char* d = nullptr;
+  char* tmp = nullptr;
+  const bool behind = gb <= (size_t)1 << 20;
+  cudaError_t e = cudaMalloc((void**)&d, cb + tb + (behind ? gb : 0));
   if (e == cudaSuccess && behind) {
-    tmp = (char*)d + cb + tl;
-  } else if (e == cudaSuccess && cudaMallocAsync(&tmp, lb, h->stream) != cudaSuccess) {
+    tmp = d + cb + tb;
+  } else if (e == cudaSuccess && cudaMalloc((void**)&tmp, gb) != cudaSuccess) {
     cudaFree(d);
     e = cudaErrorMemoryAllocation;
   }
@@ -555,25 +582,26 @@ int ensure_columns(hm_handle* h, int trans, MvPlan& P) {
     cudaGetLastError();
     return fail(HM_ERR_OOM, std::string("block product columns: ") + cudaGetErrorString(e));
   }
-  if (lb) {
-    e = cudaMemcpyAsync(tmp, leaf.data(), lb, cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess) {
-      mb_column_kernel<<<(unsigned)((leaf.size() + 31) / 32), 256, 0, h->stream>>>((const MbLeaf*)tmp,
-                                                                                  (int64_t)leaf.size(), (MbCol*)d);
-      e = cudaGetLastError();
-    }
+  uint32_t* d_n = (uint32_t*)tmp;
+  MbSeg* seg = (MbSeg*)(tmp + 16);
+  uint32_t ntile = 0;
+  e = cudaMemsetAsync(tmp, 0, gb, h->stream);
+  if (e == cudaSuccess) {
+    mb_count_kernel<<<(unsigned)((P.np1 + 255) / 256), 256, 0, h->stream>>>(P.d_p1, P.np1, seg);
+    mb_tiles_kernel<<<1, 1024, 0, h->stream>>>(seg, ncl, (MbTile*)(d + cb), d_n);
+    mb_column_kernel<<<(unsigned)((P.np1 + 31) / 32), 256, 0, h->stream>>>(P.d_p1, P.np1, seg, (MbCol*)d);
+    e = cudaGetLastError();
   }
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync((char*)d + cb, tile.data(), sizeof(MbTile) * tile.size(), cudaMemcpyHostToDevice, h->stream);
-  if (!behind) cudaFreeAsync(tmp, h->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&ntile, d_n, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);   // the caller's stream reads the table next
+  if (!behind) cudaFree(tmp);
   if (e != cudaSuccess) {
     cudaFree(d);
     return fail(HM_ERR_CUDA, std::string("block product columns: ") + cudaGetErrorString(e));
   }
   P.d_mbcol = (MbCol*)d;
-  P.d_mbtile = (MbTile*)((char*)d + cb);
-  P.nmbtile = (int64_t)tile.size();
+  P.d_mbtile = (MbTile*)(d + cb);
+  P.nmbtile = (int64_t)ntile;
   return HM_OK;
 }
 
@@ -587,7 +615,7 @@ int launch_multi(hm_handle* h, const double* d_x, double* d_y, int64_t ncols, in
     for (int64_t c = 0; c < ncols; ++c) HM_TRY(matvec_device(h, d_x + c * h->n, d_y + c * h->n, trans, st));
     return HM_OK;
   }
-  HM_TRY(ensure_columns(h, trans, P));
+  HM_TRY(ensure_columns(h, P));
   const int ld = (int)pad_to(ncols, 8 * NT);
   const int ncb = ld / (8 * NT);
   double* z = nullptr;
