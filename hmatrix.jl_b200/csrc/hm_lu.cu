@@ -1477,13 +1477,15 @@ static void recompress_pairs_t(Ctx& c, const TileLU& TL, const PairLists& W, int
   if (staged) {
     next(1);
     if (!scratch) a.out = nullptr;
-    lu_tile_core_kernel<TS><<<std::min<unsigned>(pers, 148 * 2), 128, smem(rl, true), c.st>>>(a, rl, W.smax, (TS*)nullptr);
+    lu_tile_core_kernel<TS><<<std::min<unsigned>(pers, 148 * 2), TC_THREADS, smem(rl, true), c.st>>>(a, rl, W.smax, (TS*)nullptr);
     LU_LAUNCH_CHECK();
   }
   if (scratch) {
     next(staged ? 2 : 1);
     a.out = nullptr;
-    lu_tile_core_kernel<TS><<<std::min<unsigned>(pers, (unsigned)W.blocks), 128, smem(rmax, false), c.st>>>(
+    // as many CTAs as are resident (at most 3 by their registers)
+    const unsigned res = 148 * (unsigned)std::max<size_t>(1, std::min<size_t>(3, (size_t)227 * 1024 / (smem(rmax, false) + 4096)));
+    lu_tile_core_kernel<TS><<<std::min({pers, res, (unsigned)W.blocks}), TC_THREADS, smem(rmax, false), c.st>>>(
         a, rmax, W.smax, (TS*)W.scratch);
     LU_LAUNCH_CHECK();
   }
@@ -1714,7 +1716,7 @@ static void tile_factor(Ctx& c, const hm_handle* h, TileLU& TL, const std::vecto
   PairLists ws{};
   ws.smax = smax;
   const size_t per = sizeof(double) * ((size_t)2 * smax * std::min(2 * cap, RCORE_MAX) + cap * cap);
-  ws.blocks = (int)std::max<size_t>(16, std::min<size_t>(148 * 2, ((size_t)256 << 20) / per));
+  ws.blocks = (int)std::max<size_t>(16, std::min<size_t>(148 * 3, ((size_t)256 << 20) / per));
   reserve(c, wsb, std::size(ws.list) * arena_round(sizeof(int32_t) * (size_t)T * T) + arena_round(8 * sizeof(int)) +
                       arena_round(per * ws.blocks));
   for (auto& l : ws.list) l = (int32_t*)dmalloc(c, wsb, sizeof(int32_t) * (size_t)T * T);

@@ -395,9 +395,14 @@ __global__ void __launch_bounds__(64 * WPS) lu_pair_kernel(PairArgs a) {
 // rows) or in the block's own part of a global scratch
 // ---------------------------------------------------------------------------
 // TS: the precision of the staged factors and of the QR + SVD core (FP32 when
-// the truncation tolerance is loose: the mixed-precision factorisation)
+// the truncation tolerance is loose: the mixed-precision factorisation).  Bound:
+// the latency of the QR's columns, so what counts is the warps an SM holds: the
+// 2-D cloud, n = 65536, 128 tiles of 512 rows, cores of up to 52 columns in
+// scratch, 2.45 s with 2 CTAs of 128 threads an SM, 1.79 with 2 of 256, 1.38 with
+// the 3 of 256 that are resident (4: 1.69, in two waves).
+constexpr int TC_THREADS = 256;
 template <typename TS>
-__global__ void __launch_bounds__(128) lu_tile_core_kernel(PairArgs a, int rl, int smax, TS* scratch) {
+__global__ void __launch_bounds__(TC_THREADS) lu_tile_core_kernel(PairArgs a, int rl, int smax, TS* scratch) {
   extern __shared__ double sm_raw[];
   TS* sm = reinterpret_cast<TS*>(sm_raw);
   // W (cap x cap, FP64 as in the register kernel), then the factors
@@ -407,7 +412,7 @@ __global__ void __launch_bounds__(128) lu_tile_core_kernel(PairArgs a, int rl, i
   TS* XA = base + cw;
   TS* XB = XA + (int64_t)smax * rl;
   const int nin = *a.nin;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
   for (int b = blockIdx.x; b < nin; b += gridDim.x) {
     const PairView v = pair_view(a, a.in[b]);
     const int k1 = v.k1, kb = v.kb, ka = v.ka, r = k1 + kb;
@@ -419,7 +424,7 @@ __global__ void __launch_bounds__(128) lu_tile_core_kernel(PairArgs a, int rl, i
       continue;
     }
     __syncthreads();
-    for (int e = warp; e < ka * kb; e += 4) {
+    for (int e = warp; e < ka * kb; e += nwarp) {
       const double *x = v.Bik + (int64_t)(e % ka) * v.s, *y = v.Akj + (int64_t)(e / ka) * v.s;
       double s = 0.0;
 #pragma unroll 4
