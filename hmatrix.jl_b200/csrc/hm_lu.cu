@@ -204,28 +204,8 @@ __global__ void lu_axpby_kernel(View Y, View X, double alpha, double beta) {
   }
 }
 
-// X <- L^{-1} X, L (m x m, m <= 96) lower triangular (strided: upper/transposed/
-// reversed triangles are views of this one), one thread per column of X.
-__global__ void __launch_bounds__(128) lu_trsm_lower_kernel(View L, View X, int unit) {
-  extern __shared__ double Ls[];
-  const int m = L.rows;
-  for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
-    const int i = e % m, j = e / m;
-    Ls[e] = (j <= i) ? L.p[(int64_t)i * L.rs + (int64_t)j * L.cs] : 0.0;
-  }
-  __syncthreads();
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= X.cols) return;
-  double* x = X.p + (int64_t)j * X.cs;
-  for (int i = 0; i < m; ++i) {
-    double s = x[(int64_t)i * X.rs];
-    for (int l = 0; l < i; ++l) s = fma(-Ls[i + l * m], x[(int64_t)l * X.rs], s);
-    if (!unit) s = s / Ls[i + i * m];
-    x[(int64_t)i * X.rs] = s;
-  }
-}
-
-// The same solve for triangles of at most MM rows (diagonal leaves): one warp
+// X <- L^{-1} X, L lower triangular (strided: upper/transposed/reversed
+// triangles are views of this one) of at most MM rows (diagonal leaves): one warp
 // per 32 columns of X, each column held in registers, loops fully unrolled.
 template <int MM>
 __global__ void __launch_bounds__(32) lu_trsm_small_kernel(View L, View X, int unit) {
@@ -603,13 +583,14 @@ static void axpby(Ctx& c, View Y, View X, double alpha, double beta) {
   LU_LAUNCH_CHECK();
 }
 
-// X <- L^-1 X for triangles of 97 to TRSM_ROWS rows, 32 columns a CTA, staged in
+// X <- L^-1 X for triangles of 65 to TRSM_ROWS rows, 32 columns a CTA, staged in
 // shared memory.  Larger ones are halved, with a product by all SMs between the
 // halves (trsm_lower).  One thread a column with the triangle read from L2 was a
 // chain of rows^2 / 2 dependent steps: 100 right-hand sides at n = 8192, 32 tiles
 // of 256 rows, 165 ms so, 11 now; 8 tiles of 1024 rows 730 and 11 ms; the LU of the
 // latter, whose panels take this way too, 544 and 33 ms.  Pieces of up to 512 rows:
-// 12 ms and 37 ms.
+// 12 ms and 37 ms.  The recursion's leaves of 94 rows (n = 3000, one column): 7.8
+// and 3.4 ms.
 constexpr int TRSM_ROWS = 256;
 __global__ void __launch_bounds__(256) lu_trsm_block_kernel(View L, View X, int unit) {
   extern __shared__ double sm[];
@@ -637,14 +618,6 @@ static void trsm_lower(Ctx& c, View L, View X, bool unit) {
   }
   if (L.rows <= 64) {
     lu_trsm_small_kernel<64><<<(X.cols + 31) / 32, 32, 0, c.st>>>(L, X, unit ? 1 : 0);
-    LU_LAUNCH_CHECK();
-    return;
-  }
-  if (L.rows <= 96) {
-    if (smem_attr((const void*)lu_trsm_lower_kernel, 96 * 96 * (int)sizeof(double)) != cudaSuccess)
-      throw LuError(HM_ERR_CUDA, "trsm smem attribute");
-    const size_t smem = sizeof(double) * (size_t)L.rows * L.rows;
-    lu_trsm_lower_kernel<<<(X.cols + 127) / 128, 128, smem, c.st>>>(L, X, unit ? 1 : 0);
     LU_LAUNCH_CHECK();
     return;
   }

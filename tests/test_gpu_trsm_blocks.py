@@ -39,3 +39,22 @@ def test_panels_of_large_tiles(n, maxb):
     assert L.info().lu_tiles >= 2 and np.array_equal(L.P, R.P)
     A, B = L.to_dense(), R.to_dense()
     assert np.abs(A - B).max() <= 1e-9 * np.abs(B).max()
+
+
+# the recursion's leaves above the register kernels' 64 rows, against the dense
+# solve (truncation at 1e-10, condition number below n)
+@pytest.mark.parametrize("rows", [65, 75, 96, 97, 128, 159])
+def test_leaves_of_the_recursion(rows):
+    import hmatrix as hm
+    n = 8 * rows
+    rng = np.random.default_rng(rows)
+    _, H = hm.NewHmat(hm.Params(LuMode="recursive", Geom=np.sort(rng.uniform(0, 10, n)), Kernel=hm.Cauchy(1.0),
+                                MaxBlock=2 * rows, MinBlock=rows, MaxRank=16, ConsMethod="aca2", εComp=1e-10,
+                                Tree="bisect", Shift=1.0))
+    A = H.to_dense()
+    L = hm.lu(H)
+    for nc in (1, 33):
+        Y = rng.standard_normal((n, nc))
+        for M, trans in ((A, False), (A.T, True)):
+            Z = np.linalg.solve(M, Y)
+            assert np.linalg.norm(L.solve(Y, trans=trans) - Z) <= 1e-8 * np.linalg.norm(Z)
