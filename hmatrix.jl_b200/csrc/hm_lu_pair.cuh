@@ -121,11 +121,11 @@ __global__ void __launch_bounds__(64 * WPS) lu_pair_kernel(PairArgs a) {
   constexpr int ROWS = 8, CAPW = 48;   // rows a lane; rank capacity (RCORE_MAX / 2)
   // W and A_ik W are FP64 sums of FP64 factors whatever TS is: what is subtracted
   // from A_ij must not carry the core's rounding.  FP64 cores form them in x's
-  // registers, FP32 ones WC columns at a time in registers of their own (2: 180
-  // to 226 registers, 4: 252 to 255).  In FP32 the factors of a mixed LU were 22 %
-  // further from the FP64 ones (8 tiles of 250 rows, l = 40: 2.4e-6 against 2.0e-6
-  // of the norm) and no faster (n = 8192 14.6 ms, now 14.4; 65536 200 and 211).
-  constexpr int WC = sizeof(TS) == 8 ? RMAX : 2;
+  // registers, FP32 ones a column at a time in registers of its own (n = 65536,
+  // truncation 1e-6: 191 ms; two columns at a time, 30 registers more, 211).  In
+  // FP32 the factors of a mixed LU were 22 % further from the FP64 ones (8 tiles of
+  // 250 rows, l = 40: 2.4e-6 against 2.0e-6 of the norm) and no faster (200 ms).
+  constexpr int WC = sizeof(TS) == 8 ? RMAX : 1;
   __shared__ double sW[CAPW * RMAX];   // W, ka x kb
   __shared__ TS sR[2][RMAX * RMAX];    // R of either side, then the coefficients of either output
   __shared__ TS sC[RMAX * (RMAX | 1)], sV[RMAX * (RMAX | 1)];
