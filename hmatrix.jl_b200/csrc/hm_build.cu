@@ -457,10 +457,11 @@ int build_matvec_plans(hm_handle* h) {
   // phase-2 shape until hm_autotune: row slabs, which read leaves that start at
   // any row and fill the SMs at every size; row windows only for n > 2^18 with
   // every leaf on a 64-row boundary (bisection of 2^k points), where a lane's
-  // four rows come in one vector load.  Matvec, slabs against windows: 103 and
-  // 236 us at n = 65536, 1068 and 1102 us at n = 2^18, 3813 and 3767 us at
-  // n = 2^19 (FP64), 2154 and 2040 us (FP32); off the grid, n = 100003, 262 and
-  // 957 us
+  // four rows come in one vector load.  H x on the grid, slabs against the best
+  // window shape, us: n = 65536 FP64 103 and 237, FP32 73 and 180, BF16 63 and 140;
+  // 2^17 309 and 438, 186 and 302, 144 and 234; 2^18 1065 and 1124, 609 and 681,
+  // 457 and 497; 2^19 3926 and 3776, 2193 and 2025.  Off the grid, n = 100003: FP64
+  // 262 and 957, BF16 139 and 1342
   if (!h->tune.tuned) {
     bool aligned = h->n > 1 << 18;
     if (aligned)

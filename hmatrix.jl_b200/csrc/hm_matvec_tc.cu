@@ -103,8 +103,9 @@ struct TcRoles {
   static constexpr int NPROD = 32 * PW;
   static constexpr int NH = CW / 4;                   // converters per TMEM lane: shares of a stage's columns
 };
-// phase 1: 8 producer warps take FP32 at n = 200000, 16 columns from 456 to 418
-// us; BF16 at n = 2^18, 64 columns, is faster with 4 (272 against 384 us)
+// phase 1: 8 producer warps against 4, us a call at n = 2^18: FP32 16 / 32 / 64
+// columns 1003 / 1170 / 1593 against 1056 / 1203 / 1609; BF16 689 / 748 / 1019
+// against 694 / 760 / 930
 template <typename T> using TcR1 = TcRoles<8, sizeof(T) == 4 ? 8 : 4>;
 // phase 2: 4 producer warps 660 us and 16 converter warps 597 us against 545
 // (FP32, n = 200000, 16 columns)
