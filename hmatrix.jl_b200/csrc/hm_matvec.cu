@@ -4,9 +4,10 @@
 //
 // Phase 1: one warp per low-rank leaf streams its F1 factor (B for H*x)
 //          with 16-byte loads and writes z = F1' x_seg (k values) to z[].
-// Phase 2: one CTA per window of 1024 output rows; each lane owns 4 rows and
-//          accumulates sum_r F2[:,r] z_r over the low-rank leaves and C x_seg
-//          over the dense leaves that cover its rows, and stores y.
+// Phase 2: y = sum_r F2[:,r] z_r over the low-rank leaves + C x_seg over the
+//          dense leaves, by row slabs cut at clusters (the default; the lists
+//          are made on first use), or by windows of 1024 output rows with 4
+//          rows a lane (the lists that every plan has).
 // FP64 factors are accumulated in FP64.  FP32 and BF16 factors are
 // multiplied and summed in FP32 over the few vectors (phase 1) or entries
 // (phase 2) a lane has in flight, and those FP32 partial sums are added in
